@@ -368,8 +368,10 @@ class _Flow:
             v_at = v
         self.vx, self.vy, self.cx, self.cy = v[..., 0], v[..., 1], c[:, 0], c[:, 1]
         self.dxv, self.dyv = v_at[..., 0] - c[:, :1], v_at[..., 1] - c[:, 1:]
-        self.zv = f(sc.elevation_vertex).reshape(N, 3)
-        self.zc = (self.zv[:, 0] + self.zv[:, 1] + self.zv[:, 2]) / 3.0
+        # the mean bed on the host: dry triangles are told by stage == bed, and
+        # a division by a constant is rounded once more on the device
+        z = np.asarray(sc.elevation_vertex, dtype=np.float64).reshape(N, 3)
+        self.zv, self.zc = f(z), f((z[:, 0] + z[:, 1] + z[:, 2]) / 3.0)
         self.ze = self._edges(self.zv)
         self.bcell, self.bedge = i(m.boundary_cells), i(m.boundary_edges)
         self.btag = i(m.boundary_tag)
@@ -564,7 +566,7 @@ class _Flow:
         return float(dt)
 
     def update(self, dt):
-        h = self.w - (self.zv[:, 0] + self.zv[:, 1] + self.zv[:, 2]) / 3.0
+        h = self.w - self.zc
         on = (self.eta > self.mah) & (h >= self.mah)
         hs = torch.where(on, h, 1.0)
         S = torch.where(on, -self.g * self.eta ** 2 * torch.sqrt(self.uh ** 2 + self.vh ** 2)
