@@ -189,7 +189,8 @@ static void issue_stage(Handle *h, const Stage &stg) {
     if (h->precision == SWGPU_FP64) {
         launch_flux_fp64(h->M, h->S, h->P, h->d_ctrl, flux_flags, h->stream);
         launch_update_fp64(h->M, h->S, h->P, h->d_ctrl, 0.0, update_flags, stg, h->stream);
-        launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl, dist_flags, h->stream);
+        launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl, dist_flags | kWriteEdges,
+                               h->stream);
     } else {
         launch_flux_mixed(h->M, h->S, h->X, h->P, h->d_ctrl, flux_flags, h->stream);
         if (!(flux_flags & kNoTimestep))
@@ -261,7 +262,18 @@ static int issue_distribute(Handle *h, bool with_boundary) {
                                 with_boundary ? kWriteBoundary : 0, kEulerStage, h->stream);
     }
     h->vertices_stale = false;
+    h->edges_stale = false;
     return check_launch(h, "distribute");
+}
+
+// The FP64 flux reads edge values: those of the last distribute, or, where
+// the vertex values were changed since (an upload, the stand-alone
+// extrapolation or balance), their interpolation.  The 'tsunami' algorithm's
+// edge values are its own.
+static void refresh_edges(Handle *h) {
+    if (h->precision != SWGPU_FP64 || h->P.flow_algorithm || !h->edges_stale) return;
+    launch_interpolate_fp64(h->M, h->S, h->stream);
+    h->edges_stale = false;
 }
 
 }  // namespace swgpu
@@ -296,11 +308,94 @@ static void set_block_counts(Handle *h) {
         const int64_t n =
             h->nscen > 1 ? h->scen_offsets[i + 1] - h->scen_offsets[i] : (int64_t)h->M.N;
         Ctrl *c = &h->h_ctrl[i];
-        c->blocks_flux = (unsigned)((n + h->M.shape.flux - 1) / h->M.shape.flux);
-        c->blocks_update = (unsigned)((n + h->M.shape.update - 1) / h->M.shape.update);
-        c->blocks_distribute =
-            (unsigned)((n + h->M.shape.distribute - 1) / h->M.shape.distribute);
+        // (counted in the FP64 path only)
+        const LaunchShape &s = h->M.shape;
+        const int64_t edges =
+            h->scen_edges.empty() ? 0 : h->scen_edges[i + 1] - h->scen_edges[i];
+        const auto blocks = [&](int64_t items, int64_t total, int knob) {
+            const int b = fp64_block(knob, total, s.sms);
+            return (unsigned)((items + b - 1) / b);
+        };
+        c->blocks_flux = blocks(edges, h->M.edges.E, s.flux);
+        c->blocks_update = blocks(n, h->M.N, s.update);
+        c->blocks_distribute = blocks(n, h->M.N, s.distribute);
     }
+}
+
+// The unique edges of an FP64 handle's mesh (DevEdges).
+static int build_edges(Handle *h, const swgpu_mesh *mesh, const std::vector<int> &nbr,
+                       const std::vector<uint8_t> &full, const int64_t *offsets, int nscen) {
+    const int64_t N = mesh->number_of_elements;
+    std::vector<int> left, right, te((size_t)3 * N), blk;
+    left.reserve((size_t)(N + N / 2 + 512));
+    right.reserve(left.capacity());
+    h->scen_edges.assign(1, 0);
+    const int ranges = offsets ? nscen : 1;
+    for (int s = 0; s < ranges; s++) {
+        const int64_t k0 = offsets ? offsets[s] : 0, k1 = offsets ? offsets[s + 1] : N;
+        for (int64_t k = k0; k < k1; k++)
+            for (int i = 0; i < 3; i++) {
+                const int pk = nbr[(size_t)i * N + k];
+                const int64_t n = pk >> 2;
+                if (pk >= 0 && n < k) {  // listed at its owner, the lower index
+                    te[(size_t)i * N + k] = te[(size_t)(pk & 3) * N + n] | 1;
+                    continue;
+                }
+                te[(size_t)i * N + k] = (int)left.size() << 1;
+                left.push_back(pack_neighbour((int)k, i));
+                right.push_back(pk);
+            }
+        if (offsets) {
+            while (left.size() % 256) {
+                left.push_back(-1);
+                right.push_back(0);
+            }
+            blk.resize(left.size() / 256, s);
+        }
+        h->scen_edges.push_back((int64_t)left.size());
+    }
+    const size_t E = left.size();
+    std::vector<double> n1(E), n2(E), len(E), rad(E);
+    for (size_t e = 0; e < E; e++) {
+        if (left[e] < 0) continue;
+        const int64_t k = left[e] >> 2;
+        const int i = left[e] & 3;
+        n1[e] = mesh->normals[6 * k + 2 * i];
+        n2[e] = mesh->normals[6 * k + 2 * i + 1];
+        len[e] = mesh->edgelengths[3 * k + i];
+        double r = mesh->radii[k];
+        if (right[e] >= 0) r = std::min(r, mesh->radii[right[e] >> 2]);
+        rad[e] = full[(size_t)k] ? r : pos_inf();
+    }
+    DevEdges &D = h->M.edges;
+    D.E = D.launch = (int)E;
+    int *d_left, *d_right, *d_te;
+    double *d_n1, *d_n2, *d_len, *d_rad;
+    int rc;
+    if ((rc = dalloc(h, &d_left, E)) || (rc = dalloc(h, &d_right, E)) ||
+        (rc = dalloc(h, &d_te, (size_t)3 * N)) || (rc = dalloc(h, &d_n1, E)) ||
+        (rc = dalloc(h, &d_n2, E)) || (rc = dalloc(h, &d_len, E)) ||
+        (rc = dalloc(h, &d_rad, E)) || (rc = dalloc(h, &D.f, 3 * E)) ||
+        (rc = dalloc(h, &D.ms, E)) || (rc = upload(h, d_left, left.data(), E)) ||
+        (rc = upload(h, d_right, right.data(), E)) ||
+        (rc = upload(h, d_te, te.data(), (size_t)3 * N)) ||
+        (rc = upload(h, d_n1, n1.data(), E)) || (rc = upload(h, d_n2, n2.data(), E)) ||
+        (rc = upload(h, d_len, len.data(), E)) || (rc = upload(h, d_rad, rad.data(), E)))
+        return rc;
+    if (offsets) {
+        int *d_blk;
+        if ((rc = dalloc(h, &d_blk, blk.size())) || (rc = upload(h, d_blk, blk.data(), blk.size())))
+            return rc;
+        D.blk_scen = d_blk;
+    }
+    D.left = d_left;
+    D.right = d_right;
+    D.te = d_te;
+    D.n1 = d_n1;
+    D.n2 = d_n2;
+    D.len = d_len;
+    D.rad = d_rad;
+    return SWGPU_OK;
 }
 
 // Shared by swgpu_create (offsets == nullptr, one scenario) and
@@ -529,6 +624,12 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     TRY(dalloc(h, &S.uhe, n3));
     TRY(dalloc(h, &S.vhe, n3));
     if (precision == SWGPU_FP64) {
+        TRY(build_edges(h, mesh, nbr, full, offsets, nscen));
+        double *geo;
+        TRY(dalloc(h, &geo, (size_t)kGeoPlanes * n1));
+        launch_geometry_fp64(M, geo, h->stream);
+        TRY(check_launch(h, "geometry"));
+        M.geo64 = geo;
         TRY(dalloc(h, &S.wv, n3));
         TRY(dalloc(h, &S.uhv, n3));
         TRY(dalloc(h, &S.vhv, n3));
@@ -598,6 +699,15 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     P.limiter = params->use_edge_limiter ? kLimiterEdge
                 : params->optimised_gradient_limiter ? kLimiterOptimised
                                                      : kLimiterVertex;
+    P.rise_w = P.beta_w - P.beta_w_dry;
+    P.rise_uh = P.beta_uh - P.beta_uh_dry;
+    P.rise_vh = P.beta_vh - P.beta_vh_dry;
+    P.betas_differ = P.rise_w != 0.0 || P.rise_uh != 0.0 || P.rise_vh != 0.0;
+    {
+        const auto plain = [](double x) { return x > 1.0e-100 && x < 1.0e30; };
+        P.plain_positive = plain(P.g) && plain(P.epsilon) && plain(P.H0) &&
+                           plain(P.minimum_allowed_height);
+    }
     P.f_g = (float)P.g;
     P.f_eps = (float)P.epsilon;
     P.f_H0 = (float)P.H0;
@@ -792,7 +902,7 @@ int swgpu_set_quantity(void *handle, int q, const double *centroid, const double
         if (build_mixed_geometry(h)) return fail(h, SWGPU_ECUDA, "mixed geometry upload");
     }
     if (q == SWGPU_STAGE || q == SWGPU_ELEVATION) h->mixed_from_stage = true;
-    if (q <= SWGPU_YMOMENTUM) h->vertices_stale = true;
+    if (q <= SWGPU_YMOMENTUM) h->vertices_stale = h->edges_stale = true;
     return SWGPU_OK;
 }
 
@@ -965,7 +1075,9 @@ int swgpu_compute_fluxes(void *handle, double *flux_timestep) {
     if ((rc = sync_ctrl(h))) return rc;
     reset_ftmin(h->h_ctrl, h->P);
     if ((rc = push_ctrl(h))) return rc;
+    refresh_edges(h);
     launch_flux_fp64(h->M, h->S, h->P, h->d_ctrl, kWriteMaxSpeed, h->stream);
+    launch_explicit_fp64(h->M, h->S, h->P, h->stream);
     if ((rc = check_launch(h, "compute_fluxes"))) return rc;
     if ((rc = sync_ctrl(h))) return rc;
     double ft;
@@ -1008,6 +1120,7 @@ int swgpu_extrapolate_second_order_sw(void *handle) {
     launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl, kExtrapolateOnly, h->stream);
     if ((rc = check_launch(h, "extrapolate_second_order_sw"))) return rc;
     h->vertices_stale = false;
+    h->edges_stale = true;
     if ((rc = sync_ctrl(h))) return rc;
     return device_status(h);
 }
@@ -1017,6 +1130,7 @@ int swgpu_balance_deep_and_shallow(void *handle) {
     int rc = require_fp64(h, "balance_deep_and_shallow");
     if (rc) return rc;
     launch_balance_fp64(h->M, h->S, h->P, h->stream);
+    h->edges_stale = true;
     if ((rc = check_launch(h, "balance_deep_and_shallow"))) return rc;
     CK(cudaStreamSynchronize(h->stream));
     return SWGPU_OK;
@@ -1313,6 +1427,9 @@ static int set_launch_extent(Handle *h, int n) {
         drop_graphs(h);
     }
     h->M.n_launch = n;
+    h->M.edges.launch = h->M.edges.E;
+    for (size_t i = 1; i < h->scen_edges.size() && h->nscen > 1; i++)
+        if (h->scen_offsets[i] == n) h->M.edges.launch = (int)h->scen_edges[i];
     return SWGPU_OK;
 }
 
@@ -1353,6 +1470,7 @@ static int prepare_run(Handle *h, int64_t max_steps) {
         if (h->h_ctrl[i].halt) h->h_halt_bits[i >> 5] |= 1u << (i & 31);
     if ((rc = upload(h, h->d_halt_bits, h->h_halt_bits, (size_t)nwords))) return rc;
     if ((rc = set_launch_extent(h, h->M.N))) return rc;
+    refresh_edges(h);
     return push_ctrl(h);
 }
 
@@ -1407,7 +1525,7 @@ int swgpu_profile_steps(void *handle, int64_t nsteps, double *ms) {
         CK(cudaEventRecord(ev[3], h->stream));
         if (!mixed)
             launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl,
-                                   kFused | kWriteBoundary, h->stream);
+                                   kFused | kWriteBoundary | kWriteEdges, h->stream);
         else
             launch_distribute_mixed(h->M, h->S, h->X, h->P, h->d_tags, h->d_ctrl,
                                     kFused | kWriteBoundary, kEulerStage, h->stream);

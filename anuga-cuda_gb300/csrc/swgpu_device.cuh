@@ -99,6 +99,17 @@ __host__ __device__ inline bool boundary_keeps_edge_stage(int type) {
            type == SWGPU_BC_TRANSMISSIVE_STAGE_ZERO_MOMENTUM;
 }
 
+// Programmatic dependent launch: let the next kernel of the stream start
+// its blocks as this one's finish, and wait (in the next kernel) until the
+// previous kernel has completed and its writes are visible.  Both are no-ops
+// for kernels launched without the programmatic attribute.  Every block of
+// every step kernel waits before it leaves, so a kernel that has completed
+// implies that all before it have.
+__device__ __forceinline__ void pdl_launch_dependents() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Snapshot of the time bookkeeping taken at kernel entry.
 struct StepClock {
     double dt;          // timestep of this step
@@ -186,21 +197,36 @@ __device__ __forceinline__ void publish_step_clock(Ctrl *c, const DevParams &P) 
 
 // Block-wide minimum of a positive double, then one atomicMin on its bit
 // pattern (positive IEEE doubles order like their bits) only when it lowers
-// the running minimum.  In the fused loop the last block then publishes the
-// step's clock.
+// the running minimum.  The minimum is taken on the integer pipe, the high
+// words first (an FP64 comparison costs a warp 16 clocks of its SM); a
+// negative or NaN timestep wins it as -1 and raises the status.
 template <int BLOCK = kBlock>
 __device__ __forceinline__ void block_min_timestep(double t, Ctrl *ctrl) {
-    __shared__ double wmin[BLOCK / 32];
-    for (int o = 16; o > 0; o >>= 1) t = omin(t, __shfl_xor_sync(0xffffffffu, t, o));
+    __shared__ int wmin_hi[BLOCK / 32];
+    __shared__ unsigned wmin_lo[BLOCK / 32];
+    int hi = __double2hiint(t);
+    if ((unsigned)hi > 0x7ff00000u) hi = -1;
+    unsigned lo = (unsigned)__double2loint(t);
+    const auto warp_min = [&] {
+        const int m = __reduce_min_sync(0xffffffffu, hi);
+        lo = __reduce_min_sync(0xffffffffu, hi == m ? lo : 0xffffffffu);
+        hi = m;
+    };
+    warp_min();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) wmin[warp] = t;
+    if (lane == 0) {
+        wmin_hi[warp] = hi;
+        wmin_lo[warp] = lo;
+    }
     __syncthreads();
     if (warp == 0) {
-        t = lane < (int)(blockDim.x >> 5) ? wmin[lane] : pos_inf();
-        for (int o = 16; o > 0; o >>= 1) t = omin(t, __shfl_xor_sync(0xffffffffu, t, o));
+        const bool in = lane < (int)(blockDim.x >> 5);
+        hi = in ? wmin_hi[lane] : 0x7ff00000;
+        lo = in ? wmin_lo[lane] : 0u;
+        warp_min();
         if (lane == 0) {
-            const unsigned long long bits = (unsigned long long)__double_as_longlong(t);
-            if (!(t >= 0.0)) {
+            const unsigned long long bits = ((unsigned long long)(unsigned)hi << 32) | lo;
+            if (hi < 0) {
                 set_status(ctrl, SWGPU_ENONFINITE);  // NaN reached the timestep
             } else if (bits < *(volatile unsigned long long *)&ctrl->ftmin_bits) {
                 atomicMin(&ctrl->ftmin_bits, bits);
@@ -353,6 +379,25 @@ __device__ __forceinline__ void announce_halt(Ctrl *c) {
         __threadfence();
         atomicAdd(&c->summary->halted, 1);
     }
+}
+
+// A launch of kernel k; with pdl, as a programmatic dependent of the stream's
+// previous kernel (it may start during that kernel's last wave and waits for
+// it with griddepcontrol.wait before reading what that kernel writes).
+template <typename... KArgs, typename... Args>
+static void launch_k(void (*k)(KArgs...), int grid, int block, cudaStream_t st, bool pdl,
+                     Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k, args...);
 }
 
 }  // namespace swgpu

@@ -4,24 +4,26 @@
 // reference's ANUGA C kernels so that the results agree bit for bit with
 // them on the same mesh (the file is compiled with --fmad=false: no
 // contraction into FMA).  On GB300 this path is bound by the FP64 pipe, not
-// by HBM: ~600 dependent FP64 operations per triangle-step.
+// by HBM, so what the pipe is not needed for runs elsewhere: quotients, roots
+// and comparisons on the integer pipe (swgpu_soft64.cuh, the same bits),
+// constants of the geometry from a table, each edge's flux once.
 //
 // One Euler step of the device-resident loop is three kernels:
-//   flux_fp64       central-upwind fluxes of the three edges (triangle
-//                   centric, neighbour edge values gathered), summed in
-//                   ANUGA's order, gravity_wb, per-triangle CFL timestep ->
-//                   block min -> atomicMin into Ctrl
-//   update_fp64     the step's update_timestep (evaluated once by the flux
-//                   kernel's last block), Manning
+//   flux_fp64       central-upwind flux of each edge (one thread per edge),
+//                   CFL timestep -> block min -> atomicMin into Ctrl
+//   update_fp64     the edge fluxes of each triangle summed in ANUGA's order,
+//                   gravity_wb, the step's update_timestep (evaluated once by
+//                   the flux kernel's last block), Manning
 //                   friction, the semi-implicit conserved update, protect,
 //                   centroid velocities for the next extrapolation; the last
 //                   block advances the model time
 //   distribute_fp64 second-order limited extrapolation, balance_deep_and_
 //                   shallow, boundary conditions of the triangle's boundary
-//                   edges; vertex values stored, edge values derived on use
+//                   edges; vertex and edge values stored
 #include <cstdio>
 
 #include "swgpu_device.cuh"
+#include "swgpu_soft64.cuh"
 
 namespace swgpu {
 
@@ -45,25 +47,41 @@ __device__ __forceinline__ double limited_speed(double &uh, double &h, double ep
     return u;
 }
 
-// src/anuga_HMPP/shallow_water_ext.c:302-441 (_flux_function_central).
-// Returns false if the bed is discontinuous across the edge.
-__device__ __forceinline__ bool central_flux(double wl, double uhl_in, double vhl_in, double wr,
-                                             double uhr_in, double vhr_in, double zl, double zr,
-                                             double n1, double n2, const DevParams &P, double h0,
-                                             double lim, double &f0, double &f1, double &f2,
-                                             double &ms) {
+// The two states of an edge in its own frame's order: stage and momentum
+// left and right, bed left and right, the left side's outward normal.
+struct EdgeState {
+    double wl, uhl, vhl, wr, uhr, vhr, zl, zr, n1, n2;
+};
+struct EdgeFlux {
+    double f0, f1, f2, ms;
+    bool bad;  // discontinuous bed
+};
+
+// src/anuga_HMPP/shallow_water_ext.c:302-441 (_flux_function_central) in
+// plain FP64 arithmetic, with the dry test of :4581-4587: for states that
+// are not finite or huge, and for parameters that are not positive.
+static __device__ __noinline__ EdgeFlux central_flux_any(const EdgeState &s, const DevParams &P,
+                                                         double h0, double lim) {
+    EdgeFlux r;
+    r.f0 = r.f1 = r.f2 = r.ms = 0.0;
+    r.bad = false;
+    if (P.optimise_dry_cells && fabs(s.wl - s.zl) < P.epsilon && fabs(s.wr - s.zr) < P.epsilon)
+        return r;
     // rotate into the edge frame (_rotate, :36-53)
-    const double al = n1 * uhl_in + n2 * vhl_in;
-    const double bl = -n2 * uhl_in + n1 * vhl_in;
-    const double ar = n1 * uhr_in + n2 * vhr_in;
-    const double br = -n2 * uhr_in + n1 * vhr_in;
-    if (fabs(zl - zr) > 1.0e-10) return false;
-    const double z = 0.5 * (zl + zr);
+    const double al = s.n1 * s.uhl + s.n2 * s.vhl;
+    const double bl = -s.n2 * s.uhl + s.n1 * s.vhl;
+    const double ar = s.n1 * s.uhr + s.n2 * s.vhr;
+    const double br = -s.n2 * s.uhr + s.n1 * s.vhr;
+    if (fabs(s.zl - s.zr) > 1.0e-10) {
+        r.bad = true;
+        return r;
+    }
+    const double z = 0.5 * (s.zl + s.zr);
     const double g = P.g, eps = P.epsilon;
 
-    double hl = wl - z, uhl = al;
+    double hl = s.wl - z, uhl = al;
     const double ul = limited_speed(uhl, hl, eps, h0, lim);
-    double hr = wr - z, uhr = ar;
+    double hr = s.wr - z, uhr = ar;
     const double ur = limited_speed(uhr, hr, eps, h0, lim);
     double vhl = bl, vhr = br;
     limited_speed(vhl, hl, eps, h0, lim);
@@ -84,15 +102,11 @@ __device__ __forceinline__ bool central_flux(double wl, double uhl_in, double vh
     const double fr2 = ur * vhr;
 
     const double denom = smax - smin;
-    if (denom < eps) {
-        f0 = f1 = f2 = 0.0;
-        ms = 0.0;
-        return true;
-    }
+    if (denom < eps) return r;
     const double inv = 1.0 / denom;
     const double ss = smax * smin;
     double e0 = smax * fl0 - smin * fr0;
-    e0 += ss * (wr - wl);
+    e0 += ss * (s.wr - s.wl);
     e0 *= inv;
     double e1 = smax * fl1 - smin * fr1;
     e1 += ss * (ar - al);
@@ -100,197 +114,315 @@ __device__ __forceinline__ bool central_flux(double wl, double uhl_in, double vh
     double e2 = smax * fl2 - smin * fr2;
     e2 += ss * (br - bl);
     e2 *= inv;
-    ms = omax(fabs(smax), fabs(smin));
+    r.ms = omax(fabs(smax), fabs(smin));
     // rotate back: _rotate(edgeflux, n1, -n2)
-    f0 = e0;
-    f1 = n1 * e1 + (-n2) * e2;
-    f2 = -(-n2) * e1 + n1 * e2;
-    return true;
-}
-
-struct EdgeFlux {
-    double f0, f1, f2;
-    bool skip;
-};
-
-// Flux of edge i of triangle k (src/anuga_HMPP/shallow_water_ext.c:4553-4640,
-// seen from triangle k) and its contribution to the CFL timestep.
-template <int I>
-__device__ __forceinline__ EdgeFlux edge_flux(const DevMesh &M, const DevState &S,
-                                              const DevParams &P, int k, const double (&ew)[3],
-                                              const double (&euh)[3], const double (&evh)[3],
-                                              const double (&ez)[3], double h0, double lim,
-                                              double &t, double &ms_own, int &bad) {
-    const int N = M.N;
-    EdgeFlux r;
-    const int pk = M.nbr[I * N + k];
-    double wr, uhr, vhr, zr;
-    int n = -1;
-    if (pk >= 0) {
-        n = pk >> 2;
-        const int m = pk & 3;
-        if (P.flow_algorithm) {
-            wr = S.we[m * N + n];
-            uhr = S.uhe[m * N + n];
-            vhr = S.vhe[m * N + n];
-        } else {
-            const int a = (m == 0) ? 1 : 0, b = (m == 2) ? 1 : 2;  // the other two vertices
-            wr = 0.5 * (S.wv[a * N + n] + S.wv[b * N + n]);
-            uhr = 0.5 * (S.uhv[a * N + n] + S.uhv[b * N + n]);
-            vhr = 0.5 * (S.vhv[a * N + n] + S.vhv[b * N + n]);
-        }
-        zr = S.ze[m * N + n];
-    } else {
-        const int mb = -pk - 1;
-        wr = S.wb[mb];
-        uhr = S.uhb[mb];
-        vhr = S.vhb[mb];
-        zr = ez[I];
-    }
-    const double wl = ew[I], zl = ez[I];
-    if (P.optimise_dry_cells && fabs(wl - zl) < P.epsilon && fabs(wr - zr) < P.epsilon) {
-        r.f0 = r.f1 = r.f2 = 0.0;
-        r.skip = true;
-        return r;
-    }
-    double ms;
-    if (!central_flux(wl, euh[I], evh[I], wr, uhr, vhr, zl, zr, M.normals[(2 * I) * N + k],
-                      M.normals[(2 * I + 1) * N + k], P, h0, lim, r.f0, r.f1, r.f2, ms)) {
-        bad = 1;
-        r.f0 = r.f1 = r.f2 = 0.0;
-        r.skip = true;
-        return r;
-    }
-    const double length = M.len[I * N + k];
-    r.f0 *= length;
-    r.f1 *= length;
-    r.f2 *= length;
-    r.skip = false;
-    // CFL: counted when the triangle that processes this edge first in
-    // ANUGA's loop (the lower index of the pair) is full
-    const bool full = (n >= 0 && n < k) ? M.full[n] : M.full[k];
-    if (full && ms > P.epsilon) {
-        t = omin(t, M.radii[k] / ms);
-        if (n >= 0) t = omin(t, M.radii[n] / ms);
-    }
-    if (n < 0 || n > k) ms_own = omax(ms_own, ms);
+    r.f0 = e0;
+    r.f1 = s.n1 * e1 + (-s.n2) * e2;
+    r.f2 = -(-s.n2) * e1 + s.n1 * e2;
     return r;
 }
 
-__device__ __forceinline__ void pick(int i, const EdgeFlux &a, const EdgeFlux &b,
-                                     const EdgeFlux &c, double &f0, double &f1, double &f2,
-                                     bool &skip) {
-    f0 = i == 0 ? a.f0 : (i == 1 ? b.f0 : c.f0);
-    f1 = i == 0 ? a.f1 : (i == 1 ? b.f1 : c.f1);
-    f2 = i == 0 ? a.f2 : (i == 1 ? b.f2 : c.f2);
-    skip = i == 0 ? a.skip : (i == 1 ? b.skip : c.skip);
+// limited_speed for both momentum components of one side (the second call of
+// the plain form sees the depth that the first one left) with comparisons,
+// quotients off the FP64 pipe; h finite, eps, h0 and lim positive.
+__device__ __forceinline__ double side_speed(double &uh, double &vh, double &h, double eps,
+                                             double h0, double lim) {
+    const bool shallow = lt_pos(h, lim);
+    double den = h;
+    if (shallow) {
+        if (lt_pos(h, eps)) {
+            h = uh = vh = 0.0;
+            return 0.0;
+        }
+        den = h + fdiv64(h0, h);
+    }
+    const double u = fdiv64(uh, den);
+    if (shallow) {
+        uh = u * h;
+        vh = fdiv64(vh, den) * h;
+    }
+    return u;
 }
 
-// compute_fluxes with gravity_wb ('wb_2').  Triangle k sums -flux(k,i) over
-// its edges in ANUGA's order: edges to lower-index neighbours first, by
-// neighbour index, then its remaining edges by edge index.  The central
-// flux is exactly antisymmetric in IEEE arithmetic, so -flux(k,i) equals
-// the +flux(n,m) that ANUGA's edge loop adds, and the sums agree bitwise.
-template <int BS>
-__global__ void __launch_bounds__(BS) flux_fp64(DevMesh M, DevState S, DevParams P,
+// x small enough that nothing computed from it overflows (and not NaN)
+__device__ __forceinline__ bool tame(double x) {
+    return (hi32(x) & 0x7fffffffu) < 0x52b00000u;  // below 2^300
+}
+
+// central_flux_any with the same operations in the same order, its
+// comparisons, quotients and roots on the integer pipe: 62 FP64
+// instructions where the plain form executes about 165.
+__device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevParams &P, double h0,
+                                                 double lim) {
+    if (!(P.plain_positive && tame(s.wl) && tame(s.uhl) && tame(s.vhl) && tame(s.wr) &&
+          tame(s.uhr) && tame(s.vhr) && tame(s.zl) && tame(s.zr)))
+        return central_flux_any(s, P, h0, lim);
+    EdgeFlux r;
+    r.f0 = r.f1 = r.f2 = r.ms = 0.0;
+    r.bad = false;
+    const double g = P.g, eps = P.epsilon;
+    double hl = s.wl - s.zl, hr = s.wr - s.zr;
+    if (P.optimise_dry_cells && mag_lt(hl, eps) && mag_lt(hr, eps)) return r;
+    if (bits64(s.zl) != bits64(s.zr)) {
+        // a continuous bed gives both sides the same z, which is then z_l
+        if (mag_lt(1.0e-10, s.zl - s.zr)) {
+            r.bad = true;
+            return r;
+        }
+        const double z = 0.5 * (s.zl + s.zr);
+        hl = s.wl - z;
+        hr = s.wr - z;
+    }
+    const double al = s.n1 * s.uhl + s.n2 * s.vhl;
+    const double bl = -s.n2 * s.uhl + s.n1 * s.vhl;
+    const double ar = s.n1 * s.uhr + s.n2 * s.vhr;
+    const double br = -s.n2 * s.uhr + s.n1 * s.vhr;
+    double uhl = al, vhl = bl, uhr = ar, vhr = br;
+    const double ul = side_speed(uhl, vhl, hl, eps, h0, lim);
+    const double ur = side_speed(uhr, vhr, hr, eps, h0, lim);
+    const double ghl = g * hl, ghr = g * hr;
+    const double cl = fsqrt64(ghl);
+    const double cr = fsqrt64(ghr);
+    double smax = imax(ul + cl, ur + cr);
+    if (lt_zero(smax)) smax = 0.0;
+    double smin = imin(ul - cl, ur - cr);
+    if (gt_zero(smin)) smin = 0.0;
+    const double denom = smax - smin;
+    if (lt_pos(denom, eps)) return r;
+    const double fl0 = ul * hl;
+    const double fl1 = ul * uhl + half_of(ghl) * hl;  // (0.5 g) h = (g h) / 2
+    const double fl2 = ul * vhl;
+    const double fr0 = ur * hr;
+    const double fr1 = ur * uhr + half_of(ghr) * hr;
+    const double fr2 = ur * vhr;
+    const double inv = fdiv64(1.0, denom);
+    const double ss = smax * smin;
+    double e0 = smax * fl0 - smin * fr0;
+    e0 += ss * (s.wr - s.wl);
+    e0 *= inv;
+    double e1 = smax * fl1 - smin * fr1;
+    e1 += ss * (ar - al);
+    e1 *= inv;
+    double e2 = smax * fl2 - smin * fr2;
+    e2 += ss * (br - bl);
+    e2 *= inv;
+    r.ms = fabs(mag_lt(smin, smax) ? smax : smin);
+    r.f0 = e0;
+    r.f1 = s.n1 * e1 + (-s.n2) * e2;
+    r.f2 = s.n2 * e1 + s.n1 * e2;
+    return r;
+}
+
+// compute_fluxes: the central flux of every edge, once, as its owner (the
+// triangle with the lower index, which is the one that ANUGA's loop computes
+// it for) sees it, times the edge's length; the update subtracts it from the
+// owner and adds it to the neighbour.  One thread per edge: 1.5 fluxes per
+// triangle instead of three, and equal work for every lane.
+//
+// CFL: min(r_k, r_n) / ms is the smaller of r_k / ms and r_n / ms, since a
+// correctly rounded quotient does not fall when its numerator grows; the
+// radius is infinite for an edge that does not count (owner not full).
+__global__ void __launch_bounds__(kBlock) flux_fp64(DevMesh M, DevState S, DevParams P,
                                                     Ctrl *ctrl, int flags) {
-    ctrl = block_ctrl(ctrl, M);
+    pdl_launch_dependents();
+    const DevEdges &F = M.edges;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (F.blk_scen) ctrl += F.blk_scen[(blockIdx.x * blockDim.x) >> 8];
+    int left = -1, right = 0;
+    EdgeState s;
+    double len = 0.0, rad = 0.0;
+    if (e < F.E) {
+        left = F.left[e];
+        right = F.right[e];
+        s.n1 = F.n1[e];
+        s.n2 = F.n2[e];
+        len = F.len[e];
+        rad = F.rad[e];
+    }
+    pdl_wait();
     if ((flags & kFused) && ctrl_halted(ctrl)) return;
-    const int N = M.N;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
     double t = P.evolve_max_timestep;
     int bad = 0;
-    if (k < N) {
-        const double h0 = P.H0 * P.H0;
-        const double lim = 10 * P.H0;
-        double vw[3], vu[3], vv[3], ew[3], euh[3], evh[3], ez[3];
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            vw[i] = S.wv[i * N + k];
-            vu[i] = S.uhv[i * N + k];
-            vv[i] = S.vhv[i * N + k];
-            ez[i] = S.ze[i * N + k];
-        }
-        if (P.flow_algorithm) {
-            // 'tsunami': the extrapolated edge values themselves
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                ew[i] = S.we[i * N + k];
-                euh[i] = S.uhe[i * N + k];
-                evh[i] = S.vhe[i * N + k];
-            }
+    if (left >= 0) {
+        const int N = M.N;
+        const int k = (left & 3) * N + (left >> 2);
+        s.wl = S.we[k];
+        s.uhl = S.uhe[k];
+        s.vhl = S.vhe[k];
+        s.zl = S.ze[k];
+        if (right >= 0) {
+            const int n = (right & 3) * N + (right >> 2);
+            s.wr = S.we[n];
+            s.uhr = S.uhe[n];
+            s.vhr = S.vhe[n];
+            s.zr = S.ze[n];
         } else {
-            // quantity.c:687-706 (_interpolate_from_vertices_to_edges)
-            ew[0] = 0.5 * (vw[1] + vw[2]);
-            ew[1] = 0.5 * (vw[0] + vw[2]);
-            ew[2] = 0.5 * (vw[0] + vw[1]);
-            euh[0] = 0.5 * (vu[1] + vu[2]);
-            euh[1] = 0.5 * (vu[0] + vu[2]);
-            euh[2] = 0.5 * (vu[0] + vu[1]);
-            evh[0] = 0.5 * (vv[1] + vv[2]);
-            evh[1] = 0.5 * (vv[0] + vv[2]);
-            evh[2] = 0.5 * (vv[0] + vv[1]);
+            const int mb = -right - 1;
+            s.wr = S.wb[mb];
+            s.uhr = S.uhb[mb];
+            s.vhr = S.vhb[mb];
+            s.zr = s.zl;
         }
-
-        double ms_own = 0.0;
-        const EdgeFlux F0 = edge_flux<0>(M, S, P, k, ew, euh, evh, ez, h0, lim, t, ms_own, bad);
-        const EdgeFlux F1 = edge_flux<1>(M, S, P, k, ew, euh, evh, ez, h0, lim, t, ms_own, bad);
-        const EdgeFlux F2 = edge_flux<2>(M, S, P, k, ew, euh, evh, ez, h0, lim, t, ms_own, bad);
-
-        const int code = M.order[k];
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            double f0, f1, f2;
-            bool skip;
-            pick((code >> (2 * j)) & 3, F0, F1, F2, f0, f1, f2, skip);
-            if (!skip) {
-                a0 -= f0;
-                a1 -= f1;
-                a2 -= f2;
-            }
+        const EdgeFlux r = central_flux(s, P, P.H0 * P.H0, 10 * P.H0);
+        F.f[e] = r.f0 * len;
+        F.f[F.E + e] = r.f1 * len;
+        F.f[2 * F.E + e] = r.f2 * len;
+        if (flags & kWriteMaxSpeed) F.ms[e] = r.ms;
+        bad = r.bad;
+        if (P.plain_positive ? lt_pos(P.epsilon, r.ms) && tame(r.ms) : r.ms > P.epsilon) {
+            const double q = fdiv64(rad, r.ms);
+            t = mag_lt(t, q) ? t : q;
         }
-        const double inv_area = 1.0 / M.areas[k];
-        a0 *= inv_area;
-        a1 *= inv_area;
-        a2 *= inv_area;
-
-        // gravity_wb (src/anuga_HMPP/shallow_water_ext.c:1942-2036)
-        {
-            const double g = P.g;
-            const double x0 = M.vxy[0 * N + k], y0 = M.vxy[1 * N + k];
-            const double x1 = M.vxy[2 * N + k], y1 = M.vxy[3 * N + k];
-            const double x2 = M.vxy[4 * N + k], y2 = M.vxy[5 * N + k];
-            const double det = (y2 - y0) * (x1 - x0) - (y1 - y0) * (x2 - x0);
-            double wx = (y2 - y0) * (vw[1] - vw[0]) - (y1 - y0) * (vw[2] - vw[0]);
-            wx /= det;
-            double wy = (x1 - x0) * (vw[2] - vw[0]) - (x2 - x0) * (vw[1] - vw[0]);
-            wy /= det;
-            const double avg_h = S.w[k] - S.zc[k];
-            a1 += -g * wx * avg_h;
-            a2 += -g * wy * avg_h;
-            double sidex = 0.0, sidey = 0.0;
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                const double hh = ew[i] - ez[i];
-                const double fact = -0.5 * g * hh * hh * M.len[i * N + k];
-                sidex = sidex + fact * M.normals[(2 * i) * N + k];
-                sidey = sidey + fact * M.normals[(2 * i + 1) * N + k];
-            }
-            const double area = M.areas[k];
-            a1 += -sidex / area;
-            a2 += -sidey / area;
-        }
-        S.ew[k] = a0;
-        S.euh[k] = a1;
-        S.evh[k] = a2;
-        if (flags & kWriteMaxSpeed) S.max_speed[k] = ms_own;
     }
     if (bad) set_status(ctrl, SWGPU_EBED);
     if (flags & kNoTimestep) return;  // later Runge-Kutta stage: the step's dt is set
-    block_min_timestep<BS>(t, ctrl);
+    block_min_timestep<kBlock>(t, ctrl);
     if ((flags & kFused) && threadIdx.x == 0 && last_block_done(&ctrl->done_flux, ctrl->blocks_flux))
         publish_step_clock(ctrl, P);
+}
+
+// The explicit update of triangle k: the sum of its edges' fluxes in ANUGA's
+// order (edges to lower-index neighbours first, by neighbour index, then its
+// remaining edges by edge index), over the area, and gravity_wb ('wb_2',
+// src/anuga_HMPP/shallow_water_ext.c:1942-2036).
+__device__ __forceinline__ void explicit_update(const DevMesh &M, const DevState &S,
+                                                const DevParams &P, int k, double w, double zc,
+                                                double &a0, double &a1, double &a2) {
+    const int N = M.N;
+    const DevEdges &F = M.edges;
+    double f0[3], f1[3], f2[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int te = F.te[i * N + k];
+        const u64 flip = (u64)(te & 1) << 63;  // the neighbour's side: the flux enters
+        const int e = te >> 1;
+        f0[i] = from64(bits64(F.f[e]) ^ flip);
+        f1[i] = from64(bits64(F.f[F.E + e]) ^ flip);
+        f2[i] = from64(bits64(F.f[2 * F.E + e]) ^ flip);
+    }
+    const int code = M.order[k];
+    a0 = a1 = a2 = 0.0;
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const int i = (code >> (2 * j)) & 3;
+        a0 -= i == 0 ? f0[0] : (i == 1 ? f0[1] : f0[2]);
+        a1 -= i == 0 ? f1[0] : (i == 1 ? f1[1] : f1[2]);
+        a2 -= i == 0 ? f2[0] : (i == 1 ? f2[1] : f2[2]);
+    }
+    const double *G = M.geo64 + k;
+    const double inv_area = G[kGeoInvArea * (size_t)N];
+    a0 *= inv_area;
+    a1 *= inv_area;
+    a2 *= inv_area;
+    const double g = P.g;
+    const double x10 = G[kGeoX10 * (size_t)N], y10 = G[kGeoY10 * (size_t)N];
+    const double x20 = G[kGeoX20 * (size_t)N], y20 = G[kGeoY20 * (size_t)N];
+    const double det = G[kGeoDet * (size_t)N];
+    const double w0 = S.wv[k], d1 = S.wv[N + k] - w0, d2 = S.wv[2 * N + k] - w0;
+    const double wx = fdiv64(y20 * d1 - y10 * d2, det);
+    const double wy = fdiv64(x10 * d2 - x20 * d1, det);
+    const double avg_h = w - zc;
+    a1 += -g * wx * avg_h;
+    a2 += -g * wy * avg_h;
+    double sidex = 0.0, sidey = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const double hh = S.we[i * N + k] - S.ze[i * N + k];
+        const double fact = -0.5 * g * hh * hh * M.len[i * N + k];
+        const double sx = fact * M.normals[(2 * i) * N + k];
+        const double sy = fact * M.normals[(2 * i + 1) * N + k];
+        // (0 + s is s: the sign of a zero is lost in the sum with a1 below)
+        sidex = i == 0 ? sx : sidex + sx;
+        sidey = i == 0 ? sy : sidey + sy;
+    }
+    const double area = M.areas[k];
+    a1 += fdiv64(-sidex, area);
+    a2 += fdiv64(-sidey, area);
+}
+
+// compute_fluxes as the stand-alone method: the explicit updates, and
+// max_speed (the largest speed of the edges that triangle k owns).
+__global__ void __launch_bounds__(kBlock) explicit_fp64(DevMesh M, DevState S, DevParams P) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int N = M.N;
+    if (k >= N) return;
+    double a0, a1, a2;
+    explicit_update(M, S, P, k, S.w[k], S.zc[k], a0, a1, a2);
+    S.ew[k] = a0;
+    S.euh[k] = a1;
+    S.evh[k] = a2;
+    double ms = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int pk = M.nbr[i * N + k];
+        if (pk < 0 || (pk >> 2) > k) ms = omax(ms, M.edges.ms[M.edges.te[i * N + k] >> 1]);
+    }
+    S.max_speed[k] = ms;
+}
+
+// The per-triangle constants of the FP64 path (DevMesh::geo64), with the
+// operations and the order in which ANUGA's kernels compute them on each
+// call: 1 / area and the vertex differences and determinant of gravity_wb
+// (shallow_water_ext.c:1990-2006), and the auxiliary triangle of the
+// extrapolation (:2850-2930).
+__global__ void __launch_bounds__(kBlock) geometry_fp64(DevMesh M, double *geo) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int N = M.N;
+    if (k >= N) return;
+    double *G = geo + k;
+    const auto put = [&](int plane, double v) { G[plane * (size_t)N] = v; };
+    put(kGeoInvArea, 1.0 / M.areas[k]);
+    double vx[3], vy[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        vx[i] = M.vxy[(2 * i) * N + k];
+        vy[i] = M.vxy[(2 * i + 1) * N + k];
+    }
+    put(kGeoX10, vx[1] - vx[0]);
+    put(kGeoY10, vy[1] - vy[0]);
+    put(kGeoX20, vx[2] - vx[0]);
+    put(kGeoY20, vy[2] - vy[0]);
+    put(kGeoDet, (vy[2] - vy[0]) * (vx[1] - vx[0]) - (vy[1] - vy[0]) * (vx[2] - vx[0]));
+    const double x = M.cxy[k], y = M.cxy[N + k];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        put(kGeoDxv + i, vx[i] - x);
+        put(kGeoDyv + i, vy[i] - y);
+    }
+    const int nbk = M.nb[k];
+    double dx1 = 0.0, dy1 = 0.0, dx2 = 0.0, dy2 = 0.0, inv = 0.0;  // inv 0: zero gradient
+    if (nbk <= 1) {
+        const int k0 = M.surr[k], k1 = M.surr[N + k], k2 = M.surr[2 * N + k];
+        const double x0 = M.cxy[k0], y0 = M.cxy[N + k0];
+        dx1 = M.cxy[k1] - x0;
+        dx2 = M.cxy[k2] - x0;
+        dy1 = M.cxy[N + k1] - y0;
+        dy2 = M.cxy[N + k2] - y0;
+        const double area2 = dy2 * dx1 - dy1 * dx2;
+        if (!(area2 <= 0)) inv = 1.0 / area2;
+    } else if (nbk == 2) {
+        int k1 = -1;  // the one interior neighbour: first surrogate that is not k
+#pragma unroll
+        for (int i = 2; i >= 0; i--) {
+            const int sn = M.surr[i * N + k];
+            if (sn != k) k1 = sn;
+        }
+        if (k1 >= 0) {
+            dx1 = M.cxy[k1] - x;
+            dy1 = M.cxy[N + k1] - y;
+            const double area2 = dx1 * dx1 + dy1 * dy1;
+            dx2 = 1.0 / area2;
+            dy2 = dx2 * dy1;
+            dx2 *= dx1;
+        }
+    }
+    put(kGeoDx1, dx1);
+    put(kGeoDy1, dy1);
+    put(kGeoDx2, dx2);
+    put(kGeoDy2, dy2);
+    put(kGeoInvArea2, inv);
 }
 
 // ------------------------------------------------------------- update ---
@@ -304,7 +436,7 @@ __device__ __forceinline__ double manning_S(const DevMesh &M, const DevState &S,
     const double eta = S.fric[k];
     const double eps = P.minimum_allowed_height;
     applied = false;
-    if (!(eta > eps)) return 0.0;
+    if (!lt64(eps, eta)) return 0.0;
     const double z0 = S.zv[k], z1 = S.zv[N + k], z2 = S.zv[2 * N + k];
     double zs = 1.0;
     if (P.use_sloped_mannings) {
@@ -313,20 +445,20 @@ __device__ __forceinline__ double manning_S(const DevMesh &M, const DevState &S,
         const double x2 = M.vxy[4 * N + k], y2 = M.vxy[5 * N + k];
         const double det = (y2 - y0) * (x1 - x0) - (y1 - y0) * (x2 - x0);
         double zx = (y2 - y0) * (z1 - z0) - (y1 - y0) * (z2 - z0);
-        zx /= det;
+        zx = fdiv64(zx, det);
         double zy = (x1 - x0) * (z2 - z0) - (x2 - x0) * (z1 - z0);
-        zy /= det;
-        zs = sqrt(1.0 + zx * zx + zy * zy);
+        zy = fdiv64(zy, det);
+        zs = fsqrt64(1.0 + zx * zx + zy * zy);
     }
-    const double z = (z0 + z1 + z2) / 3.0;
+    const double z = fdiv64(z0 + z1 + z2, 3.0);
     const double h = w - z;
-    if (!(h >= eps)) return 0.0;
+    if (lt64(h, eps)) return 0.0;
     double Sf;
     if (P.use_sloped_mannings)
-        Sf = -P.g * eta * eta * zs * sqrt((uh * uh + vh * vh));
+        Sf = -P.g * eta * eta * zs * fsqrt64(uh * uh + vh * vh);
     else
-        Sf = -P.g * eta * eta * sqrt((uh * uh + vh * vh));
-    Sf /= pow(h, 7.0 / 3);
+        Sf = -P.g * eta * eta * fsqrt64(uh * uh + vh * vh);
+    Sf = fdiv64(Sf, pow(h, 7.0 / 3));
     applied = true;
     return Sf;
 }
@@ -379,12 +511,12 @@ __device__ __forceinline__ double protect_swb2_one(const DevParams &P, double zc
 __device__ __forceinline__ void protect_one(const DevParams &P, double zc, double &w, double &uh,
                                             double &vh) {
     const double hc = w - zc;
-    if (!(hc < P.minimum_allowed_height)) return;
+    if (!lt64_nan(hc, P.minimum_allowed_height)) return;
     if (P.maximum_allowed_speed < P.epsilon) {
         uh = 0.0;
         vh = 0.0;
-        if (hc <= 0.0) w = zc;
-    } else if (hc <= 0.0) {
+        if (!gt_zero(hc)) w = zc;
+    } else if (!gt_zero(hc)) {
         w = zc;
         uh = 0.0;
         vh = 0.0;
@@ -398,32 +530,34 @@ __device__ __forceinline__ void protect_one(const DevParams &P, double zc, doubl
 // src/anuga_HMPP/quantity.c:769-820 (_update) on one value with a nonzero
 // semi-implicit term; returns false if the denominator is not positive.
 __device__ __forceinline__ bool semi_update(double &c, double e, double semi, double dt) {
-    if (c == 0.0)
+    if ((bits64(c) & kMag64) == 0)
         semi = 0.0;
     else
-        semi /= c;
+        semi = fdiv64(semi, c);
     c += dt * e;
     const double den = 1.0 - dt * semi;
-    if (den <= 0.0) return false;
-    c /= den;
+    if (lt64_nan(den, 0.0) || (bits64(den) & kMag64) == 0) return false;
+    c = fdiv64(c, den);
     return true;
 }
 
 // update_conserved_quantities (gpu_domain_advanced.py:1412-1442).  Fused:
-// dt from the device update_timestep, Manning friction computed here, then
-// protect (the first step of the next distribute, moved here: nothing reads
-// the centroids in between) and the centroid velocities the next
-// extrapolation reads.  API: dt given, semi-implicit terms from
-// compute_forcing_terms, no protect.
-template <int BS>
+// the explicit update gathered here from the edge fluxes (and stored, for
+// downloads), dt from the device update_timestep, Manning friction computed
+// here, then protect (the first step of the next distribute, moved here:
+// nothing reads the centroids in between) and the centroid velocities the
+// next extrapolation reads.  API: dt given, explicit and semi-implicit terms
+// from compute_fluxes and compute_forcing_terms, no protect.
+template <int BS, bool FUSED>
 __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevParams P,
                                                       Ctrl *ctrl, double dt_api, int flags,
                                                       Stage stg) {
-    const bool fused = flags & kFused;
+    pdl_launch_dependents();
     ctrl = block_ctrl(ctrl, M);
-    if (fused && ctrl_halted(ctrl)) return;
+    pdl_wait();
+    if (FUSED && ctrl_halted(ctrl)) return;
     StepClock clk;
-    if (fused) {
+    if (FUSED) {
         clk = published_step_clock(ctrl);
     } else {
         clk.dt = dt_api;
@@ -433,6 +567,18 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
     int bad = 0, nonfinite = 0;
     if (k < M.N) {
         double w = S.w[k], uh = S.uh[k], vh = S.vh[k];
+        const double zc = S.zc[k];
+        double ew, euh, evh;
+        if (FUSED) {
+            explicit_update(M, S, P, k, w, zc, ew, euh, evh);
+            S.ew[k] = ew;
+            S.euh[k] = euh;
+            S.evh[k] = evh;
+        } else {
+            ew = S.ew[k];
+            euh = S.euh[k];
+            evh = S.evh[k];
+        }
         if (stg.kind == kStageFirst) {  // backup_conserved_quantities
             S.bw[k] = w;
             S.buh[k] = uh;
@@ -452,13 +598,13 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
             S.svh[k] = 0.0;
         }
         // stage has no semi-implicit term: its denominator is exactly 1
-        w += dt * S.ew[k];
+        w += dt * ew;
         if (applied) {
-            if (!semi_update(uh, S.euh[k], su, dt)) bad = 1;
-            if (!semi_update(vh, S.evh[k], sv, dt)) bad = 1;
+            if (!semi_update(uh, euh, su, dt)) bad = 1;
+            if (!semi_update(vh, evh, sv, dt)) bad = 1;
         } else {
-            uh += dt * S.euh[k];
-            vh += dt * S.evh[k];
+            uh += dt * euh;
+            vh += dt * evh;
         }
         if (stg.kind == kStageMid || stg.kind == kStageLast) {
             // saxpy_conserved_quantities (quantity.c:749-765)
@@ -466,8 +612,7 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
             uh = stg.a * uh + stg.b * S.buh[k];
             vh = stg.a * vh + stg.b * S.bvh[k];
         }
-        if (fused) {
-            const double zc = S.zc[k];
+        if (FUSED) {
             if (P.flow_algorithm) {
                 // the stage vertex clamp of protect_swb2 is overwritten by the
                 // extrapolation that follows in the same step
@@ -477,23 +622,26 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
                 protect_one(P, zc, w, uh, vh);
             }
             if (P.extrapolate_velocity_second_order == 1) {
-                const double dk = omax(w - zc, P.minimum_allowed_height);
-                S.uvel[k] = uh / dk;
-                S.vvel[k] = vh / dk;
+                const double dk = imax(w - zc, P.minimum_allowed_height);
+                S.uvel[k] = fdiv64(uh, dk);
+                S.vvel[k] = fdiv64(vh, dk);
             }
         }
-        // NaN / Inf anywhere in the new state stops the run
-        const double big = 1.0e308;
-        if (!(fabs(w) <= big) || !(fabs(uh) <= big) || !(fabs(vh) <= big)) nonfinite = 1;
+        // NaN / Inf anywhere in the new state stops the run: beyond 1e308 in
+        // magnitude, on the integer pipe
+        const u64 big = 0x7fe1ccf385ebc8a0ull;  // the bits of 1e308
+        if ((bits64(w) & kMag64) > big || (bits64(uh) & kMag64) > big ||
+            (bits64(vh) & kMag64) > big)
+            nonfinite = 1;
         S.w[k] = w;
         S.uh[k] = uh;
         S.vh[k] = vh;
         if ((flags & kTrack) && (stg.kind == kStageEuler || stg.kind == kStageLast))
-            track_depth(S, k, w - S.zc[k], step_end_time(ctrl, clk, stg), P.track_threshold);
+            track_depth(S, k, w - zc, step_end_time(ctrl, clk, stg), P.track_threshold);
     }
     if (bad) set_status(ctrl, SWGPU_EDENOMINATOR);
     if (nonfinite) set_status(ctrl, SWGPU_ENONFINITE);
-    if (fused) {
+    if (FUSED) {
         __syncthreads();
         if (threadIdx.x == 0 && last_block_done(&ctrl->done_update, ctrl->blocks_update))
             commit_stage(ctrl, clk, P, stg);
@@ -548,8 +696,8 @@ __global__ void __launch_bounds__(kBlock) prepare_fp64(DevMesh M, DevState S, De
     S.uh[k] = uh;
     S.vh[k] = vh;
     const double dk = omax(w - zc, P.minimum_allowed_height);
-    S.uvel[k] = uh / dk;
-    S.vvel[k] = vh / dk;
+    S.uvel[k] = fdiv64(uh, dk);
+    S.vvel[k] = fdiv64(vh, dk);
 }
 
 // The centroid velocities alone: extrapolate_velocity_second_order_true
@@ -559,50 +707,43 @@ __global__ void __launch_bounds__(kBlock) velocities_fp64(DevMesh M, DevState S,
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= M.N) return;
     const double dk = omax(S.w[k] - S.zc[k], P.minimum_allowed_height);
-    S.uvel[k] = S.uh[k] / dk;
-    S.vvel[k] = S.vh[k] / dk;
+    S.uvel[k] = fdiv64(S.uh[k], dk);
+    S.vvel[k] = fdiv64(S.vh[k], dk);
 }
 
 // --------------------------------------------------------- distribute ---
 
-// src/anuga_HMPP/shallow_water_ext.c:98-148 (find_qmin_and_qmax).
+// src/anuga_HMPP/shallow_water_ext.c:98-148 (find_qmin_and_qmax); branches
+// and comparisons on the integer pipe.
 __device__ __forceinline__ void qmin_qmax(double dq0, double dq1, double dq2, double &qmin,
                                           double &qmax) {
-    if (dq0 >= 0.0) {
-        if (dq1 >= dq2) {
-            qmax = (dq1 >= 0.0) ? dq0 + dq1 : dq0;
-            qmin = dq0 + dq2;
-            if (qmin >= 0.0) qmin = 0.0;
-        } else {
-            qmax = (dq2 > 0) ? dq0 + dq2 : dq0;
-            qmin = dq0 + dq1;
-            if (qmin >= 0.0) qmin = 0.0;
-        }
+    const double s1 = dq0 + dq1, s2 = dq0 + dq2;
+    const bool above = !lt64(dq1, dq2);  // dq1 >= dq2
+    if (ge_zero(dq0)) {
+        qmax = above ? (ge_zero(dq1) ? s1 : dq0) : (gt_zero(dq2) ? s2 : dq0);
+        qmin = above ? s2 : s1;
+        if (ge_zero(qmin)) qmin = 0.0;
     } else {
-        if (dq1 <= dq2) {
-            qmin = (dq1 < 0.0) ? dq0 + dq1 : dq0;
-            qmax = dq0 + dq2;
-            if (qmax <= 0.0) qmax = 0.0;
-        } else {
-            qmin = (dq2 < 0.0) ? dq0 + dq2 : dq0;
-            qmax = dq0 + dq1;
-            if (qmax <= 0.0) qmax = 0.0;
-        }
+        const bool below = !lt64(dq2, dq1);  // dq1 <= dq2
+        qmin = below ? (lt_zero(dq1) ? s1 : dq0) : (lt_zero(dq2) ? s2 : dq0);
+        qmax = below ? s2 : s1;
+        if (!gt_zero(qmax)) qmax = 0.0;
     }
 }
 
-// src/anuga_HMPP/shallow_water_ext.c:151-181 (limit_gradient).
+// src/anuga_HMPP/shallow_water_ext.c:151-181 (limit_gradient): r0 is the
+// quotient by the last jump that is not tiny, never below zero.
 __device__ __forceinline__ void limit_jumps(double (&d)[3], double qmin, double qmax,
                                             double beta) {
-    const double TINY = 1.0e-100;
+    const u64 tiny = 0x2b2bff2ee48e0530ull;  // the bits of 1e-100
     double r = 1000.0, r0 = 1.0;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        if (d[i] < -TINY) r0 = qmin / d[i];
-        if (d[i] > TINY) r0 = qmax / d[i];
-        r = omin(r0, r);
+        if ((bits64(d[i]) & kMag64) > tiny) r0 = fdiv64(lt_zero(d[i]) ? qmin : qmax, d[i]);
+        r = mag_lt(r0, r) ? r0 : r;
     }
-    const double phi = omin(r * beta, 1.0);
+    const double rb = r * beta;
+    const double phi = lt_pos(rb, 1.0) ? rb : 1.0;
     d[0] = d[0] * phi;
     d[1] = d[1] * phi;
     d[2] = d[2] * phi;
@@ -638,17 +779,16 @@ __device__ __forceinline__ void one_nbr_jumps(double qk, double q1, double dx2, 
     double d[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) d[i] = a * dxv[i] + b * dyv[i];
-    double qmin, qmax;
-    if (dq1 >= 0.0) {
-        qmin = 0.0;
-        qmax = dq1;
-    } else {
-        qmin = dq1;
-        qmax = 0.0;
-    }
-    limit_jumps(d, qmin, qmax, beta);
+    const bool up = ge_zero(dq1);
+    limit_jumps(d, up ? 0.0 : dq1, up ? dq1 : 0.0, beta);
 #pragma unroll
     for (int i = 0; i < 3; i++) out[i] = qk + d[i];
+}
+
+// the limiter's factor of one quantity: beta_dry + (beta - beta_dry) * hfactor
+// (the same number whatever hfactor where the two are equal)
+__device__ __forceinline__ double beta_of(double dry, double rise, double hfactor) {
+    return rise == 0.0 ? dry : dry + rise * hfactor;
 }
 
 // The 'tsunami' distribute (gpu_domain_advanced.py:1755-1812): the edge
@@ -665,7 +805,9 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
                                                          const BcTag *tags, Ctrl *ctrl,
                                                          int flags) {
     const bool fused = flags & kFused;
+    pdl_launch_dependents();
     ctrl = block_ctrl(ctrl, M);
+    pdl_wait();
     if (fused && ctrl_halted(ctrl)) return;
     const int N = M.N;
     const double time = ctrl->time;
@@ -697,35 +839,32 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
             }
             if (nbk <= 1) {
                 int k0 = M.surr[k], k1 = M.surr[N + k], k2 = M.surr[2 * N + k];
-                if (S.w[k2] <= S.zc[k2]) k2 = k;
-                if (S.w[k0] <= S.zc[k0]) k0 = k;
-                if (S.w[k1] <= S.zc[k1]) k1 = k;
+                if (!lt64(S.zc[k2], S.w[k2])) k2 = k;
+                if (!lt64(S.zc[k0], S.w[k0])) k0 = k;
+                if (!lt64(S.zc[k1], S.w[k1])) k1 = k;
                 const double x0 = M.cxy[k0], y0 = M.cxy[N + k0];
                 const double dx1 = M.cxy[k1] - x0, dx2 = M.cxy[k2] - x0;
                 const double dy1 = M.cxy[N + k1] - y0, dy2 = M.cxy[N + k2] - y0;
                 const double area2 = dy2 * dx1 - dy1 * dx2;
-                if (area2 <= 0) {
+                if (!gt_zero(area2)) {
                     flat = true;
                 } else {
                     const double hc = wk - S.zc[k];
                     const double h0 = S.w[k0] - S.zc[k0];
                     const double h1 = S.w[k1] - S.zc[k1];
                     const double h2 = S.w[k2] - S.zc[k2];
-                    const double hmin = omin(omin(h0, omin(h1, h2)), hc);
-                    const double hfactor = hmin > 0.0 ? 1.0 : 0.0;
-                    if (P.optimise_dry_cells && omax(h0, omax(h1, h2)) < P.epsilon) {
+                    const double hmin = imin(imin(h0, imin(h1, h2)), hc);
+                    const double hfactor = gt_zero(hmin) ? 1.0 : 0.0;
+                    if (P.optimise_dry_cells && lt64(imax(h0, imax(h1, h2)), P.epsilon)) {
                         keep = true;
                     } else {
-                        const double inv_area2 = 1.0 / area2;
+                        const double inv_area2 = fdiv64(1.0, area2);
                         aux_jumps(wk, S.w[k0], S.w[k1], S.w[k2], dx1, dy1, dx2, dy2, inv_area2,
-                                  dxv, dyv, P.beta_w_dry + (P.beta_w - P.beta_w_dry) * hfactor,
-                                  ew);
+                                  dxv, dyv, beta_of(P.beta_w_dry, P.rise_w, hfactor), ew);
                         aux_jumps(uk, U[k0], U[k1], U[k2], dx1, dy1, dx2, dy2, inv_area2, dxv,
-                                  dyv, P.beta_uh_dry + (P.beta_uh - P.beta_uh_dry) * hfactor,
-                                  eu);
+                                  dyv, beta_of(P.beta_uh_dry, P.rise_uh, hfactor), eu);
                         aux_jumps(vk, V[k0], V[k1], V[k2], dx1, dy1, dx2, dy2, inv_area2, dxv,
-                                  dyv, P.beta_vh_dry + (P.beta_vh - P.beta_vh_dry) * hfactor,
-                                  ev);
+                                  dyv, beta_of(P.beta_vh_dry, P.rise_vh, hfactor), ev);
                     }
                 }
             } else {
@@ -741,7 +880,7 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
                 } else {
                     const double dx1 = M.cxy[k1] - x, dy1 = M.cxy[N + k1] - y;
                     const double area2 = dx1 * dx1 + dy1 * dy1;
-                    double dx2 = 1.0 / area2;
+                    double dx2 = fdiv64(1.0, area2);
                     const double dy2 = dx2 * dy1;
                     dx2 *= dx1;
                     one_nbr_jumps(wk, S.w[k1], dx2, dy2, dxv, dyv, P.beta_w, ew);
@@ -778,10 +917,12 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
         if (vel) {
 #pragma unroll
             for (int i = 0; i < 3; i++) {
-                const double de = omax(ew[i] - S.ze[i * N + k], 0.0);
+                double de = ew[i] - S.ze[i * N + k];
+                if (!gt_zero(de)) de = 0.0;
                 eu[i] = eu[i] * de;
                 ev[i] = ev[i] * de;
-                const double dv = omax(ow[i] - S.zv[i * N + k], 0.0);
+                double dv = ow[i] - S.zv[i * N + k];
+                if (!gt_zero(dv)) dv = 0.0;
                 ou[i] = ou[i] * dv;
                 ov[i] = ov[i] * dv;
             }
@@ -930,27 +1071,24 @@ __device__ __forceinline__ void balance_one(const DevParams &P, double wk, doubl
     }
 #pragma unroll
     for (int i = 0; i < 3; i++) hv[i] = ow[i] - zvk[i];
-    const double hmin = omin(hv[0], omin(hv[1], hv[2]));
-    double alpha;
+    const double hmin = imin(hv[0], imin(hv[1], hv[2]));
+    double alpha = 1.0;
     if (P.tight_slope_limiters == 0) {
-        alpha = dz > 0.0 ? omax(omin(P.alpha_balance * hmin / dz, 1.0), 0.0) : 1.0;
-    } else if (hmin < P.H0) {
-        alpha = 1.0;
+        alpha = dz > 0.0 ? omax(omin(fdiv64(P.alpha_balance * hmin, dz), 1.0), 0.0) : 1.0;
+    } else if (lt64(hmin, P.H0)) {
+        const double head = hc - P.H0;
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             const double hd = hc - hv[i];
-            if (!(hd <= 0)) alpha = omin(alpha, (hc - P.H0) / hd);
+            if (gt_zero(hd)) alpha = imin(alpha, fdiv64(head, hd));
         }
-        if (alpha > 1.0) alpha = 1.0;
-        if (alpha < 0.0) alpha = 0.0;
-    } else {
-        alpha = 1.0;
+        if (lt_zero(alpha)) alpha = 0.0;  // alpha is at most 1
     }
-    if (alpha < 1) {
+    if (lt64(alpha, 1.0)) {
         double uc = 0.0, vc = 0.0;
-        if (P.use_centroid_velocities == 1 && hc > eps) {
-            uc = uk / hc;
-            vc = vk / hc;
+        if (P.use_centroid_velocities == 1 && lt64(eps, hc)) {
+            uc = fdiv64(uk, hc);
+            vc = fdiv64(vk, hc);
         }
 #pragma unroll
         for (int i = 0; i < 3; i++) {
@@ -995,7 +1133,9 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
                                                           const BcTag *tags, Ctrl *ctrl,
                                                           int flags) {
     const bool fused = flags & kFused;
+    pdl_launch_dependents();
     ctrl = block_ctrl(ctrl, M);
+    pdl_wait();
     if (fused && ctrl_halted(ctrl)) return;
     const int N = M.N;
     const int order = (int)ctrl->order;
@@ -1031,50 +1171,49 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
             const double qv = vel ? S.vvel[k] : vk;
             const int nbk = M.nb[k];
             bool keep = false;  // dry: previous vertex values stay
-            bool flat = false;  // zero gradient: centroid values at vertices
-            if (nbk == 3) {
-                flat = true;
-            } else {
-                const double x = M.cxy[k], y = M.cxy[N + k];
+            bool flat = nbk == 3;  // zero gradient: centroid values at vertices
+            if (!flat) {
+                const double *G = M.geo64 + k;
+                const size_t n = N;
+                const double inv_area2 = G[kGeoInvArea2 * n];
                 double dxv[3], dyv[3];
 #pragma unroll
                 for (int i = 0; i < 3; i++) {
-                    dxv[i] = M.vxy[(2 * i) * N + k] - x;
-                    dyv[i] = M.vxy[(2 * i + 1) * N + k] - y;
+                    dxv[i] = G[(kGeoDxv + i) * n];
+                    dyv[i] = G[(kGeoDyv + i) * n];
                 }
+                const double dx2 = G[kGeoDx2 * n], dy2 = G[kGeoDy2 * n];
                 if (nbk <= 1) {
-                    const int k0 = M.surr[k], k1 = M.surr[N + k], k2 = M.surr[2 * N + k];
-                    const double x0 = M.cxy[k0], y0 = M.cxy[N + k0];
-                    const double dx1 = M.cxy[k1] - x0, dx2 = M.cxy[k2] - x0;
-                    const double dy1 = M.cxy[N + k1] - y0, dy2 = M.cxy[N + k2] - y0;
-                    const double area2 = dy2 * dx1 - dy1 * dx2;
-                    if (area2 <= 0) {
+                    if ((bits64(inv_area2) & kMag64) == 0) {
                         flat = true;
                     } else {
+                        const int k0 = M.surr[k], k1 = M.surr[N + k], k2 = M.surr[2 * N + k];
+                        const double dx1 = G[kGeoDx1 * n], dy1 = G[kGeoDy1 * n];
                         const double w0 = S.w[k0], w1 = S.w[k1], w2 = S.w[k2];
-                        const double hc = wk - zk;
                         const double h0 = w0 - S.zc[k0];
                         const double h1 = w1 - S.zc[k1];
                         const double h2 = w2 - S.zc[k2];
-                        const double hmin = omin(omin(h0, omin(h1, h2)), hc);
-                        double hfactor = 0.0;
-                        if (hmin > 0.001) hfactor = (hmin - 0.001) / (hmin + 0.004);
-                        if (P.optimise_dry_cells && omax(h0, omax(h1, h2)) < P.epsilon) {
+                        if (P.optimise_dry_cells && lt64(imax(h0, imax(h1, h2)), P.epsilon)) {
                             keep = true;
                         } else {
-                            const double inv_area2 = 1.0 / area2;
+                            double hfactor = 0.0;
+                            if (P.betas_differ) {
+                                const double hmin = imin(imin(h0, imin(h1, h2)), wk - zk);
+                                if (lt64(0.001, hmin))
+                                    hfactor = fdiv64(hmin - 0.001, hmin + 0.004);
+                            }
                             aux_jumps(wk, w0, w1, w2, dx1, dy1, dx2, dy2, inv_area2, dxv, dyv,
-                                      P.beta_w_dry + (P.beta_w - P.beta_w_dry) * hfactor, ow);
+                                      beta_of(P.beta_w_dry, P.rise_w, hfactor), ow);
                             const double u0 = vel ? S.uvel[k0] : S.uh[k0];
                             const double u1 = vel ? S.uvel[k1] : S.uh[k1];
                             const double u2 = vel ? S.uvel[k2] : S.uh[k2];
                             aux_jumps(qu, u0, u1, u2, dx1, dy1, dx2, dy2, inv_area2, dxv, dyv,
-                                      P.beta_uh_dry + (P.beta_uh - P.beta_uh_dry) * hfactor, ou);
+                                      beta_of(P.beta_uh_dry, P.rise_uh, hfactor), ou);
                             const double v0 = vel ? S.vvel[k0] : S.vh[k0];
                             const double v1 = vel ? S.vvel[k1] : S.vh[k1];
                             const double v2 = vel ? S.vvel[k2] : S.vh[k2];
                             aux_jumps(qv, v0, v1, v2, dx1, dy1, dx2, dy2, inv_area2, dxv, dyv,
-                                      P.beta_vh_dry + (P.beta_vh - P.beta_vh_dry) * hfactor, ov);
+                                      beta_of(P.beta_vh_dry, P.rise_vh, hfactor), ov);
                         }
                     }
                 } else {
@@ -1089,11 +1228,6 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
                         no_nbr = 1;
                         flat = true;
                     } else {
-                        const double dx1 = M.cxy[k1] - x, dy1 = M.cxy[N + k1] - y;
-                        const double area2 = dx1 * dx1 + dy1 * dy1;
-                        double dx2 = 1.0 / area2;
-                        const double dy2 = dx2 * dy1;
-                        dx2 *= dx1;
                         one_nbr_jumps(wk, S.w[k1], dx2, dy2, dxv, dyv, P.beta_w, ow);
                         one_nbr_jumps(qu, vel ? S.uvel[k1] : S.uh[k1], dx2, dy2, dxv, dyv,
                                       P.beta_w, ou);
@@ -1121,7 +1255,8 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
                 // back from velocity to momentum with the vertex depth
 #pragma unroll
                 for (int i = 0; i < 3; i++) {
-                    const double dv = omax(ow[i] - zvk[i], 0.);
+                    double dv = ow[i] - zvk[i];
+                    if (!gt_zero(dv)) dv = 0.0;
                     ou[i] = ou[i] * dv;
                     ov[i] = ov[i] * dv;
                 }
@@ -1136,16 +1271,16 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
             S.uhv[i * N + k] = ou[i];
             S.vhv[i * N + k] = ov[i];
         }
+        // interpolated edge values (quantity.c:687-706)
+        double ew[3], eu[3], ev[3];
         if (flags & kWriteEdges) {
-            S.we[k] = 0.5 * (ow[1] + ow[2]);
-            S.we[N + k] = 0.5 * (ow[0] + ow[2]);
-            S.we[2 * N + k] = 0.5 * (ow[0] + ow[1]);
-            S.uhe[k] = 0.5 * (ou[1] + ou[2]);
-            S.uhe[N + k] = 0.5 * (ou[0] + ou[2]);
-            S.uhe[2 * N + k] = 0.5 * (ou[0] + ou[1]);
-            S.vhe[k] = 0.5 * (ov[1] + ov[2]);
-            S.vhe[N + k] = 0.5 * (ov[0] + ov[2]);
-            S.vhe[2 * N + k] = 0.5 * (ov[0] + ov[1]);
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const int a = (i == 0) ? 1 : 0, b = (i == 2) ? 1 : 2;
+                S.we[i * N + k] = ew[i] = half_of(ow[a] + ow[b]);
+                S.uhe[i * N + k] = eu[i] = half_of(ou[a] + ou[b]);
+                S.vhe[i * N + k] = ev[i] = half_of(ov[a] + ov[b]);
+            }
         }
         if ((flags & kWriteBoundary) && M.nb[k] > 0) {
 #pragma unroll
@@ -1153,12 +1288,8 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
                 const int pk = M.nbr[i * N + k];
                 if (pk < 0) {
                     const int mb = -pk - 1;
-                    const int a = (i == 0) ? 1 : 0, b = (i == 2) ? 1 : 2;
-                    const double we = 0.5 * (ow[a] + ow[b]);
-                    const double uhe = 0.5 * (ou[a] + ou[b]);
-                    const double vhe = 0.5 * (ov[a] + ov[b]);
                     double wb, uhb, vhb;
-                    if (!eval_boundary(tags[M.btag[mb]], time, we, uhe, vhe,
+                    if (!eval_boundary(tags[M.btag[mb]], time, ew[i], eu[i], ev[i],
                                        M.normals[(2 * i) * N + k],
                                        M.normals[(2 * i + 1) * N + k], S.ze[i * N + k], P.g,
                                        wb, uhb, vhb)) {
@@ -1221,9 +1352,9 @@ __global__ void __launch_bounds__(kBlock) interpolate_fp64(DevMesh M, DevState S
 #pragma unroll
     for (int q = 0; q < 3; q++) {
         const double q0 = V[q][k], q1 = V[q][N + k], q2 = V[q][2 * N + k];
-        E[q][k] = 0.5 * (q1 + q2);
-        E[q][N + k] = 0.5 * (q0 + q2);
-        E[q][2 * N + k] = 0.5 * (q0 + q1);
+        E[q][k] = half_of(q1 + q2);
+        E[q][N + k] = half_of(q0 + q2);
+        E[q][2 * N + k] = half_of(q0 + q1);
     }
 }
 
@@ -1284,23 +1415,18 @@ void launch_prepare_fp64(const DevMesh &M, const DevState &S, const DevParams &P
                          cudaStream_t st) {
     prepare_fp64<<<grid_for(M.N), kBlock, 0, st>>>(M, S, P);
 }
-// Block sizes of the fused-step kernels come from M.shape.
+// Block sizes of the fused-step kernels come from M.shape (fp64_block).
 void launch_distribute_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                             const BcTag *tags, Ctrl *ctrl, int flags, cudaStream_t st) {
-    const int bs = M.shape.distribute, g = (M.n_launch + bs - 1) / bs;
-    if (P.flow_algorithm) {
-        if (bs == 128)
-            distribute_de_fp64<128><<<g, 128, 0, st>>>(M, S, P, tags, ctrl, flags);
-        else if (bs == 512)
-            distribute_de_fp64<512><<<g, 512, 0, st>>>(M, S, P, tags, ctrl, flags);
-        else
-            distribute_de_fp64<256><<<g, 256, 0, st>>>(M, S, P, tags, ctrl, flags);
-    } else if (bs == 128)
-        distribute_fp64<128><<<g, 128, 0, st>>>(M, S, P, tags, ctrl, flags);
-    else if (bs == 512)
-        distribute_fp64<512><<<g, 512, 0, st>>>(M, S, P, tags, ctrl, flags);
+    const int bs = fp64_block(M.shape.distribute, M.N, M.shape.sms);
+    const int g = (M.n_launch + bs - 1) / bs;
+    const bool pdl = M.shape.pdl && (flags & kFused);
+    if (P.flow_algorithm)
+        launch_k(bs > 256 ? distribute_de_fp64<512> : distribute_de_fp64<256>, g, bs, st, pdl, M,
+                 S, P, tags, ctrl, flags);
     else
-        distribute_fp64<256><<<g, 256, 0, st>>>(M, S, P, tags, ctrl, flags);
+        launch_k(bs > 256 ? distribute_fp64<512> : distribute_fp64<256>, g, bs, st, pdl, M, S, P,
+                 tags, ctrl, flags);
 }
 void launch_boundary_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                           const BcTag *tags, Ctrl *ctrl,
@@ -1309,13 +1435,17 @@ void launch_boundary_fp64(const DevMesh &M, const DevState &S, const DevParams &
 }
 void launch_flux_fp64(const DevMesh &M, const DevState &S, const DevParams &P, Ctrl *ctrl,
                       int flags, cudaStream_t st) {
-    const int bs = M.shape.flux, g = (M.n_launch + bs - 1) / bs;
-    if (bs == 64)
-        flux_fp64<64><<<g, 64, 0, st>>>(M, S, P, ctrl, flags);
-    else if (bs == 128)
-        flux_fp64<128><<<g, 128, 0, st>>>(M, S, P, ctrl, flags);
-    else
-        flux_fp64<256><<<g, 256, 0, st>>>(M, S, P, ctrl, flags);
+    const int bs = fp64_block(M.shape.flux, M.edges.E, M.shape.sms);
+    launch_k(flux_fp64, (M.edges.launch + bs - 1) / bs, bs, st, M.shape.pdl && (flags & kFused),
+             M, S, P, ctrl, flags);
+}
+void launch_explicit_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
+                          cudaStream_t st) {
+    const int bs = fp64_block(kBlock, M.N, M.shape.sms);
+    explicit_fp64<<<(M.N + bs - 1) / bs, bs, 0, st>>>(M, S, P);
+}
+void launch_geometry_fp64(const DevMesh &M, double *geo, cudaStream_t st) {
+    geometry_fp64<<<grid_for(M.N), kBlock, 0, st>>>(M, geo);
 }
 void launch_forcing_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                          bool explicit_target, cudaStream_t st) {
@@ -1331,13 +1461,14 @@ void launch_balance_fp64(const DevMesh &M, const DevState &S, const DevParams &P
 }
 void launch_update_fp64(const DevMesh &M, const DevState &S, const DevParams &P, Ctrl *ctrl,
                         double dt, int flags, const Stage &stage, cudaStream_t st) {
-    const int bs = M.shape.update, g = (M.n_launch + bs - 1) / bs;
-    if (bs == 128)
-        update_fp64<128><<<g, 128, 0, st>>>(M, S, P, ctrl, dt, flags, stage);
-    else if (bs == 512)
-        update_fp64<512><<<g, 512, 0, st>>>(M, S, P, ctrl, dt, flags, stage);
+    const int bs = fp64_block(M.shape.update, M.N, M.shape.sms);
+    const int g = (M.n_launch + bs - 1) / bs;
+    if (flags & kFused)
+        launch_k(bs > 256 ? update_fp64<512, true> : update_fp64<256, true>, g, bs, st,
+                 M.shape.pdl, M, S, P, ctrl, dt, flags, stage);
     else
-        update_fp64<256><<<g, 256, 0, st>>>(M, S, P, ctrl, dt, flags, stage);
+        launch_k(bs > 256 ? update_fp64<512, false> : update_fp64<256, false>, g, bs, st, false,
+                 M, S, P, ctrl, dt, flags, stage);
 }
 void launch_saxpy_fp64(const DevMesh &M, const DevState &S, double a, double b,
                        cudaStream_t st) {

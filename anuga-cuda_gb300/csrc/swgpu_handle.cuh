@@ -27,6 +27,7 @@ struct Handle {
     float *trk_hmax = nullptr, *trk_tarr = nullptr;  // tracking buffers (S.hmax/S.tarr when on)
     int nscen = 1;               // scenarios (Ctrl blocks); > 1 for an ensemble
     std::vector<int64_t> scen_offsets;  // ensemble: first triangle of each scenario, + N
+    std::vector<int64_t> scen_edges;    // FP64: first edge of each scenario, + the edge count
     int *d_blk_scen = nullptr;   // ensemble: scenario of each 256-triangle block
     Ctrl *d_ctrl = nullptr;      // [nscen]
     Ctrl *h_ctrl = nullptr;      // pinned mirror [nscen]
@@ -40,6 +41,7 @@ struct Handle {
     cudaGraphExec_t graph = nullptr;  // steps_per_graph fused steps
     bool resume_after_yield = false;
     bool vertices_stale = true;
+    bool edges_stale = true;     // FP64: edge values are not the interpolation of the vertex values
     bool mixed_from_stage = true;  // mixed: FP64 stage upload not yet converted to depth
     bool elevation_set = false;
     bool unusable = false;  // a kernel reported SWGPU_ETIMEOUT: only destroy is allowed

@@ -33,6 +33,33 @@ struct LaunchShape {
     int pdl;        // mixed kernels launched as programmatic dependents of the previous one
 };
 
+// The unique edges of the mesh (FP64 handles), in the order of their owners'
+// indices; an ensemble pads each scenario's to a multiple of 256.
+struct DevEdges {
+    int E;             // edges, padding included
+    int launch;        // edges launched: E, or those of the scenarios still running
+    const int *left;   // [E] owner and its edge, packed as DevMesh::nbr; -1 padding
+    const int *right;  // [E] neighbour and its edge, or -(boundary slot + 1)
+    const double *n1, *n2, *len;  // [E] the owner's unit normal, the length
+    const double *rad; // [E] the smaller radius of the two triangles; infinite where
+                       // the owner is not full (the edge sets no timestep)
+    const int *te;     // [3][N] edge of triangle edge i, << 1 | 1 on the neighbour's side
+    const int *blk_scen;  // ensembles: scenario of each 256 edges
+    double *f;         // [3][E] flux times length
+    double *ms;        // [E] maximum speed (written when asked for)
+};
+
+// Planes of DevMesh::geo64 (geometry_fp64).
+enum : int {
+    kGeoInvArea, kGeoX10, kGeoY10, kGeoX20, kGeoY20, kGeoDet,
+    kGeoDxv, kGeoDyv = kGeoDxv + 3,  // vertex offsets from the centroid
+    // auxiliary triangle: differences and 1/area2 (0: zero gradient); for a
+    // triangle with one neighbour Dx1, Dy1 the difference and Dx2, Dy2 the same
+    // over its squared length
+    kGeoDx1 = kGeoDyv + 3, kGeoDy1, kGeoDx2, kGeoDy2, kGeoInvArea2,
+    kGeoPlanes
+};
+
 struct DevMesh {
     int N, Nb;
     int n_launch;  // triangles the fused-step kernels are launched over: N, or for an
@@ -53,6 +80,8 @@ struct DevMesh {
     // ensembles: scenario of each 256-triangle block (scenarios start on
     // 256-triangle boundaries); nullptr for a single mesh
     const int *blk_scen;
+    DevEdges edges;            // FP64 handles
+    const double *geo64;       // [kGeoPlanes][N], FP64 handles
 };
 
 // FP64 state (both precisions keep the conserved centroid state in FP64).
@@ -124,6 +153,10 @@ struct DevParams {
     int limiter;  // kLimiterOptimised, kLimiterVertex or kLimiterEdge
     int flow_algorithm;  // 0 default, 1 'tsunami' (protect_swb2 + edge extrapolation)
     double track_threshold;  // depth that counts as arrival
+    double rise_w, rise_uh, rise_vh;  // beta - beta_dry
+    int betas_differ;    // any of them is not zero
+    int plain_positive;  // g, epsilon, H0 and minimum_allowed_height are positive and
+                         // of ordinary size (the FP64 kernels' integer comparisons)
     // FP32 copies for the mixed kernels (set on the host; FP64 arithmetic
     // on GB300 runs at 1/64 of the FP32 rate, so none is done per thread)
     float f_g, f_eps, f_H0, f_h0, f_lim, f_mah, f_mas, f_max_dt, f_alpha;
@@ -222,8 +255,13 @@ void launch_distribute_fp64(const DevMesh &M, const DevState &S, const DevParams
 void launch_boundary_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                           const BcTag *tags,
                           Ctrl *ctrl, cudaStream_t st);
+// edge fluxes from the edge values of the last distribute (or interpolation)
 void launch_flux_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                       Ctrl *ctrl, int flags, cudaStream_t st);
+// explicit updates and max_speed from the edge fluxes (the stand-alone compute_fluxes)
+void launch_explicit_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
+                          cudaStream_t st);
+void launch_geometry_fp64(const DevMesh &M, double *geo, cudaStream_t st);
 // Manning friction (S * momentum) added to the semi-implicit updates, or with
 // explicit_target to the explicit updates (manning_friction_explicit)
 void launch_forcing_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
@@ -281,5 +319,16 @@ void launch_mass_partials_mixed(const DevMesh &M, const DevState &S, const DevMi
                                 cudaStream_t st);
 
 inline int grid_for(int n) { return (n + kBlock - 1) / kBlock; }
+
+// Threads per block of an FP64 step kernel over n items: the launch shape's,
+// halved (down to a warp) while the launch has fewer than 16 blocks per SM.
+// The kernels are bound by each SM's FP64 pipe, so what counts is that every
+// SM gets the same share: 40,000 triangles in blocks of 256 are 157 blocks,
+// which leaves 147 of 152 SMs idle for half of the launch.
+inline int fp64_block(int knob, int64_t n, int sms) {
+    int b = knob;
+    while (b > 32 && (n + b - 1) / b < (int64_t)16 * sms) b >>= 1;
+    return b;
+}
 
 }  // namespace swgpu

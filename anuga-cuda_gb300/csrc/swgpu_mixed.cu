@@ -278,15 +278,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long *bar, Ctrl 
         if (mbar_try_wait(bar, parity)) break;
     return false;
 }
-// Programmatic dependent launch: let the next kernel of the stream start
-// its blocks as this one's finish, and wait (in the next kernel) until the
-// previous kernel has completed and its writes are visible.  Both are no-ops
-// for kernels launched without the programmatic attribute.
-__device__ __forceinline__ void pdl_launch_dependents() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Orders this thread's earlier generic-proxy accesses to shared memory
 // before later async-proxy (bulk copy) writes to it.
 __device__ __forceinline__ void fence_proxy_async() {
@@ -1170,25 +1161,6 @@ __global__ void mass_final_mixed(const double *partials, int n, double *out) {
 
 // Block sizes come from M.shape (the autotuner's choice; results do not
 // depend on it).
-// A launch of kernel k; with pdl, as a programmatic dependent of the stream's
-// previous kernel (it may start during that kernel's last wave and waits for
-// it with griddepcontrol.wait before reading what that kernel writes).
-template <typename... KArgs, typename... Args>
-static void launch_k(void (*k)(KArgs...), int grid, int block, cudaStream_t st, bool pdl,
-                     Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, k, args...);
-}
-
 void launch_distribute_mixed(const DevMesh &M, const DevState &S, const DevMixed &X,
                              const DevParams &P, const BcTag *tags, Ctrl *ctrl, int flags,
                              const Stage &stage, cudaStream_t st) {
