@@ -699,6 +699,9 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     P.limiter = params->use_edge_limiter ? kLimiterEdge
                 : params->optimised_gradient_limiter ? kLimiterOptimised
                                                      : kLimiterVertex;
+    P.h0 = P.H0 * P.H0;
+    P.lim = 10 * P.H0;
+    P.minus_half_g = -0.5 * P.g;
     P.rise_w = P.beta_w - P.beta_w_dry;
     P.rise_uh = P.beta_uh - P.beta_uh_dry;
     P.rise_vh = P.beta_vh - P.beta_vh_dry;

@@ -54,6 +54,7 @@ struct EdgeState {
 };
 struct EdgeFlux {
     double f0, f1, f2, ms;
+    double t;  // the edge's bound of the timestep
     bool bad;  // discontinuous bed
 };
 
@@ -61,9 +62,11 @@ struct EdgeFlux {
 // plain FP64 arithmetic, with the dry test of :4581-4587: for states that
 // are not finite or huge, and for parameters that are not positive.
 static __device__ __noinline__ EdgeFlux central_flux_any(const EdgeState &s, const DevParams &P,
-                                                         double h0, double lim) {
+                                                         double rad) {
+    const double h0 = P.h0, lim = P.lim;
     EdgeFlux r;
     r.f0 = r.f1 = r.f2 = r.ms = 0.0;
+    r.t = P.evolve_max_timestep;
     r.bad = false;
     if (P.optimise_dry_cells && fabs(s.wl - s.zl) < P.epsilon && fabs(s.wr - s.zr) < P.epsilon)
         return r;
@@ -115,33 +118,12 @@ static __device__ __noinline__ EdgeFlux central_flux_any(const EdgeState &s, con
     e2 += ss * (br - bl);
     e2 *= inv;
     r.ms = omax(fabs(smax), fabs(smin));
+    if (r.ms > eps) r.t = omin(r.t, rad / r.ms);
     // rotate back: _rotate(edgeflux, n1, -n2)
     r.f0 = e0;
     r.f1 = s.n1 * e1 + (-s.n2) * e2;
     r.f2 = -(-s.n2) * e1 + s.n1 * e2;
     return r;
-}
-
-// limited_speed for both momentum components of one side (the second call of
-// the plain form sees the depth that the first one left) with comparisons,
-// quotients off the FP64 pipe; h finite, eps, h0 and lim positive.
-__device__ __forceinline__ double side_speed(double &uh, double &vh, double &h, double eps,
-                                             double h0, double lim) {
-    const bool shallow = lt_pos(h, lim);
-    double den = h;
-    if (shallow) {
-        if (lt_pos(h, eps)) {
-            h = uh = vh = 0.0;
-            return 0.0;
-        }
-        den = h + fdiv64(h0, h);
-    }
-    const double u = fdiv64(uh, den);
-    if (shallow) {
-        uh = u * h;
-        vh = fdiv64(vh, den) * h;
-    }
-    return u;
 }
 
 // x small enough that nothing computed from it overflows (and not NaN)
@@ -152,13 +134,15 @@ __device__ __forceinline__ bool tame(double x) {
 // central_flux_any with the same operations in the same order, its
 // comparisons, quotients and roots on the integer pipe: 62 FP64
 // instructions where the plain form executes about 165.
-__device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevParams &P, double h0,
-                                                 double lim) {
+__device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevParams &P,
+                                                 double rad) {
     if (!(P.plain_positive && tame(s.wl) && tame(s.uhl) && tame(s.vhl) && tame(s.wr) &&
           tame(s.uhr) && tame(s.vhr) && tame(s.zl) && tame(s.zr)))
-        return central_flux_any(s, P, h0, lim);
+        return central_flux_any(s, P, rad);
+    const double h0 = P.h0, lim = P.lim;
     EdgeFlux r;
     r.f0 = r.f1 = r.f2 = r.ms = 0.0;
+    r.t = P.evolve_max_timestep;
     r.bad = false;
     const double g = P.g, eps = P.epsilon;
     double hl = s.wl - s.zl, hr = s.wr - s.zr;
@@ -178,11 +162,37 @@ __device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevPa
     const double ar = s.n1 * s.uhr + s.n2 * s.vhr;
     const double br = -s.n2 * s.uhr + s.n1 * s.vhr;
     double uhl = al, vhl = bl, uhr = ar, vhr = br;
-    const double ul = side_speed(uhl, vhl, hl, eps, h0, lim);
-    const double ur = side_speed(uhr, vhr, hr, eps, h0, lim);
+    // limited_speed for both momentum components of both sides (its second
+    // call sees the depth that the first one left; a zero over a positive
+    // depth is a zero)
+    double dl = hl, dr = hr;
+    const bool sl = lt_pos(hl, lim), sr = lt_pos(hr, lim);
+    if (sl || sr) {
+        const bool zl = lt_pos(hl, eps), zr = lt_pos(hr, eps);
+        if (zl) hl = uhl = vhl = 0.0;
+        if (zr) hr = uhr = vhr = 0.0;
+        dl = zl ? 1.0 : hl;
+        dr = zr ? 1.0 : hr;
+        const Two r = div2(h0, dl, h0, dr);
+        if (sl && !zl) dl = hl + r.a;
+        if (sr && !zr) dr = hr + r.b;
+    }
+    const Two u = div2(uhl, dl, uhr, dr);
+    const double ul = u.a, ur = u.b;
+    if (sl || sr) {
+        const Two v = div2(vhl, dl, vhr, dr);
+        if (sl) {
+            uhl = ul * hl;
+            vhl = v.a * hl;
+        }
+        if (sr) {
+            uhr = ur * hr;
+            vhr = v.b * hr;
+        }
+    }
     const double ghl = g * hl, ghr = g * hr;
-    const double cl = fsqrt64(ghl);
-    const double cr = fsqrt64(ghr);
+    const Two c = sqrt2(ghl, ghr);
+    const double cl = c.a, cr = c.b;
     double smax = imax(ul + cl, ur + cr);
     if (lt_zero(smax)) smax = 0.0;
     double smin = imin(ul - cl, ur - cr);
@@ -195,7 +205,11 @@ __device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevPa
     const double fr0 = ur * hr;
     const double fr1 = ur * uhr + half_of(ghr) * hr;
     const double fr2 = ur * vhr;
-    const double inv = fdiv64(1.0, denom);
+    r.ms = fabs(mag_lt(smin, smax) ? smax : smin);
+    const bool fast = lt_pos(eps, r.ms);
+    const Two iq = div2(1.0, denom, rad, fast ? r.ms : 1.0);
+    const double inv = iq.a;
+    if (fast) r.t = iq.b;
     const double ss = smax * smin;
     double e0 = smax * fl0 - smin * fr0;
     e0 += ss * (s.wr - s.wl);
@@ -206,7 +220,6 @@ __device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevPa
     double e2 = smax * fl2 - smin * fr2;
     e2 += ss * (br - bl);
     e2 *= inv;
-    r.ms = fabs(mag_lt(smin, smax) ? smax : smin);
     r.f0 = e0;
     r.f1 = s.n1 * e1 + (-s.n2) * e2;
     r.f2 = s.n2 * e1 + s.n1 * e2;
@@ -263,16 +276,13 @@ __global__ void __launch_bounds__(kBlock) flux_fp64(DevMesh M, DevState S, DevPa
             s.vhr = S.vhb[mb];
             s.zr = s.zl;
         }
-        const EdgeFlux r = central_flux(s, P, P.H0 * P.H0, 10 * P.H0);
+        const EdgeFlux r = central_flux(s, P, rad);
         F.f[e] = r.f0 * len;
         F.f[F.E + e] = r.f1 * len;
         F.f[2 * F.E + e] = r.f2 * len;
         if (flags & kWriteMaxSpeed) F.ms[e] = r.ms;
         bad = r.bad;
-        if (P.plain_positive ? lt_pos(P.epsilon, r.ms) && tame(r.ms) : r.ms > P.epsilon) {
-            const double q = fdiv64(rad, r.ms);
-            t = mag_lt(t, q) ? t : q;
-        }
+        t = lt64(t, r.t) ? t : r.t;
     }
     if (bad) set_status(ctrl, SWGPU_EBED);
     if (flags & kNoTimestep) return;  // later Runge-Kutta stage: the step's dt is set
@@ -319,16 +329,12 @@ __device__ __forceinline__ void explicit_update(const DevMesh &M, const DevState
     const double x20 = G[kGeoX20 * (size_t)N], y20 = G[kGeoY20 * (size_t)N];
     const double det = G[kGeoDet * (size_t)N];
     const double w0 = S.wv[k], d1 = S.wv[N + k] - w0, d2 = S.wv[2 * N + k] - w0;
-    const double wx = fdiv64(y20 * d1 - y10 * d2, det);
-    const double wy = fdiv64(x10 * d2 - x20 * d1, det);
     const double avg_h = w - zc;
-    a1 += -g * wx * avg_h;
-    a2 += -g * wy * avg_h;
     double sidex = 0.0, sidey = 0.0;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         const double hh = S.we[i * N + k] - S.ze[i * N + k];
-        const double fact = -0.5 * g * hh * hh * M.len[i * N + k];
+        const double fact = P.minus_half_g * hh * hh * M.len[i * N + k];
         const double sx = fact * M.normals[(2 * i) * N + k];
         const double sy = fact * M.normals[(2 * i + 1) * N + k];
         // (0 + s is s: the sign of a zero is lost in the sum with a1 below)
@@ -336,8 +342,12 @@ __device__ __forceinline__ void explicit_update(const DevMesh &M, const DevState
         sidey = i == 0 ? sy : sidey + sy;
     }
     const double area = M.areas[k];
-    a1 += fdiv64(-sidex, area);
-    a2 += fdiv64(-sidey, area);
+    const Two w_xy = div2(y20 * d1 - y10 * d2, det, x10 * d2 - x20 * d1, det);
+    const Two side = div2(-sidex, area, -sidey, area);
+    a1 += -g * w_xy.a * avg_h;
+    a2 += -g * w_xy.b * avg_h;
+    a1 += side.a;
+    a2 += side.b;
 }
 
 // compute_fluxes as the stand-alone method: the explicit updates, and
@@ -458,7 +468,7 @@ __device__ __forceinline__ double manning_S(const DevMesh &M, const DevState &S,
         Sf = -P.g * eta * eta * zs * fsqrt64(uh * uh + vh * vh);
     else
         Sf = -P.g * eta * eta * fsqrt64(uh * uh + vh * vh);
-    Sf = fdiv64(Sf, pow(h, 7.0 / 3));
+    Sf = fdiv64(Sf, pow_seven_thirds(h));
     applied = true;
     return Sf;
 }
@@ -527,17 +537,24 @@ __device__ __forceinline__ void protect_one(const DevParams &P, double zc, doubl
     }
 }
 
-// src/anuga_HMPP/quantity.c:769-820 (_update) on one value with a nonzero
-// semi-implicit term; returns false if the denominator is not positive.
-__device__ __forceinline__ bool semi_update(double &c, double e, double semi, double dt) {
-    if ((bits64(c) & kMag64) == 0)
-        semi = 0.0;
-    else
-        semi = fdiv64(semi, c);
-    c += dt * e;
-    const double den = 1.0 - dt * semi;
-    if (lt64_nan(den, 0.0) || (bits64(den) & kMag64) == 0) return false;
-    c = fdiv64(c, den);
+// src/anuga_HMPP/quantity.c:769-820 (_update) on both momenta with nonzero
+// semi-implicit terms; returns false if a denominator is not positive.
+__device__ __forceinline__ bool semi_update(double &u, double &v, double eu, double ev, double su,
+                                            double sv, double dt) {
+    const bool zu = (bits64(u) & kMag64) == 0, zv = (bits64(v) & kMag64) == 0;
+    Two s = div2(su, zu ? 1.0 : u, sv, zv ? 1.0 : v);
+    if (zu) s.a = 0.0;
+    if (zv) s.b = 0.0;
+    u += dt * eu;
+    v += dt * ev;
+    const double du = 1.0 - dt * s.a, dv = 1.0 - dt * s.b;
+    if (!(gt_zero(du) && gt_zero(dv)) &&
+        (lt64_nan(du, 0.0) || lt64_nan(dv, 0.0) || (bits64(du) & kMag64) == 0 ||
+         (bits64(dv) & kMag64) == 0))
+        return false;
+    const Two q = div2(u, du, v, dv);
+    u = q.a;
+    v = q.b;
     return true;
 }
 
@@ -600,8 +617,7 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
         // stage has no semi-implicit term: its denominator is exactly 1
         w += dt * ew;
         if (applied) {
-            if (!semi_update(uh, euh, su, dt)) bad = 1;
-            if (!semi_update(vh, evh, sv, dt)) bad = 1;
+            if (!semi_update(uh, vh, euh, evh, su, sv, dt)) bad = 1;
         } else {
             uh += dt * euh;
             vh += dt * evh;
@@ -623,8 +639,9 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
             }
             if (P.extrapolate_velocity_second_order == 1) {
                 const double dk = imax(w - zc, P.minimum_allowed_height);
-                S.uvel[k] = fdiv64(uh, dk);
-                S.vvel[k] = fdiv64(vh, dk);
+                const Two vel = div2(uh, dk, vh, dk);
+                S.uvel[k] = vel.a;
+                S.vvel[k] = vel.b;
             }
         }
         // NaN / Inf anywhere in the new state stops the run: beyond 1e308 in
@@ -696,8 +713,9 @@ __global__ void __launch_bounds__(kBlock) prepare_fp64(DevMesh M, DevState S, De
     S.uh[k] = uh;
     S.vh[k] = vh;
     const double dk = omax(w - zc, P.minimum_allowed_height);
-    S.uvel[k] = fdiv64(uh, dk);
-    S.vvel[k] = fdiv64(vh, dk);
+    const Two vel = div2(uh, dk, vh, dk);
+    S.uvel[k] = vel.a;
+    S.vvel[k] = vel.b;
 }
 
 // The centroid velocities alone: extrapolate_velocity_second_order_true
@@ -707,8 +725,9 @@ __global__ void __launch_bounds__(kBlock) velocities_fp64(DevMesh M, DevState S,
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= M.N) return;
     const double dk = omax(S.w[k] - S.zc[k], P.minimum_allowed_height);
-    S.uvel[k] = fdiv64(S.uh[k], dk);
-    S.vvel[k] = fdiv64(S.vh[k], dk);
+    const Two vel = div2(S.uh[k], dk, S.vh[k], dk);
+    S.uvel[k] = vel.a;
+    S.vvel[k] = vel.b;
 }
 
 // --------------------------------------------------------- distribute ---
@@ -736,17 +755,26 @@ __device__ __forceinline__ void qmin_qmax(double dq0, double dq1, double dq2, do
 __device__ __forceinline__ void limit_jumps(double (&d)[3], double qmin, double qmax,
                                             double beta) {
     const u64 tiny = 0x2b2bff2ee48e0530ull;  // the bits of 1e-100
+    bool on[3];
+    double top[3], low[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        on[i] = (bits64(d[i]) & kMag64) > tiny;
+        top[i] = lt_zero(d[i]) ? qmin : qmax;
+        low[i] = on[i] ? d[i] : 1.0;
+    }
+    const Three q3 = div3(top[0], low[0], top[1], low[1], top[2], low[2]);
+    const double q[3] = {q3.a, q3.b, q3.c};
     double r = 1000.0, r0 = 1.0;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        if ((bits64(d[i]) & kMag64) > tiny) r0 = fdiv64(lt_zero(d[i]) ? qmin : qmax, d[i]);
+        if (on[i]) r0 = q[i];
         r = mag_lt(r0, r) ? r0 : r;
     }
     const double rb = r * beta;
     const double phi = lt_pos(rb, 1.0) ? rb : 1.0;
-    d[0] = d[0] * phi;
-    d[1] = d[1] * phi;
-    d[2] = d[2] * phi;
+#pragma unroll
+    for (int i = 0; i < 3; i++) d[i] = d[i] * phi;
 }
 
 // Auxiliary-triangle reconstruction of one quantity
@@ -785,10 +813,18 @@ __device__ __forceinline__ void one_nbr_jumps(double qk, double q1, double dx2, 
     for (int i = 0; i < 3; i++) out[i] = qk + d[i];
 }
 
-// the limiter's factor of one quantity: beta_dry + (beta - beta_dry) * hfactor
+// the limiter's factor of each quantity: beta_dry + (beta - beta_dry) * hfactor
 // (the same number whatever hfactor where the two are equal)
-__device__ __forceinline__ double beta_of(double dry, double rise, double hfactor) {
-    return rise == 0.0 ? dry : dry + rise * hfactor;
+__device__ __forceinline__ void limiter_betas(const DevParams &P, double hfactor,
+                                              double (&beta)[3]) {
+    beta[0] = P.beta_w_dry;
+    beta[1] = P.beta_uh_dry;
+    beta[2] = P.beta_vh_dry;
+    if (P.betas_differ) {
+        beta[0] += P.rise_w * hfactor;
+        beta[1] += P.rise_uh * hfactor;
+        beta[2] += P.rise_vh * hfactor;
+    }
 }
 
 // The 'tsunami' distribute (gpu_domain_advanced.py:1755-1812): the edge
@@ -819,7 +855,9 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
         const double *V = vel ? S.vvel : S.vh;
         const double wk = S.w[k], uk = U[k], vk = V[k];
         const int nbk = M.nb[k];
-        double ew[3], eu[3], ev[3];
+        double ed[3][3];  // edge values of stage and the momenta (or velocities)
+        double (&ew)[3] = ed[0], (&eu)[3] = ed[1], (&ev)[3] = ed[2];
+        const double own[3] = {wk, uk, vk};
         bool flat = false, keep = false;
         if (nbk == 3) {
             flat = true;
@@ -858,13 +896,16 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
                     if (P.optimise_dry_cells && lt64(imax(h0, imax(h1, h2)), P.epsilon)) {
                         keep = true;
                     } else {
+                        const double q0[3] = {S.w[k0], U[k0], V[k0]};
+                        const double q1[3] = {S.w[k1], U[k1], V[k1]};
+                        const double q2[3] = {S.w[k2], U[k2], V[k2]};
+                        double beta[3];
+                        limiter_betas(P, hfactor, beta);
                         const double inv_area2 = fdiv64(1.0, area2);
-                        aux_jumps(wk, S.w[k0], S.w[k1], S.w[k2], dx1, dy1, dx2, dy2, inv_area2,
-                                  dxv, dyv, beta_of(P.beta_w_dry, P.rise_w, hfactor), ew);
-                        aux_jumps(uk, U[k0], U[k1], U[k2], dx1, dy1, dx2, dy2, inv_area2, dxv,
-                                  dyv, beta_of(P.beta_uh_dry, P.rise_uh, hfactor), eu);
-                        aux_jumps(vk, V[k0], V[k1], V[k2], dx1, dy1, dx2, dy2, inv_area2, dxv,
-                                  dyv, beta_of(P.beta_vh_dry, P.rise_vh, hfactor), ev);
+#pragma unroll
+                        for (int v = 0; v < 3; v++)
+                            aux_jumps(own[v], q0[v], q1[v], q2[v], dx1, dy1, dx2, dy2, inv_area2,
+                                      dxv, dyv, beta[v], ed[v]);
                     }
                 }
             } else {
@@ -883,9 +924,10 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
                     double dx2 = fdiv64(1.0, area2);
                     const double dy2 = dx2 * dy1;
                     dx2 *= dx1;
-                    one_nbr_jumps(wk, S.w[k1], dx2, dy2, dxv, dyv, P.beta_w, ew);
-                    one_nbr_jumps(uk, U[k1], dx2, dy2, dxv, dyv, P.beta_w, eu);
-                    one_nbr_jumps(vk, V[k1], dx2, dy2, dxv, dyv, P.beta_w, ev);
+                    const double q1[3] = {S.w[k1], U[k1], V[k1]};
+#pragma unroll
+                    for (int v = 0; v < 3; v++)
+                        one_nbr_jumps(own[v], q1[v], dx2, dy2, dxv, dyv, P.beta_w, ed[v]);
                 }
             }
         }
@@ -1059,36 +1101,46 @@ __device__ __forceinline__ bool limit_by_neighbours(const DevMesh &M, const doub
 // balance_deep_and_shallow (src/anuga_HMPP/shallow_water_ext.c:1462-1636)
 // of one triangle: centroid stage wk, bed zk, momentum uk, vk; bed vertex
 // values zvk; stage / momentum vertex values ow, ou, ov blended in place.
+// hv: the vertex depths ow - zvk.
 __device__ __forceinline__ void balance_one(const DevParams &P, double wk, double zk, double uk,
-                                            double vk, const double (&zvk)[3], double (&ow)[3],
+                                            double vk, const double (&zvk)[3],
+                                            const double (&hv)[3], double (&ow)[3],
                                             double (&ou)[3], double (&ov)[3]) {
     const double eps = 1.0e-6;
-    const double hc = wk - zk;
-    double dz = 0.0, hv[3];
+    double dz = 0.0;
     if (P.tight_slope_limiters == 0) {
 #pragma unroll
         for (int i = 0; i < 3; i++) dz = omax(dz, fabs(zvk[i] - zk));
     }
-#pragma unroll
-    for (int i = 0; i < 3; i++) hv[i] = ow[i] - zvk[i];
     const double hmin = imin(hv[0], imin(hv[1], hv[2]));
-    double alpha = 1.0;
+    double alpha = 1.0, hc = 0.0;
     if (P.tight_slope_limiters == 0) {
         alpha = dz > 0.0 ? omax(omin(fdiv64(P.alpha_balance * hmin, dz), 1.0), 0.0) : 1.0;
     } else if (lt64(hmin, P.H0)) {
+        hc = wk - zk;
         const double head = hc - P.H0;
+        double hd[3];
+        bool on[3];
 #pragma unroll
         for (int i = 0; i < 3; i++) {
-            const double hd = hc - hv[i];
-            if (gt_zero(hd)) alpha = imin(alpha, fdiv64(head, hd));
+            hd[i] = hc - hv[i];
+            on[i] = gt_zero(hd[i]);
+            if (!on[i]) hd[i] = 1.0;
         }
+        const Three q3 = div3(head, hd[0], head, hd[1], head, hd[2]);
+        const double q[3] = {q3.a, q3.b, q3.c};
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+            if (on[i]) alpha = imin(alpha, q[i]);
         if (lt_zero(alpha)) alpha = 0.0;  // alpha is at most 1
     }
     if (lt64(alpha, 1.0)) {
         double uc = 0.0, vc = 0.0;
+        if (P.tight_slope_limiters == 0) hc = wk - zk;
         if (P.use_centroid_velocities == 1 && lt64(eps, hc)) {
-            uc = fdiv64(uk, hc);
-            vc = fdiv64(vk, hc);
+            const Two c = div2(uk, hc, vk, hc);
+            uc = c.a;
+            vc = c.b;
         }
 #pragma unroll
         for (int i = 0; i < 3; i++) {
@@ -1111,15 +1163,16 @@ __global__ void __launch_bounds__(kBlock) balance_fp64(DevMesh M, DevState S, De
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = M.N;
     if (k >= N) return;
-    double zvk[3], ow[3], ou[3], ov[3];
+    double zvk[3], hv[3], ow[3], ou[3], ov[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         zvk[i] = S.zv[i * N + k];
         ow[i] = S.wv[i * N + k];
         ou[i] = S.uhv[i * N + k];
         ov[i] = S.vhv[i * N + k];
+        hv[i] = ow[i] - zvk[i];
     }
-    balance_one(P, S.w[k], S.zc[k], S.uh[k], S.vh[k], zvk, ow, ou, ov);
+    balance_one(P, S.w[k], S.zc[k], S.uh[k], S.vh[k], zvk, hv, ow, ou, ov);
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         S.wv[i * N + k] = ow[i];
@@ -1147,10 +1200,12 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
         double zvk[3];
 #pragma unroll
         for (int i = 0; i < 3; i++) zvk[i] = S.zv[i * N + k];
-        double ow[3], ou[3], ov[3];
+        double vert[3][3];  // vertex values of stage and the momenta
+        double (&ow)[3] = vert[0], (&ou)[3] = vert[1], (&ov)[3] = vert[2];
         // the stand-alone extrapolate_second_order_sw is second order with
         // the optimised limiter whatever the domain's order and limiter
         const bool extrapolate_only = flags & kExtrapolateOnly;
+        bool to_momentum = false;
         if (order == 1 && !extrapolate_only) {
 #pragma unroll
             for (int i = 0; i < 3; i++) {
@@ -1167,8 +1222,10 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
         } else {
             const bool vel = P.extrapolate_velocity_second_order == 1;
             // centroid values being extrapolated (velocity or momentum)
-            const double qu = vel ? S.uvel[k] : uk;
-            const double qv = vel ? S.vvel[k] : vk;
+            const double *U = vel ? S.uvel : S.uh, *V = vel ? S.vvel : S.vh;
+            const double qu = vel ? U[k] : uk;
+            const double qv = vel ? V[k] : vk;
+            const double own[3] = {wk, qu, qv};
             const int nbk = M.nb[k];
             bool keep = false;  // dry: previous vertex values stay
             bool flat = nbk == 3;  // zero gradient: centroid values at vertices
@@ -1202,18 +1259,15 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
                                 if (lt64(0.001, hmin))
                                     hfactor = fdiv64(hmin - 0.001, hmin + 0.004);
                             }
-                            aux_jumps(wk, w0, w1, w2, dx1, dy1, dx2, dy2, inv_area2, dxv, dyv,
-                                      beta_of(P.beta_w_dry, P.rise_w, hfactor), ow);
-                            const double u0 = vel ? S.uvel[k0] : S.uh[k0];
-                            const double u1 = vel ? S.uvel[k1] : S.uh[k1];
-                            const double u2 = vel ? S.uvel[k2] : S.uh[k2];
-                            aux_jumps(qu, u0, u1, u2, dx1, dy1, dx2, dy2, inv_area2, dxv, dyv,
-                                      beta_of(P.beta_uh_dry, P.rise_uh, hfactor), ou);
-                            const double v0 = vel ? S.vvel[k0] : S.vh[k0];
-                            const double v1 = vel ? S.vvel[k1] : S.vh[k1];
-                            const double v2 = vel ? S.vvel[k2] : S.vh[k2];
-                            aux_jumps(qv, v0, v1, v2, dx1, dy1, dx2, dy2, inv_area2, dxv, dyv,
-                                      beta_of(P.beta_vh_dry, P.rise_vh, hfactor), ov);
+                            const double q0[3] = {w0, U[k0], V[k0]};
+                            const double q1[3] = {w1, U[k1], V[k1]};
+                            const double q2[3] = {w2, U[k2], V[k2]};
+                            double beta[3];
+                            limiter_betas(P, hfactor, beta);
+#pragma unroll
+                            for (int v = 0; v < 3; v++)
+                                aux_jumps(own[v], q0[v], q1[v], q2[v], dx1, dy1, dx2, dy2,
+                                          inv_area2, dxv, dyv, beta[v], vert[v]);
                         }
                     }
                 } else {
@@ -1228,11 +1282,10 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
                         no_nbr = 1;
                         flat = true;
                     } else {
-                        one_nbr_jumps(wk, S.w[k1], dx2, dy2, dxv, dyv, P.beta_w, ow);
-                        one_nbr_jumps(qu, vel ? S.uvel[k1] : S.uh[k1], dx2, dy2, dxv, dyv,
-                                      P.beta_w, ou);
-                        one_nbr_jumps(qv, vel ? S.vvel[k1] : S.vh[k1], dx2, dy2, dxv, dyv,
-                                      P.beta_w, ov);
+                        const double q1[3] = {S.w[k1], U[k1], V[k1]};
+#pragma unroll
+                        for (int v = 0; v < 3; v++)
+                            one_nbr_jumps(own[v], q1[v], dx2, dy2, dxv, dyv, P.beta_w, vert[v]);
                     }
                 }
             }
@@ -1251,19 +1304,22 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
                     ov[i] = S.vhv[i * N + k];
                 }
             }
-            if (vel) {
-                // back from velocity to momentum with the vertex depth
+            to_momentum = vel;
+        }
+        double hv[3];
 #pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    double dv = ow[i] - zvk[i];
-                    if (!gt_zero(dv)) dv = 0.0;
-                    ou[i] = ou[i] * dv;
-                    ov[i] = ov[i] * dv;
-                }
+        for (int i = 0; i < 3; i++) hv[i] = ow[i] - zvk[i];
+        if (to_momentum) {
+            // back from velocity to momentum with the vertex depth
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const double dv = gt_zero(hv[i]) ? hv[i] : 0.0;
+                ou[i] = ou[i] * dv;
+                ov[i] = ov[i] * dv;
             }
         }
 
-        if (!(flags & kExtrapolateOnly)) balance_one(P, wk, zk, uk, vk, zvk, ow, ou, ov);
+        if (!(flags & kExtrapolateOnly)) balance_one(P, wk, zk, uk, vk, zvk, hv, ow, ou, ov);
 
 #pragma unroll
         for (int i = 0; i < 3; i++) {

@@ -153,6 +153,7 @@ struct DevParams {
     int limiter;  // kLimiterOptimised, kLimiterVertex or kLimiterEdge
     int flow_algorithm;  // 0 default, 1 'tsunami' (protect_swb2 + edge extrapolation)
     double track_threshold;  // depth that counts as arrival
+    double h0, lim, minus_half_g;     // H0^2, 10 H0, -g/2
     double rise_w, rise_uh, rise_vh;  // beta - beta_dry
     int betas_differ;    // any of them is not zero
     int plain_positive;  // g, epsilon, H0 and minimum_allowed_height are positive and

@@ -63,12 +63,12 @@ __device__ __forceinline__ double imax(double x, double y) { return lt64(y, x) ?
 __device__ __forceinline__ double imin(double x, double y) { return lt64(x, y) ? x : y; }
 
 // 0.5 * x on the integer pipe where the halved number is normal (or x zero)
+static __device__ __noinline__ double half_any(double x) { return 0.5 * x; }
 __device__ __forceinline__ double half_of(double x) {
-    const unsigned h = hi32(x), e = h & 0x7ff00000u;
-    if (e - 0x00200000u < 0x7fd00000u)  // exponent 2 .. 2046
-        return __hiloint2double((int)(h - 0x00100000u), __double2loint(x));
-    if ((bits64(x) & kMag64) == 0) return x;
-    return 0.5 * x;
+    const unsigned h = hi32(x);
+    const bool zero = (bits64(x) & kMag64) == 0;
+    if (!zero && (h & 0x7ff00000u) - 0x00200000u >= 0x7fd00000u) return half_any(x);
+    return __hiloint2double((int)(zero ? h : h - 0x00100000u), __double2loint(x));
 }
 
 // ---- division and square root ---------------------------------------------
@@ -115,27 +115,28 @@ __device__ __forceinline__ u64 mul_32x64(unsigned a, u64 b) {
 //                           < 7 2^20 2^-20.4 + 2 + 1 -> R2 in [0, 9B)
 //   q3 = floor(R2 r 2^11):  short by < 1.02 -> R3 in [0, 1.02 B)
 // N = 2^31 q1 + 2^11 q2 + q3 and R3 = 2^52 A - N B decide the rounding.
-__device__ __forceinline__ double fdiv64(double a, double b) {
+//
+// Straight-line code, so that several run interleaved (a warp alone on an SM
+// waits out the latency of every instruction of a single one): fine is
+// cleared for operands that div_any has to take.
+__device__ __forceinline__ double div_digits(double a, double b, bool &fine) {
     const unsigned ha = hi32(a), hb = hi32(b);
     const int ea = (int)((ha >> 20) & 0x7ffu), eb = (int)((hb >> 20) & 0x7ffu);
     const unsigned sign = (ha ^ hb) & 0x80000000u;
-    int e = ea - eb + 1023;
+    int e = ea - eb + 1022;
     const unsigned la = (unsigned)__double2loint(a), lb = (unsigned)__double2loint(b);
-    const bool b_normal = (unsigned)(eb - 1) < 2046u;
-    if (!(b_normal && (unsigned)(ea - 1) < 2046u && (unsigned)(e - 2) < 2043u)) {
-        if (b_normal && (((ha << 1) | la) == 0u)) return __hiloint2double((int)sign, 0);
-        return div_any(a, b);
-    }
+    const bool zero = ((ha << 1) | la) == 0u;
+    fine = (unsigned)(eb - 1) < 2046u &&
+           (zero || ((unsigned)(ea - 1) < 2046u && (unsigned)(e - 1) < 2043u));
     const unsigned mah = (ha & 0xfffffu) | 0x100000u, mbh = (hb & 0xfffffu) | 0x100000u;
     u64 A = ((u64)mah << 32) | la;
     const u64 B = ((u64)mbh << 32) | lb;
     const float r = rcp_est(lead(mbh, lb)) * 0.99999952316284f;  // 1 - 2^-21
     float af = lead(mah, la);
-    if (A < B) {
-        A += A;
-        af += af;
-        e -= 1;
-    }
+    const bool small = A < B;
+    A = small ? A + A : A;
+    af = small ? af + af : af;
+    e = small ? e - 1 : e;
     const unsigned q1 = floor23((af * r) * 2097152.0f);
     const u64 R1 = (A << 21) - mul_32x64(q1, B);
     // R / 2^33 times r / 2^52 in units of the next digit: 2^33 2^20 / 2^52
@@ -148,7 +149,44 @@ __device__ __forceinline__ double fdiv64(double a, double b) {
     N += t > B ? 1u : 0u;
     N += t > B + B + B ? 1u : 0u;
     // N in [2^52, 2^53]: its leading bit adds one to the exponent field
-    return from64(N + ((u64)(((unsigned)(e - 1) << 20) | sign) << 32));
+    N += (u64)((unsigned)e << 20) << 32;
+    return from64((zero ? 0ull : N) | ((u64)sign << 32));
+}
+
+// Two and three quotients side by side, out of line: the step kernels take
+// 13 to 25 of them, and with each in place a kernel was 35 kB of code that a
+// small mesh's one warp per SM fetched once per launch (25 us for 2,116
+// triangles' distribute).
+struct Two {
+    double a, b;
+};
+struct Three {
+    double a, b, c;
+};
+static __device__ __noinline__ Two div2(double a0, double b0, double a1, double b1) {
+    bool f0, f1;
+    Two q = {div_digits(a0, b0, f0), div_digits(a1, b1, f1)};
+    if (!(f0 && f1)) {
+        if (!f0) q.a = div_any(a0, b0);
+        if (!f1) q.b = div_any(a1, b1);
+    }
+    return q;
+}
+static __device__ __noinline__ Three div3(double a0, double b0, double a1, double b1, double a2,
+                                          double b2) {
+    bool f0, f1, f2;
+    Three q = {div_digits(a0, b0, f0), div_digits(a1, b1, f1), div_digits(a2, b2, f2)};
+    if (!(f0 && f1 && f2)) {
+        if (!f0) q.a = div_any(a0, b0);
+        if (!f1) q.b = div_any(a1, b1);
+        if (!f2) q.c = div_any(a2, b2);
+    }
+    return q;
+}
+static __device__ __noinline__ double fdiv64(double a, double b) {
+    bool fine;
+    const double q = div_digits(a, b, fine);
+    return fine ? q : div_any(a, b);
 }
 
 // sqrt(x), correctly rounded.
@@ -163,21 +201,17 @@ __device__ __forceinline__ double fdiv64(double a, double b) {
 // N = 2^31 s1 + 2^11 s2 + s3 and R3 = 2^52 X - N^2 decide the rounding (s3,
 // which leaves s2 out of its divisor, may exceed the root by up to 0.03: R3
 // is then below zero, and above -N / 2, and N stands).
-__device__ __forceinline__ double fsqrt64(double x) {
+__device__ __forceinline__ double sqrt_digits(double x, bool &fine) {
     const unsigned hx = hi32(x), lx = (unsigned)__double2loint(x);
-    // normal and positive
-    if (hx - 0x00100000u >= 0x7fe00000u) {
-        if (((hx << 1) | lx) == 0u) return x;
-        return sqrt_any(x);
-    }
+    const bool zero = ((hx << 1) | lx) == 0u;
+    fine = hx - 0x00100000u < 0x7fe00000u || zero;  // normal and positive, or a zero
     const unsigned ex = hx >> 20;
     const unsigned mh = (hx & 0xfffffu) | 0x100000u;
     u64 X = ((u64)mh << 32) | lx;
     float xf = lead(mh, lx);
-    if (!(ex & 1u)) {  // the unbiased exponent is odd
-        X += X;
-        xf += xf;
-    }
+    const bool odd = !(ex & 1u);  // the unbiased exponent
+    X = odd ? X + X : X;
+    xf = odd ? xf + xf : xf;
     const float y = rsqrt_est(xf) * 0.99999952316284f;
     const unsigned s1 = floor23((xf * y) * 2097152.0f);
     const u64 R1 = X - ((u64)s1 * s1 << 10);
@@ -192,7 +226,62 @@ __device__ __forceinline__ double fsqrt64(double x) {
     N += (i64)R3 > (i64)(3 * S + 2) ? 1u : 0u;
     // (ex - 1023) / 2 rounded down, plus the bias, less the leading bit's one
     const unsigned e = ((ex + 1023u) >> 1) - 1u;
-    return from64(N + ((u64)(e << 20) << 32));
+    N += (u64)(e << 20) << 32;
+    return zero ? x : from64(N);
+}
+static __device__ __noinline__ Two sqrt2(double x0, double x1) {
+    bool f0, f1;
+    Two r = {sqrt_digits(x0, f0), sqrt_digits(x1, f1)};
+    if (!(f0 && f1)) {
+        if (!f0) r.a = sqrt_any(x0);
+        if (!f1) r.b = sqrt_any(x1);
+    }
+    return r;
+}
+__device__ __forceinline__ double fsqrt64(double x) {
+    bool fine;
+    const double r = sqrt_digits(x, fine);
+    return fine ? r : sqrt_any(x);
+}
+
+// ---- h^(7/3) ---------------------------------------------------------------
+
+static __device__ __noinline__ double pow73_any(double h) { return pow(h, 7.0 / 3); }
+
+// h to the FP64 number nearest 7/3, within 0.52 ulp (pow: within 1): h^2 and
+// the cube root of h each as a pair, the root from an FP32 estimate c of 24
+// bits by two terms of the binomial series, c (1 + x/3 - x^2/9), x = h/c^3 - 1
+// of 2^-20, h / c^3 a quotient of the integer pipe; the exponent's own
+// rounding, 1.48e-16, by its first-order term.  14 FP64 instructions; pow
+// executes about 80.
+__device__ __forceinline__ double pow_seven_thirds(double h) {
+    const unsigned hh = hi32(h);
+    if (hh - 0x3c300000u >= 0x07900000u) return pow73_any(h);  // outside [2^-60, 2^61)
+    const float hf = __uint_as_float(__funnelshift_l((unsigned)__double2loint(h),
+                                                     hh - (896u << 20), 3));
+    float lg, cf;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(lg) : "f"(hf));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(cf) : "f"(lg * 0.33333333f));
+    const auto widen32 = [](float v) {  // normal v
+        const unsigned u = __float_as_uint(v);
+        return __hiloint2double((int)((((u & 0x7fffffffu) >> 3) + (896u << 20)) |
+                                      (u & 0x80000000u)),
+                                (int)(u << 29));
+    };
+    const double c = widen32(cf);
+    const double c2 = c * c;                   // exact: 48 bits
+    const double r = fma(-c2, c, h);           // h - c^3
+    const double x = fdiv64(r, c2 * c);
+    const double u = x * (1.0 / 3);
+    const double cl = c * fma(-u, u, u);       // the root is c + cl
+    const double p = h * h, pl = fma(h, h, -p);
+    const double q = p * c;
+    double s = fma(p, c, -q);
+    s = fma(p, cl, s);
+    s = fma(pl, c, s);
+    // 1.4802973661668753e-16 ln h = 1.0260639499e-16 log2 h (zero widens to 2^-127)
+    s = fma(q, widen32(lg * 1.0260639e-16f), s);
+    return q + s;
 }
 
 }  // namespace swgpu

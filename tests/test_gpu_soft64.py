@@ -2,7 +2,8 @@
 (csrc/swgpu_soft64.cuh) against IEEE arithmetic, bit for bit: random
 significands and exponents, significands at the ends of their range and next
 to one another, exact quotients and squares, zeros, subnormals, infinities,
-NaN, and quotients at both ends of the range."""
+NaN, and quotients at both ends of the range; and h^(7/3) against numpy's pow
+within the sum of the two's error bounds."""
 import ctypes as C
 import subprocess
 
@@ -15,32 +16,41 @@ HARNESS = r"""
 #include "swgpu_soft64.cuh"
 using namespace swgpu;
 __global__ void apply(const double *a, const double *b, long n, double *q, double *r, double *h,
-                      int *lt) {
+                      double *p, int *lt) {
     const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     q[i] = fdiv64(a[i], b[i]);
+    const Two t = div2(a[i], b[i], b[i], a[i]);
+    const Three u = div3(b[i], a[i], a[i], b[i], a[i], b[i]);
+    if (bits64(t.a) != bits64(q[i]) || bits64(u.b) != bits64(q[i]) ||
+        bits64(u.c) != bits64(q[i]) || bits64(t.b) != bits64(u.a))
+        q[i] = 12345.0;  // the three forms disagree
     r[i] = fsqrt64(a[i]);
+    const Two s = sqrt2(a[i], b[i]);
+    if (bits64(s.a) != bits64(r[i])) r[i] = 12345.0;
     h[i] = half_of(a[i]);
+    p[i] = pow_seven_thirds(fabs(a[i]));
     lt[i] = (lt64(a[i], b[i]) ? 1 : 0) | (mag_lt(a[i], b[i]) ? 2 : 0) |
             (lt_zero(a[i]) ? 4 : 0) | (gt_zero(a[i]) ? 8 : 0) |
             (lt_pos(a[i], 1.0e-3) ? 16 : 0) | (lt64_nan(a[i], b[i]) ? 32 : 0);
 }
 extern "C" int run(const double *a, const double *b, long n, double *q, double *r, double *h,
-                   int *lt) {
-    double *d[5];
+                   double *p, int *lt) {
+    double *d[6];
     int *dl;
-    for (int i = 0; i < 5; i++)
+    for (int i = 0; i < 6; i++)
         if (cudaMalloc(&d[i], n * 8)) return 1;
     if (cudaMalloc(&dl, n * 4)) return 1;
     cudaMemcpy(d[0], a, n * 8, cudaMemcpyHostToDevice);
     cudaMemcpy(d[1], b, n * 8, cudaMemcpyHostToDevice);
-    apply<<<(unsigned)((n + 255) / 256), 256>>>(d[0], d[1], n, d[2], d[3], d[4], dl);
+    apply<<<(unsigned)((n + 255) / 256), 256>>>(d[0], d[1], n, d[2], d[3], d[4], d[5], dl);
     cudaMemcpy(q, d[2], n * 8, cudaMemcpyDeviceToHost);
     cudaMemcpy(r, d[3], n * 8, cudaMemcpyDeviceToHost);
     cudaMemcpy(h, d[4], n * 8, cudaMemcpyDeviceToHost);
+    cudaMemcpy(p, d[5], n * 8, cudaMemcpyDeviceToHost);
     cudaMemcpy(lt, dl, n * 4, cudaMemcpyDeviceToHost);
     const int bad = cudaDeviceSynchronize() != cudaSuccess;
-    for (int i = 0; i < 5; i++) cudaFree(d[i]);
+    for (int i = 0; i < 6; i++) cudaFree(d[i]);
     cudaFree(dl);
     return bad;
 }
@@ -58,7 +68,7 @@ def soft64(tmp_path_factory):
                    ["-I" + B.CSRC, "-shared", str(src), "-o", so], check=True)
     lib = C.CDLL(so)
     p, ip = C.POINTER(C.c_double), C.POINTER(C.c_int)
-    lib.run.argtypes = [p, p, C.c_long, p, p, p, ip]
+    lib.run.argtypes = [p, p, C.c_long, p, p, p, p, ip]
     return lib
 
 
@@ -92,14 +102,19 @@ def test_soft64_is_ieee(kind, soft64):
     a, b = _operands(kind, rng)
     a, b = np.ascontiguousarray(a), np.ascontiguousarray(b)
     n = len(a)
-    q, r, h = np.empty(n), np.empty(n), np.empty(n)
+    q, r, h, p = (np.empty(n) for _ in range(4))
     lt = np.empty(n, np.int32)
     f = lambda x: x.ctypes.data_as(C.POINTER(C.c_double))  # noqa: E731
-    assert soft64.run(f(a), f(b), n, f(q), f(r), f(h), lt.ctypes.data_as(C.POINTER(C.c_int))) == 0
+    assert soft64.run(f(a), f(b), n, f(q), f(r), f(h), f(p),
+                      lt.ctypes.data_as(C.POINTER(C.c_int))) == 0
     with np.errstate(all="ignore"):
         for got, want in ((q, a / b), (r, np.sqrt(a)), (h, 0.5 * a)):
             same = (got.view(np.int64) == want.view(np.int64)) | (np.isnan(got) & np.isnan(want))
             assert same.all(), (a[~same][:3], b[~same][:3], got[~same][:3], want[~same][:3])
+        # h^(7/3) within 0.52 ulp, numpy's pow within one: two units apart at most
+        want = np.abs(a) ** (7.0 / 3)
+        ok = (np.abs(p.view(np.int64) - want.view(np.int64)) <= 2) | (np.isnan(p) & np.isnan(want))
+        assert ok.all(), (a[~ok][:3], p[~ok][:3], want[~ok][:3])
         num = ~(np.isnan(a) | np.isnan(b))
         want = ((a < b) * 1 + (np.abs(a) < np.abs(b)) * 2 + (a < 0) * 4 + (a > 0) * 8
                 + (a < 1.0e-3) * 16 + (a < b) * 32)
