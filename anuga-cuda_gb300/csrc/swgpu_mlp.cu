@@ -10,27 +10,21 @@
 // FP32; its outputs are the normalised maximum depth, the normalised
 // arrival time and the 90% quantile of the first output's absolute error.
 //
-// Every GEMM of the forward and backward passes is the one kernel
-// tc_gemm: a CTA of 4 warps computes a 128 x N tile (N = 256 or 16) of
-// A (M x K) times B (N x K)^T, both operands K-major in global memory.
-// Chunks of 64 along K are staged by cp.async into shared memory in the
-// canonical K-major no-swizzle layout (8-row x 16-byte core matrices, 128
-// bytes apart along K, (K/8)*128 bytes apart along M/N), double-buffered;
-// one thread issues the chunk's tcgen05.mma (kind::f16, M = 128) into an
-// FP32 accumulator in tensor memory and commits it to the stage's
-// mbarrier, which frees the stage for the chunk after next.  The epilogue
-// reads each warp's 32 TMEM lanes (its 32 rows) with tcgen05.ld and either
-//  * adds the bias, applies ReLU and stores BF16 activations (a hidden
-//    layer of the forward pass),
-//  * multiplies by the ReLU mask of the previous activations and stores
-//    BF16 gradients (the backward pass through a layer), or
-//  * adds the FP32 partial weight gradient of its slice of the batch into
-//    the gradient vector (split over the batch, K = rows).
-// Activations and gradients are stored row-major (rows x features) for the
-// next layer's A operand and, in training, also feature-major (features x
-// rows) for the weight gradients, whose K is the batch.  The 256 -> 3
-// output layer and its gradient run on the CUDA cores (head kernels).
-// Training keeps FP32 master weights updated by Adam.
+// Every matrix is kept as core-matrix images (see "blocked images"), so the
+// same bytes serve products over the features, the outputs and the rows; a
+// kernel keeps the weights of its layer in shared memory and walks tiles of
+// 128 rows, each a tcgen05.mma (kind::f16) into FP32 accumulators in tensor
+// memory read back with tcgen05.ld:
+//   mlp_layers12        features, layers 1 and 2 (W1, W2 resident)
+//   mlp_layer3_predict  layer 3 and the 256 -> 3 output layer (W3 resident)
+//   mlp_layer3_train    the same, the loss, the output layer's gradients and
+//                       the gradient back through layer 3
+//   mlp_back2           the gradient back through layer 2 (W2 resident)
+//   mlp_wgrad           the weight and bias gradients, split over the rows
+//   mlp_finish          the splits' sums in a fixed order, Adam on the FP32
+//                       master weights and the BF16 images
+// Inference is the first two, training the other five launches.  No sum
+// depends on the order in which blocks finish.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -64,17 +58,38 @@ constexpr long kOffW4 = kOffB3 + kH;
 constexpr long kOffB4 = kOffW4 + kH * kOut;
 constexpr long kNumParams = kOffB4 + kOut;
 
-// BF16 weight images in the layouts the GEMMs read as their B operand
-// (N x K, K contiguous): forward layers need W^T ([out][in]), the backward
-// pass through a layer needs W itself ([in][out]).
-struct BfWeights {
-    __nv_bfloat16 wt1[kH * kF];   // [out][in]
-    __nv_bfloat16 wt2[kH * kH];
-    __nv_bfloat16 wt3[kH * kH];
-    __nv_bfloat16 w2[kH * kH];    // [in][out]
+// ---- blocked images ---------------------------------------------------------
+//
+// Every matrix that a tensor-core product reads is kept, in global and in
+// shared memory alike, as 16-byte vectors of 8 BF16 in core-matrix order:
+//   activations and their gradients: per tile of 128 rows
+//     [feature / 8][row][8]          (64 kB for 256 features, 4 kB for 16)
+//   weights: [in / 8][out][8 in]     (128 kB for 256 x 256, 8 kB for 16 x 256)
+// Eight rows of one vector are a 128-byte core matrix, so one image serves a
+// product that runs over the features (K-major: a layer forward) and one that
+// runs over the rows (MN-major: a weight gradient) or over the outputs (a
+// layer backward): only the two strides of the descriptor change places.  A
+// tile is one contiguous bulk copy, and a warp that writes one vector per row
+// writes 512 contiguous bytes.
+
+constexpr int kTileM = 128;                      // rows per tile (TMEM lanes)
+constexpr unsigned kActStride = kTileM * 16;     // bytes between 8-feature vectors
+constexpr unsigned kActBytes = kTileM * kH * 2;  // one tile of activations
+constexpr unsigned kXBytes = kTileM * kF * 2;    // one tile of features
+constexpr unsigned kWStride = kH * 16;
+constexpr unsigned kWBytes = kH * kH * 2;
+constexpr unsigned kW1Bytes = kF * kH * 2;
+
+struct __align__(128) BfWeights {
+    __nv_bfloat16 w2[kH * kH];
     __nv_bfloat16 w3[kH * kH];
-    __nv_bfloat16 w4[kH * kOut];  // [in][out] (head, CUDA cores)
+    __nv_bfloat16 w1[kF * kH];
+    float4 w4[kH];  // the three BF16 weights of each hidden unit, widened
 };
+// place of weight (in, out) in its image
+__host__ __device__ __forceinline__ int w_at(int in, int out) {
+    return ((in >> 3) * kH + out) * 8 + (in & 7);
+}
 
 // ---- features --------------------------------------------------------------
 
@@ -86,15 +101,6 @@ struct FeatureTables {
     long long N;
 };
 
-__device__ __forceinline__ float raw_feature(int c, const float *th, const float *tr) {
-    if (c < kParams) return th[c];
-    if (c == 9) return tr[2];   // bed
-    if (c == 10) return tr[0];  // x
-    if (c == 11) return tr[1];  // y
-    if (c == 12) return tr[3];  // distance to the inflow
-    return 0.0f;
-}
-
 __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     z += 0x9E3779B97F4A7C15ull;
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -102,78 +108,76 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     return z ^ (z >> 31);
 }
 
-// Row of batch position r: given (rows), drawn uniformly from all (scenario,
-// triangle) pairs (seeded), or row0 + r (inference).
-__device__ __forceinline__ long long batch_row(const long long *rows, unsigned long long seed,
-                                               long long r, long long total, long long row0) {
-    if (rows) return rows[r];
-    if (total > 0)
-        return (long long)(mix64(seed ^ (unsigned long long)r * 0xD1B54A32D192ED03ull) %
-                           (unsigned long long)total);
-    return row0 + r;
+// The rows of a batch: given, drawn uniformly from all (scenario, triangle)
+// pairs (seeded), or consecutive from row0 (inference).
+struct Batch {
+    const long long *rows;
+    unsigned long long seed;
+    long long total;  // > 0: drawn
+    long long row0;
+    long long nrows;
+};
+__device__ __forceinline__ long long batch_row(const Batch &b, long long r) {
+    if (b.rows) return b.rows[r];
+    if (b.total > 0)
+        return (long long)(mix64(b.seed ^ (unsigned long long)r * 0xD1B54A32D192ED03ull) %
+                           (unsigned long long)b.total);
+    return b.row0 + r;
 }
 
-// Normalised BF16 features of batch rows [0, nrows): row-major xr [Bp][16]
-// and (training) feature-major xc [16][Bp]; rows nrows..Bp-1 are zero.
-// Also records each batch row's data row (training targets).
-__global__ void __launch_bounds__(256) mlp_features(FeatureTables F, const long long *rows,
-                                                    unsigned long long seed, long long total,
-                                                    long long row0, long long nrows, long long Bp,
-                                                    __nv_bfloat16 *__restrict__ xr,
-                                                    __nv_bfloat16 *__restrict__ xc,
-                                                    long long *__restrict__ row_of) {
-    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= Bp) return;
-    float v[kF];
-    if (r < nrows) {
-        const long long q = batch_row(rows, seed, r, total, row0);
-        if (row_of) row_of[r] = q;
+// Normalised BF16 features of batch row r (zero past the last row) into its
+// two vectors of the tile at x; returns the data row.
+__device__ __forceinline__ long long tile_features(const FeatureTables &F, const Batch &b,
+                                                   const float *norm, long long r, int trow,
+                                                   unsigned char *x) {
+    __align__(16) __nv_bfloat162 o[kF / 2];
+    long long q = 0;
+    if (r < b.nrows) {
+        q = batch_row(b, r);
         const long long s = q / F.N, k = q - s * F.N;
-        const float *th = F.scen + s * kParams;
-        const float *tr = F.tri + k * kTri;
+        const float4 tr = __ldg(reinterpret_cast<const float4 *>(F.tri) + k);
+        float v[kF];
 #pragma unroll
-        for (int c = 0; c < kF; c++) v[c] = (raw_feature(c, th, tr) - F.mu[c]) * F.isd[c];
+        for (int c = 0; c < kParams; c++) v[c] = __ldg(F.scen + s * kParams + c);
+        v[9] = tr.z;   // bed
+        v[10] = tr.x;
+        v[11] = tr.y;
+        v[12] = tr.w;  // distance to the inflow
+        v[13] = v[14] = v[15] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < kF; c++) v[c] = (v[c] - norm[c]) * norm[kF + c];
+#pragma unroll
+        for (int c = 0; c < kF / 2; c++) o[c] = __floats2bfloat162_rn(v[2 * c], v[2 * c + 1]);
     } else {
 #pragma unroll
-        for (int c = 0; c < kF; c++) v[c] = 0.0f;
+        for (int c = 0; c < kF / 2; c++) o[c] = __floats2bfloat162_rn(0.0f, 0.0f);
     }
-    __align__(16) __nv_bfloat16 b[kF];
-#pragma unroll
-    for (int c = 0; c < kF; c++) b[c] = __float2bfloat16(v[c]);
-    int4 *dst = reinterpret_cast<int4 *>(xr + r * kF);
-    dst[0] = reinterpret_cast<const int4 *>(b)[0];
-    dst[1] = reinterpret_cast<const int4 *>(b)[1];
-    if (xc) {
-#pragma unroll
-        for (int c = 0; c < kF; c++) xc[c * Bp + r] = b[c];
-    }
+    *reinterpret_cast<uint4 *>(x + trow * 16) = reinterpret_cast<const uint4 *>(o)[0];
+    *reinterpret_cast<uint4 *>(x + kActStride + trow * 16) = reinterpret_cast<const uint4 *>(o)[1];
+    return q;
 }
 
-// ---- tcgen05 GEMM ----------------------------------------------------------
-
-constexpr int kTileM = 128;  // rows per CTA (TMEM lanes)
-constexpr int kChunkK = 64;  // K per stage
-constexpr int kGemmThreads = 256;  // 8 warps: the epilogue splits the columns in two
+// ---- tcgen05, mbarriers, bulk copies ---------------------------------------
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
     return (unsigned)__cvta_generic_to_shared(p);
 }
 
-// Shared-memory matrix descriptor: start, leading-dimension byte offset
-// (between core matrices along K), stride byte offset (between 8-row groups
-// along M/N), descriptor version 1 (bit 46), no swizzle.
-__device__ __forceinline__ unsigned long long smem_desc(unsigned addr, unsigned lbo,
-                                                        unsigned sbo) {
+// Shared-memory matrix descriptor: start, the byte offsets between core
+// matrices along K (leading) and along M or N (stride), descriptor version 1
+// (bit 46), no swizzle.
+__device__ __forceinline__ unsigned long long smem_desc(unsigned addr, unsigned along_k,
+                                                        unsigned along_mn) {
     return (unsigned long long)((addr >> 4) & 0x3FFFu) |
-           ((unsigned long long)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((unsigned long long)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+           ((unsigned long long)((along_k >> 4) & 0x3FFFu) << 16) |
+           ((unsigned long long)((along_mn >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// kind::f16 instruction descriptor: FP32 accumulator, BF16 A and B, both
-// K-major, M = 128, N given.
-__host__ __device__ constexpr unsigned tc_idesc(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) |
-           ((unsigned)(kTileM >> 4) << 24);
+// kind::f16 instruction descriptor: FP32 accumulator, BF16 A and B (each
+// K-major or MN-major), M = 128, N given.
+__host__ __device__ constexpr unsigned tc_idesc(int n, bool a_mn, bool b_mn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)a_mn << 15) | ((unsigned)b_mn << 16) |
+           ((unsigned)(n >> 3) << 17) | ((unsigned)(kTileM >> 4) << 24);
 }
 
 __device__ __forceinline__ void tc_mma(unsigned d_tmem, unsigned long long a,
@@ -199,6 +203,14 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void proxy_fence() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+// A CTA's barrier after which the tensor core may read what its threads
+// wrote to shared memory and overwrite what they read from tensor memory.
+__device__ __forceinline__ void tc_sync() {
+    proxy_fence();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+}
 // 32 consecutive FP32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tc_ld32(unsigned taddr, float (&v)[32]) {
     unsigned r[32];
@@ -216,6 +228,24 @@ __device__ __forceinline__ void tc_ld32(unsigned taddr, float (&v)[32]) {
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
+// 8 consecutive FP32 columns at each of two places of this thread's lane
+__device__ __forceinline__ void tc_ld8x2(unsigned a, unsigned b, float (&v)[8], float (&w)[8]) {
+    unsigned r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                   "=r"(r[6]), "=r"(r[7])
+                 : "r"(a));
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+                   "=r"(r[14]), "=r"(r[15])
+                 : "r"(b));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        v[i] = __uint_as_float(r[i]);
+        w[i] = __uint_as_float(r[8 + i]);
+    }
+}
 // 16 consecutive FP32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tc_ld16(unsigned taddr, float (&v)[16]) {
     unsigned r[16];
@@ -230,10 +260,30 @@ __device__ __forceinline__ void tc_ld16(unsigned taddr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
+__device__ __forceinline__ void tmem_alloc(unsigned *base, unsigned columns) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(base)),
+                 "r"(columns)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free(unsigned base, unsigned columns) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns)
+                 : "memory");
+}
 
-__device__ __forceinline__ void mbar_init(unsigned long long *bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
+                 : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned long long *bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ bool mbar_test(unsigned long long *bar, unsigned parity) {
     unsigned ok;
@@ -246,484 +296,1073 @@ __device__ __forceinline__ bool mbar_test(unsigned long long *bar, unsigned pari
     return ok != 0;
 }
 constexpr int kTcWaitLimit = 1 << 22;
-// Bounded wait of the whole CTA for an MMA commit: every thread polls at
-// most kTcWaitLimit times; true when all saw the phase complete.
-__device__ __forceinline__ bool cta_wait(unsigned long long *bar, unsigned parity) {
-    bool ok = false;
-    for (int i = 0; i < kTcWaitLimit && !ok; i++) ok = mbar_test(bar, parity);
-    return __syncthreads_and(ok) != 0;
+// Bounded wait; on running out the status is set, what is in flight gets as
+// long again to land before its memory is given up, and false is returned.
+__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity, int *status) {
+    for (int i = 0; i < kTcWaitLimit; i++)
+        if (mbar_test(bar, parity)) return true;
+    atomicExch(status, SWGPU_ETIMEOUT);
+    for (int i = 0; i < kTcWaitLimit; i++)
+        if (mbar_test(bar, parity)) break;
+    return false;
 }
-
-// 16-byte asynchronous copy global -> shared; src_bytes 0 fills zeros.
-__device__ __forceinline__ void cp_async16(unsigned dst, const void *src, unsigned src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
-                 "r"(src_bytes)
+// The same by the whole CTA, which it also brings together: true when all
+// saw the phase complete.
+__device__ __forceinline__ bool cta_wait(unsigned long long *bar, unsigned parity, int *status) {
+    return __syncthreads_and(mbar_wait(bar, parity, status)) != 0;
+}
+// bulk copies (addresses and size multiples of 16)
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes,
+                                          unsigned long long *bar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+            "r"(smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ void bulk_store(void *dst, const void *src, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                 "r"(smem_u32(src)), "r"(bytes)
                  : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
-__device__ __forceinline__ void cp_async_commit() {
-    asm volatile("cp.async.commit_group;" ::: "memory");
+__device__ __forceinline__ void bulk_store_read() {  // the sources may be overwritten
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+__device__ __forceinline__ void bulk_store_done() {
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_launch_dependents() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// D (128 x 256) = A (a tile of activations) x W: over the features, or
+// backward over the outputs.
+__device__ __forceinline__ void mma_layer(unsigned d, unsigned a, unsigned w, bool accumulate) {
+    // 128 of the 256 features: a half that one bulk copy brings
+#pragma unroll
+    for (int kk = 0; kk < 8; kk++)
+        tc_mma(d, smem_desc(a + 2 * kActStride * kk, kActStride, 128),
+               smem_desc(w + 2 * kWStride * kk, kWStride, 128), tc_idesc(kH, false, false),
+               accumulate || kk > 0);
+}
+__device__ __forceinline__ void mma_layer_back(unsigned d, unsigned a, unsigned w) {
+#pragma unroll
+    for (int kk = 0; kk < 16; kk++)
+        tc_mma(d, smem_desc(a + 2 * kActStride * kk, kActStride, 128),
+               smem_desc(w + 256 * kk, 128, kWStride), tc_idesc(kH, false, true), kk > 0);
 }
 
-// Stages rows [r0, r0 + R) x k-range [k0, k0 + kc) of a K-major matrix
-// (row stride ld elements, nvalid valid rows) into the canonical layout at
-// smem address dst.  Vector v (8 elements) goes to byte 16 v: the 8 lanes
-// of a group take 8 consecutive rows at one k (a 128-byte core matrix),
-// consecutive groups the next k, so a warp stores 512 contiguous bytes and
-// reads 64 contiguous bytes of each of 8 rows.
-__device__ __forceinline__ void stage_operand(unsigned dst, const __nv_bfloat16 *src, long ld,
-                                              long long r0, long long nvalid, int R, long k0,
-                                              int kc) {
-    const int lg = kc == kChunkK ? 3 : 1;  // log2 of the 16-byte vectors per row (kc 64 or 16)
-    const int nvec = R << lg;
-    for (int v = threadIdx.x; v < nvec; v += kGemmThreads) {
-        const int r = (v & 7) + ((v >> (3 + lg)) << 3);
-        const int kv = (v >> 3) & ((1 << lg) - 1);
-        const long long row = r0 + r;
-        const bool in = row < nvalid;
-        const __nv_bfloat16 *p = in ? src + row * ld + k0 + 8 * kv : src;
-        cp_async16(dst + 16u * (unsigned)v, p, in ? 16u : 0u);
+// A thread's part of an epilogue: the tile row of its TMEM lane and half of
+// the columns.  Warp w reaches lanes 32 (w % 4) .. + 31 only.
+struct Part {
+    int row, col0;
+    unsigned tmem;  // its lane's first column
+};
+__device__ __forceinline__ Part my_part(unsigned tmem) {
+    const int warp = threadIdx.x >> 5;
+    Part p;
+    p.row = 32 * (warp & 3) + (threadIdx.x & 31);
+    p.col0 = 128 * (warp >> 2);
+    p.tmem = tmem + ((unsigned)(32 * (warp & 3)) << 16);
+    return p;
+}
+__device__ __forceinline__ uint4 pack8(const float *v) {
+    __align__(16) __nv_bfloat162 o[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) o[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+    return *reinterpret_cast<const uint4 *>(o);
+}
+// bias and ReLU of n columns from c0, in place
+template <int n>
+__device__ __forceinline__ void bias_relu(float (&v)[n], const float *bias, int c0) {
+#pragma unroll
+    for (int q = 0; q < n / 4; q++) {
+        const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + 4 * q);
+        v[4 * q] = fmaxf(v[4 * q] + b.x, 0.0f);
+        v[4 * q + 1] = fmaxf(v[4 * q + 1] + b.y, 0.0f);
+        v[4 * q + 2] = fmaxf(v[4 * q + 2] + b.z, 0.0f);
+        v[4 * q + 3] = fmaxf(v[4 * q + 3] + b.w, 0.0f);
+    }
+}
+// A hidden layer's epilogue: activations of the accumulator at column d into
+// the tile images at smem and / or global.
+template <bool SMEM, bool GLOBAL>
+__device__ __forceinline__ void hidden_epilogue(const Part &p, unsigned d, const float *bias,
+                                                unsigned char *smem, unsigned char *global) {
+#pragma unroll 1
+    for (int c0 = p.col0; c0 < p.col0 + 128; c0 += 32) {
+        float v[32];
+        tc_ld32(p.tmem + d + c0, v);
+        bias_relu(v, bias, c0);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint4 o = pack8(v + 8 * q);
+            const size_t at = (size_t)(c0 / 8 + q) * kActStride + p.row * 16;
+            if (SMEM) *reinterpret_cast<uint4 *>(smem + at) = o;
+            if (GLOBAL) *reinterpret_cast<uint4 *>(global + at) = o;
+        }
+    }
+}
+// Bits of the eight BF16 of a vector that are above zero (a ReLU's output).
+__device__ __forceinline__ unsigned positive8(const uint4 &u) {
+    const unsigned w[4] = {u.x, u.y, u.z, u.w};
+    unsigned m = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        m |= ((short)(w[j] & 0xffffu) > 0 ? 1u : 0u) << (2 * j);
+        m |= ((int)w[j] >> 16 > 0 ? 1u : 0u) << (2 * j + 1);
+    }
+    return m;
+}
+__device__ __forceinline__ void unpack8(const uint4 &u, float (&v)[8]) {
+    const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        v[2 * j] = __uint_as_float(w[j] << 16);
+        v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
     }
 }
 
-enum { kEpiHidden = 0, kEpiDgrad = 1, kEpiWgrad = 2, kEpiWgradT = 3 };
+// ---- layers 1 and 2 -----------------------------------------------------------
 
-struct GemmArgs {
-    const __nv_bfloat16 *A;  // M x K, K contiguous, row stride lda
-    long lda;
-    const __nv_bfloat16 *B;  // N x K, K contiguous, row stride ldb
-    long ldb;
-    long long M;             // valid rows of A (and of the output)
-    long K;                  // K of the whole product (a multiple of 16)
-    long k_per_split;        // K range of one blockIdx.y (a multiple of 64, or K)
-    // epilogue
-    const float *bias;               // hidden: [N]
-    const __nv_bfloat16 *mask;       // dgrad: previous activations [M][N] row-major
-    __nv_bfloat16 *out_row;          // hidden/dgrad: [M][N]
-    __nv_bfloat16 *out_col;          // hidden/dgrad: [N][ldc] (may be null)
-    long ldc;
-    float *grad;                     // wgrad: partials [splits][M][N] (or [splits][N][M]
-                                     // transposed), one slice per blockIdx.y
+constexpr int kThreads = 256;  // 8 warps: the epilogues split the columns in two
+
+struct Layers12 {
+    FeatureTables F;
+    Batch batch;
+    const BfWeights *W;
+    const float *b1, *b2;
+    unsigned char *h1, *h2;    // tile images (h1, x: training only)
+    unsigned char *x;
+    long long *row_of;         // training: data row of each batch row
+    int tiles;
     int *status;
 };
-
-template <int N>
-struct __align__(1024) GemmSmem {
-    __nv_bfloat16 a[2][kTileM * kChunkK];
-    __nv_bfloat16 b[2][N * kChunkK];
-    unsigned long long bar[2];
-    unsigned tmem_base;
+struct __align__(1024) Smem12 {
+    unsigned char w2[kWBytes];
+    unsigned char h[kActBytes];
+    unsigned char w1[kW1Bytes];
+    unsigned char x[kXBytes];
+    float b1[kH], b2[kH], norm[2 * kF];
+    unsigned long long wbar, mbar;
+    unsigned tmem;
 };
 
-template <int N>
-__host__ __device__ constexpr int tmem_cols() {
-    return N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256));
-}
-
-// The epilogue of one 32-column slice c0 .. c0+31 (or 16 for N = 16) of
-// this thread's row.
-// Row stride (elements) of the BF16 output tile staged in shared memory:
-// 129 words, so that a warp writing one row per lane, or reading 32
-// consecutive words of one row, touches 32 different banks.
-template <int N>
-constexpr int kStageStride = N + 2;
-
-// The epilogue of one 32-column slice c0 .. c0+31 (or 16 for N = 16) of
-// this thread's row (trow within the tile).  Weight gradients go straight to
-// their partial; activations and gradients of activations are written as
-// BF16 pairs into the shared-memory tile, stored to global memory by
-// gemm_store_tile.
-template <int N, int EPI, int W>
-__device__ __forceinline__ void gemm_epilogue(const GemmArgs &g, long long row, int trow, int c0,
-                                              const float (&v)[W], __nv_bfloat16 *stile) {
-    if (row >= g.M) return;
-    if (EPI == kEpiWgrad) {
-        float4 *dst = reinterpret_cast<float4 *>(g.grad + (long long)blockIdx.y * g.M * N +
-                                                 row * N + c0);
-#pragma unroll
-        for (int q = 0; q < W / 4; q++)
-            dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        return;
-    }
-    if (EPI == kEpiWgradT) {
-        float *dst = g.grad + (long long)blockIdx.y * g.M * N;
-#pragma unroll
-        for (int j = 0; j < W; j++) dst[(long long)(c0 + j) * g.M + row] = v[j];
-        return;
-    }
-    __align__(16) __nv_bfloat16 o[W];
-    if (EPI == kEpiHidden) {
-        const float4 *bp = reinterpret_cast<const float4 *>(g.bias + c0);
-#pragma unroll
-        for (int q = 0; q < W / 4; q++) {
-            const float4 b = __ldg(bp + q);
-            o[4 * q] = __float2bfloat16(fmaxf(v[4 * q] + b.x, 0.0f));
-            o[4 * q + 1] = __float2bfloat16(fmaxf(v[4 * q + 1] + b.y, 0.0f));
-            o[4 * q + 2] = __float2bfloat16(fmaxf(v[4 * q + 2] + b.z, 0.0f));
-            o[4 * q + 3] = __float2bfloat16(fmaxf(v[4 * q + 3] + b.w, 0.0f));
-        }
-    } else {  // dgrad: the ReLU mask of the activations this layer read
-        __align__(16) __nv_bfloat16 pm[W];
-        const int4 *src = reinterpret_cast<const int4 *>(g.mask + row * N + c0);
-#pragma unroll
-        for (int q = 0; q < W / 8; q++) reinterpret_cast<int4 *>(pm)[q] = src[q];
-#pragma unroll
-        for (int j = 0; j < W; j++)
-            o[j] = __float2bfloat16(__bfloat162float(pm[j]) > 0.0f ? v[j] : 0.0f);
-    }
-    unsigned *t32 = reinterpret_cast<unsigned *>(stile + trow * kStageStride<N> + c0);
-#pragma unroll
-    for (int j = 0; j < W / 2; j++) t32[j] = reinterpret_cast<const unsigned *>(o)[j];
-}
-
-// Stores the staged 128 x N BF16 tile: row-major (each warp writes whole
-// rows, 32 consecutive words per instruction) and, when asked,
-// feature-major (each warp writes one feature's 128 rows as 4-byte pairs,
-// 128 bytes per instruction).
-template <int N>
-__device__ __forceinline__ void gemm_store_tile(const GemmArgs &g, long long m0,
-                                                const __nv_bfloat16 *stile) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int TW = kStageStride<N> / 2;  // words per staged row
-    const unsigned *t32 = reinterpret_cast<const unsigned *>(stile);
-    for (int r = warp; r < kTileM; r += kGemmThreads / 32) {
-        const long long grow = m0 + r;
-        if (grow >= g.M) break;
-        unsigned *dst = reinterpret_cast<unsigned *>(g.out_row + grow * N);
-#pragma unroll
-        for (int j = lane; j < N / 2; j += 32) dst[j] = t32[r * TW + j];
-    }
-    if (!g.out_col) return;
-    for (int c = warp; c < N; c += kGemmThreads / 32) {
-#pragma unroll
-        for (int p = 0; p < kTileM / 64; p++) {
-            const int r = 64 * p + 2 * lane;
-            const long long grow = m0 + r;
-            __nv_bfloat16 *dst = g.out_col + (long long)c * g.ldc + grow;
-            const __nv_bfloat16 a = stile[r * kStageStride<N> + c];
-            const __nv_bfloat16 b = stile[(r + 1) * kStageStride<N> + c];
-            if (grow + 1 < g.M) {
-                __nv_bfloat162 pair;
-                pair.x = a;
-                pair.y = b;
-                *reinterpret_cast<__nv_bfloat162 *>(dst) = pair;
-            } else if (grow < g.M) {
-                *dst = a;
-            }
-        }
-    }
-}
-
-// C (128 x N tile) = A (tile rows) x B^T over this CTA's K range, then the
-// epilogue.  blockIdx.x: row tile; blockIdx.y: K split (weight gradients).
-template <int N, int EPI>
-__global__ void __launch_bounds__(kGemmThreads, 2) tc_gemm(GemmArgs g) {
+// Features, layer 1 and layer 2 of the tiles blockIdx.x, + gridDim.x, ...;
+// one CTA per SM with both weight matrices resident.  The two accumulators
+// take turns: a tile's layer 1 and layer 2 use one, while the other holds the
+// previous tile's layer 2 until its epilogue, which runs under this tile's
+// layer 2 product, has read it.
+template <bool TRAIN>
+__global__ void __launch_bounds__(kThreads, 1) mlp_layers12(Layers12 g) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    GemmSmem<N> &S = *reinterpret_cast<GemmSmem<N> *>(
-        smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const long long m0 = (long long)blockIdx.x * kTileM;
-    const long kb = (long)blockIdx.y * g.k_per_split;
-    const long ke = g.K < kb + g.k_per_split ? g.K : kb + g.k_per_split;
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_u32(&S.tmem_base)),
-                     "n"(tmem_cols<N>())
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    Smem12 &S = *reinterpret_cast<Smem12 *>(smem_raw +
+                                            ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
+    const int tid = threadIdx.x;
+    pdl_launch_dependents();
+    if (tid < 32) tmem_alloc(&S.tmem, 512);
     if (tid == 0) {
-        mbar_init(&S.bar[0]);
-        mbar_init(&S.bar[1]);
+        mbar_init(&S.wbar, 1);
+        mbar_init(&S.mbar, 1);
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const unsigned tmem = S.tmem_base;
-    const int kc = g.K < kChunkK ? (int)g.K : kChunkK;  // 64, or 16 for K = 16
-    // every K range is non-empty: the host launches ceil(K / k_per_split)
-    // splits
-    const int nk = (int)((ke - kb + kc - 1) / kc);
-    constexpr unsigned idesc = tc_idesc(N);
-    auto issue = [&](int c) {
-        const int s = c & 1;
-        const long k0 = kb + (long)c * kc;
-        stage_operand(smem_u32(S.a[s]), g.A, g.lda, m0, g.M, kTileM, k0, kc);
-        stage_operand(smem_u32(S.b[s]), g.B, g.ldb, 0, N, N, k0, kc);
-        cp_async_commit();
+    pdl_wait();
+    if (tid < kF) {
+        S.norm[tid] = g.F.mu[tid];
+        S.norm[kF + tid] = g.F.isd[tid];
+    }
+    S.b1[tid] = g.b1[tid];
+    S.b2[tid] = g.b2[tid];
+    tc_sync();
+    const unsigned tmem = S.tmem;
+    if (tid == 0) {
+        mbar_expect(&S.wbar, kWBytes + kW1Bytes);
+        bulk_load(S.w1, g.W->w1, kW1Bytes, &S.wbar);
+        bulk_load(S.w2, g.W->w2, kWBytes, &S.wbar);
+    }
+    const Part p = my_part(tmem);
+    const auto features = [&](int t) {
+        if (tid < kTileM) {
+            const long long r = (long long)t * kTileM + tid;
+            const long long q = tile_features(g.F, g.batch, S.norm, r, tid, S.x);
+            if (TRAIN) g.row_of[r] = q;
+        }
     };
-    bool ok = true;
-    int last = -1;  // the last chunk whose MMAs were committed
-    if (nk > 0) issue(0);
-    for (int c = 0; c < nk && ok; c++) {
-        if (c + 1 < nk) {
-            // stage (c+1)&1 was read by the MMAs of chunk c-1
-            if (c >= 1) ok = cta_wait(&S.bar[(c - 1) & 1], ((c - 1) >> 1) & 1);
-            if (!ok) break;
-            issue(c + 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        proxy_fence();  // the copies into shared memory, before the tensor core reads
-        tc_fence_before();
-        __syncthreads();
+    const auto layer1 = [&](unsigned d) {
+        tc_mma(tmem + d, smem_desc(smem_u32(S.x), kActStride, 128),
+               smem_desc(smem_u32(S.w1), kWStride, 128), tc_idesc(kH, false, false), false);
+        tc_commit(&S.mbar);
+    };
+    int t = blockIdx.x, last = -1;
+    unsigned phase = 0, buf = 0;
+    features(t);
+    bool ok = cta_wait(&S.wbar, 0, g.status);
+    tc_sync();
+    if (ok && tid == 0) layer1(0);
+    while (ok && t < g.tiles) {
+        const unsigned d = buf * kH;
+        ok = cta_wait(&S.mbar, phase, g.status);  // layer 1 of t, layer 2 of the last tile
+        phase ^= 1;
+        if (!ok) break;
         tc_fence_after();
+        if (TRAIN) {
+            // (x's image leaves before the next tile's features replace it)
+            if (tid < 2 * kTileM)
+                reinterpret_cast<uint4 *>(g.x + (size_t)t * kXBytes)[tid] =
+                    reinterpret_cast<const uint4 *>(S.x)[tid];
+        }
+        hidden_epilogue<true, TRAIN>(p, d, S.b1, S.h, TRAIN ? g.h1 + (size_t)t * kActBytes : nullptr);
+        tc_sync();
         if (tid == 0) {
-            const int s = c & 1;
-            const unsigned sbo = (unsigned)(kc / 8) * 128u;
-            const unsigned a0 = smem_u32(S.a[s]), b0 = smem_u32(S.b[s]);
-            for (int kk = 0; kk < kc / 16; kk++)
-                tc_mma(tmem, smem_desc(a0 + 256u * kk, 128, sbo),
-                       smem_desc(b0 + 256u * kk, 128, sbo), idesc, c > 0 || kk > 0);
-            tc_commit(&S.bar[s]);
+            mma_layer(tmem + d, smem_u32(S.h), smem_u32(S.w2), false);
+            mma_layer(tmem + d, smem_u32(S.h) + 16 * kActStride, smem_u32(S.w2) + 16 * kWStride,
+                      true);
         }
-        last = c;
+        const int next = t + gridDim.x;
+        if (next < g.tiles) features(next);
+        if (last >= 0)
+            hidden_epilogue<false, true>(p, (buf ^ 1) * kH, S.b2, nullptr,
+                                         g.h2 + (size_t)last * kActBytes);
+        if (next < g.tiles) {
+            tc_sync();
+            if (tid == 0) layer1((buf ^ 1) * kH);
+        } else if (tid == 0) {
+            tc_commit(&S.mbar);
+        }
+        last = t;
+        t = next;
+        buf ^= 1;
     }
-    if (ok && last >= 0) ok = cta_wait(&S.bar[last & 1], (last >> 1) & 1);
-    if (!ok) {
-        // status first; then let copies land (cp.async completes on its own)
-        // and give the MMAs in flight (up to the last committed chunk's) one
-        // more bounded wait before the columns are freed
-        if (tid == 0) atomicExch(g.status, SWGPU_ETIMEOUT);
-        cp_async_wait<0>();
-        if (last >= 0) cta_wait(&S.bar[last & 1], (last >> 1) & 1);
-    } else {
-        // warp w reads TMEM lanes 32 (w % 4) .. +31 (its rows; a warp may only
-        // reach its own quarter of the lanes) and half w / 4 of the columns
+    if (ok) ok = cta_wait(&S.mbar, phase, g.status);
+    if (ok) {
         tc_fence_after();
-        const int quarter = warp & 3, half = warp >> 2;
-        const int trow = 32 * quarter + lane;
-        const long long row = m0 + trow;
-        const unsigned lane_addr = tmem + ((unsigned)(32 * quarter) << 16);
-        // the operand stages are free (every MMA has completed): the output
-        // tile is staged there
-        __nv_bfloat16 *stile = &S.a[0][0];
-        static_assert(EPI == kEpiWgrad || EPI == kEpiWgradT ||
-                          kTileM * kStageStride<N> * 2 <= sizeof(S.a) + sizeof(S.b),
-                      "staged tile fits in the operand stages");
-        if (N >= 64) {
-#pragma unroll 1
-            for (int c0 = half * (N / 2); c0 < (half + 1) * (N / 2); c0 += 32) {
-                float v[32];
-                tc_ld32(lane_addr + c0, v);
-                gemm_epilogue<N, EPI, 32>(g, row, trow, c0, v, stile);
+        hidden_epilogue<false, true>(p, (buf ^ 1) * kH, S.b2, nullptr,
+                                     g.h2 + (size_t)last * kActBytes);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (tid < 32) tmem_free(tmem, 512);
+}
+
+// ---- layer 3 and the output layer --------------------------------------------
+
+struct Layer3 {
+    const BfWeights *W;
+    const float *b3, *b4;
+    const unsigned char *h2;
+    int tiles;
+    long long nrows;
+    float *y;                  // [nrows][3]
+    int *status;
+    // training
+    const float *targets;
+    const long long *row_of;
+    unsigned char *d3, *d2;    // gradients of the layers' sums, tile images
+    float *part4;              // per CTA: W4's gradient [256][3], b4's [3], the loss
+    float w_d, w_a, w_e;
+};
+constexpr int kPart4 = kH * kOut + kOut + 1;
+
+// One row's outputs over half of layer 3's features: the odd or even vectors
+// of eight (odd: the row's other thread has the rest), activations from the
+// accumulator at lane address tmem, kept as BF16 in the tile image at `image`
+// when given.  The sum's order: along the eight features of a vector, then
+// pairwise over vectors 16, 8, 4 and 2 apart (and 1 apart, odd and even, by
+// the caller).
+template <bool KEEP>
+__device__ __forceinline__ void head_half(unsigned tmem, int odd, const float *b3,
+                                          const float4 *w4, unsigned char *image,
+                                          float (&out)[kOut]) {
+    constexpr int order[8] = {0, 4, 2, 6, 1, 5, 3, 7};  // vectors 2 order + odd, and 16 more
+    float pair[kOut], quad[kOut], sum[kOut];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        float v[2][8], s[2][kOut];
+        const int c0 = 16 * order[i] + 8 * odd;
+        tc_ld8x2(tmem + c0, tmem + c0 + 128, v[0], v[1]);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int c = c0 + 128 * q;
+            bias_relu<8>(v[q], b3, c);
+            const uint4 u = pack8(v[q]);
+            if (KEEP) *reinterpret_cast<uint4 *>(image + (c >> 3) * kActStride) = u;
+            float h[8];
+            unpack8(u, h);
+#pragma unroll
+            for (int o = 0; o < kOut; o++) s[q][o] = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float4 w = w4[c + j];
+                s[q][0] = fmaf(h[j], w.x, s[q][0]);
+                s[q][1] = fmaf(h[j], w.y, s[q][1]);
+                s[q][2] = fmaf(h[j], w.z, s[q][2]);
             }
-        } else if (half == 0) {
-            float v[16];
-            tc_ld16(lane_addr, v);
-            gemm_epilogue<N, EPI, 16>(g, row, trow, 0, v, stile);
         }
-        if constexpr (EPI == kEpiHidden || EPI == kEpiDgrad) {
-            __syncthreads();
-            gemm_store_tile<N>(g, m0, stile);
+#pragma unroll
+        for (int o = 0; o < kOut; o++) {
+            const float a = s[0][o] + s[1][o];
+            if (i % 2 == 0) {
+                pair[o] = a;
+            } else {
+                const float b = pair[o] + a;
+                if (i % 4 == 1)
+                    quad[o] = b;
+                else if (i == 3)
+                    sum[o] = quad[o] + b;
+                else
+                    out[o] = sum[o] + (quad[o] + b);
+            }
+        }
+    }
+}
+
+constexpr int kThreads3 = kThreads + 32;  // inference: one more warp feeds the tensor core
+
+struct __align__(1024) Smem3 {
+    unsigned char w3[kWBytes];
+    unsigned char a[kActBytes];
+    float4 w4[kH];
+    float b3[kH];
+    float4 half[2][kTileM];  // a row's outputs over the odd vectors of features
+    unsigned long long wbar, full[2], free_[2], ready[2], drained[2];
+    unsigned tmem;
+};
+
+// Inference: outputs of the tiles blockIdx.x, + gridDim.x, ...  One warp
+// loads a tile's two halves and issues their products, each half's buffer
+// refilled as soon as its product is done; eight warps turn the accumulator
+// that is ready into outputs meanwhile.
+__global__ void __launch_bounds__(kThreads3, 1) mlp_layer3_predict(Layer3 g) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    Smem3 &S = *reinterpret_cast<Smem3 *>(smem_raw +
+                                          ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
+    const int tid = threadIdx.x;
+    pdl_launch_dependents();
+    if (tid < 32) tmem_alloc(&S.tmem, 512);
+    if (tid == 0) {
+        mbar_init(&S.wbar, 1);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&S.full[i], 1);
+            mbar_init(&S.free_[i], 1);
+            mbar_init(&S.ready[i], 1);
+            mbar_init(&S.drained[i], 8);
+        }
+    }
+    pdl_wait();
+    if (tid < kH) {
+        S.w4[tid] = g.W->w4[tid];
+        S.b3[tid] = g.b3[tid];
+    }
+    tc_sync();
+    const unsigned tmem = S.tmem;
+    const int stride = gridDim.x;
+    constexpr unsigned kHalf = kActBytes / 2;
+    if (tid >= kThreads) {
+        if (tid == kThreads) {
+            mbar_expect(&S.wbar, kWBytes);
+            bulk_load(S.w3, g.W->w3, kWBytes, &S.wbar);
+            const auto load = [&](int t, int i) {
+                mbar_expect(&S.full[i], kHalf);
+                bulk_load(S.a + i * kHalf, g.h2 + (size_t)t * kActBytes + i * kHalf, kHalf,
+                          &S.full[i]);
+            };
+            int t = blockIdx.x;
+            load(t, 0);
+            load(t, 1);
+            bool ok = mbar_wait(&S.wbar, 0, g.status);
+            for (int n = 0; ok && t < g.tiles; n++, t += stride) {
+                const unsigned buf = n & 1, ph = n & 1;
+                // the accumulator's last reader (tile n - 2) is done
+                if (n >= 2) ok = mbar_wait(&S.drained[buf], ((n >> 1) - 1) & 1, g.status);
+                tc_fence_after();
+                for (int i = 0; ok && i < 2; i++) {
+                    ok = mbar_wait(&S.full[i], ph, g.status);
+                    if (!ok) break;
+                    mma_layer(tmem + buf * kH, smem_u32(S.a) + i * kHalf,
+                              smem_u32(S.w3) + i * 16 * kWStride, i > 0);
+                    tc_commit(&S.free_[i]);
+                    if (i == 1) tc_commit(&S.ready[buf]);
+                    // the first half's buffer is refilled under the second's product
+                    if (i == 1 && t + stride < g.tiles) {
+                        ok = mbar_wait(&S.free_[0], ph, g.status);
+                        if (ok) load(t + stride, 0);
+                        if (ok) ok = mbar_wait(&S.free_[1], ph, g.status);
+                        if (ok) load(t + stride, 1);
+                    }
+                }
+            }
+        }
+    } else {
+        const Part p = my_part(tmem);
+        const int odd = p.col0 ? 1 : 0;
+        bool ok = true;
+        int n = 0;
+        for (int t = blockIdx.x; t < g.tiles; t += stride, n++) {
+            const unsigned buf = n & 1;
+            // (after a wait that ran out, the tiles left are passed without one)
+            if (ok) ok = mbar_wait(&S.ready[buf], (n >> 1) & 1, g.status);
+            ok = __all_sync(0xffffffffu, ok);
+            float acc[kOut] = {0.f, 0.f, 0.f};
+            if (ok) {
+                tc_fence_after();
+                head_half<false>(p.tmem + buf * kH, odd, S.b3, S.w4, nullptr, acc);
+                tc_fence_before();
+            }
+            __syncwarp();
+            if ((tid & 31) == 0) mbar_arrive(&S.drained[buf]);
+            if (odd) S.half[buf][p.row] = make_float4(acc[0], acc[1], acc[2], 0.f);
+            // the eight warps of the epilogue
+            asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+            const long long r = (long long)t * kTileM + p.row;
+            if (!odd && ok && r < g.nrows) {
+                const float4 o = S.half[buf][p.row];
+                g.y[r * kOut] = acc[0] + o.x + g.b4[0];
+                g.y[r * kOut + 1] = acc[1] + o.y + g.b4[1];
+                g.y[r * kOut + 2] = acc[2] + o.z + g.b4[2];
+            }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                     "n"(tmem_cols<N>())
-                     : "memory");
+    if (tid < 32) tmem_free(tmem, 512);
 }
 
-// ---- output layer (CUDA cores) --------------------------------------------
+struct __align__(1024) Smem3T {
+    unsigned char w3[kWBytes];
+    unsigned char a[kActBytes];        // h2, then h3, then its gradient
+    float4 w4[kH];
+    float b3[kH];
+    float4 half[2][kTileM];  // a row's outputs over the even and the odd vectors
+    float4 dy[kTileM];
+    float sum4[8][kOut + 1];
+    unsigned long long wbar, abar, mbar;
+    unsigned tmem;
+};
 
-constexpr int kHeadRows = 32;  // rows per block: one warp per row, 8 warps
-
-// y = H3 W4 + b4 for each row; the 8 columns of lane l are 8l .. 8l+7;
-// w4 is the block's shared copy of W4 ([in][out], BF16).
-__device__ __forceinline__ void head_forward(const __nv_bfloat16 *h, const __nv_bfloat16 *w4,
-                                             const float *b4, float (&hv)[8], float (&y)[kOut]) {
-    const int lane = threadIdx.x & 31;
-    __align__(16) __nv_bfloat16 hb[8];
-    *reinterpret_cast<int4 *>(hb) = *reinterpret_cast<const int4 *>(h + 8 * lane);
-    float acc[kOut] = {0.f, 0.f, 0.f};
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        hv[j] = __bfloat162float(hb[j]);
-#pragma unroll
-        for (int o = 0; o < kOut; o++)
-            acc[o] = fmaf(hv[j], __bfloat162float(w4[(8 * lane + j) * kOut + o]), acc[o]);
-    }
-#pragma unroll
-    for (int o = 0; o < kOut; o++) {
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) acc[o] += __shfl_xor_sync(0xffffffffu, acc[o], d);
-        y[o] = acc[o] + b4[o];
-    }
-}
-
-constexpr int kPredictRows = 64;  // rows per block of the inference head: 8 per warp
-
-__global__ void __launch_bounds__(256) mlp_head_predict(const __nv_bfloat16 *__restrict__ h3,
-                                                        const BfWeights *W, const float *params,
-                                                        long long nrows, float *__restrict__ out) {
-    __shared__ __nv_bfloat16 w4[kH * kOut];
-    for (int i = threadIdx.x; i < kH * kOut; i += blockDim.x) w4[i] = W->w4[i];
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = warp; i < kPredictRows; i += 8) {
-        const long long r = (long long)blockIdx.x * kPredictRows + i;
-        if (r >= nrows) break;
-        float hv[8], y[kOut];
-        head_forward(h3 + r * kH, w4, params + kOffB4, hv, y);
-        if (lane < kOut) out[r * kOut + lane] = y[lane];
-    }
-}
-
-// Training head: outputs, loss, dL/dy and the gradient into layer 3,
-// dz3 = (dy W4^T) * relu'(h3), stored row-major and feature-major; the
-// output layer's own gradients (W4, b4) are summed per block.  loss =
+// Training: outputs, loss, the gradients of the output layer (summed per
+// CTA), dz3 = (dy W4^T) * relu'(h3) and dz2 = (dz3 W3^T) * relu'(h2).  loss =
 // mean over rows of w_d (y0 - t0)^2 + w_a (y1 - t1)^2 + w_e rho(|y0 - t0| - y2),
 // rho the pinball loss of the kQuantile quantile, so that y2 learns that
-// quantile of the depth output's absolute error (taken as a constant).
-__global__ void __launch_bounds__(256) mlp_head_train(
-    const __nv_bfloat16 *__restrict__ h3, const BfWeights *W, const float *params,
-    const float *__restrict__ targets, const long long *__restrict__ row_of, long long nrows,
-    long long Bp, float w_d, float w_a, float w_e, float *__restrict__ y_out,
-    __nv_bfloat16 *__restrict__ dz_row, __nv_bfloat16 *__restrict__ dz_col,
-    float *__restrict__ grad, float *__restrict__ loss) {
-    // rows padded by 16 bytes: the feature-major pass reads down a column
-    __shared__ __align__(16) __nv_bfloat16 tile[kHeadRows][kH + 8];
-    __shared__ float gw4[kH * kOut];
-    __shared__ __nv_bfloat16 w4[kH * kOut];
-    __shared__ float gb4[kOut];
-    __shared__ float lsum;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < kH * kOut; i += blockDim.x) {
-        gw4[i] = 0.f;
-        w4[i] = W->w4[i];
+// quantile of the depth output's absolute error (taken as a constant).  The
+// tile's image in shared memory is h2 (layer 3's operand; its signs are kept
+// in registers), then h3 (W4's gradient), then dz3 (the next product's
+// operand and what is stored).
+__global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    Smem3T &S = *reinterpret_cast<Smem3T *>(smem_raw +
+                                            ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_launch_dependents();
+    if (tid < 32) tmem_alloc(&S.tmem, 512);
+    if (tid == 0) {
+        mbar_init(&S.wbar, 1);
+        mbar_init(&S.abar, 1);
+        mbar_init(&S.mbar, 1);
     }
-    if (threadIdx.x < kOut) gb4[threadIdx.x] = 0.f;
-    if (threadIdx.x == 0) lsum = 0.f;
-    __syncthreads();
-    const float inv_b = 1.0f / (float)nrows;
-    const long long rb = (long long)blockIdx.x * kHeadRows;
-    // this lane's share of the output layer's gradients over the warp's rows
-    float gw[8][kOut], gb[kOut] = {0.f, 0.f, 0.f}, ls = 0.f;
+    pdl_wait();
+    S.w4[tid] = g.W->w4[tid];
+    S.b3[tid] = g.b3[tid];
+    const float b4[kOut] = {g.b4[0], g.b4[1], g.b4[2]};
+    tc_sync();
+    const unsigned tmem = S.tmem;
+    const auto load = [&](int t) {
+        mbar_expect(&S.abar, kActBytes);
+        bulk_load(S.a, g.h2 + (size_t)t * kActBytes, kActBytes, &S.abar);
+    };
+    if (tid == 0) {
+        load(blockIdx.x);
+        mbar_expect(&S.wbar, kWBytes);
+        bulk_load(S.w3, g.W->w3, kWBytes, &S.wbar);
+    }
+    const Part p = my_part(tmem);
+    const int odd = p.col0 ? 1 : 0;  // this thread's vectors of eight features: 2 i + odd
+    const float inv_b = 1.0f / (float)g.nrows;
+    // W4's gradient: this thread's rows lane + 32 i of every tile, the eight
+    // features of each of the warp's four vectors
+    float gw[4][8][kOut], gb[kOut] = {0.f, 0.f, 0.f}, ls = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; j++)
+    for (int q = 0; q < 4; q++)
 #pragma unroll
-        for (int o = 0; o < kOut; o++) gw[j][o] = 0.f;
-    for (int i = warp; i < kHeadRows; i += 8) {
-        const long long r = rb + i;
-        __align__(16) __nv_bfloat16 dz[8];
-        if (r < nrows) {
-            float hv[8], y[kOut];
-            head_forward(h3 + r * kH, w4, params + kOffB4, hv, y);
-            const float *t = targets + row_of[r] * kTargets;
-            const float e0 = y[0] - t[0], e1 = y[1] - t[1];
-            const float u = fabsf(e0) - y[2];
-            const float pin = u >= 0.f ? kQuantile * u : (kQuantile - 1.f) * u;
-            const float d0 = 2.f * w_d * e0 * inv_b, d1 = 2.f * w_a * e1 * inv_b,
-                        d2 = w_e * (u < 0.f ? 1.f - kQuantile : -kQuantile) * inv_b;
-            if (lane == 0) {
-                y_out[r * kOut] = y[0];
-                y_out[r * kOut + 1] = y[1];
-                y_out[r * kOut + 2] = y[2];
-                ls += (w_d * e0 * e0 + w_a * e1 * e1 + w_e * pin) * inv_b;
+        for (int j = 0; j < 8; j++)
+#pragma unroll
+            for (int o = 0; o < kOut; o++) gw[q][j][o] = 0.f;
+    bool ok = cta_wait(&S.wbar, 0, g.status);
+    unsigned phase = 0, mphase = 0;
+    for (int t = blockIdx.x; ok && t < g.tiles; t += gridDim.x) {
+        ok = cta_wait(&S.abar, phase, g.status);
+        phase ^= 1;
+        if (!ok) break;
+        if (tid == 0) {
+            tc_fence_after();
+            mma_layer(tmem, smem_u32(S.a), smem_u32(S.w3), false);
+            mma_layer(tmem, smem_u32(S.a) + 16 * kActStride, smem_u32(S.w3) + 16 * kWStride, true);
+            tc_commit(&S.mbar);
+        }
+        // the targets while the product runs
+        const long long r = (long long)t * kTileM + p.row;
+        float t0 = 0.f, t1 = 0.f;
+        if (r < g.nrows) {
+            const float2 tt = *reinterpret_cast<const float2 *>(g.targets + g.row_of[r] * kTargets);
+            t0 = tt.x;
+            t1 = tt.y;
+        }
+        // signs of this thread's 128 features of h2: vectors 2 i + odd
+        unsigned char *image = S.a + p.row * 16;
+        unsigned mask[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            mask[q] = 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                mask[q] |= positive8(*reinterpret_cast<const uint4 *>(
+                               image + (2 * (4 * q + j) + odd) * kActStride))
+                           << (8 * j);
+        }
+        ok = cta_wait(&S.mbar, mphase, g.status);
+        mphase ^= 1;
+        if (!ok) break;
+        tc_fence_after();
+        float acc[kOut];
+        head_half<true>(p.tmem, odd, S.b3, S.w4, image, acc);
+        S.half[odd][p.row] = make_float4(acc[0], acc[1], acc[2], 0.f);
+        __syncthreads();
+        float d0 = 0.f, d1 = 0.f, d2 = 0.f;
+        if (r < g.nrows) {
+            const float4 a = S.half[0][p.row], b = S.half[1][p.row];
+            // (a + b first: the order of inference)
+            const float y0 = a.x + b.x + b4[0], y1 = a.y + b.y + b4[1], y2 = a.z + b.z + b4[2];
+            const float e0 = y0 - t0, e1 = y1 - t1;
+            const float u = fabsf(e0) - y2;
+            d0 = 2.f * g.w_d * e0 * inv_b;
+            d1 = 2.f * g.w_a * e1 * inv_b;
+            d2 = g.w_e * (u < 0.f ? 1.f - kQuantile : -kQuantile) * inv_b;
+            if (!odd) {
+                const float pin = u >= 0.f ? kQuantile * u : (kQuantile - 1.f) * u;
+                ls += (g.w_d * e0 * e0 + g.w_a * e1 * e1 + g.w_e * pin) * inv_b;
                 gb[0] += d0;
                 gb[1] += d1;
                 gb[2] += d2;
+                g.y[r * kOut] = y0;
+                g.y[r * kOut + 1] = y1;
+                g.y[r * kOut + 2] = y2;
             }
+        }
+        if (!odd) S.dy[p.row] = make_float4(d0, d1, d2, 0.f);
+        __syncthreads();
+#pragma unroll 1
+        for (int i = 0; i < kTileM; i += 32) {
+            const float4 d = S.dy[i + lane];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                float h[8];
+                unpack8(*reinterpret_cast<const uint4 *>(S.a + (4 * warp + q) * kActStride +
+                                                         (i + lane) * 16),
+                        h);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    gw[q][j][0] = fmaf(h[j], d.x, gw[q][j][0]);
+                    gw[q][j][1] = fmaf(h[j], d.y, gw[q][j][1]);
+                    gw[q][j][2] = fmaf(h[j], d.z, gw[q][j][2]);
+                }
+            }
+        }
+        __syncthreads();
+        // dz3 in h3's place
+#pragma unroll 1
+        for (int q = 0; q < 16; q++) {
+            uint4 *at = reinterpret_cast<uint4 *>(image + (2 * q + odd) * kActStride);
+            const unsigned m = positive8(*at);
+            float dz[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const int c = 8 * lane + j;
-                const float w0 = __bfloat162float(w4[c * kOut]);
-                const float w1 = __bfloat162float(w4[c * kOut + 1]);
-                const float w2 = __bfloat162float(w4[c * kOut + 2]);
-                const float g = fmaf(d0, w0, fmaf(d1, w1, d2 * w2));
-                dz[j] = __float2bfloat16(hv[j] > 0.f ? g : 0.f);
-                gw[j][0] += hv[j] * d0;
-                gw[j][1] += hv[j] * d1;
-                gw[j][2] += hv[j] * d2;
+                const float4 w = S.w4[16 * q + 8 * odd + j];
+                const float v = fmaf(d0, w.x, fmaf(d1, w.y, d2 * w.z));
+                dz[j] = (m >> j) & 1u ? v : 0.f;
             }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; j++) dz[j] = __float2bfloat16(0.f);
+            *at = pack8(dz);
         }
-        *reinterpret_cast<int4 *>(&tile[i][8 * lane]) = *reinterpret_cast<const int4 *>(dz);
+        tc_sync();
+        if (tid == 0) {
+            mma_layer_back(tmem + kH, smem_u32(S.a), smem_u32(S.w3));
+            tc_commit(&S.mbar);
+            bulk_store(g.d3 + (size_t)t * kActBytes, S.a, kActBytes);
+        }
+        ok = cta_wait(&S.mbar, mphase, g.status);
+        mphase ^= 1;
+        if (!ok) break;
+        tc_fence_after();
+        if (tid == 0) {
+            bulk_store_read();
+            if (t + (int)gridDim.x < g.tiles) load(t + gridDim.x);
+        }
+        unsigned char *d2_out = g.d2 + (size_t)t * kActBytes + p.row * 16;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int c0 = 32 * i + 8 * odd;
+            float v[2][8];
+            tc_ld8x2(p.tmem + kH + c0, p.tmem + kH + c0 + 16, v[0], v[1]);
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    v[q][j] = (mask[i >> 1] >> (16 * (i & 1) + 8 * q + j)) & 1u ? v[q][j] : 0.f;
+                *reinterpret_cast<uint4 *>(d2_out + (size_t)(4 * i + 2 * q + odd) * kActStride) =
+                    pack8(v[q]);
+            }
+        }
+        tc_fence_before();
     }
+    if (tid == 0) bulk_store_done();
+    // this CTA's sums, each over its lanes in a fixed order
+    float *out = g.part4 + (size_t)blockIdx.x * kPart4;
 #pragma unroll
-    for (int j = 0; j < 8; j++)
+    for (int q = 0; q < 4; q++)
 #pragma unroll
-        for (int o = 0; o < kOut; o++) atomicAdd(&gw4[(8 * lane + j) * kOut + o], gw[j][o]);
-    if (lane == 0) {
-        atomicAdd(&lsum, ls);
+        for (int j = 0; j < 8; j++)
 #pragma unroll
-        for (int o = 0; o < kOut; o++) atomicAdd(&gb4[o], gb[o]);
+            for (int o = 0; o < kOut; o++) {
+                float s = gw[q][j][o];
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+                if (lane == 0) out[((4 * warp + q) * 8 + j) * kOut + o] = s;
+            }
+    const float tail[kOut + 1] = {gb[0], gb[1], gb[2], ls};
+#pragma unroll
+    for (int o = 0; o <= kOut; o++) {
+        float s = tail[o];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+        if (lane == 0) S.sum4[warp][o] = s;
     }
+    tc_fence_before();
     __syncthreads();
-    // row-major rows of the block (rows up to Bp: the padding is zero)
-    for (int v = threadIdx.x; v < kHeadRows * (kH / 8); v += blockDim.x) {
-        const int i = v / (kH / 8), q = v % (kH / 8);
-        const long long r = rb + i;
-        if (r < Bp)
-            reinterpret_cast<int4 *>(dz_row + r * kH)[q] =
-                reinterpret_cast<const int4 *>(&tile[i][0])[q];
+    if (tid <= kOut) {
+        float s = 0.f;
+        for (int w = 0; w < 4; w++) s += S.sum4[w][tid];  // warps 0 .. 3 hold the rows
+        out[kH * kOut + tid] = s;
     }
-    // feature-major: 32 consecutive rows of each feature
-    for (int v = threadIdx.x; v < kH * kHeadRows; v += blockDim.x) {
-        const int c = v / kHeadRows, i = v % kHeadRows;
-        const long long r = rb + i;
-        if (r < Bp) dz_col[(long long)c * Bp + r] = tile[i][c];
-    }
-    for (int i = threadIdx.x; i < kH * kOut; i += blockDim.x)
-        atomicAdd(&grad[kOffW4 + i], gw4[i]);
-    if (threadIdx.x < kOut) atomicAdd(&grad[kOffB4 + threadIdx.x], gb4[threadIdx.x]);
-    if (threadIdx.x == 0) atomicAdd(loss, lsum);
+    if (tid < 32) tmem_free(tmem, 512);
 }
 
-// Bias gradients: sum over the batch of each feature-major gradient row,
-// each row split over gridDim.y blocks (8 rows per thread and step, as one
-// 16-byte load).
-__global__ void __launch_bounds__(256) mlp_bias_grad(const __nv_bfloat16 *__restrict__ dz_col,
-                                                     long long Bp, int nfeat,
-                                                     float *__restrict__ gb) {
-    const int f = blockIdx.x;
-    if (f >= nfeat) return;
-    float s = 0.f;
-    const int4 *p = reinterpret_cast<const int4 *>(dz_col + (long long)f * Bp);
-    const long long nv = Bp / 8;  // Bp is a multiple of the 128-row tile
-    for (long long q = blockIdx.y * (long long)blockDim.x + threadIdx.x; q < nv;
-         q += (long long)gridDim.y * blockDim.x) {
-        const int4 u = p[q];
-        const __nv_bfloat16 *b = reinterpret_cast<const __nv_bfloat16 *>(&u);
+// ---- the gradient through layer 2 ----------------------------------------------
+
+struct Back2 {
+    const BfWeights *W;
+    const unsigned char *d2, *h1;
+    unsigned char *d1;
+    int tiles;
+    int *status;
+};
+struct __align__(1024) SmemB {
+    unsigned char w2[kWBytes];
+    unsigned char a[kActBytes];
+    unsigned long long wbar, abar, mbar;
+    unsigned tmem;
+};
+
+// dz1 = (dz2 W2^T) * relu'(h1) of the tiles blockIdx.x, + gridDim.x, ...
+__global__ void __launch_bounds__(kThreads, 1) mlp_back2(Back2 g) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    SmemB &S = *reinterpret_cast<SmemB *>(smem_raw +
+                                          ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
+    const int tid = threadIdx.x;
+    pdl_launch_dependents();
+    if (tid < 32) tmem_alloc(&S.tmem, 256);
+    if (tid == 0) {
+        mbar_init(&S.wbar, 1);
+        mbar_init(&S.abar, 1);
+        mbar_init(&S.mbar, 1);
+    }
+    pdl_wait();
+    tc_sync();
+    const unsigned tmem = S.tmem;
+    const auto load = [&](int t) {
+        mbar_expect(&S.abar, kActBytes);
+        bulk_load(S.a, g.d2 + (size_t)t * kActBytes, kActBytes, &S.abar);
+    };
+    if (tid == 0) {
+        load(blockIdx.x);
+        mbar_expect(&S.wbar, kWBytes);
+        bulk_load(S.w2, g.W->w2, kWBytes, &S.wbar);
+    }
+    const Part p = my_part(tmem);
+    bool ok = cta_wait(&S.wbar, 0, g.status);
+    unsigned phase = 0;
+    for (int t = blockIdx.x; ok && t < g.tiles; t += gridDim.x, phase ^= 1) {
+        ok = cta_wait(&S.abar, phase, g.status);
+        if (!ok) break;
+        if (tid == 0) {
+            tc_fence_after();
+            mma_layer_back(tmem, smem_u32(S.a), smem_u32(S.w2));
+            tc_commit(&S.mbar);
+        }
+        unsigned mask[4];
+        const unsigned char *h = g.h1 + (size_t)t * kActBytes + p.row * 16;
 #pragma unroll
-        for (int j = 0; j < 8; j++) s += __bfloat162float(b[j]);
+        for (int q = 0; q < 4; q++) {
+            mask[q] = 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                mask[q] |= positive8(__ldg(reinterpret_cast<const uint4 *>(
+                               h + (size_t)(p.col0 / 8 + 4 * q + j) * kActStride)))
+                           << (8 * j);
+        }
+        ok = cta_wait(&S.mbar, phase, g.status);
+        if (!ok) break;
+        tc_fence_after();
+        if (tid == 0 && t + (int)gridDim.x < g.tiles) load(t + gridDim.x);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int c0 = p.col0 + 32 * i;
+            float v[32];
+            tc_ld32(p.tmem + c0, v);
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = (mask[i] >> j) & 1u ? v[j] : 0.f;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                *reinterpret_cast<uint4 *>(g.d1 + (size_t)t * kActBytes +
+                                           (size_t)(c0 / 8 + q) * kActStride + p.row * 16) =
+                    pack8(v + 8 * q);
+        }
+        tc_fence_before();
     }
-    __shared__ float sh[256];
-    sh[threadIdx.x] = s;
+    tc_fence_before();
     __syncthreads();
-    for (int t = 128; t > 0; t >>= 1) {
-        if ((int)threadIdx.x < t) sh[threadIdx.x] += sh[threadIdx.x + t];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) atomicAdd(&gb[f], sh[0]);
+    if (tid < 32) tmem_free(tmem, 256);
 }
 
-// Weight gradient from its per-split partials: out[i] += sum over s of
-// part[s][i] (the splits of the batch, in a fixed order).
-__global__ void __launch_bounds__(256) mlp_sum_partials(const float *__restrict__ part,
-                                                        int splits, long n,
-                                                        float *__restrict__ out) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    // four independent running sums (loads in flight together), fixed order
+// ---- weight gradients --------------------------------------------------------
+
+// gW3 = H2^T dZ3, gW2 = H1^T dZ2 (256 x 256: the whole of tensor memory) and
+// gW1^T = dZ1^T X, every one over the rows, in splits of four tiles (512
+// rows): an item is one split of one product, a CTA takes items in turn and
+// leaves a partial sum of each.  With a product goes the sum over the rows of
+// the layer's gradient (its bias).  The first `big` CTAs share the items of
+// W3 and W2, the others those of W1 (a ninth of the products but half of the
+// bytes).
+constexpr int kSplitTiles = 4;
+struct Wgrad {
+    const unsigned char *h1, *h2, *x, *d1, *d2, *d3;
+    int tiles, splits, big;
+    float *part;           // [2][splits][2][64][128][4] (W3, W2)
+    float *part1;          // [splits][2][4][128][4] (W1)
+    float *part_b;         // [3][splits][256] (b3, b2, b1)
+    int *status;
+};
+struct __align__(1024) SmemW {
+    unsigned char buf[3][kActBytes];
+    unsigned long long full[3], free_[3], done, drained;
+    unsigned tmem;
+};
+
+__global__ void __launch_bounds__(kThreads3, 1) mlp_wgrad(Wgrad g) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    SmemW &S = *reinterpret_cast<SmemW *>(smem_raw +
+                                          ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_launch_dependents();
+    if (tid < 32) tmem_alloc(&S.tmem, 512);
+    if (tid == 0) {
+        for (int i = 0; i < 3; i++) {
+            mbar_init(&S.full[i], 1);
+            mbar_init(&S.free_[i], 1 + 8);  // the products, and the eight summing warps
+        }
+        mbar_init(&S.done, 1);
+        mbar_init(&S.drained, 8);
+    }
+    pdl_wait();
+    tc_sync();
+    const unsigned tmem = S.tmem;
+    const bool first = (int)blockIdx.x >= g.big;  // layer 1
+    const int item0 = first ? blockIdx.x - g.big : blockIdx.x;
+    const int step = first ? gridDim.x - g.big : g.big;
+    const int items = first ? g.splits : 2 * g.splits;
+    bool ok = true;
+    if (tid >= kThreads) {
+        if (tid == kThreads) {
+            // loads: of each tile the activations (or features), then the
+            // layer's gradient, into the three buffers in turn, a tile and a
+            // half ahead of the products
+            int load_item = item0, load_tile = 0, loads = 0;
+            const auto load_next = [&](bool second) {
+                const int prod = first ? 2 : load_item / g.splits;
+                const int split = first ? load_item : load_item % g.splits;
+                const int t = split * kSplitTiles + load_tile;
+                const int i = loads % 3;
+                if (loads >= 3) ok = mbar_wait(&S.free_[i], (loads / 3 - 1) & 1, g.status);
+                if (!ok) return;
+                const unsigned bytes = first && !second ? kXBytes : kActBytes;
+                const unsigned char *src = second ? (prod == 0 ? g.d3 : (prod == 1 ? g.d2 : g.d1))
+                                                  : (prod == 0 ? g.h2 : (prod == 1 ? g.h1 : g.x));
+                mbar_expect(&S.full[i], bytes);
+                bulk_load(S.buf[i], src + (size_t)t * bytes, bytes, &S.full[i]);
+                loads++;
+                if (second) {
+                    load_tile++;
+                    if (load_tile == kSplitTiles || t + 1 == g.tiles) {
+                        load_tile = 0;
+                        load_item += step;
+                    }
+                }
+            };
+            const auto ahead = [&](int upto) {
+                while (ok && load_item < items && loads < upto) load_next(loads & 1);
+            };
+            int used = 0, n = 0;
+            ahead(3);
+            for (int item = item0; ok && item < items; item += step, n++) {
+                const int split = first ? item : item % g.splits;
+                const int t1 = min(g.tiles, (split + 1) * kSplitTiles);
+                // the accumulators' last reader
+                if (n > 0) ok = mbar_wait(&S.drained, (n - 1) & 1, g.status);
+                tc_fence_after();
+                bool more = false;
+                for (int t = split * kSplitTiles; ok && t < t1; t++) {
+                    const int ia = used % 3, ib = (used + 1) % 3;
+                    ok = mbar_wait(&S.full[ia], (used / 3) & 1, g.status);
+                    if (ok) ok = mbar_wait(&S.full[ib], ((used + 1) / 3) & 1, g.status);
+                    if (!ok) break;
+                    const unsigned a = smem_u32(S.buf[ia]), b = smem_u32(S.buf[ib]);
+                    for (int m = 0; m < 2; m++)
+                        for (int kk = 0; kk < 8; kk++) {
+                            if (!first)  // 128 inputs x 256 outputs
+                                tc_mma(tmem + kH * m,
+                                       smem_desc(a + 16 * m * kActStride + 256 * kk, 128,
+                                                 kActStride),
+                                       smem_desc(b + 256 * kk, 128, kActStride),
+                                       tc_idesc(kH, true, true), more || kk > 0);
+                            else  // 128 outputs x 16 inputs
+                                tc_mma(tmem + kH * m,
+                                       smem_desc(b + 16 * m * kActStride + 256 * kk, 128,
+                                                 kActStride),
+                                       smem_desc(a + 256 * kk, 128, kActStride),
+                                       tc_idesc(kF, true, true), more || kk > 0);
+                        }
+                    more = true;
+                    tc_commit(&S.free_[ia]);
+                    tc_commit(&S.free_[ib]);
+                    if (t + 1 == t1) tc_commit(&S.done);
+                    used += 2;
+                    ahead(used + 3);
+                }
+            }
+        }
+    } else {
+        const Part p = my_part(tmem);
+        int used = 0, n = 0;
+        for (int item = item0; item < items; item += step, n++) {
+            const int prod = first ? 2 : item / g.splits;
+            const int split = first ? item : item % g.splits;
+            const int t1 = min(g.tiles, (split + 1) * kSplitTiles);
+            // the bias: rows lane + 32 i, the eight features of the warp's four vectors
+            float gb[4][8];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) gb[q][j] = 0.f;
+            for (int t = split * kSplitTiles; t < t1; t++, used += 2) {
+                const int ia = used % 3, ib = (used + 1) % 3;
+                if (ok) ok = mbar_wait(&S.full[ia], (used / 3) & 1, g.status);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.free_[ia]);
+                if (ok) ok = mbar_wait(&S.full[ib], ((used + 1) / 3) & 1, g.status);
+#pragma unroll 1
+                for (int r = lane; ok && r < kTileM; r += 32)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        float v[8];
+                        unpack8(*reinterpret_cast<const uint4 *>(
+                                    S.buf[ib] + (4 * warp + q) * kActStride + r * 16),
+                                v);
+#pragma unroll
+                        for (int j = 0; j < 8; j++) gb[q][j] += v[j];
+                    }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&S.free_[ib]);
+            }
+            float *out_b = g.part_b + (size_t)(prod * g.splits + split) * kH;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    float s = gb[q][j];
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+                    if (lane == 0) out_b[(4 * warp + q) * 8 + j] = s;
+                }
+            if (ok) ok = mbar_wait(&S.done, n & 1, g.status);
+            ok = __all_sync(0xffffffffu, ok);
+            if (ok) {
+                tc_fence_after();
+                const int half = p.col0 >> 7;
+                if (!first) {
+#pragma unroll 1
+                    for (int m = 0; m < 2; m++) {
+                        float4 *out = reinterpret_cast<float4 *>(g.part) +
+                                      (size_t)((prod * g.splits + split) * 2 + m) * 64 * kTileM;
+#pragma unroll 1
+                        for (int c0 = p.col0; c0 < p.col0 + 128; c0 += 32) {
+                            float v[32];
+                            tc_ld32(p.tmem + kH * m + c0, v);
+#pragma unroll
+                            for (int q = 0; q < 8; q++)
+                                out[(size_t)(c0 / 4 + q) * kTileM + p.row] = make_float4(
+                                    v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                        }
+                    }
+                } else {
+                    float4 *out = reinterpret_cast<float4 *>(g.part1) +
+                                  (size_t)(split * 2 + half) * 4 * kTileM;
+                    float v[16];
+                    tc_ld16(p.tmem + kH * half, v);
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        out[(size_t)q * kTileM + p.row] =
+                            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                }
+                tc_fence_before();
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.drained);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (tid < 32) tmem_free(tmem, 512);
+}
+
+// ---- sums of the partials, Adam -------------------------------------------------
+
+struct Adam {
+    float *p, *m, *v;  // null p: gradients only
+    float lr, b1, b2, eps, c1, c2;
+};
+struct Finish {
+    const float *part, *part1, *part_b, *part4;
+    int splits, ctas4;
+    float *grad;       // null: not asked for
+    float *loss;
+    Adam adam;
+    BfWeights *W;
+};
+
+// A gradient becomes a parameter's step; returns the new parameter.
+__device__ __forceinline__ float adam_step(const Adam &a, long i, float gi) {
+    const float mi = a.b1 * a.m[i] + (1.f - a.b1) * gi;
+    const float vi = a.b2 * a.v[i] + (1.f - a.b2) * gi * gi;
+    a.m[i] = mi;
+    a.v[i] = vi;
+    const float p = a.p[i] - a.lr * (mi * a.c1) / (sqrtf(vi * a.c2) + a.eps);
+    a.p[i] = p;
+    return p;
+}
+
+constexpr int kItemsW = 4 * 2 * 2 * 64 * kTileM;       // W3 and W2, one output each
+constexpr int kItems1 = 4 * 2 * 4 * kTileM;            // W1, one input each
+constexpr int kItemsB = 3 * kH;                        // b3, b2, b1
+constexpr int kItems4 = kPart4;                        // W4, b4, the loss
+constexpr int kItems = kItemsW + kItems1 + kItemsB + kItems4;
+
+__device__ __forceinline__ float4 add4(const float4 &a, const float4 &b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+// The sum over n splits of the float4 at p, step apart: four running sums over
+// the splits k, k + 4, ... (what is left over four goes to the first), each by
+// one lane of four, all its loads in flight together; every lane returns
+// (s0 + s1) + (s2 + s3).
+__device__ __forceinline__ float4 split_sum4(const float4 *p, size_t step, int n, int lane4) {
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int n4 = n & ~3;
+#pragma unroll 16
+    for (int k = lane4; k < n4; k += 4) s = add4(s, __ldcs(p + (size_t)k * step));
+    if (lane4 == 0)
+        for (int k = n4; k < n; k++) s = add4(s, p[(size_t)k * step]);
+#pragma unroll
+    for (int d = 1; d <= 2; d <<= 1)
+        s = add4(s, make_float4(__shfl_xor_sync(0xffffffffu, s.x, d),
+                                __shfl_xor_sync(0xffffffffu, s.y, d),
+                                __shfl_xor_sync(0xffffffffu, s.z, d),
+                                __shfl_xor_sync(0xffffffffu, s.w, d)));
+    return s;
+}
+__device__ __forceinline__ float split_sum(const float *p, size_t step, int n) {
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
     int k = 0;
-    for (; k + 4 <= splits; k += 4) {
-        s0 += part[(long)k * n + i];
-        s1 += part[(long)(k + 1) * n + i];
-        s2 += part[(long)(k + 2) * n + i];
-        s3 += part[(long)(k + 3) * n + i];
+#pragma unroll 4
+    for (; k + 4 <= n; k += 4) {
+        s0 += p[(size_t)k * step];
+        s1 += p[(size_t)(k + 1) * step];
+        s2 += p[(size_t)(k + 2) * step];
+        s3 += p[(size_t)(k + 3) * step];
     }
-    for (; k < splits; k++) s0 += part[(long)k * n + i];
-    out[i] += (s0 + s1) + (s2 + s3);
+    for (; k < n; k++) s0 += p[(size_t)k * step];
+    return (s0 + s1) + (s2 + s3);
+}
+
+// One thread per parameter: the partials of every split summed in a fixed
+// order, then Adam and the BF16 image, or the gradient.  Reads 128 kB per
+// split and product half: bound by the latency of those reads, which is why
+// four lanes share the splits of four weights.
+__global__ void __launch_bounds__(256) mlp_finish(Finish g) {
+    pdl_launch_dependents();
+    pdl_wait();
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = i & 3;
+    const auto put = [&](long at, float gi, __nv_bfloat16 *image) {
+        if (g.grad) g.grad[at] = gi;
+        if (g.adam.p) {
+            const float p = adam_step(g.adam, at, gi);
+            if (image) *image = __float2bfloat16(p);
+        }
+    };
+    const auto pick = [&](const float4 &s) {
+        return j == 0 ? s.x : (j == 1 ? s.y : (j == 2 ? s.z : s.w));
+    };
+    if (i < kItemsW) {
+        i >>= 2;
+        const int row = i & 127, c4 = (i >> 7) & 63, m = (i >> 13) & 1, layer2 = i >> 14;
+        const float4 s = split_sum4(reinterpret_cast<const float4 *>(g.part) +
+                                        (size_t)(layer2 * g.splits * 2 + m) * 64 * kTileM +
+                                        (size_t)c4 * kTileM + row,
+                                    (size_t)2 * 64 * kTileM, g.splits, j);
+        const int in = m * kTileM + row, out = 4 * c4 + j;
+        put((layer2 ? kOffW2 : kOffW3) + (long)in * kH + out, pick(s),
+            (layer2 ? g.W->w2 : g.W->w3) + w_at(in, out));
+        return;
+    }
+    i -= kItemsW;
+    if (i < kItems1) {
+        i >>= 2;
+        const int row = i & 127, c4 = (i >> 7) & 3, m = i >> 9;
+        const float4 s = split_sum4(reinterpret_cast<const float4 *>(g.part1) +
+                                        (size_t)(m * 4 + c4) * kTileM + row,
+                                    (size_t)8 * kTileM, g.splits, j);
+        const int in = 4 * c4 + j, out = m * kTileM + row;
+        put(kOffW1 + (long)in * kH + out, pick(s), g.W->w1 + w_at(in, out));
+        return;
+    }
+    i -= kItems1;
+    if (i < kItemsB) {
+        const int layer = i >> 8, f = i & 255;  // 0: b3, 1: b2, 2: b1
+        put((layer == 0 ? kOffB3 : (layer == 1 ? kOffB2 : kOffB1)) + f,
+            split_sum(g.part_b + (size_t)layer * g.splits * kH + f, (size_t)kH, g.splits),
+            nullptr);
+        return;
+    }
+    i -= kItemsB;
+    if (i < kItems4) {
+        const float s = split_sum(g.part4 + i, (size_t)kPart4, g.ctas4);
+        if (i == kPart4 - 1) {
+            *g.loss = s;
+        } else {
+            const long at = kOffW4 + i;  // W4 [256][3], then b4
+            put(at, s, nullptr);
+            if (g.adam.p && i < kH * kOut)
+                reinterpret_cast<float *>(g.W->w4 + i / kOut)[i % kOut] =
+                    __bfloat162float(__float2bfloat16(g.adam.p[at]));
+        }
+    }
 }
 
 // ---- weights ----------------------------------------------------------------
@@ -732,49 +1371,32 @@ __global__ void mlp_pack_weights(const float *__restrict__ p, BfWeights *W) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < kH * kH) {
         const int in = i / kH, out = i % kH;
-        const __nv_bfloat16 a = __float2bfloat16(p[kOffW2 + i]);
-        const __nv_bfloat16 b = __float2bfloat16(p[kOffW3 + i]);
-        W->w2[i] = a;
-        W->w3[i] = b;
-        W->wt2[out * kH + in] = a;
-        W->wt3[out * kH + in] = b;
+        W->w2[w_at(in, out)] = __float2bfloat16(p[kOffW2 + i]);
+        W->w3[w_at(in, out)] = __float2bfloat16(p[kOffW3 + i]);
     }
     if (i < kF * kH) {
         const int in = i / kH, out = i % kH;
-        W->wt1[out * kF + in] = __float2bfloat16(p[kOffW1 + i]);
+        W->w1[w_at(in, out)] = __float2bfloat16(p[kOffW1 + i]);
     }
-    if (i < kH * kOut) W->w4[i] = __float2bfloat16(p[kOffW4 + i]);
-}
-
-__global__ void mlp_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                         float *__restrict__ v, long n, float lr, float b1, float b2, float eps,
-                         float c1, float c2) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+    if (i < kH) {
+        const float *w = p + kOffW4 + i * kOut;
+        W->w4[i] = make_float4(__bfloat162float(__float2bfloat16(w[0])),
+                               __bfloat162float(__float2bfloat16(w[1])),
+                               __bfloat162float(__float2bfloat16(w[2])), 0.f);
+    }
 }
 
 // ---- host side ----------------------------------------------------------------
 
 struct Buffers {  // one batch of rows (training) or one chunk (inference)
-    long long cap = 0;  // rows (a multiple of kTileM)
+    int tiles = 0;
     bool train = false;
-    __nv_bfloat16 *xr = nullptr, *xc = nullptr;
-    __nv_bfloat16 *h1 = nullptr, *h2 = nullptr, *h3 = nullptr;     // row-major
-    __nv_bfloat16 *h1c = nullptr, *h2c = nullptr;                  // feature-major
-    __nv_bfloat16 *d3 = nullptr, *d2 = nullptr, *d3c = nullptr, *d2c = nullptr, *d1c = nullptr;
+    unsigned char *h2 = nullptr;                    // tile images
+    unsigned char *x = nullptr, *h1 = nullptr, *d3 = nullptr, *d2 = nullptr, *d1 = nullptr;
     long long *row_of = nullptr;
     float *y = nullptr;
-    float *part = nullptr;  // weight-gradient partials [splits][256 x 256]
+    float *part = nullptr, *part1 = nullptr, *part_b = nullptr, *part4 = nullptr;  // partials
 };
-
-// Batch rows per K split of the weight-gradient GEMMs.
-constexpr long kWgradRows = 512;
 
 struct Mlp {
     int device = 0;
@@ -833,154 +1455,135 @@ void free_list(std::vector<void *> &v) {
     v.clear();
 }
 
-// Row buffers for `rows` rows (rounded up to the tile), reallocated only
-// when they grow or when training needs the feature-major copies.
-int ensure_buffers(Mlp *m, long long rows, bool train, std::vector<void *> &owned) {
-    const long long cap = (rows + kTileM - 1) / kTileM * kTileM;
+int wgrad_splits(int tiles) { return (tiles + kSplitTiles - 1) / kSplitTiles; }
+
+// Buffers for `tiles` tiles of 128 rows, reallocated only when they grow or
+// when training needs the gradients' images.
+int ensure_buffers(Mlp *m, int tiles, bool train, std::vector<void *> &owned) {
     Buffers &B = m->buf;
-    if (cap <= B.cap && (B.train || !train)) return SWGPU_OK;
+    if (tiles <= B.tiles && (B.train || !train)) return SWGPU_OK;
     MCK(cudaStreamSynchronize(m->stream));
     free_list(owned);
     B = Buffers{};
     int rc;
-    const size_t hr = (size_t)cap * kH;
-    if ((rc = malloc_dev(m, &B.xr, (size_t)cap * kF, &owned)) ||
-        (rc = malloc_dev(m, &B.h1, hr, &owned)) || (rc = malloc_dev(m, &B.h2, hr, &owned)) ||
-        (rc = malloc_dev(m, &B.h3, hr, &owned)) || (rc = malloc_dev(m, &B.y, (size_t)cap * kOut, &owned)))
-        return rc;
+    const size_t act = (size_t)tiles * kActBytes, rows = (size_t)tiles * kTileM;
+    if ((rc = malloc_dev(m, &B.h2, act, &owned))) return rc;
     if (train) {
-        if ((rc = malloc_dev(m, &B.xc, (size_t)cap * kF, &owned)) ||
-            (rc = malloc_dev(m, &B.h1c, hr, &owned)) || (rc = malloc_dev(m, &B.h2c, hr, &owned)) ||
-            (rc = malloc_dev(m, &B.d3, hr, &owned)) || (rc = malloc_dev(m, &B.d2, hr, &owned)) ||
-            (rc = malloc_dev(m, &B.d3c, hr, &owned)) || (rc = malloc_dev(m, &B.d2c, hr, &owned)) ||
-            (rc = malloc_dev(m, &B.d1c, hr, &owned)) ||
-            (rc = malloc_dev(m, &B.row_of, (size_t)cap, &owned)) ||
-            (rc = malloc_dev(m, &B.part, (size_t)((cap + kWgradRows - 1) / kWgradRows) * kH * kH,
-                             &owned)))
+        const size_t s = wgrad_splits(tiles);
+        if ((rc = malloc_dev(m, &B.x, (size_t)tiles * kXBytes, &owned)) ||
+            (rc = malloc_dev(m, &B.h1, act, &owned)) || (rc = malloc_dev(m, &B.d3, act, &owned)) ||
+            (rc = malloc_dev(m, &B.d2, act, &owned)) || (rc = malloc_dev(m, &B.d1, act, &owned)) ||
+            (rc = malloc_dev(m, &B.row_of, rows, &owned)) ||
+            (rc = malloc_dev(m, &B.y, rows * kOut, &owned)) ||
+            (rc = malloc_dev(m, &B.part, s * 2 * kH * kH, &owned)) ||
+            (rc = malloc_dev(m, &B.part1, s * kF * kH, &owned)) ||
+            (rc = malloc_dev(m, &B.part_b, s * 3 * kH, &owned)) ||
+            (rc = malloc_dev(m, &B.part4, (size_t)std::min(tiles, m->sms) * kPart4, &owned)))
             return rc;
     }
-    B.cap = cap;
+    B.tiles = tiles;
     B.train = train;
     return SWGPU_OK;
 }
 
-template <int N, int EPI>
-int launch_gemm(Mlp *m, const GemmArgs &g, int splits) {
-    const unsigned grid_x = (unsigned)((g.M + kTileM - 1) / kTileM);
-    const size_t smem = sizeof(GemmSmem<N>) + 1024;
-    tc_gemm<N, EPI><<<dim3(grid_x, (unsigned)splits), kGemmThreads, smem, m->stream>>>(g);
-    MCK(cudaGetLastError());
+template <typename Smem>
+constexpr size_t smem_of() {
+    return sizeof(Smem) + 1024;  // aligned up to 1024 in the kernel
+}
+
+// A launch as a programmatic dependent of the stream's previous kernel.
+template <typename Args>
+int launch(Mlp *m, void (*kernel)(Args), dim3 grid, int threads, size_t smem, const Args &args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = m->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    MCK(cudaLaunchKernelEx(&cfg, kernel, args));
     return SWGPU_OK;
 }
 
-template <int N, int EPI>
-cudaError_t gemm_attr() {
-    return cudaFuncSetAttribute(tc_gemm<N, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(GemmSmem<N>) + 1024));
+template <typename F>
+cudaError_t smem_attr(F *kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 FeatureTables tables(const Mlp *m) {
     return FeatureTables{m->scen, m->tri, m->mu, m->isd, m->N};
 }
 
-GemmArgs gemm_args(Mlp *m, const __nv_bfloat16 *A, long lda, const __nv_bfloat16 *B, long ldb,
-                   long long M, long K) {
-    GemmArgs g{};
-    g.A = A;
-    g.lda = lda;
-    g.B = B;
-    g.ldb = ldb;
-    g.M = M;
-    g.K = K;
-    g.k_per_split = K;
+// Layers 1 and 2 of a batch into the buffers.
+int layers12(Mlp *m, const Batch &batch, int tiles, bool train) {
+    Buffers &B = m->buf;
+    Layers12 g{};
+    g.F = tables(m);
+    g.batch = batch;
+    g.W = m->w;
+    g.b1 = m->params + kOffB1;
+    g.b2 = m->params + kOffB2;
+    g.h1 = B.h1;
+    g.h2 = B.h2;
+    g.x = B.x;
+    g.row_of = B.row_of;
+    g.tiles = tiles;
+    g.status = m->status;
+    return launch(m, train ? mlp_layers12<true> : mlp_layers12<false>,
+                  dim3((unsigned)std::min(tiles, m->sms)), kThreads, smem_of<Smem12>(), g);
+}
+
+Layer3 layer3(Mlp *m, int tiles, long long nrows, float *y) {
+    Layer3 g{};
+    g.W = m->w;
+    g.b3 = m->params + kOffB3;
+    g.b4 = m->params + kOffB4;
+    g.h2 = m->buf.h2;
+    g.tiles = tiles;
+    g.nrows = nrows;
+    g.y = y;
     g.status = m->status;
     return g;
 }
 
-// Forward pass of Bp rows already in buf.xr (feature-major copies when train).
-int forward(Mlp *m, long long Bp, bool train) {
-    Buffers &B = m->buf;
-    const BfWeights *W = m->w;
-    int rc;
-    GemmArgs g = gemm_args(m, B.xr, kF, W->wt1, kF, Bp, kF);
-    g.bias = m->params + kOffB1;
-    g.out_row = B.h1;
-    g.out_col = train ? B.h1c : nullptr;
-    g.ldc = Bp;
-    if ((rc = launch_gemm<kH, kEpiHidden>(m, g, 1))) return rc;
-    g = gemm_args(m, B.h1, kH, W->wt2, kH, Bp, kH);
-    g.bias = m->params + kOffB2;
-    g.out_row = B.h2;
-    g.out_col = train ? B.h2c : nullptr;
-    g.ldc = Bp;
-    if ((rc = launch_gemm<kH, kEpiHidden>(m, g, 1))) return rc;
-    g = gemm_args(m, B.h2, kH, W->wt3, kH, Bp, kH);
-    g.bias = m->params + kOffB3;
-    g.out_row = B.h3;
-    g.out_col = nullptr;
-    if ((rc = launch_gemm<kH, kEpiHidden>(m, g, 1))) return rc;
-    return SWGPU_OK;
-}
-
-// Forward, backward and the gradient vector of nrows rows (Bp padded).
+// Forward and backward of nrows rows: five launches, the last of which leaves
+// the gradient vector in m->grad or, with adam, takes the step.
 int batch_gradients(Mlp *m, const long long *d_rows, unsigned long long seed, long long nrows,
-                    float w_d, float w_a, float w_e) {
-    const long long Bp = (nrows + kTileM - 1) / kTileM * kTileM;
-    int rc = ensure_buffers(m, nrows, true, m->buf_allocs);
+                    float w_d, float w_a, float w_e, const Adam *adam) {
+    const int tiles = (int)((nrows + kTileM - 1) / kTileM);
+    int rc = ensure_buffers(m, tiles, true, m->buf_allocs);
     if (rc) return rc;
     Buffers &B = m->buf;
-    const BfWeights *W = m->w;
-    MCK(cudaMemsetAsync(m->grad, 0, sizeof(float) * kNumParams, m->stream));
-    MCK(cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
-    mlp_features<<<(unsigned)((Bp + 255) / 256), 256, 0, m->stream>>>(
-        tables(m), d_rows, seed, d_rows ? 0 : m->S * m->N, 0, nrows, Bp, B.xr, B.xc, B.row_of);
-    if ((rc = forward(m, Bp, true))) return rc;
-    mlp_head_train<<<(unsigned)((Bp + kHeadRows - 1) / kHeadRows), 256, 0, m->stream>>>(
-        B.h3, W, m->params, m->targets, B.row_of, nrows, Bp, w_d, w_a, w_e, B.y, B.d3, B.d3c,
-        m->grad, m->loss);
-    MCK(cudaGetLastError());
-    // weight gradients: one partial per split of the batch, then their sum
-    const int splits = (int)((Bp + kWgradRows - 1) / kWgradRows);
-    const dim3 bias_grid(kH, 16);
-    auto sum_parts = [&](long n, long off) {
-        mlp_sum_partials<<<(unsigned)((n + 255) / 256), 256, 0, m->stream>>>(B.part, splits, n,
-                                                                            m->grad + off);
-    };
-    // layer 3: gW3 = H2^T dZ3 (in x out), gb3; dZ2 = (dZ3 W3^T) * relu'(H2)
-    GemmArgs g = gemm_args(m, B.h2c, Bp, B.d3c, Bp, kH, Bp);
-    g.k_per_split = kWgradRows;
-    g.grad = B.part;
-    if ((rc = launch_gemm<kH, kEpiWgrad>(m, g, splits))) return rc;
-    sum_parts((long)kH * kH, kOffW3);
-    mlp_bias_grad<<<bias_grid, 256, 0, m->stream>>>(B.d3c, Bp, kH, m->grad + kOffB3);
-    g = gemm_args(m, B.d3, kH, W->w3, kH, Bp, kH);
-    g.mask = B.h2;
-    g.out_row = B.d2;
-    g.out_col = B.d2c;
-    g.ldc = Bp;
-    if ((rc = launch_gemm<kH, kEpiDgrad>(m, g, 1))) return rc;
-    // layer 2: gW2 = H1^T dZ2, gb2; dZ1 = (dZ2 W2^T) * relu'(H1)
-    g = gemm_args(m, B.h1c, Bp, B.d2c, Bp, kH, Bp);
-    g.k_per_split = kWgradRows;
-    g.grad = B.part;
-    if ((rc = launch_gemm<kH, kEpiWgrad>(m, g, splits))) return rc;
-    sum_parts((long)kH * kH, kOffW2);
-    mlp_bias_grad<<<bias_grid, 256, 0, m->stream>>>(B.d2c, Bp, kH, m->grad + kOffB2);
-    g = gemm_args(m, B.d2, kH, W->w2, kH, Bp, kH);
-    g.mask = B.h1;
-    g.out_row = B.d3;  // dZ1 row-major is not needed again: B.d3 is free
-    g.out_col = B.d1c;
-    g.ldc = Bp;
-    if ((rc = launch_gemm<kH, kEpiDgrad>(m, g, 1))) return rc;
-    // layer 1: gW1^T = dZ1^T X (out x in), stored transposed into W1 [in][out]; gb1
-    g = gemm_args(m, B.d1c, Bp, B.xc, Bp, kH, Bp);
-    g.k_per_split = kWgradRows;
-    g.grad = B.part;
-    if ((rc = launch_gemm<kF, kEpiWgradT>(m, g, splits))) return rc;
-    sum_parts((long)kF * kH, kOffW1);
-    mlp_bias_grad<<<bias_grid, 256, 0, m->stream>>>(B.d1c, Bp, kH, m->grad + kOffB1);
-    MCK(cudaGetLastError());
-    return SWGPU_OK;
+    const unsigned ctas = (unsigned)std::min(tiles, m->sms);
+    Batch batch{d_rows, seed, d_rows ? 0 : m->S * m->N, 0, nrows};
+    if ((rc = layers12(m, batch, tiles, true))) return rc;
+    Layer3 g3 = layer3(m, tiles, nrows, B.y);
+    g3.targets = m->targets;
+    g3.row_of = B.row_of;
+    g3.d3 = B.d3;
+    g3.d2 = B.d2;
+    g3.part4 = B.part4;
+    g3.w_d = w_d;
+    g3.w_a = w_a;
+    g3.w_e = w_e;
+    if ((rc = launch(m, mlp_layer3_train, dim3(ctas), kThreads, smem_of<Smem3T>(), g3))) return rc;
+    Back2 g2{m->w, B.d2, B.h1, B.d1, tiles, m->status};
+    if ((rc = launch(m, mlp_back2, dim3(ctas), kThreads, smem_of<SmemB>(), g2))) return rc;
+    // CTAs of the weight gradients: an item each while the SMs suffice; a
+    // seventh of them for layer 1
+    const int s = wgrad_splits(tiles);
+    const int big = std::max(1, std::min(2 * s, m->sms - m->sms / 7));
+    const int small = std::max(1, std::min(s, m->sms - big));
+    Wgrad gw{B.h1, B.h2, B.x, B.d1, B.d2, B.d3, tiles, s, big, B.part, B.part1, B.part_b,
+             m->status};
+    if ((rc = launch(m, mlp_wgrad, dim3((unsigned)(big + small)), kThreads3, smem_of<SmemW>(), gw)))
+        return rc;
+    Finish gf{B.part, B.part1, B.part_b, B.part4, s, (int)ctas, adam ? nullptr : m->grad, m->loss,
+              adam ? *adam : Adam{}, m->w};
+    return launch(m, mlp_finish, dim3((kItems + 255) / 256), 256, 0, gf);
 }
 
 int read_status(Mlp *m, const char *what) {
@@ -1015,10 +1618,12 @@ int swgpu_mlp_create(const float *params, const float *feature_mean,
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = gemm_attr<kH, kEpiHidden>();
-    if (e == cudaSuccess) e = gemm_attr<kH, kEpiDgrad>();
-    if (e == cudaSuccess) e = gemm_attr<kH, kEpiWgrad>();
-    if (e == cudaSuccess) e = gemm_attr<kF, kEpiWgradT>();
+    if (e == cudaSuccess) e = smem_attr(mlp_layers12<false>, smem_of<Smem12>());
+    if (e == cudaSuccess) e = smem_attr(mlp_layers12<true>, smem_of<Smem12>());
+    if (e == cudaSuccess) e = smem_attr(mlp_layer3_predict, smem_of<Smem3>());
+    if (e == cudaSuccess) e = smem_attr(mlp_layer3_train, smem_of<Smem3T>());
+    if (e == cudaSuccess) e = smem_attr(mlp_back2, smem_of<SmemB>());
+    if (e == cudaSuccess) e = smem_attr(mlp_wgrad, smem_of<SmemW>());
     if (e != cudaSuccess) {
         rc = mfail(m, SWGPU_ECUDA, "swgpu_mlp_create: %s", cudaGetErrorString(e));
         delete m;
@@ -1108,9 +1713,10 @@ int swgpu_mlp_predict(void *handle, int64_t row0, int64_t nrows, float *out_devi
     if (!m || !out_device || nrows <= 0 || row0 < 0 || row0 + nrows > m->S * m->N)
         return mfail(m, SWGPU_EINVAL, "swgpu_mlp_predict: bad rows");
     if (int rc = usable(m, "swgpu_mlp_predict")) return rc;
-    // chunks of up to 2^21 rows through row buffers (1 GB per activation)
-    const long long chunk = std::min<long long>(nrows, 1LL << 21);
-    int rc = ensure_buffers(m, chunk, false, m->buf_allocs);
+    // chunks of five tiles per SM (48 MB of layer 2's activations): what one
+    // kernel leaves, the next finds in L2
+    const long long chunk = std::min<long long>(nrows, 5LL * m->sms * kTileM);
+    int rc = ensure_buffers(m, (int)((chunk + kTileM - 1) / kTileM), false, m->buf_allocs);
     if (rc) return rc;
     cudaEvent_t a, b;
     MCK(cudaEventCreate(&a));
@@ -1118,13 +1724,11 @@ int swgpu_mlp_predict(void *handle, int64_t row0, int64_t nrows, float *out_devi
     MCK(cudaEventRecord(a, m->stream));
     for (long long r0 = 0; r0 < nrows; r0 += chunk) {
         const long long n = std::min(chunk, nrows - r0);
-        const long long Bp = (n + kTileM - 1) / kTileM * kTileM;
-        mlp_features<<<(unsigned)((Bp + 255) / 256), 256, 0, m->stream>>>(
-            tables(m), nullptr, 0, 0, row0 + r0, n, Bp, m->buf.xr, nullptr, nullptr);
-        if ((rc = forward(m, Bp, false))) return rc;
-        mlp_head_predict<<<(unsigned)((n + kPredictRows - 1) / kPredictRows), 256, 0, m->stream>>>(
-            m->buf.h3, m->w, m->params, n, out_device + r0 * kOut);
-        MCK(cudaGetLastError());
+        const int tiles = (int)((n + kTileM - 1) / kTileM);
+        if ((rc = layers12(m, Batch{nullptr, 0, 0, row0 + r0, n}, tiles, false))) return rc;
+        if ((rc = launch(m, mlp_layer3_predict, dim3((unsigned)std::min(tiles, m->sms)), kThreads3,
+                         smem_of<Smem3>(), layer3(m, tiles, n, out_device + r0 * kOut))))
+            return rc;
     }
     MCK(cudaEventRecord(b, m->stream));
     MCK(cudaEventSynchronize(b));
@@ -1155,7 +1759,8 @@ int swgpu_mlp_gradients(void *handle, const int64_t *rows, int64_t nrows, float 
     }
     MCK(cudaMemcpyAsync(m->rows, rows, sizeof(long long) * nrows, cudaMemcpyHostToDevice,
                         m->stream));
-    if ((rc = batch_gradients(m, m->rows, 0, nrows, w_depth, w_arrival, w_error))) return rc;
+    if ((rc = batch_gradients(m, m->rows, 0, nrows, w_depth, w_arrival, w_error, nullptr)))
+        return rc;
     if (outputs)
         MCK(cudaMemcpyAsync(outputs, m->buf.y, sizeof(float) * kOut * nrows,
                             cudaMemcpyDeviceToHost, m->stream));
@@ -1182,14 +1787,12 @@ int swgpu_mlp_train(void *handle, int steps, int64_t batch, uint64_t seed, float
     const float b1 = 0.9f, b2 = 0.999f;
     for (int s = 0; s < steps; s++) {
         const unsigned long long step_seed = seed * 0x9E3779B97F4A7C15ull + (unsigned)s;
-        int rc = batch_gradients(m, nullptr, step_seed, batch, w_depth, w_arrival, w_error);
+        const float c1 = 1.f / (1.f - powf(b1, (float)(m->adam_t + 1)));
+        const float c2 = 1.f / (1.f - powf(b2, (float)(m->adam_t + 1)));
+        const Adam adam{m->params, m->adam_m, m->adam_v, lr, b1, b2, 1e-8f, c1, c2};
+        int rc = batch_gradients(m, nullptr, step_seed, batch, w_depth, w_arrival, w_error, &adam);
         if (rc) return rc;
         m->adam_t++;
-        const float c1 = 1.f / (1.f - powf(b1, (float)m->adam_t));
-        const float c2 = 1.f / (1.f - powf(b2, (float)m->adam_t));
-        mlp_adam<<<(unsigned)((kNumParams + 255) / 256), 256, 0, m->stream>>>(
-            m->params, m->grad, m->adam_m, m->adam_v, kNumParams, lr, b1, b2, 1e-8f, c1, c2);
-        mlp_pack_weights<<<(kH * kH + 255) / 256, 256, 0, m->stream>>>(m->params, m->w);
     }
     MCK(cudaGetLastError());
     MCK(cudaEventRecord(b, m->stream));
