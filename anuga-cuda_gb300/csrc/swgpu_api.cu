@@ -179,6 +179,11 @@ static void reset_ftmin(Ctrl *c, const DevParams &P) {
 
 // ----------------------------------------------------------- step issue
 
+// Whether the mixed step's clock is a kernel of its own: on large meshes, where
+// a launch is a hundredth of the step and thousands of update blocks would each
+// evaluate it.
+static bool separate_clock(const Handle *h) { return h->M.N >= (1 << 20); }
+
 // One stage of a fused step: flux -> update (with the stage's backup or
 // saxpy and clock bookkeeping) -> distribute with boundary values.
 static void issue_stage(Handle *h, const Stage &stg) {
@@ -193,9 +198,12 @@ static void issue_stage(Handle *h, const Stage &stg) {
                                h->stream);
     } else {
         launch_flux_mixed(h->M, h->S, h->X, h->P, h->d_ctrl, flux_flags, h->stream);
-        if (!(flux_flags & kNoTimestep))
+        const bool clock = !(flux_flags & kNoTimestep);
+        const bool own_clock = clock && separate_clock(h);
+        if (own_clock)
             launch_step_clock_mixed(h->P, h->d_ctrl, h->nscen, h->M.shape.pdl, h->stream);
-        launch_update_mixed(h->M, h->S, h->X, h->P, h->d_ctrl, update_flags, stg, h->stream);
+        launch_update_mixed(h->M, h->S, h->X, h->P, h->d_ctrl, update_flags, stg,
+                            clock && !own_clock, h->d_tags, h->time_tags, h->stream);
         launch_distribute_mixed(h->M, h->S, h->X, h->P, h->d_tags, h->d_ctrl, dist_flags, stg,
                                 h->stream);
     }
@@ -204,20 +212,44 @@ static void issue_stage(Handle *h, const Stage &stg) {
 // The stages of one step of the handle's timestepping method (ANUGA's
 // evolve_one_euler_step / evolve_one_rk2_step / evolve_one_rk3_step followed
 // by the evolve loop's set_time, distribute and update_boundary).
-static void issue_step(Handle *h) {
+static int step_stages(const Handle *h, Stage (&s)[3]) {
     if (h->timestepping_method == SWGPU_RK2) {
-        issue_stage(h, Stage{kStageFirst, 1.0, 0.0, 1.0});
-        issue_stage(h, Stage{kStageLast, 0.5, 0.5, 1.0});
-    } else if (h->timestepping_method == SWGPU_RK3) {
-        issue_stage(h, Stage{kStageFirst, 1.0, 0.0, 1.0});
-        issue_stage(h, Stage{kStageMid, 0.25, 0.75, 0.5});
-        issue_stage(h, Stage{kStageLast, 2.0 / 3.0, 1.0 / 3.0, 1.0});
-    } else {
-        issue_stage(h, kEulerStage);
+        s[0] = Stage{kStageFirst, 1.0, 0.0, 1.0};
+        s[1] = Stage{kStageLast, 0.5, 0.5, 1.0};
+        return 2;
     }
+    if (h->timestepping_method == SWGPU_RK3) {
+        s[0] = Stage{kStageFirst, 1.0, 0.0, 1.0};
+        s[1] = Stage{kStageMid, 0.25, 0.75, 0.5};
+        s[2] = Stage{kStageLast, 2.0 / 3.0, 1.0 / 3.0, 1.0};
+        return 3;
+    }
+    s[0] = kEulerStage;
+    return 1;
+}
+static void issue_step(Handle *h) {
+    Stage s[3];
+    const int n = step_stages(h, s);
+    for (int i = 0; i < n; i++) issue_stage(h, s[i]);
+}
+
+// Mixed meshes small enough for the resident step (off with dependent_launch
+// off, which runs the step kernels one after the other).
+static bool use_resident(const Handle *h) { return h->resident.kernel && h->M.shape.pdl; }
+
+// At most `steps` steps in one launch of the resident step.
+static cudaError_t issue_resident(Handle *h, int steps) {
+    Stage s[3];
+    const int n = step_stages(h, s);
+    return launch_resident(h->M, h->S, h->X, h->P, h->d_tags, h->d_ctrl, h->nscen, h->resident,
+                           h->d_scen_first, steps, s, n, h->S.hmax ? kTrack : 0, h->stream);
 }
 
 static int issue_fused_step(Handle *h) {
+    if (use_resident(h)) {
+        CK(issue_resident(h, 1));
+        return SWGPU_OK;
+    }
     issue_step(h);
     return check_launch(h, "evolve step");
 }
@@ -750,6 +782,8 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     h->ntags = (int)(maxtag + 1);
     h->nscen = offsets ? nscen : 1;
     TRY(dalloc(h, &h->d_tags, (size_t)std::max(h->ntags, 1)));  // zero = reflective
+    if (precision == SWGPU_MIXED && h->nscen == 1)
+        TRY(dalloc(h, &h->X.tag_values, (size_t)std::max(h->ntags, 1)));
     TRY(dalloc(h, &h->d_ctrl, (size_t)h->nscen));
     TRY(dalloc(h, &h->d_summary, 1));
     const int nwords = (h->nscen + 31) / 32;
@@ -763,6 +797,24 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
         TRY(upload(h, h->d_blk_scen, blk.data(), (size_t)nblk));
         M.blk_scen = h->d_blk_scen;
         h->scen_offsets.assign(offsets, offsets + nscen + 1);
+    }
+    {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+        M.shape.sms = std::max(sms, 1);
+    }
+    if (precision == SWGPU_MIXED) {
+        int64_t largest = N;
+        if (offsets) {
+            largest = 0;
+            for (int i = 0; i < nscen; i++) largest = std::max(largest, offsets[i + 1] - offsets[i]);
+        }
+        h->resident = resident_shape(largest, h->nscen);
+        if (h->resident.kernel && offsets) {
+            const std::vector<int> first(offsets, offsets + nscen + 1);
+            TRY(dalloc(h, &h->d_scen_first, first.size()));
+            TRY(upload(h, h->d_scen_first, first.data(), first.size()));
+        }
     }
     {
         cudaError_t e = cudaMallocHost((void **)&h->h_ctrl, sizeof(Ctrl) * h->nscen);
@@ -780,14 +832,12 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     std::memset(h->h_ctrl, 0, sizeof(Ctrl) * h->nscen);
     std::memset(h->h_summary, 0, sizeof(RunSummary));
     {
-        int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
         // the mixed flux's tile: 256 triangles on meshes of many waves (fewer,
         // longer blocks: 0.9% faster at 4M), 128 on small ones (more blocks
         // for the latency-bound case: 3% faster at 40k)
         const int flux_tile = N >= (int64_t(1) << 20) ? 256 : 128;
         M.shape = LaunchShape{precision == SWGPU_MIXED ? flux_tile : kBlock, kBlock, kBlock, 0,
-                              std::max(sms, 1), 1};
+                              M.shape.sms, 1};
     }
     for (int i = 0; i < h->nscen; i++) {
         Ctrl *c = &h->h_ctrl[i];
@@ -862,6 +912,20 @@ int swgpu_set_boundary_tags(void *handle, const swgpu_boundary_tag *tags, int nt
         for (int j = 0; j < 8; j++) t[i].p[j] = tags[i].p[j];
     }
     const int n = std::max(h->ntags, 1);
+    // a mixed mesh's time-dependent tags are evaluated once per stage, by a
+    // block of the update (an ensemble's scenarios have clocks of their own)
+    int time_tags = 0;
+    if (h->X.tag_values)
+        for (int i = 0; i < std::min(ntags, h->ntags); i++)
+            if (t[i].type == SWGPU_BC_TIME_STAGE_SINE ||
+                t[i].type == SWGPU_BC_TIME_STAGE_FOURIER ||
+                t[i].type == SWGPU_BC_INFLOW_HYDROGRAPH)
+                time_tags = h->ntags;
+    if (time_tags != h->time_tags) {
+        CK(cudaStreamSynchronize(h->stream));
+        drop_graphs(h);  // the update's launch changes
+        h->time_tags = time_tags;
+    }
     return upload(h, h->d_tags, t.data(), (size_t)std::min(ntags, n));
 }
 
@@ -1517,14 +1581,16 @@ int swgpu_profile_steps(void *handle, int64_t nsteps, double *ms) {
         else
             launch_flux_mixed(h->M, h->S, h->X, h->P, h->d_ctrl, kFused, h->stream);
         CK(cudaEventRecord(ev[1], h->stream));
-        if (mixed) launch_step_clock_mixed(h->P, h->d_ctrl, h->nscen, h->M.shape.pdl, h->stream);
+        const bool own_clock = mixed && separate_clock(h);
+        if (own_clock)
+            launch_step_clock_mixed(h->P, h->d_ctrl, h->nscen, h->M.shape.pdl, h->stream);
         CK(cudaEventRecord(ev[2], h->stream));
         if (!mixed)
             launch_update_fp64(h->M, h->S, h->P, h->d_ctrl, 0.0, kFused | kFrictionInline,
                                kEulerStage, h->stream);
         else
             launch_update_mixed(h->M, h->S, h->X, h->P, h->d_ctrl, kFused | kFrictionInline,
-                                kEulerStage, h->stream);
+                                kEulerStage, !own_clock, h->d_tags, h->time_tags, h->stream);
         CK(cudaEventRecord(ev[3], h->stream));
         if (!mixed)
             launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl,
@@ -1554,12 +1620,16 @@ static int run_graphs(Handle *h, int64_t max_steps, swgpu_state *state, double *
     if (!h) return fail(h, SWGPU_EINVAL, "null handle");
     int rc = prepare_run(h, max_steps);
     if (rc) return rc;
-    if ((rc = build_graph(h))) return rc;
+    // the resident step's launches are bounded (a few ms each) so that the
+    // host looks in on them; the device stops itself within one
+    const bool resident = use_resident(h);
+    constexpr int kResidentSteps = 512;
+    if (!resident && (rc = build_graph(h))) return rc;
     // with a step budget the device stops itself after max_steps steps; the
     // host issues max_steps / steps-per-graph whole graphs and then the
     // remaining steps' kernels one by one (no capture for a remainder that
     // may differ between runs), so that no step is issued beyond the budget
-    const int spg = h->steps_per_graph;
+    const int spg = resident ? kResidentSteps : h->steps_per_graph;
     const int64_t full_graphs = max_steps > 0 ? max_steps / spg : INT64_MAX;
     const int tail = max_steps > 0 ? (int)(max_steps % spg) : 0;
     const int64_t max_graphs = max_steps > 0 ? full_graphs + (tail ? 1 : 0) : INT64_MAX;
@@ -1576,7 +1646,9 @@ static int run_graphs(Handle *h, int64_t max_steps, swgpu_state *state, double *
     int inflight = 0, slot = 0;
     bool halted = false;
     while (!halted && launched < max_graphs) {
-        if (launched < full_graphs) {
+        if (resident) {
+            e = issue_resident(h, launched < full_graphs ? spg : tail);
+        } else if (launched < full_graphs) {
             e = cudaGraphLaunch(h->graph, h->stream);
         } else {
             for (int s = 0; s < tail; s++) issue_step(h);
@@ -1602,7 +1674,7 @@ static int run_graphs(Handle *h, int64_t max_steps, swgpu_state *state, double *
             if (e != cudaSuccess) break;
             inflight--;
             if (h->h_summary->halted >= h->nscen || h->h_summary->status) halted = true;
-            if (!halted && h->nscen > 1) {
+            if (!halted && h->nscen > 1 && !resident) {
                 // ensembles: launch only up to the last scenario still running
                 // (longest-running scenarios are placed first) once that
                 // saves an eighth of the current launch

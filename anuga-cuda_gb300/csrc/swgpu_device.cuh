@@ -5,6 +5,7 @@
 #pragma once
 
 #include "swgpu_internal.cuh"
+#include "swgpu_soft64.cuh"
 
 namespace swgpu {
 
@@ -125,11 +126,14 @@ struct StepClock {
 __device__ __forceinline__ StepClock device_update_timestep(const Ctrl *c, const DevParams &P) {
     StepClock s;
     s.ftmin = __longlong_as_double((long long)c->ftmin_bits);
-    double dt = omin(P.CFL * s.ftmin, P.evolve_max_timestep);
+    // (comparisons as integers and the product by a CFL of 1 left out: an FP64
+    // instruction that a thread waits for takes about 100 clocks)
+    double dt = bits64(P.CFL) == 0x3ff0000000000000ull ? s.ftmin : P.CFL * s.ftmin;
+    dt = lt64(dt, P.evolve_max_timestep) ? dt : P.evolve_max_timestep;
     s.order = c->order;
     s.smallsteps = c->smallsteps;
     s.small_error = 0;
-    if (dt < P.evolve_min_timestep) {
+    if (lt64(dt, P.evolve_min_timestep)) {
         s.smallsteps += 1;
         if (s.smallsteps > P.max_smallsteps) {
             s.smallsteps = 0;
@@ -144,8 +148,12 @@ __device__ __forceinline__ StepClock device_update_timestep(const Ctrl *c, const
         s.smallsteps = 0;
         if (s.order == 1 && P.default_order == 2) s.order = 2;
     }
-    if (c->finaltime > 0 && c->time + dt > c->finaltime) dt = c->finaltime - c->time;
-    if (c->time + dt > c->yieldtime) dt = c->yieldtime - c->time;
+    double end = c->time + dt;
+    if (gt_zero(c->finaltime) && lt64(c->finaltime, end)) {
+        dt = c->finaltime - c->time;
+        end = c->time + dt;
+    }
+    if (lt64(c->yieldtime, end)) dt = c->yieldtime - c->time;
     s.dt = dt;
     return s;
 }
@@ -167,6 +175,12 @@ __device__ __forceinline__ Ctrl *block_ctrl(Ctrl *base, const DevMesh &M) {
     return M.blk_scen ? base + M.blk_scen[(blockIdx.x * blockDim.x) >> 8] : base;
 }
 
+// Whether this block's triangles are the first of their scenario.
+__device__ __forceinline__ bool first_of_scenario(const DevMesh &M) {
+    const unsigned k0 = blockIdx.x * blockDim.x;
+    return blockIdx.x == 0 || (M.blk_scen && M.blk_scen[(k0 - 1) >> 8] != M.blk_scen[k0 >> 8]);
+}
+
 // Called by thread 0 of each block after the block's work; returns true in
 // exactly one of the scenario's `blocks` blocks, the last to finish (all
 // other blocks' writes are then visible).  The counter is reset for the
@@ -185,14 +199,16 @@ __device__ __forceinline__ bool last_block_done(unsigned int *counter, unsigned 
 // Once all atomicMins of the step are done (FP64: the flux kernel's last
 // block; mixed: step_clock_mixed, after the flux grid): evaluate
 // update_timestep once and publish it for the update kernel.
-__device__ __forceinline__ void publish_step_clock(Ctrl *c, const DevParams &P) {
-    const StepClock s = device_update_timestep(c, P);
+__device__ __forceinline__ void publish_step_clock(Ctrl *c, const StepClock &s) {
     c->clk_dt = s.dt;
     c->clk_ftmin = s.ftmin;
     c->clk_order = s.order;
     c->clk_smallsteps = s.smallsteps;
     c->clk_small_error = s.small_error;
     c->clk_t0 = c->time;
+}
+__device__ __forceinline__ void publish_step_clock(Ctrl *c, const DevParams &P) {
+    publish_step_clock(c, device_update_timestep(c, P));
 }
 
 // Block-wide minimum of a positive double, then one atomicMin on its bit
@@ -346,9 +362,8 @@ __device__ __forceinline__ void track_depth(const DevState &S, int k, double h, 
 
 // Model time at the end of the step a stage belongs to, read by every
 // block before the stage is committed.
-__device__ __forceinline__ double step_end_time(const Ctrl *c, const StepClock &s,
-                                                const Stage &stg) {
-    return (stg.kind == kStageLast ? c->step_t0 : c->time) + s.dt;
+__device__ __forceinline__ double step_end_time(const Ctrl *c, double dt, const Stage &stg) {
+    return (stg.kind == kStageLast ? c->step_t0 : c->time) + dt;
 }
 
 // Last block of the distribute kernel: a pending stop takes effect.

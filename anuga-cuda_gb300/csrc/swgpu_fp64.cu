@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
         S.uh[k] = uh;
         S.vh[k] = vh;
         if ((flags & kTrack) && (stg.kind == kStageEuler || stg.kind == kStageLast))
-            track_depth(S, k, w - zc, step_end_time(ctrl, clk, stg), P.track_threshold);
+            track_depth(S, k, w - zc, step_end_time(ctrl, clk.dt, stg), P.track_threshold);
     }
     if (bad) set_status(ctrl, SWGPU_EDENOMINATOR);
     if (nonfinite) set_status(ctrl, SWGPU_ENONFINITE);

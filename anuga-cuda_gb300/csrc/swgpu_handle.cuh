@@ -23,12 +23,15 @@ struct Handle {
     DevParams P{};
     BcTag *d_tags = nullptr;
     int ntags = 0;
+    int time_tags = 0;           // mixed: tags evaluated once per stage (0: none depends on time)
     int steps_per_graph = kStepsPerGraph;
     float *trk_hmax = nullptr, *trk_tarr = nullptr;  // tracking buffers (S.hmax/S.tarr when on)
     int nscen = 1;               // scenarios (Ctrl blocks); > 1 for an ensemble
     std::vector<int64_t> scen_offsets;  // ensemble: first triangle of each scenario, + N
     std::vector<int64_t> scen_edges;    // FP64: first edge of each scenario, + the edge count
     int *d_blk_scen = nullptr;   // ensemble: scenario of each 256-triangle block
+    Resident resident{0, 0};     // mixed: shape of the resident step (kernel 0: too large)
+    int *d_scen_first = nullptr; // ensemble: first triangle of each scenario, + N
     Ctrl *d_ctrl = nullptr;      // [nscen]
     Ctrl *h_ctrl = nullptr;      // pinned mirror [nscen]
     RunSummary *d_summary = nullptr;

@@ -105,6 +105,12 @@ struct DevState {
                                               // depth in the mixed precision)
 };
 
+// The part of a time-dependent boundary tag's value that all its edges share:
+// the stage, or a hydrograph's unit discharge and critical depth.
+struct TagValue {
+    double a, b;
+};
+
 // Mixed-precision state.  The conserved state is FP64 depth h = w - z (so
 // depth at wet/dry fronts never comes from a difference of two large
 // stages) and FP64 momentum.  Everything the flux, limiter and
@@ -138,6 +144,8 @@ struct DevMixed {
                                    // vertex) minus bed centroid, z/w bed centroid as an
                                    // FP32 pair hi + lo
 
+    TagValue *tag_values;          // [tags] time-dependent boundaries at the stage's end (null:
+                                   // evaluated edge by edge, as for an ensemble's many clocks)
     int *surrp;                    // [3][S] DevMesh::surr in padded planes (TMA-staged)
     uint8_t *kind;                 // [S] 0 aux triangle, 1 one neighbour (slot<<2), 2 flat;
                                    // | 16: the triangle has a boundary edge
@@ -302,7 +310,19 @@ void launch_step_clock_mixed(const DevParams &P, Ctrl *ctrl, int nscen, bool pdl
                              cudaStream_t st);
 void launch_update_mixed(const DevMesh &M, const DevState &S, const DevMixed &X,
                          const DevParams &P, Ctrl *ctrl, int flags, const Stage &stage,
-                         cudaStream_t st);
+                         bool clock, const BcTag *tags, int ntags, cudaStream_t st);
+// Whole steps of meshes that a thread-block cluster holds, in one launch
+// (steps_resident): the shape for nscen scenarios of up to `largest` triangles
+// (kernel 0: they don't fit), and a launch of at most `steps` steps.  The
+// device stops by itself as in the step kernels.
+struct Resident {
+    int kernel, cluster;
+};
+Resident resident_shape(int64_t largest, int nscen);
+cudaError_t launch_resident(const DevMesh &M, const DevState &S, const DevMixed &X,
+                            const DevParams &P, const BcTag *tags, Ctrl *ctrl, int nscen,
+                            const Resident &shape, const int *scen_first, int steps,
+                            const Stage *stages, int nstages, int flags, cudaStream_t st);
 // stand-alone distribute head: (optionally) depth from the FP64 stage, then
 // protect and the FP32 centroid copies
 void launch_prepare_mixed(const DevMesh &M, const DevState &S, const DevMixed &X,

@@ -337,59 +337,42 @@ __device__ __forceinline__ void flux_tile_issue(const DevMixed &X, FluxTile<TILE
     flux_tile_issue_dynamic<TILE>(X, T, k0, span, bar);
 }
 
-// Fluxes + gravity_wb of triangle k0 + tid of a staged tile (cnt valid
-// triangles); stores the explicit updates and returns the triangle's CFL
-// timestep bound.
-template <int TILE>
-__device__ __forceinline__ float flux_tile_triangle(const DevMixed &X, const DevParams &P,
-                                                    const FluxTile<TILE> &T, int k0, int cnt) {
-    const int SP = X.S;
-    const int tid = threadIdx.x;
-    const int k = k0 + tid;
+// Fluxes + gravity_wb of one triangle: its own data and its neighbours'
+// through the view v (a staged tile, or the resident step's block); returns
+// the explicit updates and the triangle's CFL timestep bound.
+template <typename View>
+__device__ __forceinline__ float flux_triangle(const View &v, const DevParams &P, float2 &ewu,
+                                               float &evh) {
     float t = P.f_max_dt;
     const float eps = P.f_eps;
-    const float2 wsk = T.ws[tid];
+    const float2 wsk = v.ws();
     const float wk = wsk.x, lk = wsk.y;
-    const float rk = T.rad[tid].x;
+    const float rk = v.rad().x;
     float a0 = 0.f, a1 = 0.f, a2 = 0.f;  // flux sums
     float gx = 0.f, gy = 0.f;            // Green sum of edge stage jumps
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        const float2 nr = T.nrm[i][tid];
-        const int2 lq = T.lnb[i][tid];
+        const float2 nr = v.nrm(i);
+        const int2 lq = v.lnb(i);
         const float n1 = nr.x, n2 = nr.y, L = __int_as_float(lq.x);
-        const float4 el = T.es[i][tid];
+        const float4 el = v.es(i);
         const float hl = el.x, dwl = el.y, uhl = el.z, vhl = el.w;
         float hr, uhr, vhr, jump;
         const int pki = lq.y;
         if (pki >= 0) {
             // the neighbour's stored edge state: the very numbers it uses
             // itself, so both sides see the same two states
-            const int n = pki >> 2, m = pki & 3;
-            const int ln = n - k0;
-            float wn, lnn, dwn;
             float4 en;
             float2 wsn;
-            if ((unsigned)ln < (unsigned)cnt) {
-                en = T.es[m][ln];
-                wsn = T.ws[ln];
-            } else {
-                en = ro(X.es + m * SP + n);
-                wsn = ro(X.ws + n);
-            }
-            wn = wsn.x;
-            lnn = wsn.y;
+            v.far(pki, en, wsn);
+            const float wn = wsn.x, lnn = wsn.y;
             hr = en.x;
-            dwn = en.y;
+            const float dwn = en.y;
             uhr = en.z;
             vhr = en.w;
             jump = ((wn - wk) + (lnn - lk)) + (dwn - dwl);
         } else {
-            const int mb = -pki - 1;
-            hr = ro(X.hbf + mb);
-            jump = ro(X.wjb + mb);
-            uhr = ro(X.uhbf + mb);
-            vhr = ro(X.vhbf + mb);
+            v.boundary(-pki - 1, hr, jump, uhr, vhr);
         }
         gx += dwl * L * n1;
         gy += dwl * L * n2;
@@ -407,10 +390,56 @@ __device__ __forceinline__ float flux_tile_triangle(const DevMixed &X, const Dev
         // minimum without the neighbour's radius being read.
         if (ms > eps) t = ominf(t, __fdividef(rk, ms));
     }
-    const float ghc = P.f_g * T.hf[tid];
-    const float inv_area = T.rad[tid].y;
-    X.ewu[k] = make_float2(a0 * inv_area, (a1 - ghc * gx) * inv_area);
-    X.evh[k] = (a2 - ghc * gy) * inv_area;
+    const float ghc = P.f_g * v.hf();
+    const float inv_area = v.rad().y;
+    ewu = make_float2(a0 * inv_area, (a1 - ghc * gx) * inv_area);
+    evh = (a2 - ghc * gy) * inv_area;
+    return t;
+}
+
+// Triangle k0 + threadIdx.x of a staged tile of cnt triangles.
+template <int TILE>
+struct TileView {
+    const DevMixed &X;
+    const FluxTile<TILE> &T;
+    int k0, cnt;
+    __device__ float2 ws() const { return T.ws[threadIdx.x]; }
+    __device__ float hf() const { return T.hf[threadIdx.x]; }
+    __device__ float2 rad() const { return T.rad[threadIdx.x]; }
+    __device__ float2 nrm(int i) const { return T.nrm[i][threadIdx.x]; }
+    __device__ int2 lnb(int i) const { return T.lnb[i][threadIdx.x]; }
+    __device__ float4 es(int i) const { return T.es[i][threadIdx.x]; }
+    __device__ void far(int pki, float4 &en, float2 &wsn) const {
+        const int n = pki >> 2, m = pki & 3;
+        const int ln = n - k0;
+        if ((unsigned)ln < (unsigned)cnt) {
+            en = T.es[m][ln];
+            wsn = T.ws[ln];
+        } else {
+            en = ro(X.es + m * X.S + n);
+            wsn = ro(X.ws + n);
+        }
+    }
+    __device__ void boundary(int mb, float &hr, float &jump, float &uhr, float &vhr) const {
+        hr = ro(X.hbf + mb);
+        jump = ro(X.wjb + mb);
+        uhr = ro(X.uhbf + mb);
+        vhr = ro(X.vhbf + mb);
+    }
+};
+
+// Fluxes of triangle k0 + tid of a staged tile (cnt valid triangles); stores
+// the explicit updates and returns the triangle's CFL timestep bound.
+template <int TILE>
+__device__ __forceinline__ float flux_tile_triangle(const DevMixed &X, const DevParams &P,
+                                                    const FluxTile<TILE> &T, int k0, int cnt) {
+    const int k = k0 + threadIdx.x;
+    float2 ewu;
+    float evh;
+    const TileView<TILE> v{X, T, k0, cnt};
+    const float t = flux_triangle(v, P, ewu, evh);
+    X.ewu[k] = ewu;
+    X.evh[k] = evh;
     return t;
 }
 
@@ -568,26 +597,117 @@ __device__ __forceinline__ void finish_state(const DevParams &P, double &h, doub
     vvel = vhf * inv;
 }
 
+constexpr int kTimeTags = 6;  // time-dependent boundary tags of one block
+__device__ __forceinline__ bool time_dependent(int type) {
+    return type == SWGPU_BC_TIME_STAGE_SINE || type == SWGPU_BC_TIME_STAGE_FOURIER ||
+           type == SWGPU_BC_INFLOW_HYDROGRAPH;
+}
+// The model time that a stage's distribute evaluates the boundaries at.
+__device__ __forceinline__ double stage_end_time(const Ctrl *c, const Stage &stg) {
+    return c->clk_t0 + c->clk_dt * (stg.kind == kStageMid ? stg.tfrac : 1.0);
+}
+// The part of a time-dependent boundary that is the same for all of a tag's
+// edges (eval_boundary's own expressions).
+__device__ __noinline__ bool tag_value(const BcTag &T, double time, double g, TagValue &v) {
+    if (T.type == SWGPU_BC_INFLOW_HYDROGRAPH) {
+        const double q = hydrograph(T.p, time);
+        v.a = q;
+        v.b = cbrt(q * q / g);
+        return true;
+    }
+    if (time_dependent(T.type)) {
+        double u, w;
+        eval_boundary(T, time, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, g, v.a, u, w);
+        v.b = 0.0;
+        return true;
+    }
+    return false;
+}
+
 // Update: h += dt*E_h;  q += q*(r - 1) + dt*E_q*r  with r = 1/(1 - dt*S) the
 // semi-implicit Manning factor.  Increments in FP32, additions in FP64.
-template <int BS>
-__global__ void __launch_bounds__(BS, 2048 / BS) update_mixed(DevMesh M, DevState S, DevMixed X,
-                                                       DevParams P, Ctrl *ctrl, int flags,
-                                                       Stage stg) {
+// eta: Manning n, zmoff: mean bed vertex minus bed centroid; hf0, uv0, vv0
+// the FP32 depth and velocities of the state before.
+__device__ __forceinline__ void update_triangle(const DevParams &P, float dtf, float eta,
+                                                float zmoff, float hf0, float uv0, float vv0,
+                                                float ew, float euh, float evh, double &h,
+                                                double &uh, double &vh, int &bad) {
+    const float mah = P.f_mah;
+    const float uf = uv0 * omaxf(hf0, mah);
+    const float vf = vv0 * omaxf(hf0, mah);
+    float rm1 = 0.0f, r = 1.0f;  // r - 1 and r
+    if (eta > mah) {
+        const float hm = hf0 - zmoff;
+        if (hm >= mah) {
+            const float Sf = -P.f_g * eta * eta * sqrtf(uf * uf + vf * vf) *
+                             exp2f(-(7.0f / 3.0f) * __log2f(hm));
+            const float dS = dtf * Sf;  // <= 0
+            const float den = 1.0f - dS;
+            if (!(den > 0.0f)) bad = 1;
+            r = __fdividef(1.0f, den);
+            rm1 = dS * r;  // r - 1 without cancellation
+        }
+    }
+    h += widen(dtf * ew);
+    uh += widen(uf * rm1 + dtf * euh * r);
+    vh += widen(vf * rm1 + dtf * evh * r);
+}
+
+// saxpy_conserved_quantities in FP64 on depth: with a + b = 1 it is the stage
+// saxpy minus the (unchanged) bed.
+__device__ __forceinline__ void combine_stage(const Stage &stg, double bh, double bu, double bv,
+                                              double &h, double &uh, double &vh) {
+    h = fma(stg.b, bh, stg.a * h);
+    uh = fma(stg.b, bu, stg.a * uh);
+    vh = fma(stg.b, bv, stg.a * vh);
+}
+
+// CLOCK: the step's clock is evaluated here, by every block for itself and
+// published by the first, instead of by step_clock_mixed: one launch less (of
+// about 2.5 us) for an evaluation per block, which a mesh of many waves of
+// blocks would rather not repeat.  TAGS: the launch has one more block, which
+// evaluates the time-dependent boundary tags at the stage's end for the
+// distribute (a sine and a quotient in FP64, 6 us at the end of a block of the
+// distribute).
+template <bool CLOCK, bool TAGS>
+__device__ __forceinline__ void update_body(const DevMesh &M, const DevState &S, const DevMixed &X,
+                                            const DevParams &P, Ctrl *ctrl, int flags,
+                                            const Stage &stg, const BcTag *tags, int ntags) {
     pdl_launch_dependents();
-    ctrl = block_ctrl(ctrl, M);
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = k < M.N;
+    const bool tag_block = TAGS && blockIdx.x == gridDim.x - 1;
+    if (!tag_block) ctrl = block_ctrl(ctrl, M);
+    const bool in = k < M.N && !tag_block;
     // static per-triangle data before the previous kernel has finished
     const float4 us = in ? ro(X.ust + k) : make_float4(0.f, 0.f, 0.f, 0.f);
     const float eta = us.x, zmoff = us.y, zhi = us.z, zlo = us.w;
     pdl_wait();
     // a stopped scenario's threads load nothing more (the flag is settled:
-    // only the step clock kernel and the distribute change it)
-    if ((flags & kFused) && ctrl_halt_settled(ctrl)) return;
+    // only the step's clock and the distribute change it)
+    if ((flags & kFused) && ctrl_halt_settled(ctrl)) {
+        if (CLOCK && threadIdx.x == 0 && first_of_scenario(M) && ctrl->halt == 2)
+            ctrl->halt = 1;  // the last step's distribute has run
+        return;
+    }
+    __shared__ double block_dt;
+    if (CLOCK) {
+        if (threadIdx.x == 0) {
+            const StepClock c = device_update_timestep(ctrl, P);
+            block_dt = c.dt;
+            if (first_of_scenario(M) && !tag_block) publish_step_clock(ctrl, c);
+        }
+    }
+    if (tag_block) {
+        if (CLOCK) __syncthreads();
+        const double dt = CLOCK ? block_dt : ctrl->clk_dt;
+        const double time = (CLOCK ? ctrl->time : ctrl->clk_t0) +
+                            dt * (stg.kind == kStageMid ? stg.tfrac : 1.0);
+        for (int i = threadIdx.x; i < ntags; i += blockDim.x)
+            tag_value(tags[i], time, P.g, X.tag_values[i]);
+        return;
+    }
     // every load first, the control block's with them (this thread is the
     // only writer of element k)
-    const StepClock clk = published_step_clock(ctrl);
     const int kk = in ? k : 0;
     const double h0 = ro(X.hd + kk), uh0 = ro(S.uh + kk), vh0 = ro(S.vh + kk);
     const bool combine = stg.kind == kStageMid || stg.kind == kStageLast;
@@ -602,36 +722,14 @@ __global__ void __launch_bounds__(BS, 2048 / BS) update_mixed(DevMesh M, DevStat
     const float uv0 = vel0.x, vv0 = vel0.y;
     const float2 ewu = ro(X.ewu + kk);
     const float ew = ewu.x, euh = ewu.y, evh = ro(X.evh + kk);
-    const float dtf = (float)clk.dt;
+    if (CLOCK) __syncthreads();
+    const double dt = CLOCK ? block_dt : ctrl->clk_dt;
+    const float dtf = (float)dt;
     int bad = 0, nonfinite = 0;
     if (in) {
         double h = h0, uh = uh0, vh = vh0;
-        const float mah = P.f_mah;
-        const float uf = uv0 * omaxf(hf0, mah);
-        const float vf = vv0 * omaxf(hf0, mah);
-        float rm1 = 0.0f, r = 1.0f;  // r - 1 and r
-        if (eta > mah) {
-            const float hm = hf0 - zmoff;
-            if (hm >= mah) {
-                const float Sf = -P.f_g * eta * eta * sqrtf(uf * uf + vf * vf) *
-                                 exp2f(-(7.0f / 3.0f) * __log2f(hm));
-                const float dS = dtf * Sf;  // <= 0
-                const float den = 1.0f - dS;
-                if (!(den > 0.0f)) bad = 1;
-                r = __fdividef(1.0f, den);
-                rm1 = dS * r;  // r - 1 without cancellation
-            }
-        }
-        h += widen(dtf * ew);
-        uh += widen(uf * rm1 + dtf * euh * r);
-        vh += widen(vf * rm1 + dtf * evh * r);
-        if (combine) {
-            // saxpy_conserved_quantities in FP64 on depth: with a + b = 1 it
-            // is the stage saxpy minus the (unchanged) bed
-            h = stg.a * h + stg.b * bh;
-            uh = stg.a * uh + stg.b * bu;
-            vh = stg.a * vh + stg.b * bv;
-        }
+        update_triangle(P, dtf, eta, zmoff, hf0, uv0, vv0, ew, euh, evh, h, uh, vh, bad);
+        if (combine) combine_stage(stg, bh, bu, bv, h, uh, vh);
         float hf, wf, wl, uv, vv;
         finish_state(P, h, uh, vh, zhi, zlo, hf, wf, wl, uv, vv, nonfinite);
         if (stg.kind == kStageFirst) {  // backup_conserved_quantities (depth, momenta)
@@ -646,13 +744,27 @@ __global__ void __launch_bounds__(BS, 2048 / BS) update_mixed(DevMesh M, DevStat
         X.ws[k] = make_float2(wf, wl);
         X.vel[k] = make_float2(uv, vv);
         if ((flags & kTrack) && (stg.kind == kStageEuler || stg.kind == kStageLast))
-            track_depth(S, k, h, step_end_time(ctrl, clk, stg), P.track_threshold);
+            track_depth(S, k, h, step_end_time(ctrl, dt, stg), P.track_threshold);
     }
     // the stage is committed by the distribute (its scenario's first block)
     if (bad) set_status(ctrl, SWGPU_EDENOMINATOR);
     if (nonfinite) set_status(ctrl, SWGPU_ENONFINITE);
 }
 
+template <int BS, bool CLOCK>
+__global__ void __launch_bounds__(BS, 2048 / BS) update_mixed(DevMesh M, DevState S, DevMixed X,
+                                                       DevParams P, Ctrl *ctrl, int flags,
+                                                       Stage stg) {
+    update_body<CLOCK, false>(M, S, X, P, ctrl, flags, stg, nullptr, 0);
+}
+// (apart, so that the evaluation's call costs meshes without such tags nothing)
+template <int BS, bool CLOCK>
+__global__ void __launch_bounds__(BS, 2048 / BS) update_with_tags(DevMesh M, DevState S, DevMixed X,
+                                                           DevParams P, Ctrl *ctrl, int flags,
+                                                           Stage stg, const BcTag *tags,
+                                                           int ntags) {
+    update_body<CLOCK, true>(M, S, X, P, ctrl, flags, stg, tags, ntags);
+}
 
 __device__ __forceinline__ void qminmax_f(float dq0, float dq1, float dq2, float &qmin,
                                           float &qmax) {
@@ -726,29 +838,55 @@ __device__ __forceinline__ void one_jumps_f(float dq1, const C &c, float beta,
 }
 
 // Boundary values (evaluate_segment, per boundary type) of triangle k's
-// boundary edges from the edge values this thread has just stored.  Out of
+// boundary edges from the edge values this thread has just stored at es[i *
+// es_stride].  values: those of the time-dependent tags `known`, or of every
+// tag (known null), evaluated before; null: none are.  Out of
 // line: boundary triangles are rare, and the FP64 evaluation inlined would
 // raise the register pressure of every thread of the distribute.  Returns 1
 // when an edge's boundary could not be evaluated.
 __device__ __noinline__ int boundary_edges_mixed(int k, int N, int SP, double time, double g,
                                                  const int *nbr, const int *btag,
                                                  const BcTag *tags, const double *ze_,
-                                                 const float4 *es, const float2 *nrm,
+                                                 const float4 *es, int es_stride,
+                                                 const float2 *nrm,
                                                  double *wb_, double *uhb_,
                                                  double *vhb_, double *zb_, float *hbf,
-                                                 float *wjb, float *uhbf, float *vhbf) {
+                                                 float *wjb, float *uhbf, float *vhbf,
+                                                 const int *known, const TagValue *values,
+                                                 int nknown) {
     int bad = 0;
-    for (int i = 0; i < 3; i++) {
-        const int pk = ro(nbr + i * N + k);
-        if (pk >= 0) continue;
-        const int mb = -pk - 1;
-        const float4 e = es[i * SP + k];  // this thread's own stores: a plain load
+    const int pk3[3] = {ro(nbr + k), ro(nbr + N + k), ro(nbr + 2 * N + k)};
+    // a pass per boundary edge that a triangle has (one, at corners two), not
+    // per edge: the lanes of a warp have theirs at different places
+    unsigned left = (pk3[0] < 0 ? 1u : 0u) | (pk3[1] < 0 ? 2u : 0u) | (pk3[2] < 0 ? 4u : 0u);
+    while (left) {
+        const int i = __ffs(left) - 1;
+        left &= left - 1;
+        const int mb = -(i == 0 ? pk3[0] : (i == 1 ? pk3[1] : pk3[2])) - 1;
+        const float4 e = es[i * es_stride];  // this thread's own stores: a plain load
         const float hle = e.x;
         const double ze = ro(ze_ + i * N + k);
         const double we = ze + widen(hle);
-        const BcTag &T = tags[ro(btag + mb)];
+        const int tag = ro(btag + mb);
+        const BcTag &T = tags[tag];
         double wb, uhb, vhb;
-        if (!eval_boundary(T, time, we, widen(e.z), widen(e.w),
+        int have = -1;
+        if (known) {
+            for (int j = 0; j < nknown; j++)
+                if (known[j] == tag) have = j;
+        } else if (values && time_dependent(T.type)) {
+            have = tag;
+        }
+        if (have >= 0) {
+            const TagValue &tv = values[have];
+            wb = tv.a;
+            uhb = vhb = 0.0;
+            if (T.type == SWGPU_BC_INFLOW_HYDROGRAPH) {
+                wb = omax(we, ze + tv.b);
+                uhb = -tv.a * widen(ro(nrm + i * SP + k).x);
+                vhb = -tv.a * widen(ro(nrm + i * SP + k).y);
+            }
+        } else if (!eval_boundary(T, time, we, widen(e.z), widen(e.w),
                            widen(ro(nrm + i * SP + k).x), widen(ro(nrm + i * SP + k).y), ze, g,
                            wb, uhb,
                            vhb)) {
@@ -796,6 +934,204 @@ __device__ __forceinline__ V tile_or_global(const V *tile, const V *plane, int n
     const int ln = n - kb;
     return (unsigned)ln < (unsigned)cnt ? tile[ln] : ro(plane + n);
 }
+
+// Extrapolation and balance of one triangle, FP32, in stage jumps: its own
+// data and its surrogate neighbours' centroids through the view v, which
+// takes the new edge state.  kind: DevMixed::kind.
+template <typename View>
+__device__ __forceinline__ void distribute_triangle(const View &v, const DevParams &P, int order,
+                                                    int kind) {
+    const float mah = P.f_mah;
+    const float2 wsk = v.ws(), velk = v.vel();
+    const float wk = wsk.x, lk = wsk.y, hc = v.hf();
+    const float qu = velk.x, qv = velk.y;
+    const bool vel = P.extrapolate_velocity_second_order == 1;
+    const float hk = omaxf(hc, mah);
+    const float uk = qu * hk, vk = qv * hk;  // centroid momentum
+    float dw[3] = {0.f, 0.f, 0.f};  // vertex stage jumps
+    float ou[3], ov[3];             // vertex momentum (or velocity)
+    if (order != 1) {
+        const float cu = vel ? qu : uk, cv = vel ? qv : vk;
+        float du[3] = {0.f, 0.f, 0.f}, dv[3] = {0.f, 0.f, 0.f};
+        bool keep = false;  // dry neighbourhood: previous vertex values stay
+        if ((kind & 3) != 2) {
+            // reconstruction coefficients, read from the tile at each use
+            const auto c = [&](int j) {
+                const float2 g = v.gc(j >> 1);
+                return (j & 1) ? g.y : g.x;
+            };
+            if ((kind & 3) == 0) {
+                const int k0 = v.sur(0), k1 = v.sur(1), k2 = v.sur(2);
+                const float h0 = v.near_hf(k0);
+                const float h1 = v.near_hf(k1);
+                const float h2 = v.near_hf(k2);
+                const float hmin = ominf(ominf(h0, ominf(h1, h2)), hc);
+                const float hmax = omaxf(h0, omaxf(h1, h2));
+                if (P.optimise_dry_cells && hmax < P.f_eps) {
+                    keep = true;
+                } else {
+                    float hfactor = 0.0f;
+                    if (hmin > 0.001f) hfactor = (hmin - 0.001f) / (hmin + 0.004f);
+                    const float2 s0 = v.near_ws(k0);
+                    const float2 s1 = v.near_ws(k1);
+                    const float2 s2 = v.near_ws(k2);
+                    const float w0 = s0.x, w1 = s1.x, w2 = s2.x;
+                    const float l0 = s0.y, l1 = s1.y, l2 = s2.y;
+                    aux_jumps_f((w0 - wk) + (l0 - lk), (w1 - w0) + (l1 - l0), (w2 - w0) + (l2 - l0), c,
+                                P.f_beta_w_dry + (P.f_beta_w - P.f_beta_w_dry) * hfactor, dw);
+                    const float2 q0 = v.near_vel(k0);
+                    const float2 q1 = v.near_vel(k1);
+                    const float2 q2 = v.near_vel(k2);
+                    float u0 = q0.x, u1 = q1.x, u2 = q2.x;
+                    float v0 = q0.y, v1 = q1.y, v2 = q2.y;
+                    if (!vel) {
+                        u0 *= omaxf(h0, mah);
+                        v0 *= omaxf(h0, mah);
+                        u1 *= omaxf(h1, mah);
+                        v1 *= omaxf(h1, mah);
+                        u2 *= omaxf(h2, mah);
+                        v2 *= omaxf(h2, mah);
+                    }
+                    aux_jumps_f(u0 - cu, u1 - u0, u2 - u0, c,
+                                P.f_beta_uh_dry + (P.f_beta_uh - P.f_beta_uh_dry) * hfactor, du);
+                    aux_jumps_f(v0 - cv, v1 - v0, v2 - v0, c,
+                                P.f_beta_vh_dry + (P.f_beta_vh - P.f_beta_vh_dry) * hfactor, dv);
+                }
+            } else {
+                const int slot = (kind >> 2) & 3;
+                const int k1 = v.sur(slot);
+                const float h1 = v.near_hf(k1);
+                const float beta = P.f_beta_w;
+                const float2 s1 = v.near_ws(k1);
+                one_jumps_f((s1.x - wk) + (s1.y - lk),
+                            c, beta, dw);
+                const float2 q1 = v.near_vel(k1);
+                float u1 = q1.x, v1 = q1.y;
+                if (!vel) {
+                    u1 *= omaxf(h1, mah);
+                    v1 *= omaxf(h1, mah);
+                }
+                one_jumps_f(u1 - cu, c, beta, du);
+                one_jumps_f(v1 - cv, c, beta, dv);
+            }
+        }
+        if (keep) {
+            // previous vertex values, from the stored edge values of the
+            // (linear) reconstruction: v_i = e_a + e_b - e_i
+            float e0[3], e1[3], e2[3];
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const float4 e = v.es(i);  // before it is replaced
+                e0[i] = e.y;
+                e1[i] = e.z;
+                e2[i] = e.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const int a = (i == 0) ? 1 : 0, b = (i == 2) ? 1 : 2;
+                dw[i] = (e0[a] + e0[b]) - e0[i];
+                ou[i] = (e1[a] + e1[b]) - e1[i];
+                ov[i] = (e2[a] + e2[b]) - e2[i];
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                ou[i] = cu + du[i];
+                ov[i] = cv + dv[i];
+            }
+        }
+        if (vel) {
+            // velocity -> momentum with the vertex depth hc + dw - dzv
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const float d = omaxf((hc + dw[i]) - v.dzv(i), 0.0f);
+                ou[i] *= d;
+                ov[i] *= d;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            ou[i] = uk;
+            ov[i] = vk;
+        }
+    }
+    // balance_deep_and_shallow (shallow_water_ext.c:1462-1636) with vertex
+    // depth h_i = hc + (dw_i - dzv_i); the blend keeps the form
+    // dw_i <- alpha*(dw_i - dzv_i) + dzv_i
+    {
+        // the bed offsets at the vertices, read from the tile here rather
+        // than held in registers through the reconstruction
+        float dzv[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) dzv[i] = v.dzv(i);
+        float rel[3];  // h_i - hc
+#pragma unroll
+        for (int i = 0; i < 3; i++) rel[i] = dw[i] - dzv[i];
+        const float hmin = hc + ominf(rel[0], ominf(rel[1], rel[2]));
+        float alpha = 1.0f;
+        if (P.tight_slope_limiters == 0) {
+            float dz = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 3; i++) dz = omaxf(dz, fabsf(dzv[i]));
+            alpha = dz > 0.0f ? omaxf(ominf(P.f_alpha * hmin / dz, 1.0f), 0.0f) : 1.0f;
+        } else if (hmin < P.f_H0) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const float hd = -rel[i];
+                if (!(hd <= 0.0f)) alpha = ominf(alpha, (hc - P.f_H0) / hd);
+            }
+            alpha = fminf(fmaxf(alpha, 0.0f), 1.0f);
+        }
+        if (alpha < 1.0f) {
+            const float uc = hc > 1.0e-6f ? uk / hc : 0.0f;
+            const float vc = hc > 1.0e-6f ? vk / hc : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const float r = alpha * rel[i];
+                dw[i] = r + dzv[i];
+                if (P.use_centroid_velocities == 1) {
+                    ou[i] = uc * (hc + r);
+                    ov[i] = vc * (hc + r);
+                } else {
+                    ou[i] = (1.0f - alpha) * uk + alpha * ou[i];
+                    ov[i] = (1.0f - alpha) * vk + alpha * ov[i];
+                }
+            }
+        }
+    }
+    // edge values (quantity.c:687-706 interpolation) stored for the flux:
+    // depth, stage jump from the centroid, momentum
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int a = (i == 0) ? 1 : 0, b = (i == 2) ? 1 : 2;
+        v.put_es(i, make_float4(edge_depth(hc, dw[a], dw[b], v.dze(i)),
+                                       0.5f * (dw[a] + dw[b]), 0.5f * (ou[a] + ou[b]),
+                                       0.5f * (ov[a] + ov[b])));
+    }
+}
+
+// Triangle kb + threadIdx.x of a staged tile of cnt triangles.
+template <int BS>
+struct DistView {
+    const DevMixed &X;
+    const DistTile<BS> &T;
+    int kb, cnt, tid;
+    __device__ float2 ws() const { return T.ws[tid]; }
+    __device__ float hf() const { return T.hf[tid]; }
+    __device__ float2 vel() const { return T.vel[tid]; }
+    __device__ float2 gc(int i) const { return T.gc[i][tid]; }
+    __device__ float dzv(int i) const { return T.dzv[i][tid]; }
+    __device__ float dze(int i) const { return T.dze[i][tid]; }
+    __device__ int sur(int i) const { return T.sur[i][tid]; }
+    __device__ float near_hf(int n) const { return tile_or_global(T.hf, X.hf, n, kb, cnt); }
+    __device__ float2 near_ws(int n) const { return tile_or_global(T.ws, X.ws, n, kb, cnt); }
+    __device__ float2 near_vel(int n) const { return tile_or_global(T.vel, X.vel, n, kb, cnt); }
+    __device__ float4 es(int i) const { return X.es[i * X.S + kb + tid]; }
+    __device__ void put_es(int i, const float4 &e) const {
+        X.es[i * X.S + kb + tid] = e;
+    }
+};
 
 // Extrapolation + balance + boundary conditions, FP32, in stage jumps.  Each
 // block stages its tile's own planes with one-dimensional TMA bulk copies
@@ -865,8 +1201,7 @@ __global__ void __launch_bounds__(BS, 2048 / BS) distribute_mixed(DevMesh M, Dev
         order = (int)ctrl->clk_order;
         // the first block of each scenario (thread 0 alone reads the map)
         if (tid == 0 && !halted &&
-            (blockIdx.x == 0 ||
-             (M.blk_scen && M.blk_scen[(kb - 1) >> 8] != M.blk_scen[kb >> 8]))) {
+            first_of_scenario(M)) {
             commit_stage(ctrl, published_step_clock(ctrl), P, stg);
             announce_halt(ctrl);
         }
@@ -878,185 +1213,18 @@ __global__ void __launch_bounds__(BS, 2048 / BS) distribute_mixed(DevMesh M, Dev
     int bad_bc = 0;
     if (arrived && tid < cnt) {
         const int kind = T.kind[tid];
-        const float mah = P.f_mah;
-        const float2 wsk = T.ws[tid], velk = T.vel[tid];
-        const float wk = wsk.x, lk = wsk.y, hc = T.hf[tid];
-        const float qu = velk.x, qv = velk.y;
-        const bool vel = P.extrapolate_velocity_second_order == 1;
-        const float hk = omaxf(hc, mah);
-        const float uk = qu * hk, vk = qv * hk;  // centroid momentum
-        float dw[3] = {0.f, 0.f, 0.f};  // vertex stage jumps
-        float ou[3], ov[3];             // vertex momentum (or velocity)
-        if (order != 1) {
-            const float cu = vel ? qu : uk, cv = vel ? qv : vk;
-            float du[3] = {0.f, 0.f, 0.f}, dv[3] = {0.f, 0.f, 0.f};
-            bool keep = false;  // dry neighbourhood: previous vertex values stay
-            if ((kind & 3) != 2) {
-                // reconstruction coefficients, read from the tile at each use
-                const auto c = [&](int j) {
-                    const float2 g = T.gc[j >> 1][tid];
-                    return (j & 1) ? g.y : g.x;
-                };
-                if ((kind & 3) == 0) {
-                    const int k0 = T.sur[0][tid], k1 = T.sur[1][tid], k2 = T.sur[2][tid];
-                    const float h0 = tile_or_global(T.hf, X.hf, k0, kb, cnt);
-                    const float h1 = tile_or_global(T.hf, X.hf, k1, kb, cnt);
-                    const float h2 = tile_or_global(T.hf, X.hf, k2, kb, cnt);
-                    const float hmin = ominf(ominf(h0, ominf(h1, h2)), hc);
-                    const float hmax = omaxf(h0, omaxf(h1, h2));
-                    if (P.optimise_dry_cells && hmax < P.f_eps) {
-                        keep = true;
-                    } else {
-                        float hfactor = 0.0f;
-                        if (hmin > 0.001f) hfactor = (hmin - 0.001f) / (hmin + 0.004f);
-                        const float2 s0 = tile_or_global(T.ws, X.ws, k0, kb, cnt);
-                        const float2 s1 = tile_or_global(T.ws, X.ws, k1, kb, cnt);
-                        const float2 s2 = tile_or_global(T.ws, X.ws, k2, kb, cnt);
-                        const float w0 = s0.x, w1 = s1.x, w2 = s2.x;
-                        const float l0 = s0.y, l1 = s1.y, l2 = s2.y;
-                        aux_jumps_f((w0 - wk) + (l0 - lk), (w1 - w0) + (l1 - l0), (w2 - w0) + (l2 - l0), c,
-                                    P.f_beta_w_dry + (P.f_beta_w - P.f_beta_w_dry) * hfactor, dw);
-                        const float2 q0 = tile_or_global(T.vel, X.vel, k0, kb, cnt);
-                        const float2 q1 = tile_or_global(T.vel, X.vel, k1, kb, cnt);
-                        const float2 q2 = tile_or_global(T.vel, X.vel, k2, kb, cnt);
-                        float u0 = q0.x, u1 = q1.x, u2 = q2.x;
-                        float v0 = q0.y, v1 = q1.y, v2 = q2.y;
-                        if (!vel) {
-                            u0 *= omaxf(h0, mah);
-                            v0 *= omaxf(h0, mah);
-                            u1 *= omaxf(h1, mah);
-                            v1 *= omaxf(h1, mah);
-                            u2 *= omaxf(h2, mah);
-                            v2 *= omaxf(h2, mah);
-                        }
-                        aux_jumps_f(u0 - cu, u1 - u0, u2 - u0, c,
-                                    P.f_beta_uh_dry + (P.f_beta_uh - P.f_beta_uh_dry) * hfactor, du);
-                        aux_jumps_f(v0 - cv, v1 - v0, v2 - v0, c,
-                                    P.f_beta_vh_dry + (P.f_beta_vh - P.f_beta_vh_dry) * hfactor, dv);
-                    }
-                } else {
-                    const int slot = (kind >> 2) & 3;
-                    const int k1 = T.sur[slot][tid];
-                    const float h1 = tile_or_global(T.hf, X.hf, k1, kb, cnt);
-                    const float beta = P.f_beta_w;
-                    const float2 s1 = tile_or_global(T.ws, X.ws, k1, kb, cnt);
-                    one_jumps_f((s1.x - wk) + (s1.y - lk),
-                                c, beta, dw);
-                    const float2 q1 = tile_or_global(T.vel, X.vel, k1, kb, cnt);
-                    float u1 = q1.x, v1 = q1.y;
-                    if (!vel) {
-                        u1 *= omaxf(h1, mah);
-                        v1 *= omaxf(h1, mah);
-                    }
-                    one_jumps_f(u1 - cu, c, beta, du);
-                    one_jumps_f(v1 - cv, c, beta, dv);
-                }
-            }
-            if (keep) {
-                // previous vertex values, from the stored edge values of the
-                // (linear) reconstruction: v_i = e_a + e_b - e_i
-                float e0[3], e1[3], e2[3];
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    const float4 e = X.es[i * SP + k];  // this thread's own, before it stores
-                    e0[i] = e.y;
-                    e1[i] = e.z;
-                    e2[i] = e.w;
-                }
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    const int a = (i == 0) ? 1 : 0, b = (i == 2) ? 1 : 2;
-                    dw[i] = (e0[a] + e0[b]) - e0[i];
-                    ou[i] = (e1[a] + e1[b]) - e1[i];
-                    ov[i] = (e2[a] + e2[b]) - e2[i];
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    ou[i] = cu + du[i];
-                    ov[i] = cv + dv[i];
-                }
-            }
-            if (vel) {
-                // velocity -> momentum with the vertex depth hc + dw - dzv
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    const float d = omaxf((hc + dw[i]) - T.dzv[i][tid], 0.0f);
-                    ou[i] *= d;
-                    ov[i] *= d;
-                }
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                ou[i] = uk;
-                ov[i] = vk;
-            }
-        }
-        // balance_deep_and_shallow (shallow_water_ext.c:1462-1636) with vertex
-        // depth h_i = hc + (dw_i - dzv_i); the blend keeps the form
-        // dw_i <- alpha*(dw_i - dzv_i) + dzv_i
-        {
-            // the bed offsets at the vertices, read from the tile here rather
-            // than held in registers through the reconstruction
-            float dzv[3];
-#pragma unroll
-            for (int i = 0; i < 3; i++) dzv[i] = T.dzv[i][tid];
-            float rel[3];  // h_i - hc
-#pragma unroll
-            for (int i = 0; i < 3; i++) rel[i] = dw[i] - dzv[i];
-            const float hmin = hc + ominf(rel[0], ominf(rel[1], rel[2]));
-            float alpha = 1.0f;
-            if (P.tight_slope_limiters == 0) {
-                float dz = 0.0f;
-#pragma unroll
-                for (int i = 0; i < 3; i++) dz = omaxf(dz, fabsf(dzv[i]));
-                alpha = dz > 0.0f ? omaxf(ominf(P.f_alpha * hmin / dz, 1.0f), 0.0f) : 1.0f;
-            } else if (hmin < P.f_H0) {
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    const float hd = -rel[i];
-                    if (!(hd <= 0.0f)) alpha = ominf(alpha, (hc - P.f_H0) / hd);
-                }
-                alpha = fminf(fmaxf(alpha, 0.0f), 1.0f);
-            }
-            if (alpha < 1.0f) {
-                const float uc = hc > 1.0e-6f ? uk / hc : 0.0f;
-                const float vc = hc > 1.0e-6f ? vk / hc : 0.0f;
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    const float r = alpha * rel[i];
-                    dw[i] = r + dzv[i];
-                    if (P.use_centroid_velocities == 1) {
-                        ou[i] = uc * (hc + r);
-                        ov[i] = vc * (hc + r);
-                    } else {
-                        ou[i] = (1.0f - alpha) * uk + alpha * ou[i];
-                        ov[i] = (1.0f - alpha) * vk + alpha * ov[i];
-                    }
-                }
-            }
-        }
-        // edge values (quantity.c:687-706 interpolation) stored for the flux:
-        // depth, stage jump from the centroid, momentum
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const int a = (i == 0) ? 1 : 0, b = (i == 2) ? 1 : 2;
-            X.es[i * SP + k] = make_float4(edge_depth(hc, dw[a], dw[b], T.dze[i][tid]),
-                                           0.5f * (dw[a] + dw[b]), 0.5f * (ou[a] + ou[b]),
-                                           0.5f * (ov[a] + ov[b]));
-        }
+        const DistView<BS> v{X, T, kb, cnt, tid};
+        distribute_triangle(v, P, order, kind);
         if ((flags & kWriteBoundary) && (kind & 16)) {  // a boundary edge
             // the control block and the boundary's time are looked up again
             // here rather than held in registers through the reconstruction
             // (neither changes during the kernel)
             const Ctrl *c = block_ctrl(ctrls, M);
-            const double time =
-                fused ? c->clk_t0 + c->clk_dt * (stg.kind == kStageMid ? stg.tfrac : 1.0)
-                      : c->time;
+            const double time = fused ? stage_end_time(c, stg) : c->time;
             bad_bc = boundary_edges_mixed(k, N, SP, time, P.g, M.nbr, M.btag, tags, S.ze,
-                                          X.es, X.nrm, S.wb, S.uhb, S.vhb,
-                                          S.zb, X.hbf, X.wjb, X.uhbf, X.vhbf);
+                                          X.es + k, SP, X.nrm, S.wb, S.uhb, S.vhb, S.zb,
+                                          X.hbf, X.wjb, X.uhbf, X.vhbf, nullptr,
+                                          fused ? X.tag_values : nullptr, 0);
         }
     }
     if (bad_bc) set_status(block_ctrl(ctrls, M), SWGPU_EBOUNDARY);
@@ -1157,6 +1325,359 @@ __global__ void mass_final_mixed(const double *partials, int n, double *out) {
     if (threadIdx.x == 0) *out = sh[0];
 }
 
+// ---------------------------------------------------- resident small meshes ---
+
+// A whole run of steps in one launch, for meshes that one thread-block cluster
+// holds.  A step kernel by kernel costs such a mesh four launches (13.5 us a
+// step at 1,024 triangles, of which less than 3 us is work); here each thread
+// keeps one triangle, its state in registers and its block's data in shared
+// memory, where the cluster's other blocks read what they need of it, and
+// the blocks meet three times a stage at the cluster's barrier: after the flux
+// (with the timestep's minimum), after the update and after the distribute.
+// One more warp per block evaluates the step's clock, the time-dependent
+// boundary values while the update runs, and the step's commit while the
+// distribute does.  Same operations as the step kernels (flux_triangle,
+// update_triangle, distribute_triangle): the results are the same bits.  (The
+// same across the whole chip, with a barrier in global memory, lost to the step
+// kernels: a meeting of 139 blocks that exchange data took 5,800 to 9,600
+// clocks, 20 us a step.)
+
+struct ResidentArgs {
+    DevMesh M;
+    DevState S;
+    DevMixed X;
+    DevParams P;
+    const BcTag *tags;
+    Ctrl *ctrls;
+    const int *scen_first;      // ensembles: first triangle of each scenario, + the count
+    int steps;                  // at most this many
+    int nstages;
+    Stage stage[3];
+    int flags;                  // kTrack
+};
+
+constexpr int kClusterMax = 16;
+
+template <int T>
+struct __align__(16) ResidentBlock {
+    float4 es[3][T];
+    float4 ust[T];
+    float2 ws[T], vel[T], rad[T];
+    float2 nrm[3][T], gc[3][T];
+    int2 lnb[3][T];
+    float dzv[3][T], dze[3][T], hf[T];
+    int sur[3][T];
+    uint8_t kind[T];
+    Ctrl ctrl, next;            // the clock; the same after this step's commit
+    int key[kClusterMax][T / 32];  // timestep keys of every warp of the cluster
+    int error[kClusterMax];        // a thread of that block set the status
+    int my_error;
+    int ntags;
+    int tag[kTimeTags];
+    TagValue value[kTimeTags];
+};
+
+// Address of a shared-memory variable of this block in block `rank` of the
+// cluster, and loads and a store there.
+__device__ __forceinline__ unsigned cluster_at(const void *p, unsigned rank) {
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float cluster_f1(unsigned a) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 cluster_f2(unsigned a) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];"
+                 : "=f"(v.x), "=f"(v.y)
+                 : "r"(a)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 cluster_f4(unsigned a) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(a)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_put(unsigned a, int v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+// Every thread of the cluster; what was written before it is visible after.
+// (A hardware barrier of blocks that run side by side by construction: no
+// thread leaves the kernel, or the step loop, without the others.)
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int T>
+struct ResidentView {
+    const DevMixed &X;
+    ResidentBlock<T> &B;
+    int first, tid;  // the scenario's first triangle
+    unsigned rank;
+    // block and place of the scenario's triangle n
+    __device__ unsigned owner(int n, int &ln) const {
+        const unsigned r = (unsigned)(n - first) / T;
+        ln = n - first - (int)(r * T);
+        return r;
+    }
+    __device__ float2 ws() const { return B.ws[tid]; }
+    __device__ float hf() const { return B.hf[tid]; }
+    __device__ float2 vel() const { return B.vel[tid]; }
+    __device__ float2 rad() const { return B.rad[tid]; }
+    __device__ float2 nrm(int i) const { return B.nrm[i][tid]; }
+    __device__ int2 lnb(int i) const { return B.lnb[i][tid]; }
+    __device__ float2 gc(int i) const { return B.gc[i][tid]; }
+    __device__ float dzv(int i) const { return B.dzv[i][tid]; }
+    __device__ float dze(int i) const { return B.dze[i][tid]; }
+    __device__ int sur(int i) const { return B.sur[i][tid]; }
+    __device__ float4 es(int i) const { return B.es[i][tid]; }
+    __device__ void far(int pki, float4 &en, float2 &wsn) const {
+        int ln;
+        const unsigned r = owner(pki >> 2, ln);
+        if (r == rank) {
+            en = B.es[pki & 3][ln];
+            wsn = B.ws[ln];
+        } else {
+            en = cluster_f4(cluster_at(&B.es[pki & 3][ln], r));
+            wsn = cluster_f2(cluster_at(&B.ws[ln], r));
+        }
+    }
+    __device__ void boundary(int mb, float &hr, float &jump, float &uhr, float &vhr) const {
+        // this thread's own stores
+        hr = X.hbf[mb];
+        jump = X.wjb[mb];
+        uhr = X.uhbf[mb];
+        vhr = X.vhbf[mb];
+    }
+    __device__ float near_hf(int n) const {
+        int ln;
+        const unsigned r = owner(n, ln);
+        return r == rank ? B.hf[ln] : cluster_f1(cluster_at(&B.hf[ln], r));
+    }
+    __device__ float2 near_ws(int n) const {
+        int ln;
+        const unsigned r = owner(n, ln);
+        return r == rank ? B.ws[ln] : cluster_f2(cluster_at(&B.ws[ln], r));
+    }
+    __device__ float2 near_vel(int n) const {
+        int ln;
+        const unsigned r = owner(n, ln);
+        return r == rank ? B.vel[ln] : cluster_f2(cluster_at(&B.vel[ln], r));
+    }
+    __device__ void put_es(int i, const float4 &e) const { B.es[i][tid] = e; }
+};
+
+// A control block copied word by word (as a struct it takes 60 registers).
+__device__ __forceinline__ void copy_ctrl(Ctrl *to, const Ctrl *from, int first, int step) {
+    static_assert(sizeof(Ctrl) % 4 == 0, "whole words");
+#pragma unroll 1
+    for (int i = first; i < (int)(sizeof(Ctrl) / 4); i += step)
+        reinterpret_cast<unsigned *>(to)[i] = reinterpret_cast<const unsigned *>(from)[i];
+}
+
+// One cluster per scenario.
+template <int T>
+__global__ void __launch_bounds__(T + 32, 1)
+    steps_resident(const __grid_constant__ ResidentArgs A) {
+    extern __shared__ __align__(16) unsigned char resident_smem[];
+    ResidentBlock<T> &B = *reinterpret_cast<ResidentBlock<T> *>(resident_smem);
+    const DevMesh &M = A.M;
+    const DevState &S = A.S;
+    const DevMixed &X = A.X;
+    const DevParams &P = A.P;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool extra = tid >= T;
+    unsigned rank, size;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+    const int scen = blockIdx.x / size;
+    const int first = A.scen_first ? A.scen_first[scen] : 0;
+    const int end = A.scen_first ? A.scen_first[scen + 1] : M.N;
+    const int k = first + (int)rank * T + tid;
+    Ctrl *ctrl = A.ctrls + scen;
+    if (ctrl->halt) return;  // the whole cluster: only the host clears it, between runs
+    const bool in = !extra && k < end;
+    double h = 0.0, uh = 0.0, vh = 0.0;
+    float evh = 0.f;
+    float2 ewu = make_float2(0.f, 0.f);
+    if (extra) copy_ctrl(&B.ctrl, ctrl, lane, 32);
+    if (tid == T) B.my_error = B.ntags = 0;
+    if (tid < kClusterMax) B.error[tid] = 0;
+    if (!extra) B.kind[tid] = in ? X.kind[k] : 2;
+    if (in) {
+        const int SP = X.S;
+        h = X.hd[k];
+        uh = S.uh[k];
+        vh = S.vh[k];
+        B.ust[tid] = ro(X.ust + k);
+        B.ws[tid] = X.ws[k];
+        B.vel[tid] = X.vel[k];
+        B.hf[tid] = X.hf[k];
+        B.rad[tid] = ro(X.rad + k);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            B.es[i][tid] = X.es[i * SP + k];
+            B.nrm[i][tid] = ro(X.nrm + i * SP + k);
+            B.gc[i][tid] = ro(X.gc + i * SP + k);
+            B.dzv[i][tid] = ro(X.dzv + i * SP + k);
+            B.dze[i][tid] = ro(X.dze + i * SP + k);
+            B.sur[i][tid] = ro(X.surrp + i * SP + k);
+            B.lnb[i][tid] = ro(X.lnb + i * SP + k);
+        }
+    }
+    __syncthreads();
+    // the block's time-dependent boundary tags
+    if (in && (B.kind[tid] & 16)) {
+        for (int i = 0; i < 3; i++) {
+            const int pk = B.lnb[i][tid].y;
+            if (pk >= 0) continue;
+            const int tag = ro(M.btag - pk - 1);
+            if (!time_dependent(A.tags[tag].type)) continue;
+            bool known = false;
+            const int have = min(*(volatile int *)&B.ntags, kTimeTags);
+            for (int j = 0; j < have; j++) known |= *(volatile int *)&B.tag[j] == tag;
+            if (!known) {
+                const int at = atomicAdd(&B.ntags, 1);  // (a tag may come in twice)
+                if (at < kTimeTags) *(volatile int *)&B.tag[at] = tag;
+            }
+        }
+    }
+    cluster_meet();
+    const int ntags = min(B.ntags, kTimeTags);
+    const ResidentView<T> v{X, B, first, tid, rank};
+    for (int step = 0; step < A.steps; step++) {
+        double bh = 0.0, bu = 0.0, bv = 0.0;
+        for (int g = 0; g < A.nstages; g++) {
+            const Stage &stg = A.stage[g];
+            // ---- flux, the minimum timestep, the step's clock
+            if (!extra) {
+                float t = P.f_max_dt;
+                if (in) t = flux_triangle(v, P, ewu, evh);
+                const int key = __reduce_min_sync(0xffffffffu, timestep_key(t));
+                if (lane < (int)size) cluster_put(cluster_at(&B.key[rank][warp], lane), key);
+            }
+            cluster_meet();
+            if (g == 0) {
+                if (extra) {
+                    int key = 0x7f7fffff;
+                    for (int i = lane; i < (int)size * (T / 32); i += 32)
+                        key = min(key, (&B.key[0][0])[i]);
+                    key = __reduce_min_sync(0xffffffffu, key);
+                    if (lane == 0) {
+                        if (key < 0) {  // a NaN or negative timestep
+                            set_status(ctrl, SWGPU_ENONFINITE);
+                            B.my_error = 1;
+                        } else {
+                            const u64 bits = bits64(widen(__int_as_float(key)));
+                            if (bits < B.ctrl.ftmin_bits) B.ctrl.ftmin_bits = bits;
+                        }
+                        publish_step_clock(&B.ctrl, P);
+                    }
+                }
+                __syncthreads();
+            }
+            const StepClock clk = published_step_clock(&B.ctrl);
+            // ---- update; the boundary tags' values
+            if (!extra) {
+                int bad = 0, nonfinite = 0;
+                if (in) {
+                    const double h0 = h, uh0 = uh, vh0 = vh;
+                    if (stg.kind == kStageFirst) {
+                        bh = h0;
+                        bu = uh0;
+                        bv = vh0;
+                    }
+                    const float4 us = B.ust[tid];
+                    const float2 vel0 = B.vel[tid];
+                    update_triangle(P, (float)clk.dt, us.x, us.y, B.hf[tid], vel0.x, vel0.y, ewu.x,
+                                    ewu.y, evh, h, uh, vh, bad);
+                    if (stg.kind == kStageMid || stg.kind == kStageLast)
+                        combine_stage(stg, bh, bu, bv, h, uh, vh);
+                    float hf, wf, wl, uv, vv;
+                    finish_state(P, h, uh, vh, us.z, us.w, hf, wf, wl, uv, vv, nonfinite);
+                    B.hf[tid] = hf;
+                    B.ws[tid] = make_float2(wf, wl);
+                    B.vel[tid] = make_float2(uv, vv);
+                    if ((A.flags & kTrack) && (stg.kind == kStageEuler || stg.kind == kStageLast))
+                        track_depth(S, k, h, step_end_time(&B.ctrl, clk.dt, stg), P.track_threshold);
+                }
+                if (bad) set_status(ctrl, SWGPU_EDENOMINATOR);
+                if (nonfinite) set_status(ctrl, SWGPU_ENONFINITE);
+                if (bad || nonfinite) B.my_error = 1;
+            } else if (lane < ntags) {
+                tag_value(A.tags[B.tag[lane]], stage_end_time(&B.ctrl, stg), P.g, B.value[lane]);
+            }
+            cluster_meet();
+            // ---- distribute and boundary values; the stage's commit
+            if (!extra) {
+                if (in) {
+                    const int kind = B.kind[tid];
+                    distribute_triangle(v, P, (int)clk.order, kind);
+                    if ((kind & 16) &&
+                        boundary_edges_mixed(k, M.N, X.S, stage_end_time(&B.ctrl, stg), P.g, M.nbr,
+                                             M.btag, A.tags, S.ze, &B.es[0][tid], T, X.nrm, S.wb,
+                                             S.uhb, S.vhb, S.zb, X.hbf, X.wjb, X.uhbf, X.vhbf,
+                                             B.tag, B.value, ntags)) {
+                        set_status(ctrl, SWGPU_EBOUNDARY);
+                        B.my_error = 1;
+                    }
+                }
+            } else {
+                // errors up to the update; one in the distribute shows a step later
+                if (lane < (int)size)
+                    cluster_put(cluster_at(&B.error[rank], lane), *(volatile int *)&B.my_error);
+                copy_ctrl(&B.next, &B.ctrl, lane, 32);
+                __syncwarp();
+                if (lane == 0) commit_stage(&B.next, clk, P, stg);
+            }
+            cluster_meet();
+            if (extra) {
+                if (__any_sync(0xffffffffu, lane < (int)size && B.error[lane] != 0)) {
+                    // some block's thread set the status: commit with it
+                    if (lane == 0) {
+                        B.my_error = 1;
+                        B.ctrl.status = *(volatile int *)&ctrl->status;
+                    }
+                    __syncwarp();
+                    copy_ctrl(&B.next, &B.ctrl, lane, 32);
+                    __syncwarp();
+                    if (lane == 0) commit_stage(&B.next, clk, P, stg);
+                    __syncwarp();
+                }
+                copy_ctrl(&B.ctrl, &B.next, lane, 32);
+            }
+            __syncthreads();
+        }
+        if (B.ctrl.halt_pending) break;  // the same in every block of the cluster
+    }
+    // the state as the step kernels leave it
+    if (in) {
+        X.hd[k] = h;
+        S.uh[k] = uh;
+        S.vh[k] = vh;
+        X.hf[k] = B.hf[tid];
+        X.ws[k] = B.ws[tid];
+        X.vel[k] = B.vel[tid];
+#pragma unroll
+        for (int i = 0; i < 3; i++) X.es[i * X.S + k] = B.es[i][tid];
+    }
+    cluster_meet();  // (every block has read the control block's status for the last time)
+    if (tid == 0 && rank == 0) {
+        const int status = *(volatile int *)&ctrl->status;  // set by any block
+        copy_ctrl(ctrl, &B.ctrl, 0, 1);
+        ctrl->status = status ? status : B.ctrl.status;
+        apply_pending_halt(ctrl);
+    }
+}
+
 // ------------------------------------------------------------ launches ---
 
 // Block sizes come from M.shape (the autotuner's choice; results do not
@@ -1202,21 +1723,109 @@ void launch_flux_mixed(const DevMesh &M, const DevState &, const DevMixed &X, co
     else
         launch_k(flux_mixed<128>, g, 128, st, pdl, M, X, P, ctrl, flags);
 }
+// The shapes of the resident step: threads per block, smallest first (a mesh
+// spread over more SMs has fewer warps to wait for on each).
+struct ResidentShape {
+    int threads;
+    void (*kernel)(ResidentArgs);
+    size_t smem;
+};
+template <int T>
+static ResidentShape resident_of() {
+    return {T, steps_resident<T>, sizeof(ResidentBlock<T>)};
+}
+static const ResidentShape kResidentShapes[] = {resident_of<128>(), resident_of<256>(),
+                                                resident_of<512>()};
+
+static cudaLaunchConfig_t resident_config(const ResidentShape &r, int cluster, int nscen,
+                                          cudaStream_t st, cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(cluster * nscen));
+    cfg.blockDim = dim3((unsigned)(r.threads + 32));
+    cfg.dynamicSmemBytes = r.smem;
+    cfg.stream = st;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)cluster;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+Resident resident_shape(int64_t largest, int nscen) {
+    int i = -1;
+    for (const ResidentShape &r : kResidentShapes) {
+        i++;
+        int cluster = 1;
+        while ((int64_t)cluster * r.threads < largest) cluster *= 2;
+        if (cluster > kClusterMax) continue;
+        int fit = 0;
+        cudaLaunchAttribute attr[1];
+        const cudaLaunchConfig_t cfg = resident_config(r, cluster, nscen, nullptr, attr);
+        if (cudaFuncSetAttribute(r.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)r.smem) != cudaSuccess ||
+            cudaFuncSetAttribute(r.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&fit, r.kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return Resident{0, 0};
+        }
+        // an ensemble of more scenarios than run at once goes kernel by kernel
+        if (fit < nscen) return Resident{0, 0};
+        return Resident{i + 1, cluster};
+    }
+    return Resident{0, 0};
+}
+cudaError_t launch_resident(const DevMesh &M, const DevState &S, const DevMixed &X,
+                            const DevParams &P, const BcTag *tags, Ctrl *ctrl, int nscen,
+                            const Resident &shape, const int *scen_first, int steps,
+                            const Stage *stages, int nstages, int flags, cudaStream_t st) {
+    const ResidentShape &r = kResidentShapes[shape.kernel - 1];
+    ResidentArgs A{};
+    A.M = M;
+    A.S = S;
+    A.X = X;
+    A.P = P;
+    A.tags = tags;
+    A.ctrls = ctrl;
+    A.scen_first = scen_first;
+    A.steps = steps;
+    A.nstages = nstages;
+    for (int i = 0; i < nstages; i++) A.stage[i] = stages[i];
+    A.flags = flags;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = resident_config(r, shape.cluster, nscen, st, attr);
+    return cudaLaunchKernelEx(&cfg, r.kernel, A);
+}
 void launch_step_clock_mixed(const DevParams &P, Ctrl *ctrl, int nscen, bool pdl,
                              cudaStream_t st) {
     launch_k(step_clock_mixed, (nscen + 127) / 128, 128, st, pdl, ctrl, nscen, P);
 }
 void launch_update_mixed(const DevMesh &M, const DevState &S, const DevMixed &X,
                          const DevParams &P, Ctrl *ctrl, int flags, const Stage &stage,
-                         cudaStream_t st) {
+                         bool clock, const BcTag *tags, int ntags, cudaStream_t st) {
     const int bs = M.shape.update, g = (M.n_launch + bs - 1) / bs;
     const bool pdl = M.shape.pdl;
-    if (bs == 128)
-        launch_k(update_mixed<128>, g, 128, st, pdl, M, S, X, P, ctrl, flags, stage);
-    else if (bs == 512)
-        launch_k(update_mixed<512>, g, 512, st, pdl, M, S, X, P, ctrl, flags, stage);
-    else
-        launch_k(update_mixed<256>, g, 256, st, pdl, M, S, X, P, ctrl, flags, stage);
+    const auto launch = [&](auto plain, auto with_tags) {
+        if (ntags > 0)
+            launch_k(with_tags, g + 1, bs, st, pdl, M, S, X, P, ctrl, flags, stage, tags, ntags);
+        else
+            launch_k(plain, g, bs, st, pdl, M, S, X, P, ctrl, flags, stage);
+    };
+    if (clock) {
+        if (bs == 128)
+            launch(update_mixed<128, true>, update_with_tags<128, true>);
+        else if (bs == 512)
+            launch(update_mixed<512, true>, update_with_tags<512, true>);
+        else
+            launch(update_mixed<256, true>, update_with_tags<256, true>);
+    } else {
+        if (bs == 128)
+            launch(update_mixed<128, false>, update_with_tags<128, false>);
+        else if (bs == 512)
+            launch(update_mixed<512, false>, update_with_tags<512, false>);
+        else
+            launch(update_mixed<256, false>, update_with_tags<256, false>);
+    }
 }
 void launch_prepare_mixed(const DevMesh &M, const DevState &S, const DevMixed &X,
                           const DevParams &P, int from_stage, cudaStream_t st) {

@@ -234,7 +234,10 @@ typedef struct {
     int32_t dependent_launch; /* mixed kernels: each step kernel is launched as a
                                  programmatic dependent of the previous one, so
                                  its blocks start (and fetch the static planes)
-                                 during that kernel's last wave */
+                                 during that kernel's last wave; 0 also runs
+                                 small mixed meshes kernel by kernel, which
+                                 otherwise take whole steps in one resident
+                                 launch, without the knobs above */
 } swgpu_launch_config;
 
 int swgpu_get_launch_config(void *handle, swgpu_launch_config *config);
