@@ -822,6 +822,7 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
         if (e == cudaSuccess)
             e = cudaMallocHost((void **)&h->h_halt_bits, sizeof(unsigned) * ((h->nscen + 31) / 32));
         if (e == cudaSuccess) e = cudaMallocHost((void **)&h->h_scalar, 4 * sizeof(double));
+        if (e == cudaSuccess) e = cudaMallocHost((void **)&h->h_watch, 2 * sizeof(Ctrl));
         if (e != cudaSuccess) {
             fail(h, SWGPU_ENOMEM, "pinned host allocation: %s", cudaGetErrorString(e));
             g_create_error = h->err;
@@ -885,6 +886,7 @@ int swgpu_destroy(void *handle) {
     if (h->h_summary) cudaFreeHost(h->h_summary);
     if (h->h_halt_bits) cudaFreeHost(h->h_halt_bits);
     if (h->h_scalar) cudaFreeHost(h->h_scalar);
+    if (h->h_watch) cudaFreeHost(h->h_watch);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return SWGPU_OK;
@@ -1616,90 +1618,110 @@ int swgpu_profile_steps(void *handle, int64_t nsteps, double *ms) {
     return finish_run(h, nullptr);
 }
 
+// Steps to the next yield or final time as of control block c, at the CFL
+// timestep of its last step (before any clamp): at most `most`.
+static int64_t steps_left(const Handle *h, const Ctrl &c, int64_t most) {
+    double stop = c.yieldtime;
+    if (c.finaltime > 0) stop = std::min(stop, c.finaltime);
+    if (stop >= 1.0e299) return most;
+    const double dt = std::min(h->P.CFL * c.flux_timestep, h->P.evolve_max_timestep);
+    if (!(dt > 0)) return std::min<int64_t>(most, 4);  // no step taken yet
+    const double n = std::ceil((stop - c.time) / dt);
+    if (!(n < (double)most)) return most;
+    return std::max<int64_t>(1, (int64_t)n);
+}
+
+// The run: units of steps issued until the device has stopped, two in flight,
+// so that the host waits on the copies that follow one while the other runs.
+//
+// With a step budget the device stops itself after max_steps steps, and no
+// step is issued beyond it: whole graphs, then kernels one by one (no capture
+// for a remainder that may differ between runs).  One mesh's steps to the next
+// yield or final time are estimated from its last known clock and no more than
+// those are issued either: a step past a stop is empty launches (5 us a stage),
+// of which a yield inside a graph with another behind it left up to 31 steps'
+// worth.  The resident step stops within a launch: its units are long (a few
+// ms).
+static int run_units(Handle *h, int64_t max_steps, cudaEvent_t (&ev)[2]) {
+    const bool resident = use_resident(h);
+    constexpr int kResidentSteps = 512;
+    const int64_t unit = resident ? kResidentSteps : h->steps_per_graph;
+    const bool watch = !resident && h->nscen == 1;
+    int64_t budget = max_steps > 0 ? max_steps : INT64_MAX;  // steps not issued yet
+    int64_t ahead = 0;               // steps issued past the clock that h_ctrl shows
+    int64_t issued[2] = {0, 0};      // steps of the unit that each event follows
+    int inflight = 0, slot = 0, rc;
+    for (;;) {
+        int64_t steps = std::min(budget, unit);
+        if (watch) steps = std::min(steps, steps_left(h, *h->h_ctrl, ahead + unit) - ahead);
+        if (steps <= 0 && inflight == 0) steps = std::min<int64_t>(budget, 1);
+        if (steps > 0) {
+            if (resident) {
+                CK(issue_resident(h, (int)steps));
+            } else if (steps == unit) {
+                CK(cudaGraphLaunch(h->graph, h->stream));
+            } else {
+                for (int64_t s = 0; s < steps; s++) issue_step(h);
+                CK(cudaGetLastError());
+            }
+            CK(cudaMemcpyAsync(h->h_summary, h->d_summary, sizeof(RunSummary),
+                               cudaMemcpyDeviceToHost, h->stream));
+            if (h->nscen > 1)
+                CK(cudaMemcpyAsync(h->h_halt_bits, h->d_halt_bits,
+                                   sizeof(unsigned) * ((h->nscen + 31) / 32),
+                                   cudaMemcpyDeviceToHost, h->stream));
+            if (watch)
+                CK(cudaMemcpyAsync(h->h_watch + slot, h->d_ctrl, sizeof(Ctrl),
+                                   cudaMemcpyDeviceToHost, h->stream));
+            CK(cudaEventRecord(ev[slot], h->stream));
+            if (budget != INT64_MAX) budget -= steps;
+            issued[slot] = steps;
+            ahead += steps;
+            inflight++;
+            slot ^= 1;
+            if (inflight < 2 && budget > 0) continue;
+        }
+        const int oldest = inflight == 2 ? slot : slot ^ 1;
+        CK(cudaEventSynchronize(ev[oldest]));
+        inflight--;
+        if (watch) {
+            *h->h_ctrl = h->h_watch[oldest];
+            ahead -= issued[oldest];
+        }
+        if (h->h_summary->halted >= h->nscen || h->h_summary->status) return SWGPU_OK;
+        if (budget == 0 && inflight == 0) return SWGPU_OK;
+        if (h->nscen > 1 && !resident) {
+            // ensembles: launch only up to the last scenario still running
+            // (longest-running scenarios are placed first) once that
+            // saves an eighth of the current launch
+            int last = h->nscen - 1;
+            while (last > 0 && (h->h_halt_bits[last >> 5] >> (last & 31) & 1u)) last--;
+            const int extent = (int)h->scen_offsets[(size_t)last + 1];
+            if (extent <= h->M.n_launch - h->M.n_launch / 8) {
+                CK(cudaStreamSynchronize(h->stream));
+                inflight = 0;
+                if ((rc = set_launch_extent(h, extent)) || (rc = build_graph(h))) return rc;
+            }
+        }
+    }
+}
+
 static int run_graphs(Handle *h, int64_t max_steps, swgpu_state *state, double *elapsed_ms) {
     if (!h) return fail(h, SWGPU_EINVAL, "null handle");
     int rc = prepare_run(h, max_steps);
     if (rc) return rc;
-    // the resident step's launches are bounded (a few ms each) so that the
-    // host looks in on them; the device stops itself within one
-    const bool resident = use_resident(h);
-    constexpr int kResidentSteps = 512;
-    if (!resident && (rc = build_graph(h))) return rc;
-    // with a step budget the device stops itself after max_steps steps; the
-    // host issues max_steps / steps-per-graph whole graphs and then the
-    // remaining steps' kernels one by one (no capture for a remainder that
-    // may differ between runs), so that no step is issued beyond the budget
-    const int spg = resident ? kResidentSteps : h->steps_per_graph;
-    const int64_t full_graphs = max_steps > 0 ? max_steps / spg : INT64_MAX;
-    const int tail = max_steps > 0 ? (int)(max_steps % spg) : 0;
-    const int64_t max_graphs = max_steps > 0 ? full_graphs + (tail ? 1 : 0) : INT64_MAX;
-    // keep two graphs in flight: while graph i runs, the host waits on the
-    // control-block copy that follows graph i-1
+    if (!use_resident(h) && (rc = build_graph(h))) return rc;
     cudaEvent_t ev[2], t0, t1;
     CK(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
     CK(cudaEventCreate(&t0));
     CK(cudaEventCreate(&t1));
-    CK(cudaEventRecord(t0, h->stream));
-    int64_t launched = 0;
-    cudaError_t e = cudaSuccess;
-    int inflight = 0, slot = 0;
-    bool halted = false;
-    while (!halted && launched < max_graphs) {
-        if (resident) {
-            e = issue_resident(h, launched < full_graphs ? spg : tail);
-        } else if (launched < full_graphs) {
-            e = cudaGraphLaunch(h->graph, h->stream);
-        } else {
-            for (int s = 0; s < tail; s++) issue_step(h);
-            e = cudaGetLastError();
-        }
-        if (e != cudaSuccess) break;
-        e = cudaMemcpyAsync(h->h_summary, h->d_summary, sizeof(RunSummary),
-                            cudaMemcpyDeviceToHost, h->stream);
-        if (e != cudaSuccess) break;
-        if (h->nscen > 1) {
-            e = cudaMemcpyAsync(h->h_halt_bits, h->d_halt_bits,
-                                sizeof(unsigned) * ((h->nscen + 31) / 32),
-                                cudaMemcpyDeviceToHost, h->stream);
-            if (e != cudaSuccess) break;
-        }
-        e = cudaEventRecord(ev[slot], h->stream);
-        if (e != cudaSuccess) break;
-        launched++;
-        inflight++;
-        slot ^= 1;
-        if (inflight == 2) {
-            e = cudaEventSynchronize(ev[slot]);  // the older of the two
-            if (e != cudaSuccess) break;
-            inflight--;
-            if (h->h_summary->halted >= h->nscen || h->h_summary->status) halted = true;
-            if (!halted && h->nscen > 1 && !resident) {
-                // ensembles: launch only up to the last scenario still running
-                // (longest-running scenarios are placed first) once that
-                // saves an eighth of the current launch
-                int last = h->nscen - 1;
-                while (last > 0 && (h->h_halt_bits[last >> 5] >> (last & 31) & 1u)) last--;
-                const int extent = (int)h->scen_offsets[(size_t)last + 1];
-                if (extent <= h->M.n_launch - h->M.n_launch / 8) {
-                    e = cudaStreamSynchronize(h->stream);
-                    if (e != cudaSuccess) break;
-                    inflight = 0;
-                    if ((rc = set_launch_extent(h, extent)) || (rc = build_graph(h))) {
-                        cudaEventDestroy(ev[0]);
-                        cudaEventDestroy(ev[1]);
-                        cudaEventDestroy(t0);
-                        cudaEventDestroy(t1);
-                        return rc;
-                    }
-                }
-            }
-        }
-    }
+    cudaError_t e = cudaEventRecord(t0, h->stream);
+    if (e == cudaSuccess) rc = run_units(h, max_steps, ev);
     if (e == cudaSuccess) e = cudaEventRecord(t1, h->stream);
-    cudaError_t e2 = cudaStreamSynchronize(h->stream);
+    const cudaError_t e2 = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) e = e2;
-    if (e == cudaSuccess && elapsed_ms) {
+    if (e == cudaSuccess && !rc && elapsed_ms) {
         float ms = 0.f;
         e = cudaEventElapsedTime(&ms, t0, t1);
         *elapsed_ms = ms;
@@ -1708,6 +1730,7 @@ static int run_graphs(Handle *h, int64_t max_steps, swgpu_state *state, double *
     cudaEventDestroy(ev[1]);
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
+    if (rc) return rc;
     if (e != cudaSuccess) return fail(h, SWGPU_ECUDA, "evolve_run: %s", cudaGetErrorString(e));
     return finish_run(h, state);
 }

@@ -34,6 +34,7 @@ struct Handle {
     int *d_scen_first = nullptr; // ensemble: first triangle of each scenario, + N
     Ctrl *d_ctrl = nullptr;      // [nscen]
     Ctrl *h_ctrl = nullptr;      // pinned mirror [nscen]
+    Ctrl *h_watch = nullptr;     // pinned: the clock after each of the two units in flight
     RunSummary *d_summary = nullptr;
     RunSummary *h_summary = nullptr;  // pinned
     unsigned int *d_halt_bits = nullptr;  // one bit per scenario
