@@ -9,6 +9,8 @@
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -77,6 +79,19 @@ static std::vector<T> to_planes(const U *src, int64_t N, int width) {
         for (int j = 0; j < width; j++) out[(size_t)j * N + k] = (T)src[k * width + j];
     return out;
 }
+// The same for a caller's [N][3] values on their way to the device, through
+// memory that is not cleared first.
+static int upload_planes3(Handle *h, double *dst, const double *src, int64_t N) {
+    std::unique_ptr<double[]> out(new (std::nothrow) double[(size_t)3 * N]);
+    if (!out) return fail(h, SWGPU_ENOMEM, "host memory for %lld triangles", (long long)N);
+    double *a = out.get(), *b = a + N, *c = b + N;
+    for (int64_t k = 0; k < N; k++) {
+        a[k] = src[3 * k];
+        b[k] = src[3 * k + 1];
+        c[k] = src[3 * k + 2];
+    }
+    return upload(h, dst, out.get(), (size_t)3 * N);
+}
 
 static int check_launch(Handle *h, const char *what) {
     cudaError_t e = cudaGetLastError();
@@ -98,19 +113,38 @@ static int check_usable(Handle *h) {
     return SWGPU_OK;
 }
 
+// Waits for the stream and brings the control blocks to their pinned mirror.
 static int sync_ctrl(Handle *h) {
     if (int rc = check_usable(h)) return rc;
     CK(cudaMemcpyAsync(h->h_ctrl, h->d_ctrl, sizeof(Ctrl) * h->nscen, cudaMemcpyDeviceToHost,
                        h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    h->ctrl_current = true;
+    h->push_pending = false;
     return SWGPU_OK;
 }
 
+// The mirror to read: nothing to wait for while no kernel that was issued
+// since the last sync_ctrl may have changed the device's (a trip of about
+// 10 us, of which a single small step made a dozen).
+static int read_ctrl(Handle *h) { return h->ctrl_current ? check_usable(h) : sync_ctrl(h); }
+
+// The mirror to change: a copy from it to the device has to be done with it.
+static int edit_ctrl(Handle *h) {
+    if (int rc = read_ctrl(h)) return rc;
+    if (h->push_pending) {
+        CK(cudaStreamSynchronize(h->stream));
+        h->push_pending = false;
+    }
+    return SWGPU_OK;
+}
+
+// The mirror to the device, in stream order.
 static int push_ctrl(Handle *h) {
     if (int rc = check_usable(h)) return rc;
     CK(cudaMemcpyAsync(h->d_ctrl, h->h_ctrl, sizeof(Ctrl) * h->nscen, cudaMemcpyHostToDevice,
                        h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    h->push_pending = true;
     return SWGPU_OK;
 }
 
@@ -283,6 +317,7 @@ static void drop_graphs(Handle *h) {
 // distribute as the stand-alone method: protect + velocities, then the
 // extrapolation/balance pass with edge values materialised.
 static int issue_distribute(Handle *h, bool with_boundary) {
+    h->ctrl_current = false;
     if (h->precision == SWGPU_FP64) {
         launch_prepare_fp64(h->M, h->S, h->P, h->d_ctrl, h->stream);
         launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl,
@@ -881,6 +916,8 @@ int swgpu_destroy(void *handle) {
     Handle *h = static_cast<Handle *>(handle);
     if (h->stream) cudaStreamSynchronize(h->stream);
     drop_graphs(h);
+    for (cudaEvent_t e : h->events)
+        if (e) cudaEventDestroy(e);
     for (void *p : h->allocs) cudaFree(p);
     if (h->h_ctrl) cudaFreeHost(h->h_ctrl);
     if (h->h_summary) cudaFreeHost(h->h_summary);
@@ -949,12 +986,10 @@ int swgpu_set_quantity(void *handle, int q, const double *centroid, const double
     int rc = upload(h, c, centroid, (size_t)N);
     if (rc) return rc;
     if (v && vertex) {
-        auto pv = to_planes<double>(vertex, N, 3);
-        if ((rc = upload(h, v, pv.data(), (size_t)3 * N))) return rc;
+        if ((rc = upload_planes3(h, v, vertex, N))) return rc;
     }
     if (e && edge) {
-        auto pe = to_planes<double>(edge, N, 3);
-        if ((rc = upload(h, e, pe.data(), (size_t)3 * N))) return rc;
+        if ((rc = upload_planes3(h, e, edge, N))) return rc;
     } else if (q == SWGPU_ELEVATION && vertex) {
         // quantity.c:687-706: bed edge values from the bed vertex values
         std::vector<double> pe((size_t)3 * N);
@@ -1109,14 +1144,13 @@ int swgpu_protect(void *handle) {
     if (rc) return rc;
     launch_prepare_fp64(h->M, h->S, h->P, h->d_ctrl, h->stream);
     if ((rc = check_launch(h, "protect"))) return rc;
-    CK(cudaStreamSynchronize(h->stream));
     return SWGPU_OK;
 }
 
 int swgpu_distribute_to_vertices_and_edges(void *handle) {
     Handle *h = static_cast<Handle *>(handle);
     if (!h) return fail(h, SWGPU_EINVAL, "null handle");
-    int rc = sync_ctrl(h);  // current _order_ lives in the control block
+    int rc = check_usable(h);
     if (rc) return rc;
     if ((rc = issue_distribute(h, false))) return rc;
     if ((rc = sync_ctrl(h))) return rc;
@@ -1129,6 +1163,7 @@ int swgpu_update_boundary(void *handle) {
     if (h->precision == SWGPU_MIXED && !h->mixed_from_stage) {
         launch_vertices_from_mixed(h->M, h->S, h->X, h->stream);
     }
+    h->ctrl_current = false;
     launch_boundary_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl, h->stream);
     int rc = check_launch(h, "update_boundary");
     if (rc) return rc;
@@ -1141,9 +1176,10 @@ int swgpu_compute_fluxes(void *handle, double *flux_timestep) {
     int rc = require_fp64(h, "compute_fluxes");
     if (rc) return rc;
     if ((rc = require_single(h, "compute_fluxes"))) return rc;
-    if ((rc = sync_ctrl(h))) return rc;
+    if ((rc = edit_ctrl(h))) return rc;
     reset_ftmin(h->h_ctrl, h->P);
     if ((rc = push_ctrl(h))) return rc;
+    h->ctrl_current = false;
     refresh_edges(h);
     launch_flux_fp64(h->M, h->S, h->P, h->d_ctrl, kWriteMaxSpeed, h->stream);
     launch_explicit_fp64(h->M, h->S, h->P, h->stream);
@@ -1163,7 +1199,6 @@ int swgpu_compute_forcing_terms(void *handle) {
     if (rc) return rc;
     launch_forcing_fp64(h->M, h->S, h->P, false, h->stream);
     if ((rc = check_launch(h, "compute_forcing_terms"))) return rc;
-    CK(cudaStreamSynchronize(h->stream));
     return SWGPU_OK;
 }
 
@@ -1173,7 +1208,6 @@ int swgpu_manning_friction_explicit(void *handle) {
     if (rc) return rc;
     launch_forcing_fp64(h->M, h->S, h->P, true, h->stream);
     if ((rc = check_launch(h, "manning_friction_explicit"))) return rc;
-    CK(cudaStreamSynchronize(h->stream));
     return SWGPU_OK;
 }
 
@@ -1185,6 +1219,7 @@ int swgpu_extrapolate_second_order_sw(void *handle) {
         return fail(h, SWGPU_EINVAL,
                     "extrapolate_second_order_sw: the 'tsunami' flow algorithm extrapolates "
                     "to edges inside distribute_to_vertices_and_edges");
+    h->ctrl_current = false;
     if (h->P.extrapolate_velocity_second_order) launch_velocities_fp64(h->M, h->S, h->P, h->stream);
     launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl, kExtrapolateOnly, h->stream);
     if ((rc = check_launch(h, "extrapolate_second_order_sw"))) return rc;
@@ -1201,7 +1236,6 @@ int swgpu_balance_deep_and_shallow(void *handle) {
     launch_balance_fp64(h->M, h->S, h->P, h->stream);
     h->edges_stale = true;
     if ((rc = check_launch(h, "balance_deep_and_shallow"))) return rc;
-    CK(cudaStreamSynchronize(h->stream));
     return SWGPU_OK;
 }
 
@@ -1210,6 +1244,7 @@ int swgpu_update_conserved_quantities(void *handle, double timestep) {
     int rc = require_fp64(h, "update_conserved_quantities");
     if (rc) return rc;
     if ((rc = require_single(h, "update_conserved_quantities"))) return rc;
+    h->ctrl_current = false;
     launch_update_fp64(h->M, h->S, h->P, h->d_ctrl, timestep, 0, kEulerStage, h->stream);
     if ((rc = check_launch(h, "update_conserved_quantities"))) return rc;
     if ((rc = sync_ctrl(h))) return rc;
@@ -1224,7 +1259,6 @@ int swgpu_backup_conserved_quantities(void *handle) {
     CK(cudaMemcpyAsync(h->S.bw, h->S.w, bytes, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->S.buh, h->S.uh, bytes, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->S.bvh, h->S.vh, bytes, cudaMemcpyDeviceToDevice, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
     return SWGPU_OK;
 }
 
@@ -1235,7 +1269,6 @@ int swgpu_saxpy_conserved_quantities(void *handle, double a, double b) {
     launch_saxpy_fp64(h->M, h->S, a, b, h->stream);
     if ((rc = check_launch(h, "saxpy_conserved_quantities"))) return rc;
     h->vertices_stale = true;
-    CK(cudaStreamSynchronize(h->stream));
     return SWGPU_OK;
 }
 
@@ -1260,7 +1293,6 @@ int swgpu_update_other_quantities(void *handle) {
     launch_other_quantities(h->M, h->S, h->stream);
     int rc = check_launch(h, "update_other_quantities");
     if (rc) return rc;
-    CK(cudaStreamSynchronize(h->stream));
     return SWGPU_OK;
 }
 
@@ -1279,7 +1311,7 @@ int swgpu_mass(void *handle, double *mass) {
 int swgpu_get_state(void *handle, swgpu_state *state) {
     Handle *h = static_cast<Handle *>(handle);
     if (!h || !state) return fail(h, SWGPU_EINVAL, "null argument");
-    int rc = sync_ctrl(h);
+    int rc = read_ctrl(h);
     if (rc) return rc;
     fill_state(h->h_ctrl, state);
     return SWGPU_OK;
@@ -1290,7 +1322,7 @@ int swgpu_ensemble_get_state(void *handle, int scenario, swgpu_state *state) {
     if (!h || !state) return fail(h, SWGPU_EINVAL, "null argument");
     if (scenario < 0 || scenario >= h->nscen)
         return fail(h, SWGPU_EINVAL, "scenario %d of %d", scenario, h->nscen);
-    int rc = sync_ctrl(h);
+    int rc = read_ctrl(h);
     if (rc) return rc;
     fill_state(&h->h_ctrl[scenario], state);
     return SWGPU_OK;
@@ -1299,7 +1331,7 @@ int swgpu_ensemble_get_state(void *handle, int scenario, swgpu_state *state) {
 int swgpu_ensemble_set_finaltimes(void *handle, const double *finaltimes) {
     Handle *h = static_cast<Handle *>(handle);
     if (!h || !finaltimes) return fail(h, SWGPU_EINVAL, "null argument");
-    int rc = sync_ctrl(h);
+    int rc = edit_ctrl(h);
     if (rc) return rc;
     for (int i = 0; i < h->nscen; i++) {
         if (finaltimes[i] > 0 && finaltimes[i] < h->h_ctrl[i].time)
@@ -1430,7 +1462,7 @@ int swgpu_set_state(void *handle, const swgpu_state *s) {
     Handle *h = static_cast<Handle *>(handle);
     if (!h || !s) return fail(h, SWGPU_EINVAL, "null argument");
     if (s->order != 1 && s->order != 2) return fail(h, SWGPU_EINVAL, "order must be 1 or 2");
-    int rc = sync_ctrl(h);
+    int rc = edit_ctrl(h);
     if (rc) return rc;
     Ctrl *c = h->h_ctrl;
     c->time = s->time;
@@ -1455,7 +1487,7 @@ int swgpu_evolve_start(void *handle, double starttime, double yieldstep, double 
     if (!(yieldstep > 0)) return fail(h, SWGPU_EINVAL, "yieldstep must be > 0");
     if (finaltime > 0 && finaltime < starttime)
         return fail(h, SWGPU_EINVAL, "finaltime before starttime");
-    int rc = sync_ctrl(h);
+    int rc = check_usable(h);
     if (rc) return rc;
     // first distribute with the current order (gpu_domain_advanced.py:2476)
     if ((rc = issue_distribute(h, false))) return rc;
@@ -1506,7 +1538,7 @@ static int set_launch_extent(Handle *h, int n) {
 // those that stopped at a yield move to the next yield point
 // (gpu_domain_advanced.py:2649-2654).
 static int prepare_run(Handle *h, int64_t max_steps) {
-    int rc = sync_ctrl(h);
+    int rc = edit_ctrl(h);
     if (rc) return rc;
     if ((rc = device_status(h))) return rc;
     int running = 0;
@@ -1532,15 +1564,22 @@ static int prepare_run(Handle *h, int64_t max_steps) {
     if (running == 0) return fail(h, SWGPU_EINVAL, "evolve already reached finaltime");
     h->h_summary->halted = h->nscen - running;
     h->h_summary->status = 0;
-    if ((rc = upload(h, h->d_summary, h->h_summary, 1))) return rc;
-    const int nwords = (h->nscen + 31) / 32;
-    for (int w = 0; w < nwords; w++) h->h_halt_bits[w] = 0u;
-    for (int i = 0; i < h->nscen; i++)
-        if (h->h_ctrl[i].halt) h->h_halt_bits[i >> 5] |= 1u << (i & 31);
-    if ((rc = upload(h, h->d_halt_bits, h->h_halt_bits, (size_t)nwords))) return rc;
+    // (pinned, and free: the last run's end waited for the stream)
+    CK(cudaMemcpyAsync(h->d_summary, h->h_summary, sizeof(RunSummary), cudaMemcpyHostToDevice,
+                       h->stream));
+    if (h->nscen > 1) {
+        const int nwords = (h->nscen + 31) / 32;
+        for (int w = 0; w < nwords; w++) h->h_halt_bits[w] = 0u;
+        for (int i = 0; i < h->nscen; i++)
+            if (h->h_ctrl[i].halt) h->h_halt_bits[i >> 5] |= 1u << (i & 31);
+        CK(cudaMemcpyAsync(h->d_halt_bits, h->h_halt_bits, sizeof(unsigned) * (size_t)nwords,
+                           cudaMemcpyHostToDevice, h->stream));
+    }
     if ((rc = set_launch_extent(h, h->M.N))) return rc;
     refresh_edges(h);
-    return push_ctrl(h);
+    if ((rc = push_ctrl(h))) return rc;
+    h->ctrl_current = false;
+    return SWGPU_OK;
 }
 
 static int finish_run(Handle *h, swgpu_state *state) {
@@ -1642,7 +1681,8 @@ static int64_t steps_left(const Handle *h, const Ctrl &c, int64_t most) {
 // of which a yield inside a graph with another behind it left up to 31 steps'
 // worth.  The resident step stops within a launch: its units are long (a few
 // ms).
-static int run_units(Handle *h, int64_t max_steps, cudaEvent_t (&ev)[2]) {
+static int run_units(Handle *h, int64_t max_steps) {
+    cudaEvent_t *ev = h->events;
     const bool resident = use_resident(h);
     constexpr int kResidentSteps = 512;
     const int64_t unit = resident ? kResidentSteps : h->steps_per_graph;
@@ -1664,6 +1704,8 @@ static int run_units(Handle *h, int64_t max_steps, cudaEvent_t (&ev)[2]) {
                 for (int64_t s = 0; s < steps; s++) issue_step(h);
                 CK(cudaGetLastError());
             }
+            // a budget's last unit: the caller waits for it
+            if (steps == budget) return SWGPU_OK;
             CK(cudaMemcpyAsync(h->h_summary, h->d_summary, sizeof(RunSummary),
                                cudaMemcpyDeviceToHost, h->stream));
             if (h->nscen > 1)
@@ -1679,7 +1721,7 @@ static int run_units(Handle *h, int64_t max_steps, cudaEvent_t (&ev)[2]) {
             ahead += steps;
             inflight++;
             slot ^= 1;
-            if (inflight < 2 && budget > 0) continue;
+            if (inflight < 2) continue;
         }
         const int oldest = inflight == 2 ? slot : slot ^ 1;
         CK(cudaEventSynchronize(ev[oldest]));
@@ -1689,7 +1731,6 @@ static int run_units(Handle *h, int64_t max_steps, cudaEvent_t (&ev)[2]) {
             ahead -= issued[oldest];
         }
         if (h->h_summary->halted >= h->nscen || h->h_summary->status) return SWGPU_OK;
-        if (budget == 0 && inflight == 0) return SWGPU_OK;
         if (h->nscen > 1 && !resident) {
             // ensembles: launch only up to the last scenario still running
             // (longest-running scenarios are placed first) once that
@@ -1711,28 +1752,25 @@ static int run_graphs(Handle *h, int64_t max_steps, swgpu_state *state, double *
     int rc = prepare_run(h, max_steps);
     if (rc) return rc;
     if (!use_resident(h) && (rc = build_graph(h))) return rc;
-    cudaEvent_t ev[2], t0, t1;
-    CK(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
-    CK(cudaEventCreate(&t0));
-    CK(cudaEventCreate(&t1));
-    cudaError_t e = cudaEventRecord(t0, h->stream);
-    if (e == cudaSuccess) rc = run_units(h, max_steps, ev);
-    if (e == cudaSuccess) e = cudaEventRecord(t1, h->stream);
-    const cudaError_t e2 = cudaStreamSynchronize(h->stream);
-    if (e == cudaSuccess) e = e2;
-    if (e == cudaSuccess && !rc && elapsed_ms) {
+    for (int i = 0; i < 4; i++)
+        if (!h->events[i])
+            CK(cudaEventCreateWithFlags(&h->events[i],
+                                        i < 2 ? cudaEventDisableTiming : cudaEventDefault));
+    if (elapsed_ms) CK(cudaEventRecord(h->events[2], h->stream));
+    rc = run_units(h, max_steps);
+    cudaError_t e = cudaSuccess;
+    if (!rc && elapsed_ms) e = cudaEventRecord(h->events[3], h->stream);
+    if (rc || e != cudaSuccess) {
+        cudaStreamSynchronize(h->stream);
+        return rc ? rc : fail(h, SWGPU_ECUDA, "evolve_run: %s", cudaGetErrorString(e));
+    }
+    rc = finish_run(h, state);  // waits for the stream
+    if (elapsed_ms && (rc == SWGPU_OK || h->ctrl_current)) {
         float ms = 0.f;
-        e = cudaEventElapsedTime(&ms, t0, t1);
+        CK(cudaEventElapsedTime(&ms, h->events[2], h->events[3]));
         *elapsed_ms = ms;
     }
-    cudaEventDestroy(ev[0]);
-    cudaEventDestroy(ev[1]);
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
-    if (rc) return rc;
-    if (e != cudaSuccess) return fail(h, SWGPU_ECUDA, "evolve_run: %s", cudaGetErrorString(e));
-    return finish_run(h, state);
+    return rc;
 }
 
 int swgpu_evolve_one_step(void *handle, swgpu_state *state) {

@@ -35,6 +35,9 @@ struct Handle {
     Ctrl *d_ctrl = nullptr;      // [nscen]
     Ctrl *h_ctrl = nullptr;      // pinned mirror [nscen]
     Ctrl *h_watch = nullptr;     // pinned: the clock after each of the two units in flight
+    bool ctrl_current = false;   // h_ctrl holds what d_ctrl does
+    bool push_pending = false;   // a copy of h_ctrl to the device may still be reading it
+    cudaEvent_t events[4] = {nullptr, nullptr, nullptr, nullptr};  // units in flight; run timing
     RunSummary *d_summary = nullptr;
     RunSummary *h_summary = nullptr;  // pinned
     unsigned int *d_halt_bits = nullptr;  // one bit per scenario
