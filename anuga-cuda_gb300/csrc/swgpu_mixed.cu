@@ -48,71 +48,56 @@ __device__ __forceinline__ T ro(const T *p) {
 // Exact FP32 -> FP64 widening on the integer pipe (inputs are flushed to
 // zero when denormal, as this unit compiles with -ftz).
 __device__ __forceinline__ double widen(float x) {
-    const unsigned u = __float_as_uint(x);
-    const unsigned e = (u >> 23) & 0xffu;
-    const unsigned long long sign = (unsigned long long)(u >> 31) << 63;
-    const unsigned long long mant = (unsigned long long)(u & 0x7fffffu) << 29;
-    const unsigned long long ex =
-        e == 0 ? 0ull : (e == 0xffu ? 0x7ffull : (unsigned long long)(e + 896u));
-    const unsigned long long bits = e == 0 ? sign : (sign | (ex << 52) | mant);
-    return __longlong_as_double((long long)bits);
+    const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+    unsigned hi = (m >> 3) + (896u << 20), lo = m << 29;
+    if (m < 0x00800000u) hi = lo = 0u;
+    if (m >= 0x7f800000u) hi |= 0x7ff00000u;  // infinity, NaN
+    return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
+}
+
+// FP64 -> FP32 on the integer pipe, for a magnitude (high word h without its
+// sign, low word l) outside FP32's normal range: below it zero, above infinity,
+// NaN stays NaN.
+__device__ __forceinline__ unsigned narrow_outside(unsigned h, unsigned l) {
+    if (h > 0x7ff00000u || (h == 0x7ff00000u && l)) return 0x7fc00000u;
+    return h < (897u << 20) ? 0u : 0x7f800000u;
 }
 
 // FP64 -> FP32 narrowing, round to nearest even, on the integer pipe
 // (results below the FP32 normal range flush to zero, overflow gives
 // infinity, NaN stays NaN).
 __device__ __forceinline__ float narrow(double x) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const unsigned sign = (unsigned)(b >> 63) << 31;
-    const unsigned ed = (unsigned)((b >> 52) & 0x7ffu);
-    const int e = (int)ed - 896;
-    const unsigned long long frac = b & 0xfffffffffffffull;
-    unsigned r;
-    if (ed == 0x7ffu) {
-        r = sign | 0x7f800000u | (frac ? 0x400000u : 0u);
-    } else if (e <= 0) {
-        r = sign;
-    } else if (e >= 255) {
-        r = sign | 0x7f800000u;
-    } else {
-        const unsigned m = (unsigned)(frac >> 29);
-        const unsigned long long rest = frac & 0x1fffffffull;  // the 29 dropped bits
-        r = ((unsigned)e << 23) | m;
-        // round half to even; a carry out of the mantissa bumps the exponent
-        // (up to infinity) as it should
-        if (rest > 0x10000000ull || (rest == 0x10000000ull && (m & 1u))) r += 1u;
-        r |= sign;
-    }
-    return __uint_as_float(r);
+    const unsigned hx = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+    const unsigned h = hx & 0x7fffffffu;
+    unsigned r = __funnelshift_l(l, h - (896u << 20), 3);  // the leading 24 bits
+    // the 29 dropped bits round half to even; a carry out of the significand
+    // bumps the exponent (up to infinity) as it should
+    r += ((l & 0x1fffffffu) + 0x0fffffffu + (r & 1u)) >> 29;
+    if (h - (897u << 20) >= (254u << 20)) r = narrow_outside(h, l);
+    return __uint_as_float(r | (hx & 0x80000000u));
 }
 
 // x as an FP32 pair on the integer pipe: hi = x rounded to nearest (as
 // narrow), lo = the exact remainder x - hi rounded to nearest.  lo is zero
 // where x lies outside FP32's normal range or the remainder falls below it.
 __device__ __forceinline__ void split_double(double x, float &hi, float &lo) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const unsigned sign = (unsigned)(b >> 63) << 31;
-    const unsigned ed = (unsigned)((b >> 52) & 0x7ffu);
-    const int e = (int)ed - 896;
-    if (ed == 0x7ffu || e <= 0 || e >= 255) {
-        hi = narrow(x);
-        lo = 0.0f;
-        return;
-    }
-    const unsigned long long frac = b & 0xfffffffffffffull;
-    const unsigned m = (unsigned)(frac >> 29);
-    int rest = (int)(frac & 0x1fffffffull);  // the 29 dropped bits
-    unsigned r = ((unsigned)e << 23) | m;
-    if (rest > 0x10000000 || (rest == 0x10000000 && (m & 1u))) {
-        r += 1u;  // rounded up: the remainder is negative
-        rest -= 0x20000000;
-    }
-    hi = __uint_as_float(r | sign);
-    // remainder = rest * 2^(ed - 1075): one rounding (int -> float), then an
-    // exact scaling by a power of two (flushed to zero below FP32's range)
-    const int se = (int)ed - 1075 + 127;
+    const unsigned hx = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+    const unsigned h = hx & 0x7fffffffu, sign = hx & 0x80000000u;
+    unsigned r = __funnelshift_l(l, h - (896u << 20), 3);
+    const unsigned up = ((l & 0x1fffffffu) + 0x0fffffffu + (r & 1u)) >> 29;
+    r += up;
+    // rounded up: the remainder is negative
+    const int rest = (int)(l & 0x1fffffffu) - (int)(up << 29);
+    // remainder = rest * 2^(exponent - 1075): one rounding (int -> float), then
+    // an exact scaling by a power of two (flushed to zero below FP32's range)
+    const int se = (int)(h >> 20) - 1075 + 127;
     const float scale = se > 0 ? __uint_as_float((unsigned)se << 23) : 0.0f;
     lo = __uint_as_float(__float_as_uint(__fmul_rn(__int2float_rn(rest), scale)) ^ sign);
+    if (h - (897u << 20) >= (254u << 20)) {
+        r = narrow_outside(h, l);
+        lo = 0.0f;
+    }
+    hi = __uint_as_float(r | sign);
 }
 
 // (ah + al) + (bh + bl) as an FP32 pair hi + lo (TwoSum of the high parts,
@@ -766,29 +751,14 @@ __global__ void __launch_bounds__(BS, 2048 / BS) update_with_tags(DevMesh M, Dev
     update_body<CLOCK, true>(M, S, X, P, ctrl, flags, stg, tags, ntags);
 }
 
+// find_qmin_and_qmax (shallow_water_ext.c:98-148): the extremes of 0, dq0,
+// dq0 + dq1 and dq0 + dq2 (a sum does not fall when a term grows, so its
+// branches on the terms pick these).
 __device__ __forceinline__ void qminmax_f(float dq0, float dq1, float dq2, float &qmin,
                                           float &qmax) {
-    if (dq0 >= 0.0f) {
-        if (dq1 >= dq2) {
-            qmax = (dq1 >= 0.0f) ? dq0 + dq1 : dq0;
-            qmin = dq0 + dq2;
-            if (qmin >= 0.0f) qmin = 0.0f;
-        } else {
-            qmax = (dq2 > 0.0f) ? dq0 + dq2 : dq0;
-            qmin = dq0 + dq1;
-            if (qmin >= 0.0f) qmin = 0.0f;
-        }
-    } else {
-        if (dq1 <= dq2) {
-            qmin = (dq1 < 0.0f) ? dq0 + dq1 : dq0;
-            qmax = dq0 + dq2;
-            if (qmax <= 0.0f) qmax = 0.0f;
-        } else {
-            qmin = (dq2 < 0.0f) ? dq0 + dq2 : dq0;
-            qmax = dq0 + dq1;
-            if (qmax <= 0.0f) qmax = 0.0f;
-        }
-    }
+    const float s1 = dq0 + dq1, s2 = dq0 + dq2;
+    qmin = fminf(fminf(0.0f, dq0), fminf(s1, s2));
+    qmax = fmaxf(fmaxf(0.0f, dq0), fmaxf(s1, s2));
 }
 
 // a / b from the approximate reciprocal and one Newton correction of the
@@ -808,8 +778,7 @@ __device__ __forceinline__ void limit_f(float (&d)[3], float qmin, float qmax, f
     float r = 1000.0f, r0 = 1.0f;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        if (d[i] < -TINY) r0 = div_refined(qmin, d[i]);
-        if (d[i] > TINY) r0 = div_refined(qmax, d[i]);
+        if (fabsf(d[i]) > TINY) r0 = div_refined(d[i] < 0.0f ? qmin : qmax, d[i]);
         r = ominf(r0, r);
     }
     const float phi = ominf(r * beta, 1.0f);
@@ -965,20 +934,26 @@ __device__ __forceinline__ void distribute_triangle(const View &v, const DevPara
                 const float h0 = v.near_hf(k0);
                 const float h1 = v.near_hf(k1);
                 const float h2 = v.near_hf(k2);
-                const float hmin = ominf(ominf(h0, ominf(h1, h2)), hc);
                 const float hmax = omaxf(h0, omaxf(h1, h2));
                 if (P.optimise_dry_cells && hmax < P.f_eps) {
                     keep = true;
                 } else {
-                    float hfactor = 0.0f;
-                    if (hmin > 0.001f) hfactor = (hmin - 0.001f) / (hmin + 0.004f);
+                    float bw = P.f_beta_w_dry, bu = P.f_beta_uh_dry, bv = P.f_beta_vh_dry;
+                    if (P.betas_differ) {
+                        const float hmin = ominf(ominf(h0, ominf(h1, h2)), hc);
+                        float hfactor = 0.0f;
+                        if (hmin > 0.001f) hfactor = (hmin - 0.001f) / (hmin + 0.004f);
+                        bw += (P.f_beta_w - P.f_beta_w_dry) * hfactor;
+                        bu += (P.f_beta_uh - P.f_beta_uh_dry) * hfactor;
+                        bv += (P.f_beta_vh - P.f_beta_vh_dry) * hfactor;
+                    }
                     const float2 s0 = v.near_ws(k0);
                     const float2 s1 = v.near_ws(k1);
                     const float2 s2 = v.near_ws(k2);
                     const float w0 = s0.x, w1 = s1.x, w2 = s2.x;
                     const float l0 = s0.y, l1 = s1.y, l2 = s2.y;
-                    aux_jumps_f((w0 - wk) + (l0 - lk), (w1 - w0) + (l1 - l0), (w2 - w0) + (l2 - l0), c,
-                                P.f_beta_w_dry + (P.f_beta_w - P.f_beta_w_dry) * hfactor, dw);
+                    aux_jumps_f((w0 - wk) + (l0 - lk), (w1 - w0) + (l1 - l0), (w2 - w0) + (l2 - l0), c, bw,
+                                dw);
                     const float2 q0 = v.near_vel(k0);
                     const float2 q1 = v.near_vel(k1);
                     const float2 q2 = v.near_vel(k2);
@@ -992,10 +967,8 @@ __device__ __forceinline__ void distribute_triangle(const View &v, const DevPara
                         u2 *= omaxf(h2, mah);
                         v2 *= omaxf(h2, mah);
                     }
-                    aux_jumps_f(u0 - cu, u1 - u0, u2 - u0, c,
-                                P.f_beta_uh_dry + (P.f_beta_uh - P.f_beta_uh_dry) * hfactor, du);
-                    aux_jumps_f(v0 - cv, v1 - v0, v2 - v0, c,
-                                P.f_beta_vh_dry + (P.f_beta_vh - P.f_beta_vh_dry) * hfactor, dv);
+                    aux_jumps_f(u0 - cu, u1 - u0, u2 - u0, c, bu, du);
+                    aux_jumps_f(v0 - cv, v1 - v0, v2 - v0, c, bv, dv);
                 }
             } else {
                 const int slot = (kind >> 2) & 3;
