@@ -15,15 +15,17 @@
 // kernel keeps the weights of its layer in shared memory and walks tiles of
 // 128 rows, each a tcgen05.mma (kind::f16) into FP32 accumulators in tensor
 // memory read back with tcgen05.ld:
-//   mlp_layers12        features, layers 1 and 2 (W1, W2 resident)
-//   mlp_layer3_predict  layer 3 and the 256 -> 3 output layer (W3 resident)
-//   mlp_layer3_train    the same, the loss, the output layer's gradients and
-//                       the gradient back through layer 3
+//   mlp_predict         inference: the whole network (half of each matrix
+//                       resident in each CTA of a pair)
+//   mlp_layers12        training: features, layers 1 and 2 (W1, W2 resident)
+//   mlp_layer3_train    layer 3 and the 256 -> 3 output layer, the loss, the
+//                       output layer's gradients and the gradient back through
+//                       layer 3 (W3 resident)
 //   mlp_back2           the gradient back through layer 2 (W2 resident)
 //   mlp_wgrad           the weight and bias gradients, split over the rows
 //   mlp_finish          the splits' sums in a fixed order, Adam on the FP32
 //                       master weights and the BF16 images
-// Inference is the first two, training the other five launches.  No sum
+// Inference is the first, training the other five launches.  No sum
 // depends on the order in which blocks finish.
 #include <cuda_bf16.h>
 
@@ -246,6 +248,45 @@ __device__ __forceinline__ void tc_ld8x2(unsigned a, unsigned b, float (&v)[8], 
         w[i] = __uint_as_float(r[8 + i]);
     }
 }
+// 8 consecutive FP32 columns of this thread's lane at each of 8 places, 32
+// columns apart
+__device__ __forceinline__ void tc_ld8x8(unsigned taddr, float (&v)[8][8]) {
+    unsigned r[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[i][0]), "=r"(r[i][1]), "=r"(r[i][2]), "=r"(r[i][3]), "=r"(r[i][4]),
+                       "=r"(r[i][5]), "=r"(r[i][6]), "=r"(r[i][7])
+                     : "r"(taddr + 32 * i));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[i][j] = __uint_as_float(r[i][j]);
+}
+// 32 columns of 32 lanes (rows) by a warp, a thread's part being four rows of
+// two neighbouring columns in every eight: v[b][i] is row 8 i + lane / 4 of
+// columns 8 b + 2 (lane % 4) and the next.
+__device__ __forceinline__ void tc_ld_quads(unsigned taddr, float2 (&v)[4][4]) {
+    unsigned r[2][16];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
+            "%13,%14,%15}, [%16];"
+            : "=r"(r[i][0]), "=r"(r[i][1]), "=r"(r[i][2]), "=r"(r[i][3]), "=r"(r[i][4]),
+              "=r"(r[i][5]), "=r"(r[i][6]), "=r"(r[i][7]), "=r"(r[i][8]), "=r"(r[i][9]),
+              "=r"(r[i][10]), "=r"(r[i][11]), "=r"(r[i][12]), "=r"(r[i][13]), "=r"(r[i][14]),
+              "=r"(r[i][15])
+            : "r"(taddr + ((unsigned)(16 * i) << 16)));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            v[b][i] = make_float2(__uint_as_float(r[i >> 1][4 * b + 2 * (i & 1)]),
+                                  __uint_as_float(r[i >> 1][4 * b + 2 * (i & 1) + 1]));
+}
 // 16 consecutive FP32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tc_ld16(unsigned taddr, float (&v)[16]) {
     unsigned r[16];
@@ -306,6 +347,27 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned pari
         if (mbar_test(bar, parity)) break;
     return false;
 }
+// Arrives at the barrier that CTA `rank` of the cluster has where this one
+// has `bar`.  It passes on that this CTA's own shared and tensor memory is
+// ready for the tensor core (the caller's proxy_fence and tc_fence_before),
+// no data that the other CTA's threads read: a release at cluster scope would
+// first wait for the warp's stores to global memory (1,000 clocks and more).
+__device__ __forceinline__ void mbar_arrive_at(unsigned long long *bar, unsigned rank) {
+    asm volatile(
+        "{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %0, %1;\n"
+        " mbarrier.arrive.shared::cluster.b64 _, [a];\n}" ::"r"(smem_u32(bar)),
+        "r"(rank)
+        : "memory");
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
 // The same by the whole CTA, which it also brings together: true when all
 // saw the phase complete.
 __device__ __forceinline__ bool cta_wait(unsigned long long *bar, unsigned parity, int *status) {
@@ -354,17 +416,20 @@ __device__ __forceinline__ void mma_layer_back(unsigned d, unsigned a, unsigned 
                smem_desc(w + 256 * kk, 128, kWStride), tc_idesc(kH, false, true), kk > 0);
 }
 
-// A thread's part of an epilogue: the tile row of its TMEM lane and half of
-// the columns.  Warp w reaches lanes 32 (w % 4) .. + 31 only.
+// A thread's part of an epilogue: the tile row of its TMEM lane and one of
+// `groups` equal parts of the columns.  Warp w reaches lanes 32 (w % 4) .. + 31
+// only.
 struct Part {
-    int row, col0;
+    int row, group, col0;
     unsigned tmem;  // its lane's first column
 };
+template <int groups>
 __device__ __forceinline__ Part my_part(unsigned tmem) {
     const int warp = threadIdx.x >> 5;
     Part p;
     p.row = 32 * (warp & 3) + (threadIdx.x & 31);
-    p.col0 = 128 * (warp >> 2);
+    p.group = warp >> 2;
+    p.col0 = kH / groups * p.group;
     p.tmem = tmem + ((unsigned)(32 * (warp & 3)) << 16);
     return p;
 }
@@ -374,25 +439,50 @@ __device__ __forceinline__ uint4 pack8(const float *v) {
     for (int j = 0; j < 4; j++) o[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
     return *reinterpret_cast<const uint4 *>(o);
 }
+// two FP32 operations in one instruction
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
+        " add.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
+        " mov.b64 z, {%6, %7};\n fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
 // bias and ReLU of n columns from c0, in place
 template <int n>
 __device__ __forceinline__ void bias_relu(float (&v)[n], const float *bias, int c0) {
 #pragma unroll
     for (int q = 0; q < n / 4; q++) {
         const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + 4 * q);
-        v[4 * q] = fmaxf(v[4 * q] + b.x, 0.0f);
-        v[4 * q + 1] = fmaxf(v[4 * q + 1] + b.y, 0.0f);
-        v[4 * q + 2] = fmaxf(v[4 * q + 2] + b.z, 0.0f);
-        v[4 * q + 3] = fmaxf(v[4 * q + 3] + b.w, 0.0f);
+        const float2 lo = add2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(b.x, b.y));
+        const float2 hi = add2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(b.z, b.w));
+        v[4 * q] = fmaxf(lo.x, 0.0f);
+        v[4 * q + 1] = fmaxf(lo.y, 0.0f);
+        v[4 * q + 2] = fmaxf(hi.x, 0.0f);
+        v[4 * q + 3] = fmaxf(hi.y, 0.0f);
     }
 }
+// A layer's epilogue is a chain of tensor memory read, arithmetic and store
+// per 32 columns: sixteen warps, four on a scheduler, hide one another's.  (A
+// training step of 32,768 rows: 108 us with eight, 104 with sixteen.)
+constexpr int kGroups = 4;
+constexpr int kThreads = 128 * kGroups;
+
 // A hidden layer's epilogue: activations of the accumulator at column d into
-// the tile images at smem and / or global.
-template <bool SMEM, bool GLOBAL>
+// the tile images at global and, when asked for, smem.
+template <bool SMEM>
 __device__ __forceinline__ void hidden_epilogue(const Part &p, unsigned d, const float *bias,
                                                 unsigned char *smem, unsigned char *global) {
 #pragma unroll 1
-    for (int c0 = p.col0; c0 < p.col0 + 128; c0 += 32) {
+    for (int c0 = p.col0; c0 < p.col0 + kH / kGroups; c0 += 32) {
         float v[32];
         tc_ld32(p.tmem + d + c0, v);
         bias_relu(v, bias, c0);
@@ -401,7 +491,7 @@ __device__ __forceinline__ void hidden_epilogue(const Part &p, unsigned d, const
             const uint4 o = pack8(v + 8 * q);
             const size_t at = (size_t)(c0 / 8 + q) * kActStride + p.row * 16;
             if (SMEM) *reinterpret_cast<uint4 *>(smem + at) = o;
-            if (GLOBAL) *reinterpret_cast<uint4 *>(global + at) = o;
+            *reinterpret_cast<uint4 *>(global + at) = o;
         }
     }
 }
@@ -427,16 +517,14 @@ __device__ __forceinline__ void unpack8(const uint4 &u, float (&v)[8]) {
 
 // ---- layers 1 and 2 -----------------------------------------------------------
 
-constexpr int kThreads = 256;  // 8 warps: the epilogues split the columns in two
-
 struct Layers12 {
     FeatureTables F;
     Batch batch;
     const BfWeights *W;
     const float *b1, *b2;
-    unsigned char *h1, *h2;    // tile images (h1, x: training only)
+    unsigned char *h1, *h2;    // tile images
     unsigned char *x;
-    long long *row_of;         // training: data row of each batch row
+    long long *row_of;         // data row of each batch row
     int tiles;
     int *status;
 };
@@ -450,12 +538,11 @@ struct __align__(1024) Smem12 {
     unsigned tmem;
 };
 
-// Features, layer 1 and layer 2 of the tiles blockIdx.x, + gridDim.x, ...;
+// Training: features, layer 1 and layer 2 of the tiles blockIdx.x, + gridDim.x, ...;
 // one CTA per SM with both weight matrices resident.  The two accumulators
 // take turns: a tile's layer 1 and layer 2 use one, while the other holds the
 // previous tile's layer 2 until its epilogue, which runs under this tile's
 // layer 2 product, has read it.
-template <bool TRAIN>
 __global__ void __launch_bounds__(kThreads, 1) mlp_layers12(Layers12 g) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     Smem12 &S = *reinterpret_cast<Smem12 *>(smem_raw +
@@ -472,8 +559,10 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layers12(Layers12 g) {
         S.norm[tid] = g.F.mu[tid];
         S.norm[kF + tid] = g.F.isd[tid];
     }
-    S.b1[tid] = g.b1[tid];
-    S.b2[tid] = g.b2[tid];
+    if (tid < kH) {
+        S.b1[tid] = g.b1[tid];
+        S.b2[tid] = g.b2[tid];
+    }
     tc_sync();
     const unsigned tmem = S.tmem;
     if (tid == 0) {
@@ -481,12 +570,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layers12(Layers12 g) {
         bulk_load(S.w1, g.W->w1, kW1Bytes, &S.wbar);
         bulk_load(S.w2, g.W->w2, kWBytes, &S.wbar);
     }
-    const Part p = my_part(tmem);
+    const Part p = my_part<kGroups>(tmem);
     const auto features = [&](int t) {
         if (tid < kTileM) {
             const long long r = (long long)t * kTileM + tid;
             const long long q = tile_features(g.F, g.batch, S.norm, r, tid, S.x);
-            if (TRAIN) g.row_of[r] = q;
+            g.row_of[r] = q;
         }
     };
     const auto layer1 = [&](unsigned d) {
@@ -506,13 +595,11 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layers12(Layers12 g) {
         phase ^= 1;
         if (!ok) break;
         tc_fence_after();
-        if (TRAIN) {
-            // (x's image leaves before the next tile's features replace it)
-            if (tid < 2 * kTileM)
-                reinterpret_cast<uint4 *>(g.x + (size_t)t * kXBytes)[tid] =
-                    reinterpret_cast<const uint4 *>(S.x)[tid];
-        }
-        hidden_epilogue<true, TRAIN>(p, d, S.b1, S.h, TRAIN ? g.h1 + (size_t)t * kActBytes : nullptr);
+        // (x's image leaves before the next tile's features replace it)
+        if (tid < 2 * kTileM)
+            reinterpret_cast<uint4 *>(g.x + (size_t)t * kXBytes)[tid] =
+                reinterpret_cast<const uint4 *>(S.x)[tid];
+        hidden_epilogue<true>(p, d, S.b1, S.h, g.h1 + (size_t)t * kActBytes);
         tc_sync();
         if (tid == 0) {
             mma_layer(tmem + d, smem_u32(S.h), smem_u32(S.w2), false);
@@ -522,7 +609,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layers12(Layers12 g) {
         const int next = t + gridDim.x;
         if (next < g.tiles) features(next);
         if (last >= 0)
-            hidden_epilogue<false, true>(p, (buf ^ 1) * kH, S.b2, nullptr,
+            hidden_epilogue<false>(p, (buf ^ 1) * kH, S.b2, nullptr,
                                          g.h2 + (size_t)last * kActBytes);
         if (next < g.tiles) {
             tc_sync();
@@ -537,7 +624,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layers12(Layers12 g) {
     if (ok) ok = cta_wait(&S.mbar, phase, g.status);
     if (ok) {
         tc_fence_after();
-        hidden_epilogue<false, true>(p, (buf ^ 1) * kH, S.b2, nullptr,
+        hidden_epilogue<false>(p, (buf ^ 1) * kH, S.b2, nullptr,
                                      g.h2 + (size_t)last * kActBytes);
     }
     tc_fence_before();
@@ -555,7 +642,6 @@ struct Layer3 {
     long long nrows;
     float *y;                  // [nrows][3]
     int *status;
-    // training
     const float *targets;
     const long long *row_of;
     unsigned char *d3, *d2;    // gradients of the layers' sums, tile images
@@ -564,29 +650,28 @@ struct Layer3 {
 };
 constexpr int kPart4 = kH * kOut + kOut + 1;
 
-// One row's outputs over half of layer 3's features: the odd or even vectors
-// of eight (odd: the row's other thread has the rest), activations from the
-// accumulator at lane address tmem, kept as BF16 in the tile image at `image`
-// when given.  The sum's order: along the eight features of a vector, then
-// pairwise over vectors 16, 8, 4 and 2 apart (and 1 apart, odd and even, by
-// the caller).
-template <bool KEEP>
-__device__ __forceinline__ void head_half(unsigned tmem, int odd, const float *b3,
-                                          const float4 *w4, unsigned char *image,
-                                          float (&out)[kOut]) {
-    constexpr int order[8] = {0, 4, 2, 6, 1, 5, 3, 7};  // vectors 2 order + odd, and 16 more
-    float pair[kOut], quad[kOut], sum[kOut];
+// One row's outputs over a quarter of layer 3's features: every fourth vector
+// of eight from vector `quarter` on (the row's other threads have the rest),
+// activations from the accumulator at lane address tmem, kept as BF16 in the
+// tile image at `image`.  The sum's order: along the eight features
+// of a vector, then pairwise over vectors 16, 8 and 4 apart (and 2 and 1
+// apart in row_outputs).
+__device__ __forceinline__ void head_quarter(unsigned tmem, int quarter, const float *b3,
+                                             const float4 *w4, unsigned char *image,
+                                             float (&out)[kOut]) {
+    constexpr int order[4] = {0, 2, 1, 3};  // vectors 4 order + quarter, and 16 more
+    float pair[kOut], sum[kOut];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < 4; i++) {
         float v[2][8], s[2][kOut];
-        const int c0 = 16 * order[i] + 8 * odd;
+        const int c0 = 32 * order[i] + 8 * quarter;
         tc_ld8x2(tmem + c0, tmem + c0 + 128, v[0], v[1]);
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             const int c = c0 + 128 * q;
             bias_relu<8>(v[q], b3, c);
             const uint4 u = pack8(v[q]);
-            if (KEEP) *reinterpret_cast<uint4 *>(image + (c >> 3) * kActStride) = u;
+            *reinterpret_cast<uint4 *>(image + (c >> 3) * kActStride) = u;
             float h[8];
             unpack8(u, h);
 #pragma unroll
@@ -602,130 +687,22 @@ __device__ __forceinline__ void head_half(unsigned tmem, int odd, const float *b
 #pragma unroll
         for (int o = 0; o < kOut; o++) {
             const float a = s[0][o] + s[1][o];
-            if (i % 2 == 0) {
+            if (i % 2 == 0)
                 pair[o] = a;
-            } else {
-                const float b = pair[o] + a;
-                if (i % 4 == 1)
-                    quad[o] = b;
-                else if (i == 3)
-                    sum[o] = quad[o] + b;
-                else
-                    out[o] = sum[o] + (quad[o] + b);
-            }
+            else if (i == 1)
+                sum[o] = pair[o] + a;
+            else
+                out[o] = sum[o] + (pair[o] + a);
         }
     }
 }
-
-constexpr int kThreads3 = kThreads + 32;  // inference: one more warp feeds the tensor core
-
-struct __align__(1024) Smem3 {
-    unsigned char w3[kWBytes];
-    unsigned char a[kActBytes];
-    float4 w4[kH];
-    float b3[kH];
-    float4 half[2][kTileM];  // a row's outputs over the odd vectors of features
-    unsigned long long wbar, full[2], free_[2], ready[2], drained[2];
-    unsigned tmem;
-};
-
-// Inference: outputs of the tiles blockIdx.x, + gridDim.x, ...  One warp
-// loads a tile's two halves and issues their products, each half's buffer
-// refilled as soon as its product is done; eight warps turn the accumulator
-// that is ready into outputs meanwhile.
-__global__ void __launch_bounds__(kThreads3, 1) mlp_layer3_predict(Layer3 g) {
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    Smem3 &S = *reinterpret_cast<Smem3 *>(smem_raw +
-                                          ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
-    const int tid = threadIdx.x;
-    pdl_launch_dependents();
-    if (tid < 32) tmem_alloc(&S.tmem, 512);
-    if (tid == 0) {
-        mbar_init(&S.wbar, 1);
-        for (int i = 0; i < 2; i++) {
-            mbar_init(&S.full[i], 1);
-            mbar_init(&S.free_[i], 1);
-            mbar_init(&S.ready[i], 1);
-            mbar_init(&S.drained[i], 8);
-        }
-    }
-    pdl_wait();
-    if (tid < kH) {
-        S.w4[tid] = g.W->w4[tid];
-        S.b3[tid] = g.b3[tid];
-    }
-    tc_sync();
-    const unsigned tmem = S.tmem;
-    const int stride = gridDim.x;
-    constexpr unsigned kHalf = kActBytes / 2;
-    if (tid >= kThreads) {
-        if (tid == kThreads) {
-            mbar_expect(&S.wbar, kWBytes);
-            bulk_load(S.w3, g.W->w3, kWBytes, &S.wbar);
-            const auto load = [&](int t, int i) {
-                mbar_expect(&S.full[i], kHalf);
-                bulk_load(S.a + i * kHalf, g.h2 + (size_t)t * kActBytes + i * kHalf, kHalf,
-                          &S.full[i]);
-            };
-            int t = blockIdx.x;
-            load(t, 0);
-            load(t, 1);
-            bool ok = mbar_wait(&S.wbar, 0, g.status);
-            for (int n = 0; ok && t < g.tiles; n++, t += stride) {
-                const unsigned buf = n & 1, ph = n & 1;
-                // the accumulator's last reader (tile n - 2) is done
-                if (n >= 2) ok = mbar_wait(&S.drained[buf], ((n >> 1) - 1) & 1, g.status);
-                tc_fence_after();
-                for (int i = 0; ok && i < 2; i++) {
-                    ok = mbar_wait(&S.full[i], ph, g.status);
-                    if (!ok) break;
-                    mma_layer(tmem + buf * kH, smem_u32(S.a) + i * kHalf,
-                              smem_u32(S.w3) + i * 16 * kWStride, i > 0);
-                    tc_commit(&S.free_[i]);
-                    if (i == 1) tc_commit(&S.ready[buf]);
-                    // the first half's buffer is refilled under the second's product
-                    if (i == 1 && t + stride < g.tiles) {
-                        ok = mbar_wait(&S.free_[0], ph, g.status);
-                        if (ok) load(t + stride, 0);
-                        if (ok) ok = mbar_wait(&S.free_[1], ph, g.status);
-                        if (ok) load(t + stride, 1);
-                    }
-                }
-            }
-        }
-    } else {
-        const Part p = my_part(tmem);
-        const int odd = p.col0 ? 1 : 0;
-        bool ok = true;
-        int n = 0;
-        for (int t = blockIdx.x; t < g.tiles; t += stride, n++) {
-            const unsigned buf = n & 1;
-            // (after a wait that ran out, the tiles left are passed without one)
-            if (ok) ok = mbar_wait(&S.ready[buf], (n >> 1) & 1, g.status);
-            ok = __all_sync(0xffffffffu, ok);
-            float acc[kOut] = {0.f, 0.f, 0.f};
-            if (ok) {
-                tc_fence_after();
-                head_half<false>(p.tmem + buf * kH, odd, S.b3, S.w4, nullptr, acc);
-                tc_fence_before();
-            }
-            __syncwarp();
-            if ((tid & 31) == 0) mbar_arrive(&S.drained[buf]);
-            if (odd) S.half[buf][p.row] = make_float4(acc[0], acc[1], acc[2], 0.f);
-            // the eight warps of the epilogue
-            asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
-            const long long r = (long long)t * kTileM + p.row;
-            if (!odd && ok && r < g.nrows) {
-                const float4 o = S.half[buf][p.row];
-                g.y[r * kOut] = acc[0] + o.x + g.b4[0];
-                g.y[r * kOut + 1] = acc[1] + o.y + g.b4[1];
-                g.y[r * kOut + 2] = acc[2] + o.z + g.b4[2];
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (tid < 32) tmem_free(tmem, 512);
+// A row's outputs from its four quarters' sums.
+__device__ __forceinline__ void row_outputs(const float4 (&part)[kGroups][kTileM], int row,
+                                            const float *b4, float (&y)[kOut]) {
+    const float4 a = part[0][row], b = part[1][row], c = part[2][row], d = part[3][row];
+    y[0] = (a.x + c.x) + (b.x + d.x) + b4[0];
+    y[1] = (a.y + c.y) + (b.y + d.y) + b4[1];
+    y[2] = (a.z + c.z) + (b.z + d.z) + b4[2];
 }
 
 struct __align__(1024) Smem3T {
@@ -733,9 +710,9 @@ struct __align__(1024) Smem3T {
     unsigned char a[kActBytes];        // h2, then h3, then its gradient
     float4 w4[kH];
     float b3[kH];
-    float4 half[2][kTileM];  // a row's outputs over the even and the odd vectors
+    float4 quarter[kGroups][kTileM];  // a row's outputs by parts
     float4 dy[kTileM];
-    float sum4[8][kOut + 1];
+    float sum4[4][kOut + 1];
     unsigned long long wbar, abar, mbar;
     unsigned tmem;
 };
@@ -761,8 +738,10 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
         mbar_init(&S.mbar, 1);
     }
     pdl_wait();
-    S.w4[tid] = g.W->w4[tid];
-    S.b3[tid] = g.b3[tid];
+    if (tid < kH) {
+        S.w4[tid] = g.W->w4[tid];
+        S.b3[tid] = g.b3[tid];
+    }
     const float b4[kOut] = {g.b4[0], g.b4[1], g.b4[2]};
     tc_sync();
     const unsigned tmem = S.tmem;
@@ -775,14 +754,16 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
         mbar_expect(&S.wbar, kWBytes);
         bulk_load(S.w3, g.W->w3, kWBytes, &S.wbar);
     }
-    const Part p = my_part(tmem);
-    const int odd = p.col0 ? 1 : 0;  // this thread's vectors of eight features: 2 i + odd
+    const Part p = my_part<kGroups>(tmem);
+    // this thread's vectors of eight features: 4 i + p.group, i below kMine
+    constexpr int kMine = kH / 8 / kGroups;
     const float inv_b = 1.0f / (float)g.nrows;
     // W4's gradient: this thread's rows lane + 32 i of every tile, the eight
-    // features of each of the warp's four vectors
-    float gw[4][8][kOut], gb[kOut] = {0.f, 0.f, 0.f}, ls = 0.f;
+    // features of each of the warp's two vectors
+    constexpr int kWarpVecs = kH / 8 / (kThreads / 32);
+    float gw[kWarpVecs][8][kOut], gb[kOut] = {0.f, 0.f, 0.f}, ls = 0.f;
 #pragma unroll
-    for (int q = 0; q < 4; q++)
+    for (int q = 0; q < kWarpVecs; q++)
 #pragma unroll
         for (int j = 0; j < 8; j++)
 #pragma unroll
@@ -807,16 +788,16 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
             t0 = tt.x;
             t1 = tt.y;
         }
-        // signs of this thread's 128 features of h2: vectors 2 i + odd
+        // signs of this thread's features of h2
         unsigned char *image = S.a + p.row * 16;
-        unsigned mask[4];
+        unsigned mask[kMine / 4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < kMine / 4; q++) {
             mask[q] = 0;
 #pragma unroll
             for (int j = 0; j < 4; j++)
                 mask[q] |= positive8(*reinterpret_cast<const uint4 *>(
-                               image + (2 * (4 * q + j) + odd) * kActStride))
+                               image + (4 * (4 * q + j) + p.group) * kActStride))
                            << (8 * j);
         }
         ok = cta_wait(&S.mbar, mphase, g.status);
@@ -824,39 +805,38 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
         if (!ok) break;
         tc_fence_after();
         float acc[kOut];
-        head_half<true>(p.tmem, odd, S.b3, S.w4, image, acc);
-        S.half[odd][p.row] = make_float4(acc[0], acc[1], acc[2], 0.f);
+        head_quarter(p.tmem, p.group, S.b3, S.w4, image, acc);
+        S.quarter[p.group][p.row] = make_float4(acc[0], acc[1], acc[2], 0.f);
         __syncthreads();
         float d0 = 0.f, d1 = 0.f, d2 = 0.f;
         if (r < g.nrows) {
-            const float4 a = S.half[0][p.row], b = S.half[1][p.row];
-            // (a + b first: the order of inference)
-            const float y0 = a.x + b.x + b4[0], y1 = a.y + b.y + b4[1], y2 = a.z + b.z + b4[2];
-            const float e0 = y0 - t0, e1 = y1 - t1;
-            const float u = fabsf(e0) - y2;
+            float y[kOut];
+            row_outputs(S.quarter, p.row, b4, y);
+            const float e0 = y[0] - t0, e1 = y[1] - t1;
+            const float u = fabsf(e0) - y[2];
             d0 = 2.f * g.w_d * e0 * inv_b;
             d1 = 2.f * g.w_a * e1 * inv_b;
             d2 = g.w_e * (u < 0.f ? 1.f - kQuantile : -kQuantile) * inv_b;
-            if (!odd) {
+            if (p.group == 0) {
                 const float pin = u >= 0.f ? kQuantile * u : (kQuantile - 1.f) * u;
                 ls += (g.w_d * e0 * e0 + g.w_a * e1 * e1 + g.w_e * pin) * inv_b;
                 gb[0] += d0;
                 gb[1] += d1;
                 gb[2] += d2;
-                g.y[r * kOut] = y0;
-                g.y[r * kOut + 1] = y1;
-                g.y[r * kOut + 2] = y2;
+                g.y[r * kOut] = y[0];
+                g.y[r * kOut + 1] = y[1];
+                g.y[r * kOut + 2] = y[2];
             }
         }
-        if (!odd) S.dy[p.row] = make_float4(d0, d1, d2, 0.f);
+        if (p.group == 0) S.dy[p.row] = make_float4(d0, d1, d2, 0.f);
         __syncthreads();
 #pragma unroll 1
         for (int i = 0; i < kTileM; i += 32) {
             const float4 d = S.dy[i + lane];
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
+            for (int q = 0; q < kWarpVecs; q++) {
                 float h[8];
-                unpack8(*reinterpret_cast<const uint4 *>(S.a + (4 * warp + q) * kActStride +
+                unpack8(*reinterpret_cast<const uint4 *>(S.a + (kWarpVecs * warp + q) * kActStride +
                                                          (i + lane) * 16),
                         h);
 #pragma unroll
@@ -870,13 +850,13 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
         __syncthreads();
         // dz3 in h3's place
 #pragma unroll 1
-        for (int q = 0; q < 16; q++) {
-            uint4 *at = reinterpret_cast<uint4 *>(image + (2 * q + odd) * kActStride);
+        for (int q = 0; q < kMine; q++) {
+            uint4 *at = reinterpret_cast<uint4 *>(image + (4 * q + p.group) * kActStride);
             const unsigned m = positive8(*at);
             float dz[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const float4 w = S.w4[16 * q + 8 * odd + j];
+                const float4 w = S.w4[32 * q + 8 * p.group + j];
                 const float v = fmaf(d0, w.x, fmaf(d1, w.y, d2 * w.z));
                 dz[j] = (m >> j) & 1u ? v : 0.f;
             }
@@ -898,16 +878,16 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
         }
         unsigned char *d2_out = g.d2 + (size_t)t * kActBytes + p.row * 16;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int c0 = 32 * i + 8 * odd;
+        for (int i = 0; i < kMine / 2; i++) {
+            const int c0 = 64 * i + 8 * p.group;
             float v[2][8];
-            tc_ld8x2(p.tmem + kH + c0, p.tmem + kH + c0 + 16, v[0], v[1]);
+            tc_ld8x2(p.tmem + kH + c0, p.tmem + kH + c0 + 32, v[0], v[1]);
 #pragma unroll
             for (int q = 0; q < 2; q++) {
 #pragma unroll
                 for (int j = 0; j < 8; j++)
                     v[q][j] = (mask[i >> 1] >> (16 * (i & 1) + 8 * q + j)) & 1u ? v[q][j] : 0.f;
-                *reinterpret_cast<uint4 *>(d2_out + (size_t)(4 * i + 2 * q + odd) * kActStride) =
+                *reinterpret_cast<uint4 *>(d2_out + (size_t)(8 * i + 4 * q + p.group) * kActStride) =
                     pack8(v[q]);
             }
         }
@@ -917,7 +897,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
     // this CTA's sums, each over its lanes in a fixed order
     float *out = g.part4 + (size_t)blockIdx.x * kPart4;
 #pragma unroll
-    for (int q = 0; q < 4; q++)
+    for (int q = 0; q < kWarpVecs; q++)
 #pragma unroll
         for (int j = 0; j < 8; j++)
 #pragma unroll
@@ -925,7 +905,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
                 float s = gw[q][j][o];
 #pragma unroll
                 for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-                if (lane == 0) out[((4 * warp + q) * 8 + j) * kOut + o] = s;
+                if (lane == 0) out[((kWarpVecs * warp + q) * 8 + j) * kOut + o] = s;
             }
     const float tail[kOut + 1] = {gb[0], gb[1], gb[2], ls};
 #pragma unroll
@@ -933,13 +913,13 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
         float s = tail[o];
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-        if (lane == 0) S.sum4[warp][o] = s;
+        if (lane == 0 && warp < 4) S.sum4[warp][o] = s;  // (the first group's rows)
     }
     tc_fence_before();
     __syncthreads();
     if (tid <= kOut) {
         float s = 0.f;
-        for (int w = 0; w < 4; w++) s += S.sum4[w][tid];  // warps 0 .. 3 hold the rows
+        for (int w = 0; w < 4; w++) s += S.sum4[w][tid];
         out[kH * kOut + tid] = s;
     }
     if (tid < 32) tmem_free(tmem, 512);
@@ -986,7 +966,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_back2(Back2 g) {
         mbar_expect(&S.wbar, kWBytes);
         bulk_load(S.w2, g.W->w2, kWBytes, &S.wbar);
     }
-    const Part p = my_part(tmem);
+    const Part p = my_part<kGroups>(tmem);
     bool ok = cta_wait(&S.wbar, 0, g.status);
     unsigned phase = 0;
     for (int t = blockIdx.x; ok && t < g.tiles; t += gridDim.x, phase ^= 1) {
@@ -997,10 +977,11 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_back2(Back2 g) {
             mma_layer_back(tmem, smem_u32(S.a), smem_u32(S.w2));
             tc_commit(&S.mbar);
         }
-        unsigned mask[4];
+        constexpr int kParts = kH / kGroups / 32;  // of 32 columns
+        unsigned mask[kParts];
         const unsigned char *h = g.h1 + (size_t)t * kActBytes + p.row * 16;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < kParts; q++) {
             mask[q] = 0;
 #pragma unroll
             for (int j = 0; j < 4; j++)
@@ -1013,7 +994,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_back2(Back2 g) {
         tc_fence_after();
         if (tid == 0 && t + (int)gridDim.x < g.tiles) load(t + gridDim.x);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < kParts; i++) {
             const int c0 = p.col0 + 32 * i;
             float v[32];
             tc_ld32(p.tmem + c0, v);
@@ -1042,6 +1023,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_back2(Back2 g) {
 // W3 and W2, the others those of W1 (a ninth of the products but half of the
 // bytes).
 constexpr int kSplitTiles = 4;
+constexpr int kThreadsW = 256;  // eight warps sum and store; one more feeds the tensor core
 struct Wgrad {
     const unsigned char *h1, *h2, *x, *d1, *d2, *d3;
     int tiles, splits, big;
@@ -1056,7 +1038,7 @@ struct __align__(1024) SmemW {
     unsigned tmem;
 };
 
-__global__ void __launch_bounds__(kThreads3, 1) mlp_wgrad(Wgrad g) {
+__global__ void __launch_bounds__(kThreadsW + 32, 1) mlp_wgrad(Wgrad g) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     SmemW &S = *reinterpret_cast<SmemW *>(smem_raw +
                                           ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
@@ -1079,8 +1061,8 @@ __global__ void __launch_bounds__(kThreads3, 1) mlp_wgrad(Wgrad g) {
     const int step = first ? gridDim.x - g.big : g.big;
     const int items = first ? g.splits : 2 * g.splits;
     bool ok = true;
-    if (tid >= kThreads) {
-        if (tid == kThreads) {
+    if (tid >= kThreadsW) {
+        if (tid == kThreadsW) {
             // loads: of each tile the activations (or features), then the
             // layer's gradient, into the three buffers in turn, a tile and a
             // half ahead of the products
@@ -1149,7 +1131,7 @@ __global__ void __launch_bounds__(kThreads3, 1) mlp_wgrad(Wgrad g) {
             }
         }
     } else {
-        const Part p = my_part(tmem);
+        const Part p = my_part<2>(tmem);
         int used = 0, n = 0;
         for (int item = item0; item < items; item += step, n++) {
             const int prod = first ? 2 : item / g.splits;
@@ -1365,6 +1347,358 @@ __global__ void __launch_bounds__(256) mlp_finish(Finish g) {
     }
 }
 
+// ---- inference ---------------------------------------------------------------
+
+// The whole network in one launch, activations never leaving the SM: no SM's
+// shared memory holds W1, W2 and W3 (264 kB), so the two CTAs of a cluster
+// hold half of the outputs' columns of each, and their products are of 256
+// rows (cta_group::2): 128 rows of each CTA's own against both halves.
+//
+// X and Y are the two accumulators (256 columns each, all of tensor memory)
+// and h the tile's activations in shared memory, whose halves (128 features)
+// are written and multiplied one after the other.  Tile n has P = X and Q = Y
+// for even n, the other way round for odd:
+//   product warp (of the first CTA)      sixteen epilogue warps (of both)
+//                                          P -> h half 0 (layer 1)
+//     layer 2, half 0: h -> Q              Q -> registers (n - 1's layer 3)
+//     layer 2, half 1                      P -> h half 1
+//                                          outputs of n - 1, two of their
+//                                            four parts
+//     layer 1 of n + 1 -> Q, half 0        Q -> h half 0 (layer 2)
+//     layer 3, half 0: h -> P              Q -> h half 1
+//     layer 1 of n + 1 -> Q, half 1        outputs of n - 1, the other two
+//     layer 3, half 1: h -> P
+// The products hide the outputs of the tile before.  Two warps compute
+// features a tile ahead.
+//
+// Clocks per tile and SM, of which the products are 4,200 (3.2 million rows):
+//   12,800  layers 1 and 2, then layer 3 and the outputs, as launches of five
+//           tiles an SM with layer 2's activations through L2: every launch
+//           reloads the weights, and of a tile's 6,100 + 4,400 clocks its
+//           features, the products' issue and layer 1's epilogue come one
+//           after the other
+//   15,000  one CTA of a pair layers 1 and 2, the other layer 3, through a
+//           ring in L2: an SM stores 32 bytes a clock, 2,000 clocks a tile
+//    8,700  this: 1,130 -> 740 us
+// What is left is the chain of a tile's three products and the halves of
+// epilogues between them (about 600 clocks each, and 300 for every hand-over
+// between the CTAs); shared memory has no room for a second tile of h.
+constexpr int kFeatureWarps = 2;
+constexpr int kThreadsP = kThreads + 32 + 32 * kFeatureWarps;
+constexpr int kPairRows = 2 * kTileM;
+
+struct Predict {
+    FeatureTables F;
+    Batch batch;
+    const BfWeights *W;
+    const float *b1, *b2, *b3, *b4;
+    float *y;   // [nrows][3]
+    int pairs;  // of tiles
+    int *status;
+};
+struct __align__(1024) SmemP {
+    unsigned char w2[kWBytes / 2], w3[kWBytes / 2];  // [in / 8][this CTA's 128 outputs][8 in]
+    unsigned char h[kActBytes];
+    unsigned char w1[2][kW1Bytes / 4];  // the same of each half of layer 1's outputs
+    unsigned char x[2][kXBytes];
+    float4 w4xy[kH / 2];  // features c and c + 128: the weights of output 0, of output 1
+    float2 w4z[kH / 2];   // and of output 2
+    float b1[kH], b2[kH], b3[kH], norm[2 * kF];
+    float4 quarter[kGroups][kTileM];  // a row's outputs by parts
+    // the first CTA's: what the warps of both have done
+    unsigned long long hfull[2], qfree, xfull[2], other_w;
+    // products done (both CTAs'); this CTA's own
+    unsigned long long l1done, l2done, h0free, l3done, xfree[2], wbar, parts;
+    unsigned tmem;
+};
+
+template <int n>
+__device__ __forceinline__ void tc_mma_pair(unsigned d_tmem, unsigned long long a,
+                                            unsigned long long b, bool accumulate) {
+    // as tc_idesc, M = 256
+    constexpr unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) |
+                               ((unsigned)(kPairRows >> 4) << 24);
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "l"(a), "l"(b), "r"(idesc), "r"((unsigned)accumulate)
+        : "memory");
+}
+// Arrives at the barrier of both CTAs when the products so far are done.
+__device__ __forceinline__ void tc_commit_pair(unsigned long long *bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
+        " [%0], %1;" ::"r"(smem_u32(bar)),
+        "h"((unsigned short)3)
+        : "memory");
+}
+// 128 of the 256 features of a layer; a, w: the first of each CTA's own
+__device__ __forceinline__ void mma_half_pair(unsigned d, unsigned a, unsigned w,
+                                              bool accumulate) {
+#pragma unroll
+    for (int kk = 0; kk < 8; kk++)
+        tc_mma_pair<kH>(d, smem_desc(a + 2 * kActStride * kk, kActStride, 128),
+                        smem_desc(w + kWStride * kk, kWStride / 2, 128), accumulate || kk > 0);
+}
+__device__ __forceinline__ void tmem_alloc_pair(unsigned *base) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     smem_u32(base))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free_pair(unsigned base) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(base) : "memory");
+}
+
+// relu(v + bias) of two features as BF16
+__device__ __forceinline__ unsigned relu_pair(float2 v, float2 bias) {
+    const float2 h = add2(v, bias);
+    const __nv_bfloat162 o = __floats2bfloat162_rn(fmaxf(h.x, 0.0f), fmaxf(h.y, 0.0f));
+    return *reinterpret_cast<const unsigned *>(&o);
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsP, 1) mlp_predict(Predict g) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    SmemP &S = *reinterpret_cast<SmemP *>(smem_raw +
+                                          ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned rank = cluster_rank();
+    const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
+    constexpr int kWarps = kThreads / 32;  // of the epilogue
+    pdl_launch_dependents();
+    if (tid < 32) tmem_alloc_pair(&S.tmem);
+    if (tid == 0) {
+        mbar_init(&S.wbar, 1);
+        mbar_init(&S.other_w, 1);
+        mbar_init(&S.parts, kWarps);
+        mbar_init(&S.qfree, 2 * kWarps);
+        mbar_init(&S.l1done, 1);
+        mbar_init(&S.l2done, 1);
+        mbar_init(&S.l3done, 1);
+        mbar_init(&S.h0free, 1);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&S.hfull[i], 2 * kWarps);
+            mbar_init(&S.xfull[i], 2 * kFeatureWarps);
+            mbar_init(&S.xfree[i], 1);
+        }
+    }
+    pdl_wait();
+    if (tid < kF) {
+        S.norm[tid] = g.F.mu[tid];
+        S.norm[kF + tid] = g.F.isd[tid];
+    }
+    if (tid < kH) {
+        S.b1[tid] = g.b1[tid];
+        S.b2[tid] = g.b2[tid];
+        S.b3[tid] = g.b3[tid];
+    }
+    if (tid < kH / 2) {
+        const float4 a = g.W->w4[tid], b = g.W->w4[tid + kH / 2];
+        S.w4xy[tid] = make_float4(a.x, b.x, a.y, b.y);
+        S.w4z[tid] = make_float2(a.z, b.z);
+    }
+    tc_sync();
+    cluster_sync();
+    const unsigned tmem = S.tmem;
+    bool ok = true;
+    if (warp == kWarps) {
+        if (lane == 0) {
+            // this CTA's columns of the weights
+            mbar_expect(&S.wbar, kWBytes + kW1Bytes / 2);
+            constexpr unsigned kCols = kWStride / 2;  // bytes of 128 outputs, 8 inputs
+            const auto load = [&](unsigned char *dst, const void *src, int vecs, unsigned from,
+                                  unsigned bytes) {
+                for (int i = 0; i < vecs; i++)
+                    bulk_load(dst + i * bytes,
+                              static_cast<const unsigned char *>(src) + i * kWStride + from, bytes,
+                              &S.wbar);
+            };
+            for (int half = 0; half < 2; half++)
+                load(S.w1[half], g.W->w1, kF / 8, half * kCols + rank * (kCols / 2), kCols / 2);
+            load(S.w2, g.W->w2, kH / 8, rank * kCols, kCols);
+            load(S.w3, g.W->w3, kH / 8, rank * kCols, kCols);
+            ok = mbar_wait(&S.wbar, 0, g.status);
+            if (ok && rank != 0) mbar_arrive_at(&S.other_w, 0);
+            const unsigned h = smem_u32(S.h), w2 = smem_u32(S.w2), w3 = smem_u32(S.w3);
+            const auto wait = [&](unsigned long long *bar, unsigned parity) {
+                ok = ok && mbar_wait(bar, parity, g.status);
+                tc_fence_after();
+            };
+            const auto layer1 = [&](int n, int half) {
+                wait(&S.xfull[n & 1], (n >> 1) & 1);
+                if (!ok) return;
+                tc_mma_pair<kH / 2>(tmem + (n & 1) * kH + half * (kH / 2),
+                                    smem_desc(smem_u32(S.x[n & 1]), kActStride, 128),
+                                    smem_desc(smem_u32(S.w1[half]), kCols / 2, 128), false);
+                if (half) tc_commit_pair(&S.xfree[n & 1]);
+            };
+            int n = 0, t = first;
+            if (rank != 0) t = g.pairs;
+            if (ok && t < g.pairs) {
+                wait(&S.other_w, 0);
+                layer1(0, 0);
+                layer1(0, 1);
+                if (ok) tc_commit_pair(&S.l1done);
+            }
+            for (; ok && t < g.pairs; t += stride, n++) {
+                const unsigned p = tmem + (n & 1) * kH, q = tmem + (~n & 1) * kH;
+                const bool more = t + stride < g.pairs;
+                wait(&S.hfull[0], 0);
+                if (n) wait(&S.qfree, (n - 1) & 1);
+                if (!ok) break;
+                mma_half_pair(q, h, w2, false);
+                wait(&S.hfull[1], 0);
+                if (!ok) break;
+                mma_half_pair(q, h + 16 * kActStride, w2 + 16 * kCols, true);
+                tc_commit_pair(&S.l2done);
+                wait(&S.hfull[0], 1);  // (Q's first half has been read)
+                if (more) layer1(n + 1, 0);
+                if (!ok) break;
+                mma_half_pair(p, h, w3, false);
+                tc_commit_pair(&S.h0free);
+                wait(&S.hfull[1], 1);  // (and its second)
+                if (more) layer1(n + 1, 1);
+                if (!ok) break;
+                mma_half_pair(p, h + 16 * kActStride, w3 + 16 * kCols, true);
+                tc_commit_pair(&S.l3done);
+            }
+        }
+    } else if (warp > kWarps) {
+        const int row = tid - kThreads - 32;
+        int n = 0;
+        for (int t = first; ok && t < g.pairs; t += stride, n++) {
+            const int b = n & 1;
+            if (n >= 2) ok = __all_sync(~0u, mbar_wait(&S.xfree[b], ((n >> 1) - 1) & 1, g.status));
+            if (!ok) break;
+#pragma unroll
+            for (int i = row; i < kTileM; i += 32 * kFeatureWarps)
+                tile_features(g.F, g.batch, S.norm,
+                              (long long)t * kPairRows + (int)rank * kTileM + i, i, S.x[b]);
+            proxy_fence();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_at(&S.xfull[b], 0);
+        }
+    } else {
+        const Part p = my_part<kGroups>(tmem);
+        const int c0 = 32 * p.group;  // this warp's columns of each half of a layer
+        const int row0 = 32 * (warp & 3) + lane / 4;  // the first of this thread's four rows
+        const float b4[kOut] = {g.b4[0], g.b4[1], g.b4[2]};
+        const auto wait = [&](unsigned long long *bar, unsigned parity) {
+            if (ok) ok = __all_sync(~0u, mbar_wait(bar, parity, g.status));
+            tc_fence_after();
+        };
+        const int quad = lane & 3;
+        const auto hidden_half = [&](unsigned acc, int half, const float *bias) {
+            const int c = 128 * half + c0;
+            float2 v[4][4];
+            tc_ld_quads(p.tmem + acc + c, v);
+            unsigned char *out = S.h + (c / 8) * kActStride + row0 * 16 + quad * 4;
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const float2 bb = *reinterpret_cast<const float2 *>(bias + c + 8 * b + 2 * quad);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    *reinterpret_cast<unsigned *>(out + b * kActStride + i * 128) =
+                        relu_pair(v[b][i], bb);
+            }
+            proxy_fence();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_at(&S.hfull[half], 0);
+        };
+        // Layer 3 of tile n as BF16, which frees its accumulator: of the row of
+        // this thread's lane, h3[m] is vector 4 m + group of eight features.
+        uint4 h3[8];
+        const auto read_layer3 = [&](int n) {
+            wait(&S.l3done, n & 1);
+            if (!ok) return;
+            float v[8][8];
+            tc_ld8x8(p.tmem + (n & 1) * kH + 8 * p.group, v);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_at(&S.qfree, 0);
+#pragma unroll
+            for (int m = 0; m < 8; m++) {
+                bias_relu<8>(v[m], S.b3, 32 * m + 8 * p.group);
+                h3[m] = pack8(v[m]);
+            }
+        };
+        // Outputs of tile n: head_quarter's sums, those of two vectors 16 apart
+        // side by side in the two halves of an instruction.
+        const auto outputs = [&](int n) {
+            constexpr int order[4] = {0, 2, 1, 3};
+            float pair[kOut], sum[kOut], y[kOut];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int m = order[i], c = 32 * m + 8 * p.group;
+                const unsigned lo[4] = {h3[m].x, h3[m].y, h3[m].z, h3[m].w};
+                const unsigned hi[4] = {h3[m + 4].x, h3[m + 4].y, h3[m + 4].z, h3[m + 4].w};
+                float2 s[kOut];
+#pragma unroll
+                for (int o = 0; o < kOut; o++) s[o] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const unsigned a = j & 1 ? lo[j / 2] & 0xffff0000u : lo[j / 2] << 16;
+                    const unsigned b = j & 1 ? hi[j / 2] & 0xffff0000u : hi[j / 2] << 16;
+                    const float2 h = make_float2(__uint_as_float(a), __uint_as_float(b));
+                    const float4 w = S.w4xy[c + j];
+                    s[0] = fma2(h, make_float2(w.x, w.y), s[0]);
+                    s[1] = fma2(h, make_float2(w.z, w.w), s[1]);
+                    s[2] = fma2(h, S.w4z[c + j], s[2]);
+                }
+#pragma unroll
+                for (int o = 0; o < kOut; o++) {
+                    const float a = s[o].x + s[o].y;
+                    if (i % 2 == 0)
+                        pair[o] = a;
+                    else if (i == 1)
+                        sum[o] = pair[o] + a;
+                    else
+                        y[o] = sum[o] + (pair[o] + a);
+                }
+            }
+            S.quarter[p.group][p.row] = make_float4(y[0], y[1], y[2], 0.f);
+            // (a part is written again after layer 3 of the next tile, for which
+            // all of the warps have gone on)
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.parts);
+            if (p.group != (n & (kGroups - 1))) return;
+            wait(&S.parts, n & 1);
+            const long long r = (long long)(first + n * stride) * kPairRows + (int)rank * kTileM +
+                                p.row;
+            if (ok && r < g.batch.nrows) {
+                row_outputs(S.quarter, p.row, b4, y);
+                g.y[r * kOut] = y[0];
+                g.y[r * kOut + 1] = y[1];
+                g.y[r * kOut + 2] = y[2];
+            }
+        };
+        int n = 0;
+        for (int t = first; ok && t < g.pairs; t += stride, n++) {
+            const unsigned P = (n & 1) * kH, Q = (~n & 1) * kH;
+            if (n)
+                wait(&S.h0free, (n - 1) & 1);  // (and layer 1's first half)
+            else
+                wait(&S.l1done, 0);
+            if (!ok) break;
+            hidden_half(P, 0, S.b1);
+            if (n) read_layer3(n - 1);  // (and so layer 1's second half)
+            if (!ok) break;
+            hidden_half(P, 1, S.b1);
+            if (n) outputs(n - 1);
+            wait(&S.l2done, n & 1);
+            if (!ok) break;
+            hidden_half(Q, 0, S.b2);
+            hidden_half(Q, 1, S.b2);
+        }
+        if (ok && n) read_layer3(n - 1);
+        if (ok && n) outputs(n - 1);
+    }
+    tc_fence_before();
+    cluster_sync();  // both are done with tensor memory and with each other's barriers
+    if (tid < 32) tmem_free_pair(tmem);
+}
+
 // ---- weights ----------------------------------------------------------------
 
 __global__ void mlp_pack_weights(const float *__restrict__ p, BfWeights *W) {
@@ -1390,7 +1724,6 @@ __global__ void mlp_pack_weights(const float *__restrict__ p, BfWeights *W) {
 
 struct Buffers {  // one batch of rows (training) or one chunk (inference)
     int tiles = 0;
-    bool train = false;
     unsigned char *h2 = nullptr;                    // tile images
     unsigned char *x = nullptr, *h1 = nullptr, *d3 = nullptr, *d2 = nullptr, *d1 = nullptr;
     long long *row_of = nullptr;
@@ -1459,30 +1792,27 @@ int wgrad_splits(int tiles) { return (tiles + kSplitTiles - 1) / kSplitTiles; }
 
 // Buffers for `tiles` tiles of 128 rows, reallocated only when they grow or
 // when training needs the gradients' images.
-int ensure_buffers(Mlp *m, int tiles, bool train, std::vector<void *> &owned) {
+int ensure_buffers(Mlp *m, int tiles, std::vector<void *> &owned) {
     Buffers &B = m->buf;
-    if (tiles <= B.tiles && (B.train || !train)) return SWGPU_OK;
+    if (tiles <= B.tiles) return SWGPU_OK;
     MCK(cudaStreamSynchronize(m->stream));
     free_list(owned);
     B = Buffers{};
     int rc;
     const size_t act = (size_t)tiles * kActBytes, rows = (size_t)tiles * kTileM;
-    if ((rc = malloc_dev(m, &B.h2, act, &owned))) return rc;
-    if (train) {
-        const size_t s = wgrad_splits(tiles);
-        if ((rc = malloc_dev(m, &B.x, (size_t)tiles * kXBytes, &owned)) ||
-            (rc = malloc_dev(m, &B.h1, act, &owned)) || (rc = malloc_dev(m, &B.d3, act, &owned)) ||
-            (rc = malloc_dev(m, &B.d2, act, &owned)) || (rc = malloc_dev(m, &B.d1, act, &owned)) ||
-            (rc = malloc_dev(m, &B.row_of, rows, &owned)) ||
-            (rc = malloc_dev(m, &B.y, rows * kOut, &owned)) ||
-            (rc = malloc_dev(m, &B.part, s * 2 * kH * kH, &owned)) ||
-            (rc = malloc_dev(m, &B.part1, s * kF * kH, &owned)) ||
-            (rc = malloc_dev(m, &B.part_b, s * 3 * kH, &owned)) ||
-            (rc = malloc_dev(m, &B.part4, (size_t)std::min(tiles, m->sms) * kPart4, &owned)))
-            return rc;
-    }
+    const size_t s = wgrad_splits(tiles);
+    if ((rc = malloc_dev(m, &B.h2, act, &owned)) ||
+        (rc = malloc_dev(m, &B.x, (size_t)tiles * kXBytes, &owned)) ||
+        (rc = malloc_dev(m, &B.h1, act, &owned)) || (rc = malloc_dev(m, &B.d3, act, &owned)) ||
+        (rc = malloc_dev(m, &B.d2, act, &owned)) || (rc = malloc_dev(m, &B.d1, act, &owned)) ||
+        (rc = malloc_dev(m, &B.row_of, rows, &owned)) ||
+        (rc = malloc_dev(m, &B.y, rows * kOut, &owned)) ||
+        (rc = malloc_dev(m, &B.part, s * 2 * kH * kH, &owned)) ||
+        (rc = malloc_dev(m, &B.part1, s * kF * kH, &owned)) ||
+        (rc = malloc_dev(m, &B.part_b, s * 3 * kH, &owned)) ||
+        (rc = malloc_dev(m, &B.part4, (size_t)std::min(tiles, m->sms) * kPart4, &owned)))
+        return rc;
     B.tiles = tiles;
-    B.train = train;
     return SWGPU_OK;
 }
 
@@ -1518,7 +1848,7 @@ FeatureTables tables(const Mlp *m) {
 }
 
 // Layers 1 and 2 of a batch into the buffers.
-int layers12(Mlp *m, const Batch &batch, int tiles, bool train) {
+int layers12(Mlp *m, const Batch &batch, int tiles) {
     Buffers &B = m->buf;
     Layers12 g{};
     g.F = tables(m);
@@ -1532,8 +1862,8 @@ int layers12(Mlp *m, const Batch &batch, int tiles, bool train) {
     g.row_of = B.row_of;
     g.tiles = tiles;
     g.status = m->status;
-    return launch(m, train ? mlp_layers12<true> : mlp_layers12<false>,
-                  dim3((unsigned)std::min(tiles, m->sms)), kThreads, smem_of<Smem12>(), g);
+    return launch(m, mlp_layers12, dim3((unsigned)std::min(tiles, m->sms)), kThreads,
+                  smem_of<Smem12>(), g);
 }
 
 Layer3 layer3(Mlp *m, int tiles, long long nrows, float *y) {
@@ -1554,12 +1884,12 @@ Layer3 layer3(Mlp *m, int tiles, long long nrows, float *y) {
 int batch_gradients(Mlp *m, const long long *d_rows, unsigned long long seed, long long nrows,
                     float w_d, float w_a, float w_e, const Adam *adam) {
     const int tiles = (int)((nrows + kTileM - 1) / kTileM);
-    int rc = ensure_buffers(m, tiles, true, m->buf_allocs);
+    int rc = ensure_buffers(m, tiles, m->buf_allocs);
     if (rc) return rc;
     Buffers &B = m->buf;
     const unsigned ctas = (unsigned)std::min(tiles, m->sms);
     Batch batch{d_rows, seed, d_rows ? 0 : m->S * m->N, 0, nrows};
-    if ((rc = layers12(m, batch, tiles, true))) return rc;
+    if ((rc = layers12(m, batch, tiles))) return rc;
     Layer3 g3 = layer3(m, tiles, nrows, B.y);
     g3.targets = m->targets;
     g3.row_of = B.row_of;
@@ -1579,7 +1909,7 @@ int batch_gradients(Mlp *m, const long long *d_rows, unsigned long long seed, lo
     const int small = std::max(1, std::min(s, m->sms - big));
     Wgrad gw{B.h1, B.h2, B.x, B.d1, B.d2, B.d3, tiles, s, big, B.part, B.part1, B.part_b,
              m->status};
-    if ((rc = launch(m, mlp_wgrad, dim3((unsigned)(big + small)), kThreads3, smem_of<SmemW>(), gw)))
+    if ((rc = launch(m, mlp_wgrad, dim3((unsigned)(big + small)), kThreadsW + 32, smem_of<SmemW>(), gw)))
         return rc;
     Finish gf{B.part, B.part1, B.part_b, B.part4, s, (int)ctas, adam ? nullptr : m->grad, m->loss,
               adam ? *adam : Adam{}, m->w};
@@ -1618,9 +1948,8 @@ int swgpu_mlp_create(const float *params, const float *feature_mean,
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = smem_attr(mlp_layers12<false>, smem_of<Smem12>());
-    if (e == cudaSuccess) e = smem_attr(mlp_layers12<true>, smem_of<Smem12>());
-    if (e == cudaSuccess) e = smem_attr(mlp_layer3_predict, smem_of<Smem3>());
+    if (e == cudaSuccess) e = smem_attr(mlp_predict, smem_of<SmemP>());
+    if (e == cudaSuccess) e = smem_attr(mlp_layers12, smem_of<Smem12>());
     if (e == cudaSuccess) e = smem_attr(mlp_layer3_train, smem_of<Smem3T>());
     if (e == cudaSuccess) e = smem_attr(mlp_back2, smem_of<SmemB>());
     if (e == cudaSuccess) e = smem_attr(mlp_wgrad, smem_of<SmemW>());
@@ -1713,21 +2042,21 @@ int swgpu_mlp_predict(void *handle, int64_t row0, int64_t nrows, float *out_devi
     if (!m || !out_device || nrows <= 0 || row0 < 0 || row0 + nrows > m->S * m->N)
         return mfail(m, SWGPU_EINVAL, "swgpu_mlp_predict: bad rows");
     if (int rc = usable(m, "swgpu_mlp_predict")) return rc;
-    // chunks of five tiles per SM (48 MB of layer 2's activations): what one
-    // kernel leaves, the next finds in L2
-    const long long chunk = std::min<long long>(nrows, 5LL * m->sms * kTileM);
-    int rc = ensure_buffers(m, (int)((chunk + kTileM - 1) / kTileM), false, m->buf_allocs);
-    if (rc) return rc;
+    const int most = std::max(1, m->sms / 2);  // pairs of CTAs
+    int rc = SWGPU_OK;
     cudaEvent_t a, b;
     MCK(cudaEventCreate(&a));
     MCK(cudaEventCreate(&b));
     MCK(cudaEventRecord(a, m->stream));
+    const long long chunk = (1LL << 24) * kTileM;  // (the tiles of a launch are counted in an int)
     for (long long r0 = 0; r0 < nrows; r0 += chunk) {
         const long long n = std::min(chunk, nrows - r0);
-        const int tiles = (int)((n + kTileM - 1) / kTileM);
-        if ((rc = layers12(m, Batch{nullptr, 0, 0, row0 + r0, n}, tiles, false))) return rc;
-        if ((rc = launch(m, mlp_layer3_predict, dim3((unsigned)std::min(tiles, m->sms)), kThreads3,
-                         smem_of<Smem3>(), layer3(m, tiles, n, out_device + r0 * kOut))))
+        const int pairs = (int)((n + kPairRows - 1) / kPairRows);
+        const Predict g{tables(m), Batch{nullptr, 0, 0, row0 + r0, n}, m->w, m->params + kOffB1,
+                        m->params + kOffB2, m->params + kOffB3, m->params + kOffB4,
+                        out_device + r0 * kOut, pairs, m->status};
+        if ((rc = launch(m, mlp_predict, dim3(2u * (unsigned)std::min(pairs, most)), kThreadsP,
+                         smem_of<SmemP>(), g)))
             return rc;
     }
     MCK(cudaEventRecord(b, m->stream));
