@@ -817,8 +817,24 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     h->ntags = (int)(maxtag + 1);
     h->nscen = offsets ? nscen : 1;
     TRY(dalloc(h, &h->d_tags, (size_t)std::max(h->ntags, 1)));  // zero = reflective
-    if (precision == SWGPU_MIXED && h->nscen == 1)
-        TRY(dalloc(h, &h->X.tag_values, (size_t)std::max(h->ntags, 1)));
+    if (precision == SWGPU_MIXED) {
+        TRY(dalloc(h, &h->d_tag_values, (size_t)std::max(h->ntags, 1)));
+        if (offsets) {
+            const int unused = -2, several = -1;
+            h->tag_scen.assign((size_t)std::max(h->ntags, 1), unused);
+            for (int64_t m = 0; m < mesh->number_of_boundary_elements; m++) {
+                int &t = h->tag_scen[(size_t)mesh->boundary_tag[m]];
+                const int owner = tri_scen[(size_t)mesh->boundary_cells[m]];
+                t = t == unused || t == owner ? owner : several;
+            }
+            std::vector<int> scen(h->tag_scen);
+            for (int &t : scen) t = std::max(t, 0);
+            int *d = nullptr;
+            TRY(dalloc(h, &d, scen.size()));
+            TRY(upload(h, d, scen.data(), scen.size()));
+            h->X.tag_scen = d;
+        }
+    }
     TRY(dalloc(h, &h->d_ctrl, (size_t)h->nscen));
     TRY(dalloc(h, &h->d_summary, 1));
     const int nwords = (h->nscen + 31) / 32;
@@ -951,19 +967,24 @@ int swgpu_set_boundary_tags(void *handle, const swgpu_boundary_tag *tags, int nt
         for (int j = 0; j < 8; j++) t[i].p[j] = tags[i].p[j];
     }
     const int n = std::max(h->ntags, 1);
-    // a mixed mesh's time-dependent tags are evaluated once per stage, by a
-    // block of the update (an ensemble's scenarios have clocks of their own)
+    // a mixed mesh's time-dependent tags are evaluated once per stage, by blocks
+    // of the update (unless scenarios, which have clocks of their own, share one)
     int time_tags = 0;
-    if (h->X.tag_values)
+    bool shared = false;
+    if (h->d_tag_values)
         for (int i = 0; i < std::min(ntags, h->ntags); i++)
             if (t[i].type == SWGPU_BC_TIME_STAGE_SINE ||
                 t[i].type == SWGPU_BC_TIME_STAGE_FOURIER ||
-                t[i].type == SWGPU_BC_INFLOW_HYDROGRAPH)
+                t[i].type == SWGPU_BC_INFLOW_HYDROGRAPH) {
                 time_tags = h->ntags;
+                shared = shared || (!h->tag_scen.empty() && h->tag_scen[(size_t)i] == -1);
+            }
+    if (shared) time_tags = 0;
     if (time_tags != h->time_tags) {
         CK(cudaStreamSynchronize(h->stream));
         drop_graphs(h);  // the update's launch changes
         h->time_tags = time_tags;
+        h->X.tag_values = time_tags ? h->d_tag_values : nullptr;
     }
     return upload(h, h->d_tags, t.data(), (size_t)std::min(ntags, n));
 }

@@ -24,6 +24,8 @@ struct Handle {
     BcTag *d_tags = nullptr;
     int ntags = 0;
     int time_tags = 0;           // mixed: tags evaluated once per stage (0: none depends on time)
+    TagValue *d_tag_values = nullptr;  // mixed: X.tag_values where time_tags is set
+    std::vector<int> tag_scen;   // ensemble: scenario whose edges have the tag (-1: several)
     int steps_per_graph = kStepsPerGraph;
     float *trk_hmax = nullptr, *trk_tarr = nullptr;  // tracking buffers (S.hmax/S.tarr when on)
     int nscen = 1;               // scenarios (Ctrl blocks); > 1 for an ensemble

@@ -145,7 +145,8 @@ struct DevMixed {
                                    // FP32 pair hi + lo
 
     TagValue *tag_values;          // [tags] time-dependent boundaries at the stage's end (null:
-                                   // evaluated edge by edge, as for an ensemble's many clocks)
+                                   // evaluated edge by edge)
+    const int *tag_scen;           // ensembles: [tags] the scenario whose edges have the tag
     int *surrp;                    // [3][S] DevMesh::surr in padded planes (TMA-staged)
     uint8_t *kind;                 // [S] 0 aux triangle, 1 one neighbour (slot<<2), 2 flat;
                                    // | 16: the triangle has a boundary edge
