@@ -109,6 +109,10 @@ __host__ __device__ inline bool boundary_keeps_edge_stage(int type) {
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// The same at the place `when` (0, kStartMid, kStartEnd) of a mixed step kernel.
+__device__ __forceinline__ void pdl_launch_at(int when, int flags) {
+    if ((flags & (kStartMid | kStartEnd)) == when) pdl_launch_dependents();
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Snapshot of the time bookkeeping taken at kernel entry.

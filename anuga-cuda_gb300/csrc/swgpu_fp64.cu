@@ -237,7 +237,6 @@ __device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevPa
 // radius is infinite for an edge that does not count (owner not full).
 __global__ void __launch_bounds__(kBlock) flux_fp64(DevMesh M, DevState S, DevParams P,
                                                     Ctrl *ctrl, int flags) {
-    pdl_launch_dependents();
     const DevEdges &F = M.edges;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (F.blk_scen) ctrl += F.blk_scen[(blockIdx.x * blockDim.x) >> 8];
@@ -286,6 +285,7 @@ __global__ void __launch_bounds__(kBlock) flux_fp64(DevMesh M, DevState S, DevPa
     }
     if (bad) set_status(ctrl, SWGPU_EBED);
     if (flags & kNoTimestep) return;  // later Runge-Kutta stage: the step's dt is set
+    pdl_launch_dependents();
     block_min_timestep<kBlock>(t, ctrl);
     if ((flags & kFused) && threadIdx.x == 0 && last_block_done(&ctrl->done_flux, ctrl->blocks_flux))
         publish_step_clock(ctrl, P);
@@ -353,7 +353,6 @@ __device__ __forceinline__ void explicit_update(const DevMesh &M, const DevState
 // compute_fluxes as the stand-alone method: the explicit updates, and
 // max_speed (the largest speed of the edges that triangle k owns).
 __global__ void __launch_bounds__(kBlock) explicit_fp64(DevMesh M, DevState S, DevParams P) {
-    pdl_launch_dependents();
     pdl_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = M.N;
@@ -569,7 +568,6 @@ template <int BS, bool FUSED>
 __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevParams P,
                                                       Ctrl *ctrl, double dt_api, int flags,
                                                       Stage stg) {
-    pdl_launch_dependents();
     ctrl = block_ctrl(ctrl, M);
     pdl_wait();
     if (FUSED && ctrl_halted(ctrl)) return;
@@ -659,6 +657,7 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
     if (bad) set_status(ctrl, SWGPU_EDENOMINATOR);
     if (nonfinite) set_status(ctrl, SWGPU_ENONFINITE);
     if (FUSED) {
+        pdl_launch_dependents();
         __syncthreads();
         if (threadIdx.x == 0 && last_block_done(&ctrl->done_update, ctrl->blocks_update))
             commit_stage(ctrl, clk, P, stg);
@@ -841,7 +840,6 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
                                                          const BcTag *tags, Ctrl *ctrl,
                                                          int flags) {
     const bool fused = flags & kFused;
-    pdl_launch_dependents();
     ctrl = block_ctrl(ctrl, M);
     pdl_wait();
     if (fused && ctrl_halted(ctrl)) return;
@@ -1003,6 +1001,7 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
     if (bad_bc) set_status(ctrl, SWGPU_EBOUNDARY);
     if (no_nbr) set_status(ctrl, SWGPU_EMESH);
     if (fused) {
+        pdl_launch_dependents();
         __syncthreads();
         if (threadIdx.x == 0 && last_block_done(&ctrl->done_distribute, ctrl->blocks_distribute))
             apply_pending_halt(ctrl);
@@ -1186,7 +1185,6 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
                                                           const BcTag *tags, Ctrl *ctrl,
                                                           int flags) {
     const bool fused = flags & kFused;
-    pdl_launch_dependents();
     ctrl = block_ctrl(ctrl, M);
     pdl_wait();
     if (fused && ctrl_halted(ctrl)) return;
@@ -1363,6 +1361,7 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
     if (bad_bc) set_status(ctrl, SWGPU_EBOUNDARY);
     if (no_nbr) set_status(ctrl, SWGPU_EMESH);
     if (fused) {
+        pdl_launch_dependents();
         __syncthreads();
         if (threadIdx.x == 0 && last_block_done(&ctrl->done_distribute, ctrl->blocks_distribute)) apply_pending_halt(ctrl);
     }
@@ -1476,7 +1475,7 @@ void launch_distribute_fp64(const DevMesh &M, const DevState &S, const DevParams
                             const BcTag *tags, Ctrl *ctrl, int flags, cudaStream_t st) {
     const int bs = fp64_block(M.shape.distribute, M.N, M.shape.sms);
     const int g = (M.n_launch + bs - 1) / bs;
-    const bool pdl = M.shape.pdl && (flags & kFused);
+    const bool pdl = M.shape.pdl && (flags & kFused) && overlap_fp64(M.n_launch, M.shape.sms);
     if (P.flow_algorithm)
         launch_k(bs > 256 ? distribute_de_fp64<512> : distribute_de_fp64<256>, g, bs, st, pdl, M,
                  S, P, tags, ctrl, flags);
@@ -1492,8 +1491,8 @@ void launch_boundary_fp64(const DevMesh &M, const DevState &S, const DevParams &
 void launch_flux_fp64(const DevMesh &M, const DevState &S, const DevParams &P, Ctrl *ctrl,
                       int flags, cudaStream_t st) {
     const int bs = fp64_block(M.shape.flux, M.edges.E, M.shape.sms);
-    launch_k(flux_fp64, (M.edges.launch + bs - 1) / bs, bs, st, M.shape.pdl && (flags & kFused),
-             M, S, P, ctrl, flags);
+    const bool pdl = M.shape.pdl && (flags & kFused) && overlap_fp64(M.n_launch, M.shape.sms);
+    launch_k(flux_fp64, (M.edges.launch + bs - 1) / bs, bs, st, pdl, M, S, P, ctrl, flags);
 }
 void launch_explicit_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                           cudaStream_t st) {
@@ -1521,7 +1520,8 @@ void launch_update_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
     const int g = (M.n_launch + bs - 1) / bs;
     if (flags & kFused)
         launch_k(bs > 256 ? update_fp64<512, true> : update_fp64<256, true>, g, bs, st,
-                 M.shape.pdl, M, S, P, ctrl, dt, flags, stage);
+                 M.shape.pdl && overlap_fp64(M.n_launch, M.shape.sms), M, S, P, ctrl, dt, flags,
+                 stage);
     else
         launch_k(bs > 256 ? update_fp64<512, false> : update_fp64<256, false>, g, bs, st, false,
                  M, S, P, ctrl, dt, flags, stage);

@@ -228,6 +228,8 @@ enum : int {
     kTrack = 64,          // update records maximum depth and arrival time (whole steps)
     kExtrapolateOnly = 128,  // FP64 distribute: the second-order extrapolation alone
                              // (extrapolate_second_order_sw), no balance, vertex values only
+    kStartMid = 256,  // mixed: the next kernel may start once a block's data has arrived,
+    kStartEnd = 512,  // ... or at a block's end; else from the start (start_flag)
 };
 
 // One stage of a fused step.  An Euler step is one stage; ANUGA's RK2 and
@@ -351,6 +353,26 @@ inline int fp64_block(int knob, int64_t n, int sms) {
     int b = knob;
     while (b > 32 && (n + b - 1) / b < (int64_t)16 * sms) b >>= 1;
     return b;
+}
+
+// When the next step kernel may start (kStartMid, kStartEnd; 0: at once), and
+// whether an FP64 one overlaps this one at all.  A block that starts early
+// prepares (and prefetches) under the previous kernel, but it holds its place:
+// where a kernel has a few blocks per SM, those of the next go where there is
+// room at that moment, and the SM that gets most of them holds up the step.
+// Mixed, microseconds per step with the start at once / once the block's data
+// has arrived / at its end: 10,000 triangles 12.5 / 11.2 / 12.3, 79,524
+// 19.2 / 13.4 / 13.8, 102,400 19.7 / 13.7 / 14.3, 160,000 20.7 / 20.9 / 17.5,
+// 202,500 20.2 / 20.4 / 19.6, 250,000 23.2 / 23.7 / 23.6, a million
+// 76.6 / 79.1 / 81.3.  FP64 (which prepares nothing, so starts at a block's
+// end), overlapped / not: 1,024 27.4 / 28.4, 10,000 32.5 / 32.6, 14,400
+// 36.7 / 33.5, 48,400 62.4 / 51.7, 67,600 71.1 / 72.3, 320,356 270.7 / 272.6
+// (at once: 20,164 67.7, 40,000 65.8).
+inline int start_flag(int64_t n, int sms) {
+    return n <= (int64_t)840 * sms ? kStartMid : (n <= (int64_t)1450 * sms ? kStartEnd : 0);
+}
+inline bool overlap_fp64(int64_t n, int sms) {
+    return n <= (int64_t)80 * sms || n >= (int64_t)420 * sms;
 }
 
 }  // namespace swgpu

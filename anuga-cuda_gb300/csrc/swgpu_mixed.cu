@@ -432,10 +432,12 @@ __device__ __forceinline__ float flux_tile_triangle(const DevMixed &X, const Dev
 // stages its tile of TILE triangles with one-dimensional TMA bulk copies into
 // shared memory; neighbours inside the tile (most of them, in Morton order)
 // are read from shared memory, the others from global memory.
-template <int TILE>
-__global__ void __launch_bounds__(TILE, 1536 / TILE) flux_mixed(DevMesh M, DevMixed X, DevParams P,
-                                                        Ctrl *ctrl, int flags) {
-    pdl_launch_dependents();
+// LATE: the next kernel starts where the flags say (start_flag), else at once.
+// (Apart: the test of the flags costs a mesh that starts it at once 2%.)
+template <int TILE, bool LATE>
+__device__ __forceinline__ void flux_body(const DevMesh &M, const DevMixed &X, const DevParams &P,
+                                          Ctrl *ctrl, int flags) {
+    if (!LATE) pdl_launch_dependents();
     ctrl = block_ctrl(ctrl, M);
     __shared__ FluxTile<TILE> T;
     __shared__ __align__(8) unsigned long long bar;
@@ -474,13 +476,25 @@ __global__ void __launch_bounds__(TILE, 1536 / TILE) flux_mixed(DevMesh M, DevMi
     __shared__ unsigned long long ft_seen;
     if (tid == 0) ft_seen = *(volatile unsigned long long *)&ctrl->ftmin_bits;
     const bool arrived = mbar_wait_bounded(&bar, ctrl);
+    if (LATE) pdl_launch_at(kStartMid, flags);
     if (halted) return;
     float t = P.f_max_dt;
     if (arrived && tid < cnt) t = flux_tile_triangle<TILE>(X, P, T, k0, cnt);
+    if (LATE) pdl_launch_at(kStartEnd, flags);
     if (flags & kNoTimestep) return;  // later Runge-Kutta stage: the step's dt is set
     // the step's clock is evaluated from the minimum by step_clock_mixed once
     // this grid has completed: no block waits on a count of finished blocks
     block_min_timestep_f<TILE>(t, ctrl, &ft_seen);
+}
+template <int TILE>
+__global__ void __launch_bounds__(TILE, 1536 / TILE) flux_mixed(DevMesh M, DevMixed X, DevParams P,
+                                                        Ctrl *ctrl, int flags) {
+    flux_body<TILE, false>(M, X, P, ctrl, flags);
+}
+template <int TILE>
+__global__ void __launch_bounds__(TILE, 1536 / TILE) flux_late(DevMesh M, DevMixed X, DevParams P,
+                                                       Ctrl *ctrl, int flags) {
+    flux_body<TILE, true>(M, X, P, ctrl, flags);
 }
 
 // The same fluxes with persistent blocks: each block walks tiles
@@ -656,16 +670,18 @@ __device__ __forceinline__ void combine_stage(const Stage &stg, double bh, doubl
 // time (a sine and a quotient in FP64, 6 us at the end of a block of the
 // distribute: eight harbours of 128,000 triangles in all took 25.6 us a step
 // with it there, 23.9 with it here).
-template <bool CLOCK, bool TAGS>
+template <bool CLOCK, bool TAGS, bool LATE>
 __device__ __forceinline__ void update_body(const DevMesh &M, const DevState &S, const DevMixed &X,
                                             const DevParams &P, Ctrl *ctrl, int flags,
                                             const Stage &stg, const BcTag *tags, int ntags) {
-    pdl_launch_dependents();
+    if (!LATE) pdl_launch_dependents();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (TAGS) {
         const int blocks = (ntags + (int)blockDim.x - 1) / (int)blockDim.x;
         const int b = (int)blockIdx.x - ((int)gridDim.x - blocks);
         if (b >= 0) {
+            // (at once: the evaluation outlasts the other blocks' work)
+            if (LATE) pdl_launch_dependents();
             pdl_wait();
             const int i = b * (int)blockDim.x + (int)threadIdx.x;
             if (i >= ntags || !time_dependent(tags[i].type)) return;
@@ -691,6 +707,7 @@ __device__ __forceinline__ void update_body(const DevMesh &M, const DevState &S,
             ctrl->halt = 1;  // the last step's distribute has run
         return;
     }
+    if (LATE) pdl_launch_at(kStartMid, flags);
     __shared__ double block_dt;
     if (CLOCK) {
         if (threadIdx.x == 0) {
@@ -739,6 +756,7 @@ __device__ __forceinline__ void update_body(const DevMesh &M, const DevState &S,
         if ((flags & kTrack) && (stg.kind == kStageEuler || stg.kind == kStageLast))
             track_depth(S, k, h, step_end_time(ctrl, dt, stg), P.track_threshold);
     }
+    if (LATE) pdl_launch_at(kStartEnd, flags);
     // the stage is committed by the distribute (its scenario's first block)
     if (bad) set_status(ctrl, SWGPU_EDENOMINATOR);
     if (nonfinite) set_status(ctrl, SWGPU_ENONFINITE);
@@ -748,15 +766,21 @@ template <int BS, bool CLOCK>
 __global__ void __launch_bounds__(BS, 2048 / BS) update_mixed(DevMesh M, DevState S, DevMixed X,
                                                        DevParams P, Ctrl *ctrl, int flags,
                                                        Stage stg) {
-    update_body<CLOCK, false>(M, S, X, P, ctrl, flags, stg, nullptr, 0);
+    update_body<CLOCK, false, false>(M, S, X, P, ctrl, flags, stg, nullptr, 0);
+}
+template <int BS, bool CLOCK>
+__global__ void __launch_bounds__(BS, 2048 / BS) update_late(DevMesh M, DevState S, DevMixed X,
+                                                      DevParams P, Ctrl *ctrl, int flags,
+                                                      Stage stg) {
+    update_body<CLOCK, false, true>(M, S, X, P, ctrl, flags, stg, nullptr, 0);
 }
 // (apart, so that the evaluation's call costs meshes without such tags nothing)
-template <int BS, bool CLOCK>
+template <int BS, bool CLOCK, bool LATE>
 __global__ void __launch_bounds__(BS, 2048 / BS) update_with_tags(DevMesh M, DevState S, DevMixed X,
                                                            DevParams P, Ctrl *ctrl, int flags,
                                                            Stage stg, const BcTag *tags,
                                                            int ntags) {
-    update_body<CLOCK, true>(M, S, X, P, ctrl, flags, stg, tags, ntags);
+    update_body<CLOCK, true, LATE>(M, S, X, P, ctrl, flags, stg, tags, ntags);
 }
 
 // find_qmin_and_qmax (shallow_water_ext.c:98-148): the extremes of 0, dq0,
@@ -1123,12 +1147,13 @@ struct DistView {
 // scenario, once the update grid has completed; every block takes the
 // stage's order and end time from the step's clock (clk_*), which the commit
 // does not write, so no block depends on when the commit runs.
-template <int BS>
-__global__ void __launch_bounds__(BS, 2048 / BS) distribute_mixed(DevMesh M, DevState S, DevMixed X,
-                                                           DevParams P, const BcTag *tags,
-                                                           Ctrl *ctrls, int flags, Stage stg) {
+template <int BS, bool LATE>
+__device__ __forceinline__ void distribute_body(const DevMesh &M, const DevState &S,
+                                                const DevMixed &X, const DevParams &P,
+                                                const BcTag *tags, Ctrl *ctrls, int flags,
+                                                const Stage &stg) {
     const bool fused = flags & kFused;
-    pdl_launch_dependents();
+    if (!LATE) pdl_launch_dependents();
     Ctrl *ctrl = block_ctrl(ctrls, M);
     __shared__ DistTile<BS> T;
     __shared__ __align__(8) unsigned long long bar;
@@ -1190,6 +1215,7 @@ __global__ void __launch_bounds__(BS, 2048 / BS) distribute_mixed(DevMesh M, Dev
         order = (int)ctrl->order;
     }
     const bool arrived = mbar_wait_bounded(&bar, ctrl);
+    if (LATE) pdl_launch_at(kStartMid, flags);
     if (halted) return;
     int bad_bc = 0;
     if (arrived && tid < cnt) {
@@ -1208,7 +1234,20 @@ __global__ void __launch_bounds__(BS, 2048 / BS) distribute_mixed(DevMesh M, Dev
                                           fused ? X.tag_values : nullptr, 0);
         }
     }
+    if (LATE) pdl_launch_at(kStartEnd, flags);
     if (bad_bc) set_status(block_ctrl(ctrls, M), SWGPU_EBOUNDARY);
+}
+template <int BS>
+__global__ void __launch_bounds__(BS, 2048 / BS) distribute_mixed(DevMesh M, DevState S, DevMixed X,
+                                                           DevParams P, const BcTag *tags,
+                                                           Ctrl *ctrls, int flags, Stage stg) {
+    distribute_body<BS, false>(M, S, X, P, tags, ctrls, flags, stg);
+}
+template <int BS>
+__global__ void __launch_bounds__(BS, 2048 / BS) distribute_late(DevMesh M, DevState S, DevMixed X,
+                                                          DevParams P, const BcTag *tags,
+                                                          Ctrl *ctrls, int flags, Stage stg) {
+    distribute_body<BS, true>(M, S, X, P, tags, ctrls, flags, stg);
 }
 
 // update_timestep (the step's clock) of each running scenario, evaluated
@@ -1668,12 +1707,17 @@ void launch_distribute_mixed(const DevMesh &M, const DevState &S, const DevMixed
                              const Stage &stage, cudaStream_t st) {
     const int bs = M.shape.distribute, g = (M.n_launch + bs - 1) / bs;
     const bool pdl = M.shape.pdl;
+    const int start = start_flag(M.n_launch, M.shape.sms);
+    const auto launch = [&](auto early, auto late) {
+        launch_k(start ? late : early, g, bs, st, pdl, M, S, X, P, tags, ctrl, flags | start,
+                 stage);
+    };
     if (bs == 128)
-        launch_k(distribute_mixed<128>, g, 128, st, pdl, M, S, X, P, tags, ctrl, flags, stage);
+        launch(distribute_mixed<128>, distribute_late<128>);
     else if (bs == 512)
-        launch_k(distribute_mixed<512>, g, 512, st, pdl, M, S, X, P, tags, ctrl, flags, stage);
+        launch(distribute_mixed<512>, distribute_late<512>);
     else
-        launch_k(distribute_mixed<256>, g, 256, st, pdl, M, S, X, P, tags, ctrl, flags, stage);
+        launch(distribute_mixed<256>, distribute_late<256>);
 }
 void launch_flux_mixed(const DevMesh &M, const DevState &, const DevMixed &X, const DevParams &P,
                        Ctrl *ctrl, int flags, cudaStream_t st) {
@@ -1697,12 +1741,16 @@ void launch_flux_mixed(const DevMesh &M, const DevState &, const DevMixed &X, co
             launch_k(flux_mixed_pipelined<128>, grid, 128, st, pdl, M, X, P, ctrl, flags, g);
         return;
     }
+    const int start = start_flag(M.n_launch, M.shape.sms);
+    const auto launch = [&](auto early, auto late) {
+        launch_k(start ? late : early, g, t, st, pdl, M, X, P, ctrl, flags | start);
+    };
     if (t == 64)
-        launch_k(flux_mixed<64>, g, 64, st, pdl, M, X, P, ctrl, flags);
+        launch(flux_mixed<64>, flux_late<64>);
     else if (t == 256)
-        launch_k(flux_mixed<256>, g, 256, st, pdl, M, X, P, ctrl, flags);
+        launch(flux_mixed<256>, flux_late<256>);
     else
-        launch_k(flux_mixed<128>, g, 128, st, pdl, M, X, P, ctrl, flags);
+        launch(flux_mixed<128>, flux_late<128>);
 }
 // The shapes of the resident step: threads per block, smallest first (a mesh
 // spread over more SMs has fewer warps to wait for on each).
@@ -1786,26 +1834,34 @@ void launch_update_mixed(const DevMesh &M, const DevState &S, const DevMixed &X,
                          bool clock, const BcTag *tags, int ntags, cudaStream_t st) {
     const int bs = M.shape.update, g = (M.n_launch + bs - 1) / bs;
     const bool pdl = M.shape.pdl;
-    const auto launch = [&](auto plain, auto with_tags) {
+    const int start = start_flag(M.n_launch, M.shape.sms);
+    const auto launch = [&](auto early, auto late, auto tags_early, auto tags_late) {
         if (ntags > 0)
-            launch_k(with_tags, g + (ntags + bs - 1) / bs, bs, st, pdl, M, S, X, P, ctrl, flags, stage, tags, ntags);
+            launch_k(start ? tags_late : tags_early, g + (ntags + bs - 1) / bs, bs, st, pdl, M, S, X,
+                     P, ctrl, flags | start, stage, tags, ntags);
         else
-            launch_k(plain, g, bs, st, pdl, M, S, X, P, ctrl, flags, stage);
+            launch_k(start ? late : early, g, bs, st, pdl, M, S, X, P, ctrl, flags | start, stage);
     };
     if (clock) {
         if (bs == 128)
-            launch(update_mixed<128, true>, update_with_tags<128, true>);
+            launch(update_mixed<128, true>, update_late<128, true>,
+                   update_with_tags<128, true, false>, update_with_tags<128, true, true>);
         else if (bs == 512)
-            launch(update_mixed<512, true>, update_with_tags<512, true>);
+            launch(update_mixed<512, true>, update_late<512, true>,
+                   update_with_tags<512, true, false>, update_with_tags<512, true, true>);
         else
-            launch(update_mixed<256, true>, update_with_tags<256, true>);
+            launch(update_mixed<256, true>, update_late<256, true>,
+                   update_with_tags<256, true, false>, update_with_tags<256, true, true>);
     } else {
         if (bs == 128)
-            launch(update_mixed<128, false>, update_with_tags<128, false>);
+            launch(update_mixed<128, false>, update_late<128, false>,
+                   update_with_tags<128, false, false>, update_with_tags<128, false, true>);
         else if (bs == 512)
-            launch(update_mixed<512, false>, update_with_tags<512, false>);
+            launch(update_mixed<512, false>, update_late<512, false>,
+                   update_with_tags<512, false, false>, update_with_tags<512, false, true>);
         else
-            launch(update_mixed<256, false>, update_with_tags<256, false>);
+            launch(update_mixed<256, false>, update_late<256, false>,
+                   update_with_tags<256, false, false>, update_with_tags<256, false, true>);
     }
 }
 void launch_prepare_mixed(const DevMesh &M, const DevState &S, const DevMixed &X,
