@@ -379,13 +379,10 @@ static void set_block_counts(Handle *h) {
         const LaunchShape &s = h->M.shape;
         const int64_t edges =
             h->scen_edges.empty() ? 0 : h->scen_edges[i + 1] - h->scen_edges[i];
-        const auto blocks = [&](int64_t items, int64_t total, int knob) {
-            const int b = fp64_block(knob, total, s.sms);
-            return (unsigned)((items + b - 1) / b);
-        };
-        c->blocks_flux = blocks(edges, h->M.edges.E, s.flux);
-        c->blocks_update = blocks(n, h->M.N, s.update);
-        c->blocks_distribute = blocks(n, h->M.N, s.distribute);
+        const auto blocks = [&](int64_t items, int b) { return (unsigned)((items + b - 1) / b); };
+        c->blocks_flux = blocks(edges, fp64_block(s.flux, h->M.edges.E, s.sms));
+        c->blocks_update = blocks(n, fp64_block(s.update, h->M.N, s.sms));
+        c->blocks_distribute = blocks(n, distribute_tile_fp64(s.distribute, h->M.N, s.sms));
     }
 }
 

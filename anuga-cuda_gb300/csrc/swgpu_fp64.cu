@@ -1101,10 +1101,12 @@ __device__ __forceinline__ bool limit_by_neighbours(const DevMesh &M, const doub
 // of one triangle: centroid stage wk, bed zk, momentum uk, vk; bed vertex
 // values zvk; stage / momentum vertex values ow, ou, ov blended in place.
 // hv: the vertex depths ow - zvk.
-__device__ __forceinline__ void balance_one(const DevParams &P, double wk, double zk, double uk,
-                                            double vk, const double (&zvk)[3],
-                                            const double (&hv)[3], double (&ow)[3],
-                                            double (&ou)[3], double (&ov)[3]) {
+struct Balance {
+    double alpha, hc, uc, vc;  // blend, centroid depth and velocities (alpha below 1 only)
+};
+__device__ __forceinline__ Balance balance_of(const DevParams &P, double wk, double zk, double uk,
+                                              double vk, const double (&zvk)[3],
+                                              const double (&hv)[3]) {
     const double eps = 1.0e-6;
     double dz = 0.0;
     if (P.tight_slope_limiters == 0) {
@@ -1133,26 +1135,40 @@ __device__ __forceinline__ void balance_one(const DevParams &P, double wk, doubl
             if (on[i]) alpha = imin(alpha, q[i]);
         if (lt_zero(alpha)) alpha = 0.0;  // alpha is at most 1
     }
+    double uc = 0.0, vc = 0.0;
     if (lt64(alpha, 1.0)) {
-        double uc = 0.0, vc = 0.0;
         if (P.tight_slope_limiters == 0) hc = wk - zk;
         if (P.use_centroid_velocities == 1 && lt64(eps, hc)) {
             const Two c = div2(uk, hc, vk, hc);
             uc = c.a;
             vc = c.b;
         }
+    }
+    return Balance{alpha, hc, uc, vc};
+}
+// One vertex of it (alpha below 1).
+__device__ __forceinline__ void balance_vertex(const DevParams &P, const Balance &B, double uk,
+                                               double vk, double zv, double hv, double &ow,
+                                               double &ou, double &ov) {
+    ow = zv + (1 - B.alpha) * B.hc + B.alpha * hv;
+    if (P.use_centroid_velocities == 1) {
+        const double h = ow - zv;
+        ou = B.uc * h;
+        ov = B.vc * h;
+    } else {
+        ou = (1 - B.alpha) * uk + B.alpha * ou;
+        ov = (1 - B.alpha) * vk + B.alpha * ov;
+    }
+}
+__device__ __forceinline__ void balance_one(const DevParams &P, double wk, double zk, double uk,
+                                            double vk, const double (&zvk)[3],
+                                            const double (&hv)[3], double (&ow)[3],
+                                            double (&ou)[3], double (&ov)[3]) {
+    const Balance B = balance_of(P, wk, zk, uk, vk, zvk, hv);
+    if (lt64(B.alpha, 1.0)) {
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            ow[i] = zvk[i] + (1 - alpha) * hc + alpha * hv[i];
-            if (P.use_centroid_velocities == 1) {
-                const double h = ow[i] - zvk[i];
-                ou[i] = uc * h;
-                ov[i] = vc * h;
-            } else {
-                ou[i] = (1 - alpha) * uk + alpha * ou[i];
-                ov[i] = (1 - alpha) * vk + alpha * ov[i];
-            }
-        }
+        for (int i = 0; i < 3; i++)
+            balance_vertex(P, B, uk, vk, zvk[i], hv[i], ow[i], ou[i], ov[i]);
     }
 }
 
@@ -1367,6 +1383,341 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
     }
 }
 
+// Boundary values of boundary edge mb, edge i of triangle k, from its edge
+// values; returns 1 where they could not be evaluated.
+__device__ __forceinline__ int boundary_edge(const DevMesh &M, const DevState &S,
+                                             const DevParams &P, const BcTag *tags, double time,
+                                             int k, int i, int mb, double we, double uhe,
+                                             double vhe) {
+    const int N = M.N;
+    const double ze = S.ze[i * N + k];
+    double wb, uhb, vhb;
+    int bad = 0;
+    if (!eval_boundary(tags[M.btag[mb]], time, we, uhe, vhe, M.normals[(2 * i) * N + k],
+                       M.normals[(2 * i + 1) * N + k], ze, P.g, wb, uhb, vhb)) {
+        bad = 1;
+        wb = uhb = vhb = 0.0;
+    }
+    S.wb[mb] = wb;
+    S.uhb[mb] = uhb;
+    S.vhb[mb] = vhb;
+    S.zb[mb] = ze;
+    return bad;
+}
+
+// distribute_fp64 and distribute_de_fp64 with three threads per triangle, one
+// for each quantity in the reconstruction and for each vertex and edge after
+// it, in three warps that meet through shared memory.  A mesh that leaves the
+// SMs few warps is bound by the chain of FP64 operations and quotients of one
+// triangle (an operation that a warp waits for takes about 100 clocks, its
+// pipe 16): a third of the operations per thread, three times the warps.  The
+// depths and the balance's blend are computed by all three, so a mesh that
+// fills the FP64 pipe is better off with a thread per triangle (distribute_split;
+// microseconds per step, three threads / one: 1,024 triangles 28.9 / 35.9, 4,096
+// 28.8 / 36.1, 14,400 32.5 / 36.9, 20,164 37.4 / 39.5, 28,900 43.0 / 42.4, 40,000
+// 54.8 / 50.7, 160,000 164 / 152).
+__global__ void __launch_bounds__(3 * kSplitTile) distribute_split_fp64(DevMesh M, DevState S,
+                                                                        DevParams P,
+                                                                        const BcTag *tags,
+                                                                        Ctrl *ctrl, int flags) {
+    const bool fused = flags & kFused;
+    const int k0 = blockIdx.x * kSplitTile;
+    if (M.blk_scen) ctrl += M.blk_scen[k0 >> 8];
+    pdl_wait();
+    if (fused && ctrl_halted(ctrl)) return;
+    const int N = M.N;
+    const int role = threadIdx.x / kSplitTile, t = threadIdx.x % kSplitTile, k = k0 + t;
+    __shared__ double vert[3][3][kSplitTile];  // [quantity][vertex], then balanced
+    const bool in = k < N;
+    int bad_bc = 0, no_nbr = 0;
+    bool to_momentum = false;
+    double wk = 0.0, zk = 0.0, zvk[3] = {0.0, 0.0, 0.0};
+    if (in) {
+        const int order = (int)ctrl->order;
+        wk = S.w[k];
+        zk = S.zc[k];
+#pragma unroll
+        for (int i = 0; i < 3; i++) zvk[i] = S.zv[i * N + k];
+        const bool extrapolate_only = flags & kExtrapolateOnly;
+        const bool vel = P.extrapolate_velocity_second_order == 1;
+        const double *mom = role == 1 ? S.uh : S.vh;
+        double out[3];
+        if (order == 1 && !extrapolate_only) {
+            const double q = role == 0 ? wk : mom[k];
+#pragma unroll
+            for (int i = 0; i < 3; i++) out[i] = q;
+        } else if (P.limiter != kLimiterOptimised && !extrapolate_only) {
+            if (!limit_by_neighbours(M, role == 0 ? S.w : mom, k,
+                                     role == 0 ? P.beta_w : (role == 1 ? P.beta_uh : P.beta_vh),
+                                     P.limiter == kLimiterEdge, out))
+                no_nbr = 1;
+        } else {
+            const double *Q = role == 0 ? S.w : (!vel ? mom : (role == 1 ? S.uvel : S.vvel));
+            const double own = Q[k];
+            const int nbk = M.nb[k];
+            bool keep = false;
+            bool flat = nbk == 3;
+            if (!flat) {
+                const double *G = M.geo64 + k;
+                const size_t n = N;
+                const double inv_area2 = G[kGeoInvArea2 * n];
+                double dxv[3], dyv[3];
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    dxv[i] = G[(kGeoDxv + i) * n];
+                    dyv[i] = G[(kGeoDyv + i) * n];
+                }
+                const double dx2 = G[kGeoDx2 * n], dy2 = G[kGeoDy2 * n];
+                if (nbk <= 1) {
+                    if ((bits64(inv_area2) & kMag64) == 0) {
+                        flat = true;
+                    } else {
+                        const int k0n = M.surr[k], k1n = M.surr[N + k], k2n = M.surr[2 * N + k];
+                        const double dx1 = G[kGeoDx1 * n], dy1 = G[kGeoDy1 * n];
+                        const double q0 = Q[k0n], q1 = Q[k1n], q2 = Q[k2n];
+                        const double h0 = S.w[k0n] - S.zc[k0n];
+                        const double h1 = S.w[k1n] - S.zc[k1n];
+                        const double h2 = S.w[k2n] - S.zc[k2n];
+                        if (P.optimise_dry_cells && lt64(imax(h0, imax(h1, h2)), P.epsilon)) {
+                            keep = true;
+                        } else {
+                            double hfactor = 0.0;
+                            if (P.betas_differ) {
+                                const double hmin = imin(imin(h0, imin(h1, h2)), wk - zk);
+                                if (lt64(0.001, hmin))
+                                    hfactor = fdiv64(hmin - 0.001, hmin + 0.004);
+                            }
+                            double beta[3];
+                            limiter_betas(P, hfactor, beta);
+                            aux_jumps(own, q0, q1, q2, dx1, dy1, dx2, dy2, inv_area2, dxv, dyv,
+                                      role == 0 ? beta[0] : (role == 1 ? beta[1] : beta[2]), out);
+                        }
+                    }
+                } else {
+                    int k1 = -1;
+#pragma unroll
+                    for (int i = 2; i >= 0; i--) {
+                        const int sn = M.surr[i * N + k];
+                        if (sn != k) k1 = sn;
+                    }
+                    if (k1 < 0) {
+                        no_nbr = 1;
+                        flat = true;
+                    } else {
+                        one_nbr_jumps(own, Q[k1], dx2, dy2, dxv, dyv, P.beta_w, out);
+                    }
+                }
+            }
+            if (flat) {
+#pragma unroll
+                for (int i = 0; i < 3; i++) out[i] = own;
+            } else if (keep) {
+                const double *before = role == 0 ? S.wv : (role == 1 ? S.uhv : S.vhv);
+#pragma unroll
+                for (int i = 0; i < 3; i++) out[i] = before[i * N + k];
+            }
+            to_momentum = vel;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) vert[role][i][t] = out[i];
+    }
+    __syncthreads();
+    // vertex `role`
+    double ow = 0.0, ou = 0.0, ov = 0.0;
+    if (in) {
+        double hv[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) hv[i] = vert[0][i][t] - zvk[i];
+        const double h = role == 0 ? hv[0] : (role == 1 ? hv[1] : hv[2]);
+        const double zv = role == 0 ? zvk[0] : (role == 1 ? zvk[1] : zvk[2]);
+        ow = vert[0][role][t];
+        ou = vert[1][role][t];
+        ov = vert[2][role][t];
+        if (to_momentum) {
+            const double dv = gt_zero(h) ? h : 0.0;
+            ou = ou * dv;
+            ov = ov * dv;
+        }
+        if (!(flags & kExtrapolateOnly)) {
+            const double uk = S.uh[k], vk = S.vh[k];
+            const Balance B = balance_of(P, wk, zk, uk, vk, zvk, hv);
+            if (lt64(B.alpha, 1.0)) balance_vertex(P, B, uk, vk, zv, h, ow, ou, ov);
+        }
+        S.wv[role * N + k] = ow;
+        S.uhv[role * N + k] = ou;
+        S.vhv[role * N + k] = ov;
+    }
+    if (flags & kWriteEdges) {
+        __syncthreads();
+        vert[0][role][t] = ow;
+        vert[1][role][t] = ou;
+        vert[2][role][t] = ov;
+        __syncthreads();
+        if (in) {
+            // edge `role`
+            const int a = role == 0 ? 1 : 0, b = role == 2 ? 1 : 2;
+            const double we = half_of(vert[0][a][t] + vert[0][b][t]);
+            const double uhe = half_of(vert[1][a][t] + vert[1][b][t]);
+            const double vhe = half_of(vert[2][a][t] + vert[2][b][t]);
+            S.we[role * N + k] = we;
+            S.uhe[role * N + k] = uhe;
+            S.vhe[role * N + k] = vhe;
+            if (flags & kWriteBoundary) {
+                const int pk = M.nbr[role * N + k];
+                if (pk < 0)
+                    bad_bc = boundary_edge(M, S, P, tags, ctrl->time, k, role, -pk - 1, we, uhe,
+                                           vhe);
+            }
+        }
+    }
+    if (bad_bc) set_status(ctrl, SWGPU_EBOUNDARY);
+    if (no_nbr) set_status(ctrl, SWGPU_EMESH);
+    if (fused) {
+        pdl_launch_dependents();
+        __syncthreads();
+        if (threadIdx.x == 0 && last_block_done(&ctrl->done_distribute, ctrl->blocks_distribute))
+            apply_pending_halt(ctrl);
+    }
+}
+
+__global__ void __launch_bounds__(3 * kSplitTile) distribute_de_split_fp64(DevMesh M, DevState S,
+                                                                           DevParams P,
+                                                                           const BcTag *tags,
+                                                                           Ctrl *ctrl, int flags) {
+    const bool fused = flags & kFused;
+    const int first = blockIdx.x * kSplitTile;
+    if (M.blk_scen) ctrl += M.blk_scen[first >> 8];
+    pdl_wait();
+    if (fused && ctrl_halted(ctrl)) return;
+    const int N = M.N;
+    const int role = threadIdx.x / kSplitTile, t = threadIdx.x % kSplitTile, k = first + t;
+    __shared__ double edge[3][3][kSplitTile];  // [quantity][edge]
+    const bool in = k < N;
+    const bool vel = P.extrapolate_velocity_second_order == 1;
+    int bad_bc = 0, no_nbr = 0;
+    if (in) {
+        const double *mom = role == 1 ? (vel ? S.uvel : S.uh) : (vel ? S.vvel : S.vh);
+        const double *Q = role == 0 ? S.w : mom;
+        const double own = Q[k];
+        const int nbk = M.nb[k];
+        double out[3];
+        bool flat = false, keep = false;
+        if (nbk == 3) {
+            flat = true;
+        } else {
+            const double x = M.cxy[k], y = M.cxy[N + k];
+            double vx[3], vy[3], dxv[3], dyv[3];
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                vx[i] = M.vxy[(2 * i) * N + k];
+                vy[i] = M.vxy[(2 * i + 1) * N + k];
+            }
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const int a = (i + 1) % 3, b = (i + 2) % 3;
+                dxv[i] = half_of(vx[a] + vx[b]) - x;  // edge midpoint offsets
+                dyv[i] = half_of(vy[a] + vy[b]) - y;
+            }
+            if (nbk <= 1) {
+                int k0 = M.surr[k], k1 = M.surr[N + k], k2 = M.surr[2 * N + k];
+                if (!lt64(S.zc[k2], S.w[k2])) k2 = k;
+                if (!lt64(S.zc[k0], S.w[k0])) k0 = k;
+                if (!lt64(S.zc[k1], S.w[k1])) k1 = k;
+                const double x0 = M.cxy[k0], y0 = M.cxy[N + k0];
+                const double dx1 = M.cxy[k1] - x0, dx2 = M.cxy[k2] - x0;
+                const double dy1 = M.cxy[N + k1] - y0, dy2 = M.cxy[N + k2] - y0;
+                const double area2 = dy2 * dx1 - dy1 * dx2;
+                if (!gt_zero(area2)) {
+                    flat = true;
+                } else {
+                    const double hc = S.w[k] - S.zc[k];
+                    const double h0 = S.w[k0] - S.zc[k0];
+                    const double h1 = S.w[k1] - S.zc[k1];
+                    const double h2 = S.w[k2] - S.zc[k2];
+                    const double hmin = imin(imin(h0, imin(h1, h2)), hc);
+                    const double hfactor = gt_zero(hmin) ? 1.0 : 0.0;
+                    if (P.optimise_dry_cells && lt64(imax(h0, imax(h1, h2)), P.epsilon)) {
+                        keep = true;
+                    } else {
+                        double beta[3];
+                        limiter_betas(P, hfactor, beta);
+                        const double inv_area2 = fdiv64(1.0, area2);
+                        aux_jumps(own, Q[k0], Q[k1], Q[k2], dx1, dy1, dx2, dy2, inv_area2, dxv,
+                                  dyv, role == 0 ? beta[0] : (role == 1 ? beta[1] : beta[2]), out);
+                    }
+                }
+            } else {
+                int k1 = -1;
+#pragma unroll
+                for (int i = 2; i >= 0; i--) {
+                    const int sn = M.surr[i * N + k];
+                    if (sn != k) k1 = sn;
+                }
+                if (k1 < 0) {
+                    no_nbr = 1;
+                    flat = true;
+                } else {
+                    const double dx1 = M.cxy[k1] - x, dy1 = M.cxy[N + k1] - y;
+                    const double area2 = dx1 * dx1 + dy1 * dy1;
+                    double dx2 = fdiv64(1.0, area2);
+                    const double dy2 = dx2 * dy1;
+                    dx2 *= dx1;
+                    one_nbr_jumps(own, Q[k1], dx2, dy2, dxv, dyv, P.beta_w, out);
+                }
+            }
+        }
+        if (flat) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) out[i] = own;
+        } else if (keep) {
+            const double *before = role == 0 ? S.we : (role == 1 ? S.uhe : S.vhe);
+#pragma unroll
+            for (int i = 0; i < 3; i++) out[i] = before[i * N + k];
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) edge[role][i][t] = out[i];
+    }
+    __syncthreads();
+    if (in) {
+        // edge and vertex `role`
+        const int a = role == 0 ? 1 : 0, b = role == 2 ? 1 : 2;
+        const double we = edge[0][role][t];
+        double ue = edge[1][role][t], ve = edge[2][role][t];
+        const double ow = edge[0][a][t] + edge[0][b][t] - we;
+        double ou = edge[1][a][t] + edge[1][b][t] - ue;
+        double ov = edge[2][a][t] + edge[2][b][t] - ve;
+        if (vel) {
+            double de = we - S.ze[role * N + k];
+            if (!gt_zero(de)) de = 0.0;
+            ue = ue * de;
+            ve = ve * de;
+            double dv = ow - S.zv[role * N + k];
+            if (!gt_zero(dv)) dv = 0.0;
+            ou = ou * dv;
+            ov = ov * dv;
+        }
+        S.we[role * N + k] = we;
+        S.uhe[role * N + k] = ue;
+        S.vhe[role * N + k] = ve;
+        S.wv[role * N + k] = ow;
+        S.uhv[role * N + k] = ou;
+        S.vhv[role * N + k] = ov;
+        if (flags & kWriteBoundary) {
+            const int pk = M.nbr[role * N + k];
+            if (pk < 0)
+                bad_bc = boundary_edge(M, S, P, tags, ctrl->time, k, role, -pk - 1, we, ue, ve);
+        }
+    }
+    if (bad_bc) set_status(ctrl, SWGPU_EBOUNDARY);
+    if (no_nbr) set_status(ctrl, SWGPU_EMESH);
+    if (fused) {
+        pdl_launch_dependents();
+        __syncthreads();
+        if (threadIdx.x == 0 && last_block_done(&ctrl->done_distribute, ctrl->blocks_distribute))
+            apply_pending_halt(ctrl);
+    }
+}
+
 // update_boundary as a stand-alone pass over boundary slots, from the
 // stored vertex values (gpu_domain_advanced.py:2006-2108).
 __global__ void __launch_bounds__(kBlock) boundary_fp64(DevMesh M, DevState S, DevParams P,
@@ -1473,15 +1824,20 @@ void launch_prepare_fp64(const DevMesh &M, const DevState &S, const DevParams &P
 // Block sizes of the fused-step kernels come from M.shape (fp64_block).
 void launch_distribute_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                             const BcTag *tags, Ctrl *ctrl, int flags, cudaStream_t st) {
-    const int bs = fp64_block(M.shape.distribute, M.N, M.shape.sms);
-    const int g = (M.n_launch + bs - 1) / bs;
+    const int tile = distribute_tile_fp64(M.shape.distribute, M.N, M.shape.sms);
+    const int g = (M.n_launch + tile - 1) / tile;
     const bool pdl = M.shape.pdl && (flags & kFused) && overlap_fp64(M.n_launch, M.shape.sms);
+    if (distribute_split(M.N, M.shape.sms)) {
+        launch_k(P.flow_algorithm ? distribute_de_split_fp64 : distribute_split_fp64, g, 3 * tile,
+                 st, pdl, M, S, P, tags, ctrl, flags);
+        return;
+    }
     if (P.flow_algorithm)
-        launch_k(bs > 256 ? distribute_de_fp64<512> : distribute_de_fp64<256>, g, bs, st, pdl, M,
-                 S, P, tags, ctrl, flags);
+        launch_k(tile > 256 ? distribute_de_fp64<512> : distribute_de_fp64<256>, g, tile, st, pdl,
+                 M, S, P, tags, ctrl, flags);
     else
-        launch_k(bs > 256 ? distribute_fp64<512> : distribute_fp64<256>, g, bs, st, pdl, M, S, P,
-                 tags, ctrl, flags);
+        launch_k(tile > 256 ? distribute_fp64<512> : distribute_fp64<256>, g, tile, st, pdl, M, S,
+                 P, tags, ctrl, flags);
 }
 void launch_boundary_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                           const BcTag *tags, Ctrl *ctrl,

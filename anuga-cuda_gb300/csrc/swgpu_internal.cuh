@@ -355,6 +355,14 @@ inline int fp64_block(int knob, int64_t n, int sms) {
     return b;
 }
 
+// Whether the FP64 distribute takes three threads per triangle
+// (distribute_split_fp64), and the triangles of one of its blocks.
+constexpr int kSplitTile = 32;
+inline bool distribute_split(int64_t n, int sms) { return n <= (int64_t)160 * sms; }
+inline int distribute_tile_fp64(int knob, int64_t n, int sms) {
+    return distribute_split(n, sms) ? kSplitTile : fp64_block(knob, n, sms);
+}
+
 // When the next step kernel may start (kStartMid, kStartEnd; 0: at once), and
 // whether an FP64 one overlaps this one at all.  A block that starts early
 // prepares (and prefetches) under the previous kernel, but it holds its place:
