@@ -229,7 +229,7 @@ static void issue_stage(Handle *h, const Stage &stg) {
         launch_flux_fp64(h->M, h->S, h->P, h->d_ctrl, flux_flags, h->stream);
         launch_update_fp64(h->M, h->S, h->P, h->d_ctrl, 0.0, update_flags, stg, h->stream);
         launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl, dist_flags | kWriteEdges,
-                               h->stream);
+                               stg, h->stream);
     } else {
         launch_flux_mixed(h->M, h->S, h->X, h->P, h->d_ctrl, flux_flags, h->stream);
         const bool clock = !(flux_flags & kNoTimestep);
@@ -321,7 +321,8 @@ static int issue_distribute(Handle *h, bool with_boundary) {
     if (h->precision == SWGPU_FP64) {
         launch_prepare_fp64(h->M, h->S, h->P, h->d_ctrl, h->stream);
         launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl,
-                               kWriteEdges | (with_boundary ? kWriteBoundary : 0), h->stream);
+                               kWriteEdges | (with_boundary ? kWriteBoundary : 0), kEulerStage,
+                               h->stream);
     } else {
         launch_prepare_mixed(h->M, h->S, h->X, h->P, h->mixed_from_stage ? 1 : 0, h->stream);
         h->mixed_from_stage = false;
@@ -368,22 +369,14 @@ int swgpu_device_info(char *buf, int buflen) {
     return SWGPU_OK;
 }
 
-// Blocks of each scenario in one launch of each fused-step kernel (the
-// last-block-done counts) for the handle's launch shape.
+// Blocks of each scenario in one launch of the FP64 flux (its last-block-done
+// count) for the handle's launch shape.
 static void set_block_counts(Handle *h) {
-    for (int i = 0; i < h->nscen; i++) {
-        const int64_t n =
-            h->nscen > 1 ? h->scen_offsets[i + 1] - h->scen_offsets[i] : (int64_t)h->M.N;
-        Ctrl *c = &h->h_ctrl[i];
-        // (counted in the FP64 path only)
-        const LaunchShape &s = h->M.shape;
-        const int64_t edges =
-            h->scen_edges.empty() ? 0 : h->scen_edges[i + 1] - h->scen_edges[i];
-        const auto blocks = [&](int64_t items, int b) { return (unsigned)((items + b - 1) / b); };
-        c->blocks_flux = blocks(edges, fp64_block(s.flux, h->M.edges.E, s.sms));
-        c->blocks_update = blocks(n, fp64_block(s.update, h->M.N, s.sms));
-        c->blocks_distribute = blocks(n, distribute_tile_fp64(s.distribute, h->M.N, s.sms));
-    }
+    if (h->scen_edges.empty()) return;  // mixed
+    const int b = fp64_block(h->M.shape.flux, h->M.edges.E, h->M.shape.sms);
+    for (int i = 0; i < h->nscen; i++)
+        h->h_ctrl[i].blocks_flux =
+            (unsigned)((h->scen_edges[i + 1] - h->scen_edges[i] + b - 1) / b);
 }
 
 // The unique edges of an FP64 handle's mesh (DevEdges).
@@ -1239,7 +1232,8 @@ int swgpu_extrapolate_second_order_sw(void *handle) {
                     "to edges inside distribute_to_vertices_and_edges");
     h->ctrl_current = false;
     if (h->P.extrapolate_velocity_second_order) launch_velocities_fp64(h->M, h->S, h->P, h->stream);
-    launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl, kExtrapolateOnly, h->stream);
+    launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl, kExtrapolateOnly, kEulerStage,
+                           h->stream);
     if ((rc = check_launch(h, "extrapolate_second_order_sw"))) return rc;
     h->vertices_stale = false;
     h->edges_stale = true;
@@ -1526,7 +1520,6 @@ int swgpu_evolve_start(void *handle, double starttime, double yieldstep, double 
         c->stop_reason = kStopNone;
         c->status = 0;
         c->budget = -1;
-        c->done_update = c->done_distribute = 0;
         reset_ftmin(c, h->P);
     }
     if ((rc = push_ctrl(h))) return rc;
@@ -1653,7 +1646,7 @@ int swgpu_profile_steps(void *handle, int64_t nsteps, double *ms) {
         CK(cudaEventRecord(ev[3], h->stream));
         if (!mixed)
             launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl,
-                                   kFused | kWriteBoundary | kWriteEdges, h->stream);
+                                   kFused | kWriteBoundary | kWriteEdges, kEulerStage, h->stream);
         else
             launch_distribute_mixed(h->M, h->S, h->X, h->P, h->d_tags, h->d_ctrl,
                                     kFused | kWriteBoundary, kEulerStage, h->stream);

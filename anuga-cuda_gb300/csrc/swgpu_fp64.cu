@@ -15,11 +15,11 @@
 //                   gravity_wb, the step's update_timestep (evaluated once by
 //                   the flux kernel's last block), Manning
 //                   friction, the semi-implicit conserved update, protect,
-//                   centroid velocities for the next extrapolation; the last
-//                   block advances the model time
+//                   centroid velocities for the next extrapolation
 //   distribute_fp64 second-order limited extrapolation, balance_deep_and_
 //                   shallow, boundary conditions of the triangle's boundary
-//                   edges; vertex and edge values stored
+//                   edges; vertex and edge values stored; the scenario's
+//                   first block commits the step (time, counters, a stop)
 #include <cstdio>
 
 #include "swgpu_device.cuh"
@@ -570,7 +570,11 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
                                                       Stage stg) {
     ctrl = block_ctrl(ctrl, M);
     pdl_wait();
-    if (FUSED && ctrl_halted(ctrl)) return;
+    if (FUSED && ctrl_halted(ctrl)) {
+        if (threadIdx.x == 0 && first_of_scenario(M) && ctrl->halt == 2)
+            ctrl->halt = 1;  // the last step's distribute has run
+        return;
+    }
     StepClock clk;
     if (FUSED) {
         clk = published_step_clock(ctrl);
@@ -656,12 +660,8 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
     }
     if (bad) set_status(ctrl, SWGPU_EDENOMINATOR);
     if (nonfinite) set_status(ctrl, SWGPU_ENONFINITE);
-    if (FUSED) {
-        pdl_launch_dependents();
-        __syncthreads();
-        if (threadIdx.x == 0 && last_block_done(&ctrl->done_update, ctrl->blocks_update))
-            commit_stage(ctrl, clk, P, stg);
-    }
+    // the stage is committed by the distribute (its scenario's first block)
+    if (FUSED) pdl_launch_dependents();
 }
 
 __global__ void __launch_bounds__(kBlock) track_reset(int N, float *hmax, float *tarr) {
@@ -838,13 +838,17 @@ __device__ __forceinline__ void limiter_betas(const DevParams &P, double hfactor
 template <int BS>
 __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, DevParams P,
                                                          const BcTag *tags, Ctrl *ctrl,
-                                                         int flags) {
+                                                         int flags, Stage stg) {
     const bool fused = flags & kFused;
     ctrl = block_ctrl(ctrl, M);
     pdl_wait();
-    if (fused && ctrl_halted(ctrl)) return;
+    if (fused && ctrl_halt_settled(ctrl) == 1) return;
+    if (fused && threadIdx.x == 0 && first_of_scenario(M, blockIdx.x * blockDim.x)) {
+        commit_stage(ctrl, published_step_clock(ctrl), P, stg);
+        announce_halt(ctrl);
+    }
     const int N = M.N;
-    const double time = ctrl->time;
+    const double time = fused ? committed_time(ctrl, stg) : ctrl->time;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     int bad_bc = 0, no_nbr = 0;
     if (k < N) {
@@ -1000,12 +1004,7 @@ __global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, 
     }
     if (bad_bc) set_status(ctrl, SWGPU_EBOUNDARY);
     if (no_nbr) set_status(ctrl, SWGPU_EMESH);
-    if (fused) {
-        pdl_launch_dependents();
-        __syncthreads();
-        if (threadIdx.x == 0 && last_block_done(&ctrl->done_distribute, ctrl->blocks_distribute))
-            apply_pending_halt(ctrl);
-    }
+    if (fused) pdl_launch_dependents();
 }
 
 // distribute_to_vertices_and_edges for triangle k: extrapolation of the
@@ -1199,14 +1198,18 @@ __global__ void __launch_bounds__(kBlock) balance_fp64(DevMesh M, DevState S, De
 template <int BS>
 __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, DevParams P,
                                                           const BcTag *tags, Ctrl *ctrl,
-                                                          int flags) {
+                                                          int flags, Stage stg) {
     const bool fused = flags & kFused;
     ctrl = block_ctrl(ctrl, M);
     pdl_wait();
-    if (fused && ctrl_halted(ctrl)) return;
+    if (fused && ctrl_halt_settled(ctrl) == 1) return;
+    if (fused && threadIdx.x == 0 && first_of_scenario(M, blockIdx.x * blockDim.x)) {
+        commit_stage(ctrl, published_step_clock(ctrl), P, stg);
+        announce_halt(ctrl);
+    }
     const int N = M.N;
-    const int order = (int)ctrl->order;
-    const double time = ctrl->time;
+    const int order = (int)(fused ? ctrl->clk_order : ctrl->order);
+    const double time = fused ? committed_time(ctrl, stg) : ctrl->time;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     int bad_bc = 0, no_nbr = 0;
     if (k < N) {
@@ -1376,11 +1379,7 @@ __global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, Dev
     }
     if (bad_bc) set_status(ctrl, SWGPU_EBOUNDARY);
     if (no_nbr) set_status(ctrl, SWGPU_EMESH);
-    if (fused) {
-        pdl_launch_dependents();
-        __syncthreads();
-        if (threadIdx.x == 0 && last_block_done(&ctrl->done_distribute, ctrl->blocks_distribute)) apply_pending_halt(ctrl);
-    }
+    if (fused) pdl_launch_dependents();
 }
 
 // Boundary values of boundary edge mb, edge i of triangle k, from its edge
@@ -1419,12 +1418,16 @@ __device__ __forceinline__ int boundary_edge(const DevMesh &M, const DevState &S
 __global__ void __launch_bounds__(3 * kSplitTile) distribute_split_fp64(DevMesh M, DevState S,
                                                                         DevParams P,
                                                                         const BcTag *tags,
-                                                                        Ctrl *ctrl, int flags) {
+                                                                        Ctrl *ctrl, int flags, Stage stg) {
     const bool fused = flags & kFused;
     const int k0 = blockIdx.x * kSplitTile;
     if (M.blk_scen) ctrl += M.blk_scen[k0 >> 8];
     pdl_wait();
-    if (fused && ctrl_halted(ctrl)) return;
+    if (fused && ctrl_halt_settled(ctrl) == 1) return;
+    if (fused && threadIdx.x == 0 && first_of_scenario(M, blockIdx.x * kSplitTile)) {
+        commit_stage(ctrl, published_step_clock(ctrl), P, stg);
+        announce_halt(ctrl);
+    }
     const int N = M.N;
     const int role = threadIdx.x / kSplitTile, t = threadIdx.x % kSplitTile, k = k0 + t;
     __shared__ double vert[3][3][kSplitTile];  // [quantity][vertex], then balanced
@@ -1433,7 +1436,7 @@ __global__ void __launch_bounds__(3 * kSplitTile) distribute_split_fp64(DevMesh 
     bool to_momentum = false;
     double wk = 0.0, zk = 0.0, zvk[3] = {0.0, 0.0, 0.0};
     if (in) {
-        const int order = (int)ctrl->order;
+        const int order = (int)(fused ? ctrl->clk_order : ctrl->order);
         wk = S.w[k];
         zk = S.zc[k];
 #pragma unroll
@@ -1565,30 +1568,30 @@ __global__ void __launch_bounds__(3 * kSplitTile) distribute_split_fp64(DevMesh 
             if (flags & kWriteBoundary) {
                 const int pk = M.nbr[role * N + k];
                 if (pk < 0)
-                    bad_bc = boundary_edge(M, S, P, tags, ctrl->time, k, role, -pk - 1, we, uhe,
+                    bad_bc = boundary_edge(M, S, P, tags,
+                                       fused ? committed_time(ctrl, stg) : ctrl->time, k, role, -pk - 1, we, uhe,
                                            vhe);
             }
         }
     }
     if (bad_bc) set_status(ctrl, SWGPU_EBOUNDARY);
     if (no_nbr) set_status(ctrl, SWGPU_EMESH);
-    if (fused) {
-        pdl_launch_dependents();
-        __syncthreads();
-        if (threadIdx.x == 0 && last_block_done(&ctrl->done_distribute, ctrl->blocks_distribute))
-            apply_pending_halt(ctrl);
-    }
+    if (fused) pdl_launch_dependents();
 }
 
 __global__ void __launch_bounds__(3 * kSplitTile) distribute_de_split_fp64(DevMesh M, DevState S,
                                                                            DevParams P,
                                                                            const BcTag *tags,
-                                                                           Ctrl *ctrl, int flags) {
+                                                                           Ctrl *ctrl, int flags, Stage stg) {
     const bool fused = flags & kFused;
     const int first = blockIdx.x * kSplitTile;
     if (M.blk_scen) ctrl += M.blk_scen[first >> 8];
     pdl_wait();
-    if (fused && ctrl_halted(ctrl)) return;
+    if (fused && ctrl_halt_settled(ctrl) == 1) return;
+    if (fused && threadIdx.x == 0 && first_of_scenario(M, blockIdx.x * kSplitTile)) {
+        commit_stage(ctrl, published_step_clock(ctrl), P, stg);
+        announce_halt(ctrl);
+    }
     const int N = M.N;
     const int role = threadIdx.x / kSplitTile, t = threadIdx.x % kSplitTile, k = first + t;
     __shared__ double edge[3][3][kSplitTile];  // [quantity][edge]
@@ -1705,17 +1708,13 @@ __global__ void __launch_bounds__(3 * kSplitTile) distribute_de_split_fp64(DevMe
         if (flags & kWriteBoundary) {
             const int pk = M.nbr[role * N + k];
             if (pk < 0)
-                bad_bc = boundary_edge(M, S, P, tags, ctrl->time, k, role, -pk - 1, we, ue, ve);
+                bad_bc = boundary_edge(M, S, P, tags,
+                                       fused ? committed_time(ctrl, stg) : ctrl->time, k, role, -pk - 1, we, ue, ve);
         }
     }
     if (bad_bc) set_status(ctrl, SWGPU_EBOUNDARY);
     if (no_nbr) set_status(ctrl, SWGPU_EMESH);
-    if (fused) {
-        pdl_launch_dependents();
-        __syncthreads();
-        if (threadIdx.x == 0 && last_block_done(&ctrl->done_distribute, ctrl->blocks_distribute))
-            apply_pending_halt(ctrl);
-    }
+    if (fused) pdl_launch_dependents();
 }
 
 // update_boundary as a stand-alone pass over boundary slots, from the
@@ -1823,21 +1822,22 @@ void launch_prepare_fp64(const DevMesh &M, const DevState &S, const DevParams &P
 }
 // Block sizes of the fused-step kernels come from M.shape (fp64_block).
 void launch_distribute_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
-                            const BcTag *tags, Ctrl *ctrl, int flags, cudaStream_t st) {
+                            const BcTag *tags, Ctrl *ctrl, int flags, const Stage &stage,
+                            cudaStream_t st) {
     const int tile = distribute_tile_fp64(M.shape.distribute, M.N, M.shape.sms);
     const int g = (M.n_launch + tile - 1) / tile;
     const bool pdl = M.shape.pdl && (flags & kFused) && overlap_fp64(M.n_launch, M.shape.sms);
     if (distribute_split(M.N, M.shape.sms)) {
         launch_k(P.flow_algorithm ? distribute_de_split_fp64 : distribute_split_fp64, g, 3 * tile,
-                 st, pdl, M, S, P, tags, ctrl, flags);
+                 st, pdl, M, S, P, tags, ctrl, flags, stage);
         return;
     }
     if (P.flow_algorithm)
         launch_k(tile > 256 ? distribute_de_fp64<512> : distribute_de_fp64<256>, g, tile, st, pdl,
-                 M, S, P, tags, ctrl, flags);
+                 M, S, P, tags, ctrl, flags, stage);
     else
         launch_k(tile > 256 ? distribute_fp64<512> : distribute_fp64<256>, g, tile, st, pdl, M, S,
-                 P, tags, ctrl, flags);
+                 P, tags, ctrl, flags, stage);
 }
 void launch_boundary_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                           const BcTag *tags, Ctrl *ctrl,

@@ -185,22 +185,21 @@ struct RunSummary {
     int status;
 };
 
-// Device-resident evolve bookkeeping, one per scenario.  FP64 path: written by the
-// last block of the update kernel (time, order, counters) and the last block of
-// the distribute kernel (halt).  Mixed path: the step clock kernel publishes the
-// clock, the first block of the scenario in the distribute commits the stage.
-// Read by every kernel at entry.
+// Device-resident evolve bookkeeping, one per scenario.  The step's clock is
+// published after the flux grid (FP64: by its last block; mixed: by the update
+// or the step clock kernel), the first block of the scenario in the distribute
+// commits the stage.  Read by every kernel at entry.
 struct __align__(16) Ctrl {
     unsigned long long ftmin_bits;  // minimum flux timestep of this step (bits of a positive double)
     double time, yieldtime, finaltime, yieldstep, timestep, flux_timestep;
     double rec_max, rec_min, time_epsilon;
     long long order, smallsteps, steps_since_yield, total_steps;
     long long budget;               // steps left in this run; < 0 = unlimited
-    int halt;                       // nonzero: kernels return at entry
-    int halt_pending;               // stop reason raised by update, applied after distribute
+    int halt;                       // nonzero: kernels return at entry (2: see announce_halt)
+    int halt_pending;               // stop reason raised by the commit
     int stop_reason;
     int status;                     // first device-side failure (swgpu_status)
-    unsigned int done_update, done_distribute, done_flux;
+    unsigned int done_flux;
     int clk_small_error;            // the step's update_timestep, evaluated once
     double clk_dt, clk_ftmin;       // after the flux grid (FP64: its last block;
     long long clk_order, clk_smallsteps;  // mixed: step_clock_mixed) and read by
@@ -208,8 +207,6 @@ struct __align__(16) Ctrl {
     double clk_t0;                  // model time when that clock was evaluated
     double step_t0;                 // time at the start of a Runge-Kutta step
     unsigned int blocks_flux;       // blocks of this scenario in one flux launch
-    unsigned int blocks_update;     // ... in one update launch
-    unsigned int blocks_distribute; // ... in one distribute launch
     RunSummary *summary;            // shared by all scenarios of a handle
     unsigned int *halt_bits;        // one bit per scenario, set when it halts
     int scen;                       // this scenario's index
@@ -263,7 +260,8 @@ __host__ __device__ inline double pos_inf() { return 1.0e300 * 1.0e300; }
 void launch_prepare_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                          Ctrl *ctrl, cudaStream_t st);
 void launch_distribute_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
-                            const BcTag *tags, Ctrl *ctrl, int flags, cudaStream_t st);
+                            const BcTag *tags, Ctrl *ctrl, int flags, const Stage &stage,
+                            cudaStream_t st);
 void launch_boundary_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                           const BcTag *tags,
                           Ctrl *ctrl, cudaStream_t st);
