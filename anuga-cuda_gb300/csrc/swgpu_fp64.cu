@@ -12,8 +12,8 @@
 //   flux_fp64       central-upwind flux of each edge (one thread per edge),
 //                   CFL timestep -> block min -> atomicMin into Ctrl
 //   update_fp64     the edge fluxes of each triangle summed in ANUGA's order,
-//                   gravity_wb, the step's update_timestep (evaluated once by
-//                   the flux kernel's last block), Manning
+//                   gravity_wb, the step's update_timestep (evaluated here or
+//                   once by the flux kernel's last block), Manning
 //                   friction, the semi-implicit conserved update, protect,
 //                   centroid velocities for the next extrapolation
 //   distribute_fp64 second-order limited extrapolation, balance_deep_and_
@@ -287,7 +287,8 @@ __global__ void __launch_bounds__(kBlock) flux_fp64(DevMesh M, DevState S, DevPa
     if (flags & kNoTimestep) return;  // later Runge-Kutta stage: the step's dt is set
     pdl_launch_dependents();
     block_min_timestep<kBlock>(t, ctrl);
-    if ((flags & kFused) && threadIdx.x == 0 && last_block_done(&ctrl->done_flux, ctrl->blocks_flux))
+    if ((flags & (kFused | kClock)) == (kFused | kClock) && threadIdx.x == 0 &&
+        last_block_done(&ctrl->done_flux, ctrl->blocks_flux))
         publish_step_clock(ctrl, P);
 }
 
@@ -575,15 +576,17 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
             ctrl->halt = 1;  // the last step's distribute has run
         return;
     }
-    StepClock clk;
-    if (FUSED) {
-        clk = published_step_clock(ctrl);
-    } else {
-        clk.dt = dt_api;
+    __shared__ double block_dt;
+    const bool own_clock = FUSED && (flags & kClock);
+    if (own_clock && threadIdx.x == 0) {
+        const StepClock c = device_update_timestep(ctrl, P);
+        block_dt = c.dt;
+        if (first_of_scenario(M)) publish_step_clock(ctrl, c);
     }
-    const double dt = clk.dt;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     int bad = 0, nonfinite = 0;
+    if (own_clock) __syncthreads();
+    const double dt = own_clock ? block_dt : (FUSED ? ctrl->clk_dt : dt_api);
     if (k < M.N) {
         double w = S.w[k], uh = S.uh[k], vh = S.vh[k];
         const double zc = S.zc[k];
@@ -656,7 +659,7 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
         S.uh[k] = uh;
         S.vh[k] = vh;
         if ((flags & kTrack) && (stg.kind == kStageEuler || stg.kind == kStageLast))
-            track_depth(S, k, w - zc, step_end_time(ctrl, clk.dt, stg), P.track_threshold);
+            track_depth(S, k, w - zc, step_end_time(ctrl, dt, stg), P.track_threshold);
     }
     if (bad) set_status(ctrl, SWGPU_EDENOMINATOR);
     if (nonfinite) set_status(ctrl, SWGPU_ENONFINITE);
@@ -1848,6 +1851,7 @@ void launch_flux_fp64(const DevMesh &M, const DevState &S, const DevParams &P, C
                       int flags, cudaStream_t st) {
     const int bs = fp64_block(M.shape.flux, M.edges.E, M.shape.sms);
     const bool pdl = M.shape.pdl && (flags & kFused) && overlap_fp64(M.n_launch, M.shape.sms);
+    if (!update_clock_fp64(M.N, M.shape.sms)) flags |= kClock;
     launch_k(flux_fp64, (M.edges.launch + bs - 1) / bs, bs, st, pdl, M, S, P, ctrl, flags);
 }
 void launch_explicit_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
@@ -1874,6 +1878,10 @@ void launch_update_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                         double dt, int flags, const Stage &stage, cudaStream_t st) {
     const int bs = fp64_block(M.shape.update, M.N, M.shape.sms);
     const int g = (M.n_launch + bs - 1) / bs;
+    // (a later Runge-Kutta stage has the step's clock)
+    if ((stage.kind == kStageEuler || stage.kind == kStageFirst) &&
+        update_clock_fp64(M.N, M.shape.sms))
+        flags |= kClock;
     if (flags & kFused)
         launch_k(bs > 256 ? update_fp64<512, true> : update_fp64<256, true>, g, bs, st,
                  M.shape.pdl && overlap_fp64(M.n_launch, M.shape.sms), M, S, P, ctrl, dt, flags,
