@@ -1034,6 +1034,7 @@ struct Wgrad {
 };
 struct __align__(1024) SmemW {
     unsigned char buf[3][kActBytes];
+    unsigned char x[3][kXBytes];  // layer 1's features, with its gradient's buffer
     unsigned long long full[3], free_[3], done, drained;
     unsigned tmem;
 };
@@ -1060,25 +1061,30 @@ __global__ void __launch_bounds__(kThreadsW + 32, 1) mlp_wgrad(Wgrad g) {
     const int item0 = first ? blockIdx.x - g.big : blockIdx.x;
     const int step = first ? gridDim.x - g.big : g.big;
     const int items = first ? g.splits : 2 * g.splits;
+    const int per_tile = first ? 1 : 2;  // buffers
     bool ok = true;
     if (tid >= kThreadsW) {
         if (tid == kThreadsW) {
-            // loads: of each tile the activations (or features), then the
-            // layer's gradient, into the three buffers in turn, a tile and a
-            // half ahead of the products
+            // loads, into the three buffers in turn: of each tile the
+            // activations, then the layer's gradient, a tile and a half ahead
+            // of the products; of layer 1 its gradient with the tile's
+            // features, three tiles ahead (with the features in a buffer of
+            // their own, and so a tile and a half, an item of layer 1 took
+            // 22,000 clocks and the launch 38 us; so 30)
             int load_item = item0, load_tile = 0, loads = 0;
-            const auto load_next = [&](bool second) {
+            const auto load_next = [&] {
                 const int prod = first ? 2 : load_item / g.splits;
                 const int split = first ? load_item : load_item % g.splits;
                 const int t = split * kSplitTiles + load_tile;
                 const int i = loads % 3;
+                const bool second = first || (loads & 1);
                 if (loads >= 3) ok = mbar_wait(&S.free_[i], (loads / 3 - 1) & 1, g.status);
                 if (!ok) return;
-                const unsigned bytes = first && !second ? kXBytes : kActBytes;
+                mbar_expect(&S.full[i], first ? kXBytes + kActBytes : kActBytes);
+                if (first) bulk_load(S.x[i], g.x + (size_t)t * kXBytes, kXBytes, &S.full[i]);
                 const unsigned char *src = second ? (prod == 0 ? g.d3 : (prod == 1 ? g.d2 : g.d1))
-                                                  : (prod == 0 ? g.h2 : (prod == 1 ? g.h1 : g.x));
-                mbar_expect(&S.full[i], bytes);
-                bulk_load(S.buf[i], src + (size_t)t * bytes, bytes, &S.full[i]);
+                                                  : (prod == 0 ? g.h2 : g.h1);
+                bulk_load(S.buf[i], src + (size_t)t * kActBytes, kActBytes, &S.full[i]);
                 loads++;
                 if (second) {
                     load_tile++;
@@ -1089,7 +1095,7 @@ __global__ void __launch_bounds__(kThreadsW + 32, 1) mlp_wgrad(Wgrad g) {
                 }
             };
             const auto ahead = [&](int upto) {
-                while (ok && load_item < items && loads < upto) load_next(loads & 1);
+                while (ok && load_item < items && loads < upto) load_next();
             };
             int used = 0, n = 0;
             ahead(3);
@@ -1101,11 +1107,13 @@ __global__ void __launch_bounds__(kThreadsW + 32, 1) mlp_wgrad(Wgrad g) {
                 tc_fence_after();
                 bool more = false;
                 for (int t = split * kSplitTiles; ok && t < t1; t++) {
-                    const int ia = used % 3, ib = (used + 1) % 3;
+                    const int ia = used % 3, ib = (used + per_tile - 1) % 3;
                     ok = mbar_wait(&S.full[ia], (used / 3) & 1, g.status);
-                    if (ok) ok = mbar_wait(&S.full[ib], ((used + 1) / 3) & 1, g.status);
+                    if (ok && !first)
+                        ok = mbar_wait(&S.full[ib], ((used + 1) / 3) & 1, g.status);
                     if (!ok) break;
-                    const unsigned a = smem_u32(S.buf[ia]), b = smem_u32(S.buf[ib]);
+                    const unsigned a = smem_u32(first ? S.x[ia] : S.buf[ia]),
+                                   b = smem_u32(S.buf[ib]);
                     for (int m = 0; m < 2; m++)
                         for (int kk = 0; kk < 8; kk++) {
                             if (!first)  // 128 inputs x 256 outputs
@@ -1122,10 +1130,10 @@ __global__ void __launch_bounds__(kThreadsW + 32, 1) mlp_wgrad(Wgrad g) {
                                        tc_idesc(kF, true, true), more || kk > 0);
                         }
                     more = true;
-                    tc_commit(&S.free_[ia]);
+                    if (!first) tc_commit(&S.free_[ia]);
                     tc_commit(&S.free_[ib]);
                     if (t + 1 == t1) tc_commit(&S.done);
-                    used += 2;
+                    used += per_tile;
                     ahead(used + 3);
                 }
             }
@@ -1143,12 +1151,14 @@ __global__ void __launch_bounds__(kThreadsW + 32, 1) mlp_wgrad(Wgrad g) {
             for (int q = 0; q < 4; q++)
 #pragma unroll
                 for (int j = 0; j < 8; j++) gb[q][j] = 0.f;
-            for (int t = split * kSplitTiles; t < t1; t++, used += 2) {
-                const int ia = used % 3, ib = (used + 1) % 3;
+            for (int t = split * kSplitTiles; t < t1; t++, used += per_tile) {
+                const int ia = used % 3, ib = (used + per_tile - 1) % 3;
                 if (ok) ok = mbar_wait(&S.full[ia], (used / 3) & 1, g.status);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&S.free_[ia]);
-                if (ok) ok = mbar_wait(&S.full[ib], ((used + 1) / 3) & 1, g.status);
+                if (!first) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&S.free_[ia]);
+                    if (ok) ok = mbar_wait(&S.full[ib], ((used + 1) / 3) & 1, g.status);
+                }
 #pragma unroll 1
                 for (int r = lane; ok && r < kTileM; r += 32)
 #pragma unroll
@@ -1722,7 +1732,7 @@ __global__ void mlp_pack_weights(const float *__restrict__ p, BfWeights *W) {
 
 // ---- host side ----------------------------------------------------------------
 
-struct Buffers {  // one batch of rows (training) or one chunk (inference)
+struct Buffers {  // one batch of rows (training)
     int tiles = 0;
     unsigned char *h2 = nullptr;                    // tile images
     unsigned char *x = nullptr, *h1 = nullptr, *d3 = nullptr, *d2 = nullptr, *d1 = nullptr;
