@@ -187,8 +187,8 @@ struct RunSummary {
 
 // Device-resident evolve bookkeeping, one per scenario.  The step's clock is
 // published after the flux grid (FP64: by its last block or the update; mixed: by
-// the update or the step clock kernel), the first block of the scenario in the distribute
-// commits the stage.  Read by every kernel at entry.
+// the update or the step clock kernel), the first block of the scenario in the
+// distribute commits the stage.  Read by every kernel at entry.
 struct __align__(16) Ctrl {
     unsigned long long ftmin_bits;  // minimum flux timestep of this step (bits of a positive double)
     double time, yieldtime, finaltime, yieldstep, timestep, flux_timestep;
@@ -201,9 +201,8 @@ struct __align__(16) Ctrl {
     int status;                     // first device-side failure (swgpu_status)
     unsigned int done_flux;
     int clk_small_error;            // the step's update_timestep, evaluated once
-    double clk_dt, clk_ftmin;       // after the flux grid (FP64: its last block;
-    long long clk_order, clk_smallsteps;  // mixed: step_clock_mixed) and read by
-                                          // the update and distribute kernels
+    double clk_dt, clk_ftmin;       // after the flux grid and read by the update
+    long long clk_order, clk_smallsteps;  // and distribute kernels
     double clk_t0;                  // model time when that clock was evaluated
     double step_t0;                 // time at the start of a Runge-Kutta step
     unsigned int blocks_flux;       // blocks of this scenario in one flux launch

@@ -705,6 +705,42 @@ __device__ __forceinline__ void row_outputs(const float4 (&part)[kGroups][kTileM
     y[2] = (a.z + c.z) + (b.z + d.z) + b4[2];
 }
 
+// Sums over a warp's lanes of n values each; this lane is left with those from
+// index lanes_first on in v[0 ..] (32 values: one, 48: three, in both lanes of
+// a pair).  Lanes half a warp apart share the values between them, each adding
+// its half, then lanes a quarter apart: the additions are those of a butterfly
+// over every value (48 values in 48 shuffles instead of 240, which took 6,000
+// clocks at the end of mlp_layer3_train).
+template <int n, int d = 16, int N>
+__device__ __forceinline__ void lane_sums(float (&v)[N]) {
+    if constexpr (n % 2 == 0) {
+        const bool up = threadIdx.x & d;
+#pragma unroll
+        for (int i = 0; i < n / 2; i++) {
+            const float mine = up ? v[n / 2 + i] : v[i], other = up ? v[i] : v[n / 2 + i];
+            v[i] = mine + __shfl_xor_sync(0xffffffffu, other, d);
+        }
+        if constexpr (d > 1) lane_sums<n / 2, d / 2>(v);
+    } else {
+#pragma unroll
+        for (int i = 0; i < n; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], d);
+        if constexpr (d > 1) lane_sums<n, d / 2>(v);
+    }
+}
+// The index of v[0] then, and whether this lane is the first to have it.
+template <int n, int d = 16>
+__device__ __forceinline__ int lanes_first(bool &own) {
+    if constexpr (n % 2 == 0) {
+        int i = threadIdx.x & d ? n / 2 : 0;
+        if constexpr (d > 1) i += lanes_first<n / 2, d / 2>(own);
+        return i;
+    } else {
+        own = own && !(threadIdx.x & d);
+        if constexpr (d > 1) return lanes_first<n, d / 2>(own);
+        return 0;
+    }
+}
+
 struct __align__(1024) Smem3T {
     unsigned char w3[kWBytes];
     unsigned char a[kActBytes];        // h2, then h3, then its gradient
@@ -896,17 +932,22 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_layer3_train(Layer3 g) {
     if (tid == 0) bulk_store_done();
     // this CTA's sums, each over its lanes in a fixed order
     float *out = g.part4 + (size_t)blockIdx.x * kPart4;
+    {
+        constexpr int n = kWarpVecs * 8 * kOut;  // 48: three are left to a pair of lanes
+        float v[n];
 #pragma unroll
-    for (int q = 0; q < kWarpVecs; q++)
+        for (int q = 0; q < kWarpVecs; q++)
 #pragma unroll
-        for (int j = 0; j < 8; j++)
+            for (int j = 0; j < 8; j++)
 #pragma unroll
-            for (int o = 0; o < kOut; o++) {
-                float s = gw[q][j][o];
+                for (int o = 0; o < kOut; o++) v[(q * 8 + j) * kOut + o] = gw[q][j][o];
+        lane_sums<n>(v);
+        bool own = true;
+        const int at = lanes_first<n>(own);
+        if (own)
 #pragma unroll
-                for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-                if (lane == 0) out[((kWarpVecs * warp + q) * 8 + j) * kOut + o] = s;
-            }
+            for (int o = 0; o < kOut; o++) out[n * warp + at + o] = v[o];
+    }
     const float tail[kOut + 1] = {gb[0], gb[1], gb[2], ls};
 #pragma unroll
     for (int o = 0; o <= kOut; o++) {
@@ -1174,15 +1215,15 @@ __global__ void __launch_bounds__(kThreadsW + 32, 1) mlp_wgrad(Wgrad g) {
                 if (lane == 0) mbar_arrive(&S.free_[ib]);
             }
             float *out_b = g.part_b + (size_t)(prod * g.splits + split) * kH;
+            float v[32];
 #pragma unroll
             for (int q = 0; q < 4; q++)
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    float s = gb[q][j];
-#pragma unroll
-                    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-                    if (lane == 0) out_b[(4 * warp + q) * 8 + j] = s;
-                }
+                for (int j = 0; j < 8; j++) v[8 * q + j] = gb[q][j];
+            lane_sums<32>(v);
+            bool own = true;
+            const int at = lanes_first<32>(own);
+            out_b[32 * warp + at] = v[0];
             if (ok) ok = mbar_wait(&S.done, n & 1, g.status);
             ok = __all_sync(0xffffffffu, ok);
             if (ok) {
