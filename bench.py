@@ -64,7 +64,6 @@ MIXED_BYTES = {"flux": 128, "update": 104, "distribute": 114}
 # DRAM bytes (read + write) per launch from one ncu capture of the 4,000,000-
 # triangle mesh (1000x1000 cells); scaled by the triangles for other meshes
 NCU_TRAFFIC_4M = {"flux": 509.35e6, "update": 377.39e6, "distribute": 520.23e6}
-FP64_BYTES = {"flux": 296, "update": 120, "distribute": 253}
 MODEL_BYTES = {"mixed": 368, "fp64": 568}   # whole-step byte model
 ACC_STEPS = 1000                             # steps of the mixed-vs-FP64 accuracy check
 WET_FLOOR = 0.01                             # m: wet triangles of the per-element depth error
@@ -74,7 +73,7 @@ WET_FLOOR = 0.01                             # m: wet triangles of the per-eleme
 # FP64 at 1/64 of the FP32 rate, 2 thread instructions per SM per clock
 # (DADD, DMUL, DFMA and the pipe's other instructions one slot each):
 # 152 SMs x 2 x 2.07 GHz
-FP64_PIPE_INST = {"flux": 494.99, "update": 166.79, "distribute": 317.03}
+FP64_PIPE_INST = {"flux": 94.48, "update": 95.00, "distribute": 138.99}
 FP64_PIPE_PEAK = 152 * 2 * 2.07e9
 
 
@@ -693,9 +692,10 @@ def main():
                      "step_model_frac": MODEL_BYTES["mixed"] * N / (mixed_ms / K / 1000.0) / 1e9
                      / peak_gbs},
         "clocks": r["mixed"]["clocks"],
-        # the timed region issues K steps of 4 kernels (flux, step clock,
-        # update, distribute): whole graphs of 16 steps, then the remainder
-        "gpu_launches": 4 * K,
+        # the timed region issues K steps of 3 kernels (flux, update, distribute)
+        # and, at 2^20 triangles and more, the step clock's: whole graphs of 16
+        # steps, then the remainder
+        "gpu_launches": (4 if N >= 1 << 20 else 3) * K,
         "host_cpu": host_cpu(),
     }
     if out["e2e"]:
