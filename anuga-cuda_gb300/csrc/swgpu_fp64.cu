@@ -232,10 +232,18 @@ __device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevPa
 // owner and adds it to the neighbour.  One thread per edge: 1.5 fluxes per
 // triangle instead of three, and equal work for every lane.
 //
+// PER_SM: blocks of 256 that the registers leave room for, here and in the
+// distribute.  With three, at 80 registers (24 and 34 words spilled, which L1
+// holds), the FP64 pipe of a large mesh finds a ready warp more often than with
+// two at 97 and 127 (a million triangles: flux 224 -> 205 us, distribute 318 ->
+// 304; four: 202 and 310); a mesh without that many warps only has the spills
+// (2,132 triangles: 26.7 -> 27.7 us a stage).
+//
 // CFL: min(r_k, r_n) / ms is the smaller of r_k / ms and r_n / ms, since a
 // correctly rounded quotient does not fall when its numerator grows; the
 // radius is infinite for an edge that does not count (owner not full).
-__global__ void __launch_bounds__(kBlock) flux_fp64(DevMesh M, DevState S, DevParams P,
+template <int PER_SM>
+__global__ void __launch_bounds__(kBlock, PER_SM) flux_fp64(DevMesh M, DevState S, DevParams P,
                                                     Ctrl *ctrl, int flags) {
     const DevEdges &F = M.edges;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -838,8 +846,8 @@ __device__ __forceinline__ void limiter_betas(const DevParams &P, double hfactor
 // (v_i = e_j + e_k - e_i), momenta back from velocities with the edge and
 // vertex depths; cells skipped as dry keep their previous edge values.  Edge
 // values are always stored (the flux reads them), then the boundary values.
-template <int BS>
-__global__ void __launch_bounds__(BS) distribute_de_fp64(DevMesh M, DevState S, DevParams P,
+template <int BS, int PER_SM>
+__global__ void __launch_bounds__(BS, PER_SM * 256 / BS) distribute_de_fp64(DevMesh M, DevState S, DevParams P,
                                                          const BcTag *tags, Ctrl *ctrl,
                                                          int flags, Stage stg) {
     const bool fused = flags & kFused;
@@ -1198,8 +1206,8 @@ __global__ void __launch_bounds__(kBlock) balance_fp64(DevMesh M, DevState S, De
     }
 }
 
-template <int BS>
-__global__ void __launch_bounds__(BS) distribute_fp64(DevMesh M, DevState S, DevParams P,
+template <int BS, int PER_SM>
+__global__ void __launch_bounds__(BS, PER_SM * 256 / BS) distribute_fp64(DevMesh M, DevState S, DevParams P,
                                                           const BcTag *tags, Ctrl *ctrl,
                                                           int flags, Stage stg) {
     const bool fused = flags & kFused;
@@ -1835,12 +1843,15 @@ void launch_distribute_fp64(const DevMesh &M, const DevState &S, const DevParams
                  st, pdl, M, S, P, tags, ctrl, flags, stage);
         return;
     }
+    const bool dense = dense_fp64(M.N, M.shape.sms);
     if (P.flow_algorithm)
-        launch_k(tile > 256 ? distribute_de_fp64<512> : distribute_de_fp64<256>, g, tile, st, pdl,
-                 M, S, P, tags, ctrl, flags, stage);
+        launch_k(tile > 256 ? distribute_de_fp64<512, 2>
+                            : (dense ? distribute_de_fp64<256, 3> : distribute_de_fp64<256, 2>),
+                 g, tile, st, pdl, M, S, P, tags, ctrl, flags, stage);
     else
-        launch_k(tile > 256 ? distribute_fp64<512> : distribute_fp64<256>, g, tile, st, pdl, M, S,
-                 P, tags, ctrl, flags, stage);
+        launch_k(tile > 256 ? distribute_fp64<512, 2>
+                            : (dense ? distribute_fp64<256, 3> : distribute_fp64<256, 2>),
+                 g, tile, st, pdl, M, S, P, tags, ctrl, flags, stage);
 }
 void launch_boundary_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                           const BcTag *tags, Ctrl *ctrl,
@@ -1852,7 +1863,8 @@ void launch_flux_fp64(const DevMesh &M, const DevState &S, const DevParams &P, C
     const int bs = fp64_block(M.shape.flux, M.edges.E, M.shape.sms);
     const bool pdl = M.shape.pdl && (flags & kFused) && overlap_fp64(M.n_launch, M.shape.sms);
     if (!update_clock_fp64(M.N, M.shape.sms)) flags |= kClock;
-    launch_k(flux_fp64, (M.edges.launch + bs - 1) / bs, bs, st, pdl, M, S, P, ctrl, flags);
+    launch_k(dense_fp64(M.N, M.shape.sms) ? flux_fp64<3> : flux_fp64<1>,
+             (M.edges.launch + bs - 1) / bs, bs, st, pdl, M, S, P, ctrl, flags);
 }
 void launch_explicit_fp64(const DevMesh &M, const DevState &S, const DevParams &P,
                           cudaStream_t st) {

@@ -361,6 +361,12 @@ inline int distribute_tile_fp64(int knob, int64_t n, int sms) {
     return distribute_split(n, sms) ? kSplitTile : fp64_block(knob, n, sms);
 }
 
+// Whether the FP64 kernels are built for warps in flight rather than for
+// registers (PER_SM at flux_fp64): microseconds per step with / without, 40,000
+// triangles 47.7 / 47.4, 57,600 56.9 / 56.8, 79,524 79.8 / 83.7, a million
+// 759 / 775.
+inline bool dense_fp64(int64_t n, int sms) { return n >= (int64_t)420 * sms; }
+
 // Whether the FP64 step's clock is evaluated by every block of the update for
 // itself (while its loads are on their way), instead of by the flux's last
 // block to finish: 1,024 triangles 23.5 us a step instead of 24.3, 79,524 83.2

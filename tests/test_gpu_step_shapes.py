@@ -1,6 +1,6 @@
 """The step kernels on both sides of the mesh sizes where their shape changes:
-three threads per triangle or one in the FP64 distribute, and where in a kernel
-(or whether) the next one starts."""
+three threads per triangle or one in the FP64 distribute, more or fewer registers
+in the FP64 kernels, and where in a kernel (or whether) the next one starts."""
 import dataclasses
 
 import numpy as np
@@ -35,7 +35,7 @@ TOL = 1.0e-12
 
 
 @pytest.mark.parametrize("flow", [0, 1])
-@pytest.mark.parametrize("size", ["one_block", "ragged", "split", "single"])
+@pytest.mark.parametrize("size", ["one_block", "ragged", "split", "single", "dense"])
 def test_fp64_distribute_shapes_match_oracle(size, flow, oracle_mod, swgpu_built):
     from anuga_cuda import DEFAULT, scenarios
     line = 160 * _sms()
@@ -44,7 +44,7 @@ def test_fp64_distribute_shapes_match_oracle(size, flow, oracle_mod, swgpu_built
     elif size == "ragged":
         sc = scenarios.small_basin(41, 23, seed=5)
     else:
-        sc = _scene(line, size == "single")
+        sc = _scene(420 * _sms() if size == "dense" else line, size != "split")
     sc = dataclasses.replace(sc, friction=np.zeros(sc.N))
     p = DEFAULT.replace(flow_algorithm=flow)
     od = oracle_from_scenario(oracle_mod, sc, p)
