@@ -130,12 +130,16 @@ static int sync_ctrl(Handle *h) {
 static int read_ctrl(Handle *h) { return h->ctrl_current ? check_usable(h) : sync_ctrl(h); }
 
 // The mirror to change: a copy from it to the device has to be done with it.
+// From here on it is not the device's until push_ctrl: a call that is refused
+// or fails in between leaves its changes behind, and the next one reads the
+// device again.
 static int edit_ctrl(Handle *h) {
     if (int rc = read_ctrl(h)) return rc;
     if (h->push_pending) {
         CK(cudaStreamSynchronize(h->stream));
         h->push_pending = false;
     }
+    h->ctrl_current = false;
     return SWGPU_OK;
 }
 
@@ -145,6 +149,7 @@ static int push_ctrl(Handle *h) {
     CK(cudaMemcpyAsync(h->d_ctrl, h->h_ctrl, sizeof(Ctrl) * h->nscen, cudaMemcpyHostToDevice,
                        h->stream));
     h->push_pending = true;
+    h->ctrl_current = true;
     return SWGPU_OK;
 }
 
@@ -1195,7 +1200,7 @@ int swgpu_compute_fluxes(void *handle, double *flux_timestep) {
     launch_flux_fp64(h->M, h->S, h->P, h->d_ctrl, kWriteMaxSpeed, h->stream);
     launch_explicit_fp64(h->M, h->S, h->P, h->stream);
     if ((rc = check_launch(h, "compute_fluxes"))) return rc;
-    if ((rc = sync_ctrl(h))) return rc;
+    if ((rc = edit_ctrl(h))) return rc;
     double ft;
     std::memcpy(&ft, &h->h_ctrl->ftmin_bits, sizeof ft);
     h->h_ctrl->flux_timestep = ft;
@@ -1345,11 +1350,11 @@ int swgpu_ensemble_set_finaltimes(void *handle, const double *finaltimes) {
     if (!h || !finaltimes) return fail(h, SWGPU_EINVAL, "null argument");
     int rc = edit_ctrl(h);
     if (rc) return rc;
-    for (int i = 0; i < h->nscen; i++) {
+    for (int i = 0; i < h->nscen; i++)
         if (finaltimes[i] > 0 && finaltimes[i] < h->h_ctrl[i].time)
             return fail(h, SWGPU_EINVAL, "scenario %d: finaltime before its time", i);
+    for (int i = 0; i < h->nscen; i++)
         h->h_ctrl[i].finaltime = finaltimes[i] > 0 ? finaltimes[i] : -1.0;
-    }
     return push_ctrl(h);
 }
 
@@ -1416,8 +1421,9 @@ int swgpu_set_launch_config(void *handle, const swgpu_launch_config *cfg) {
         return fail(h, SWGPU_EINVAL,
                     "launch config: flux 64/128/256 (at most 128 pipelined), update and "
                     "distribute 128/256/512 (at most 256 for an ensemble), 1..64 steps per graph");
-    int rc = sync_ctrl(h);
+    int rc = edit_ctrl(h);
     if (rc) return rc;
+    CK(cudaStreamSynchronize(h->stream));
     drop_graphs(h);  // recaptured with the new shape on the next run
     h->M.shape.flux = cfg->flux_block;
     h->M.shape.update = cfg->update_block;
@@ -1503,7 +1509,7 @@ int swgpu_evolve_start(void *handle, double starttime, double yieldstep, double 
     if (rc) return rc;
     // first distribute with the current order (gpu_domain_advanced.py:2476)
     if ((rc = issue_distribute(h, false))) return rc;
-    if ((rc = sync_ctrl(h))) return rc;
+    if ((rc = edit_ctrl(h))) return rc;
     for (int i = 0; i < h->nscen; i++) {
         Ctrl *c = &h->h_ctrl[i];
         c->time = starttime;
