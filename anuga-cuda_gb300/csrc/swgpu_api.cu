@@ -100,6 +100,14 @@ static int check_launch(Handle *h, const char *what) {
     return SWGPU_OK;
 }
 
+// The end of a method that puts kernels or copies on the stream: its status is
+// that of its own work (a failure would else come up in a later call).
+static int finish(Handle *h, const char *what) {
+    if (int rc = check_launch(h, what)) return rc;
+    CK(cudaStreamSynchronize(h->stream));
+    return SWGPU_OK;
+}
+
 // A handle whose kernels reported SWGPU_ETIMEOUT (a bounded wait for a
 // tile's bulk copies ran out twice) may have left copies in flight into the
 // shared memory of blocks that have exited; nothing it computes afterwards
@@ -1159,8 +1167,7 @@ int swgpu_protect(void *handle) {
     int rc = require_fp64(h, "protect");
     if (rc) return rc;
     launch_prepare_fp64(h->M, h->S, h->P, h->d_ctrl, h->stream);
-    if ((rc = check_launch(h, "protect"))) return rc;
-    return SWGPU_OK;
+    return finish(h, "protect");
 }
 
 int swgpu_distribute_to_vertices_and_edges(void *handle) {
@@ -1200,7 +1207,7 @@ int swgpu_compute_fluxes(void *handle, double *flux_timestep) {
     launch_flux_fp64(h->M, h->S, h->P, h->d_ctrl, kWriteMaxSpeed, h->stream);
     launch_explicit_fp64(h->M, h->S, h->P, h->stream);
     if ((rc = check_launch(h, "compute_fluxes"))) return rc;
-    if ((rc = edit_ctrl(h))) return rc;
+    if ((rc = sync_ctrl(h)) || (rc = edit_ctrl(h))) return rc;
     double ft;
     std::memcpy(&ft, &h->h_ctrl->ftmin_bits, sizeof ft);
     h->h_ctrl->flux_timestep = ft;
@@ -1214,8 +1221,7 @@ int swgpu_compute_forcing_terms(void *handle) {
     int rc = require_fp64(h, "compute_forcing_terms");
     if (rc) return rc;
     launch_forcing_fp64(h->M, h->S, h->P, false, h->stream);
-    if ((rc = check_launch(h, "compute_forcing_terms"))) return rc;
-    return SWGPU_OK;
+    return finish(h, "compute_forcing_terms");
 }
 
 int swgpu_manning_friction_explicit(void *handle) {
@@ -1223,8 +1229,7 @@ int swgpu_manning_friction_explicit(void *handle) {
     int rc = require_fp64(h, "manning_friction_explicit");
     if (rc) return rc;
     launch_forcing_fp64(h->M, h->S, h->P, true, h->stream);
-    if ((rc = check_launch(h, "manning_friction_explicit"))) return rc;
-    return SWGPU_OK;
+    return finish(h, "manning_friction_explicit");
 }
 
 int swgpu_extrapolate_second_order_sw(void *handle) {
@@ -1252,8 +1257,7 @@ int swgpu_balance_deep_and_shallow(void *handle) {
     if (rc) return rc;
     launch_balance_fp64(h->M, h->S, h->P, h->stream);
     h->edges_stale = true;
-    if ((rc = check_launch(h, "balance_deep_and_shallow"))) return rc;
-    return SWGPU_OK;
+    return finish(h, "balance_deep_and_shallow");
 }
 
 int swgpu_update_conserved_quantities(void *handle, double timestep) {
@@ -1276,7 +1280,7 @@ int swgpu_backup_conserved_quantities(void *handle) {
     CK(cudaMemcpyAsync(h->S.bw, h->S.w, bytes, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->S.buh, h->S.uh, bytes, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->S.bvh, h->S.vh, bytes, cudaMemcpyDeviceToDevice, h->stream));
-    return SWGPU_OK;
+    return finish(h, "backup_conserved_quantities");
 }
 
 int swgpu_saxpy_conserved_quantities(void *handle, double a, double b) {
@@ -1284,9 +1288,8 @@ int swgpu_saxpy_conserved_quantities(void *handle, double a, double b) {
     int rc = require_fp64(h, "saxpy_conserved_quantities");
     if (rc) return rc;
     launch_saxpy_fp64(h->M, h->S, a, b, h->stream);
-    if ((rc = check_launch(h, "saxpy_conserved_quantities"))) return rc;
     h->vertices_stale = true;
-    return SWGPU_OK;
+    return finish(h, "saxpy_conserved_quantities");
 }
 
 int swgpu_set_timestepping_method(void *handle, int method) {
@@ -1308,9 +1311,7 @@ int swgpu_update_other_quantities(void *handle) {
     if (h->precision == SWGPU_MIXED && !h->mixed_from_stage)
         launch_stage_from_mixed(h->M, h->S, h->X, h->stream);
     launch_other_quantities(h->M, h->S, h->stream);
-    int rc = check_launch(h, "update_other_quantities");
-    if (rc) return rc;
-    return SWGPU_OK;
+    return finish(h, "update_other_quantities");
 }
 
 int swgpu_mass(void *handle, double *mass) {

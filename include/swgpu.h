@@ -13,6 +13,9 @@
  *   - Every function returns an int status: SWGPU_OK (0) or a SWGPU_E*
  *     code.  swgpu_last_error() gives the message of the last failure on a
  *     handle.  Nothing in the library aborts, traps or exits.
+ *   - A call returns when its kernels and its copies of the caller's data are
+ *     done, and its status is theirs.  Clocks and final times that a call
+ *     sets reach the device in stream order, before any later work.
  *   - Host arrays use ANUGA's layout: triangle k, edge/vertex i at [3k+i],
  *     normals and vertex coordinates at [6k+2i] (x) and [6k+2i+1] (y),
  *     indices as int64 (ANUGA's `long`).  The library copies them; it never
