@@ -164,11 +164,11 @@ __device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevPa
     double uhl = al, vhl = bl, uhr = ar, vhr = br;
     // limited_speed for both momentum components of both sides (its second
     // call sees the depth that the first one left; a zero over a positive
-    // depth is a zero)
+    // depth is a zero).  Epsilon may lie above lim: it cuts a side below both.
     double dl = hl, dr = hr;
     const bool sl = lt_pos(hl, lim), sr = lt_pos(hr, lim);
     if (sl || sr) {
-        const bool zl = lt_pos(hl, eps), zr = lt_pos(hr, eps);
+        const bool zl = sl && lt_pos(hl, eps), zr = sr && lt_pos(hr, eps);
         if (zl) hl = uhl = vhl = 0.0;
         if (zr) hr = uhr = vhr = 0.0;
         dl = zl ? 1.0 : hl;
