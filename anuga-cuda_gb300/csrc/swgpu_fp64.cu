@@ -454,7 +454,7 @@ __device__ __forceinline__ double manning_S(const DevMesh &M, const DevState &S,
     const double eta = S.fric[k];
     const double eps = P.minimum_allowed_height;
     applied = false;
-    if (!lt64(eps, eta)) return 0.0;
+    if (!gt64_nan(eta, eps)) return 0.0;  // (a triangle without a value, NaN, has none)
     const double z0 = S.zv[k], z1 = S.zv[N + k], z2 = S.zv[2 * N + k];
     double zs = 1.0;
     if (P.use_sloped_mannings) {
@@ -470,7 +470,7 @@ __device__ __forceinline__ double manning_S(const DevMesh &M, const DevState &S,
     }
     const double z = fdiv64(z0 + z1 + z2, 3.0);
     const double h = w - z;
-    if (lt64(h, eps)) return 0.0;
+    if (lt64(h, eps) || nan64(h)) return 0.0;
     double Sf;
     if (P.use_sloped_mannings)
         Sf = -P.g * eta * eta * zs * fsqrt64(uh * uh + vh * vh);

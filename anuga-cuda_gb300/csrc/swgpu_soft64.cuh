@@ -52,10 +52,13 @@ __device__ __forceinline__ i64 order64(double x) {
 }
 __device__ __forceinline__ bool lt64(double x, double y) { return order64(x) < order64(y); }
 
-// x < y also where x may be NaN (then false)
-__device__ __forceinline__ bool lt64_nan(double x, double y) {
-    return lt64(x, y) && (bits64(x) & kMag64) <= 0x7ff0000000000000ull;
+__device__ __forceinline__ bool nan64(double x) {
+    return (bits64(x) & kMag64) > 0x7ff0000000000000ull;
 }
+// x < y also where x may be NaN (then false)
+__device__ __forceinline__ bool lt64_nan(double x, double y) { return lt64(x, y) && !nan64(x); }
+// x > y also where x may be NaN (then false)
+__device__ __forceinline__ bool gt64_nan(double x, double y) { return lt64(y, x) && !nan64(x); }
 
 // The larger and smaller of two, the second on ties (x > y ? x : y and
 // x < y ? x : y, as src/anuga_HMPP/util_ext.h:45-59).
