@@ -651,7 +651,8 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
                 protect_one(P, zc, w, uh, vh);
             }
             if (P.extrapolate_velocity_second_order == 1) {
-                const double dk = imax(w - zc, P.minimum_allowed_height);
+                const double dw = w - zc, mah = P.minimum_allowed_height;
+                const double dk = gt64_nan(dw, mah) ? dw : mah;
                 const Two vel = div2(uh, dk, vh, dk);
                 S.uvel[k] = vel.a;
                 S.vvel[k] = vel.b;
@@ -742,6 +743,43 @@ __global__ void __launch_bounds__(kBlock) velocities_fp64(DevMesh M, DevState S,
 
 // --------------------------------------------------------- distribute ---
 
+// The limiter in plain FP64 arithmetic (find_qmin_and_qmax and limit_gradient,
+// src/anuga_HMPP/shallow_water_ext.c:98-181): for a gradient with an infinity or
+// a NaN, whose comparisons the integer forms below do not have.
+__device__ __forceinline__ Three limit_plain(double d0, double d1, double d2, double qmin,
+                                             double qmax, double beta) {
+    const double TINY = 1.0e-100, d[3] = {d0, d1, d2};
+    double r = 1000.0, r0 = 1.0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        if (d[i] < -TINY) r0 = qmin / d[i];
+        if (d[i] > TINY) r0 = qmax / d[i];
+        r = omin(r0, r);
+    }
+    const double phi = omin(r * beta, 1.0);
+    return Three{d0 * phi, d1 * phi, d2 * phi};
+}
+static __device__ __noinline__ Three aux_limit_any(double d0, double d1, double d2, double dq0,
+                                                   double dq1, double dq2, double beta) {
+    const double s1 = dq0 + dq1, s2 = dq0 + dq2;
+    double qmin, qmax;
+    if (dq0 >= 0.0) {
+        qmax = dq1 >= dq2 ? (dq1 >= 0.0 ? s1 : dq0) : (dq2 > 0.0 ? s2 : dq0);
+        qmin = dq1 >= dq2 ? s2 : s1;
+        if (qmin >= 0.0) qmin = 0.0;
+    } else {
+        qmin = dq1 <= dq2 ? (dq1 < 0.0 ? s1 : dq0) : (dq2 < 0.0 ? s2 : dq0);
+        qmax = dq1 <= dq2 ? s2 : s1;
+        if (qmax <= 0.0) qmax = 0.0;
+    }
+    return limit_plain(d0, d1, d2, qmin, qmax, beta);
+}
+static __device__ __noinline__ Three one_limit_any(double d0, double d1, double d2, double dq1,
+                                                   double beta) {
+    const bool up = dq1 >= 0.0;
+    return limit_plain(d0, d1, d2, up ? 0.0 : dq1, up ? dq1 : 0.0, beta);
+}
+
 // src/anuga_HMPP/shallow_water_ext.c:98-148 (find_qmin_and_qmax); branches
 // and comparisons on the integer pipe.
 __device__ __forceinline__ void qmin_qmax(double dq0, double dq1, double dq2, double &qmin,
@@ -801,9 +839,16 @@ __device__ __forceinline__ void aux_jumps(double qk, double q0, double q1, doubl
     double d[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) d[i] = a * dxv[i] + b * dyv[i];
-    double qmin, qmax;
-    qmin_qmax(dq0, dq1, dq2, qmin, qmax);
-    limit_jumps(d, qmin, qmax, beta);
+    if (finite64(a, b)) {
+        double qmin, qmax;
+        qmin_qmax(dq0, dq1, dq2, qmin, qmax);
+        limit_jumps(d, qmin, qmax, beta);
+    } else {
+        const Three t = aux_limit_any(d[0], d[1], d[2], dq0, dq1, dq2, beta);
+        d[0] = t.a;
+        d[1] = t.b;
+        d[2] = t.c;
+    }
 #pragma unroll
     for (int i = 0; i < 3; i++) out[i] = qk + d[i];
 }
@@ -817,10 +862,27 @@ __device__ __forceinline__ void one_nbr_jumps(double qk, double q1, double dx2, 
     double d[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) d[i] = a * dxv[i] + b * dyv[i];
-    const bool up = ge_zero(dq1);
-    limit_jumps(d, up ? 0.0 : dq1, up ? dq1 : 0.0, beta);
+    if (finite64(a, b)) {
+        const bool up = ge_zero(dq1);
+        limit_jumps(d, up ? 0.0 : dq1, up ? dq1 : 0.0, beta);
+    } else {
+        const Three t = one_limit_any(d[0], d[1], d[2], dq1, beta);
+        d[0] = t.a;
+        d[1] = t.b;
+        d[2] = t.c;
+    }
 #pragma unroll
     for (int i = 0; i < 3; i++) out[i] = qk + d[i];
+}
+
+// omax(h0, omax(h1, h2)) < epsilon of the surrogate neighbours' depths: a NaN
+// gives way to the other operand, unless it is the last.
+__device__ __forceinline__ bool dry_neighbours(double h0, double h1, double h2, double eps) {
+    return (lt64(h0, eps) || nan64(h0)) && (lt64(h1, eps) || nan64(h1)) && lt64_nan(h2, eps);
+}
+// omin(omin(h0, omin(h1, h2)), hc): the depth that the limiter's factors follow
+__device__ __forceinline__ double least_depth(double h0, double h1, double h2, double hc) {
+    return imin_nan(imin_nan(h0, imin_nan(h1, h2)), hc);
 }
 
 // the limiter's factor of each quantity: beta_dry + (beta - beta_dry) * hfactor
@@ -890,9 +952,9 @@ __global__ void __launch_bounds__(BS, PER_SM * 256 / BS) distribute_de_fp64(DevM
             }
             if (nbk <= 1) {
                 int k0 = M.surr[k], k1 = M.surr[N + k], k2 = M.surr[2 * N + k];
-                if (!lt64(S.zc[k2], S.w[k2])) k2 = k;
-                if (!lt64(S.zc[k0], S.w[k0])) k0 = k;
-                if (!lt64(S.zc[k1], S.w[k1])) k1 = k;
+                if (le64_nan(S.w[k2], S.zc[k2])) k2 = k;
+                if (le64_nan(S.w[k0], S.zc[k0])) k0 = k;
+                if (le64_nan(S.w[k1], S.zc[k1])) k1 = k;
                 const double x0 = M.cxy[k0], y0 = M.cxy[N + k0];
                 const double dx1 = M.cxy[k1] - x0, dx2 = M.cxy[k2] - x0;
                 const double dy1 = M.cxy[N + k1] - y0, dy2 = M.cxy[N + k2] - y0;
@@ -904,9 +966,10 @@ __global__ void __launch_bounds__(BS, PER_SM * 256 / BS) distribute_de_fp64(DevM
                     const double h0 = S.w[k0] - S.zc[k0];
                     const double h1 = S.w[k1] - S.zc[k1];
                     const double h2 = S.w[k2] - S.zc[k2];
-                    const double hmin = imin(imin(h0, imin(h1, h2)), hc);
-                    const double hfactor = gt_zero(hmin) ? 1.0 : 0.0;
-                    if (P.optimise_dry_cells && lt64(imax(h0, imax(h1, h2)), P.epsilon)) {
+                    double hfactor = 0.0;
+                    if (P.betas_differ && gt64_nan(least_depth(h0, h1, h2, hc), 0.0))
+                        hfactor = 1.0;
+                    if (P.optimise_dry_cells && dry_neighbours(h0, h1, h2, P.epsilon)) {
                         keep = true;
                     } else {
                         const double q0[3] = {S.w[k0], U[k0], V[k0]};
@@ -972,12 +1035,10 @@ __global__ void __launch_bounds__(BS, PER_SM * 256 / BS) distribute_de_fp64(DevM
         if (vel) {
 #pragma unroll
             for (int i = 0; i < 3; i++) {
-                double de = ew[i] - S.ze[i * N + k];
-                if (!gt_zero(de)) de = 0.0;
+                const double de = above_zero(ew[i] - S.ze[i * N + k]);
                 eu[i] = eu[i] * de;
                 ev[i] = ev[i] * de;
-                double dv = ow[i] - S.zv[i * N + k];
-                if (!gt_zero(dv)) dv = 0.0;
+                const double dv = above_zero(ow[i] - S.zv[i * N + k]);
                 ou[i] = ou[i] * dv;
                 ov[i] = ov[i] * dv;
             }
@@ -1123,11 +1184,17 @@ __device__ __forceinline__ Balance balance_of(const DevParams &P, double wk, dou
 #pragma unroll
         for (int i = 0; i < 3; i++) dz = omax(dz, fabs(zvk[i] - zk));
     }
-    const double hmin = imin(hv[0], imin(hv[1], hv[2]));
+    // (comparisons as the reference's have it where a depth is NaN)
     double alpha = 1.0, hc = 0.0;
     if (P.tight_slope_limiters == 0) {
-        alpha = dz > 0.0 ? omax(omin(fdiv64(P.alpha_balance * hmin, dz), 1.0), 0.0) : 1.0;
-    } else if (lt64(hmin, P.H0)) {
+        const double hmin = imin_nan(hv[0], imin_nan(hv[1], hv[2]));
+        if (dz > 0.0) {
+            // omax(omin(q, 1), 0), which the compiler, given so, makes 0 of a NaN q
+            const double q = fdiv64(P.alpha_balance * hmin, dz);
+            alpha = above_zero(lt64_nan(q, 1.0) ? q : 1.0);
+        }
+    } else if ((lt64_nan(hv[0], P.H0) || lt64_nan(hv[1], P.H0) || lt64(hv[2], P.H0)) &&
+               !nan64(hv[2])) {  // omin(hv[0], omin(hv[1], hv[2])) < H0
         hc = wk - zk;
         const double head = hc - P.H0;
         double hd[3];
@@ -1135,20 +1202,21 @@ __device__ __forceinline__ Balance balance_of(const DevParams &P, double wk, dou
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             hd[i] = hc - hv[i];
-            on[i] = gt_zero(hd[i]);
+            on[i] = gt_zero(hd[i]) || nan64(hd[i]);
             if (!on[i]) hd[i] = 1.0;
         }
         const Three q3 = div3(head, hd[0], head, hd[1], head, hd[2]);
         const double q[3] = {q3.a, q3.b, q3.c};
 #pragma unroll
         for (int i = 0; i < 3; i++)
-            if (on[i]) alpha = imin(alpha, q[i]);
-        if (lt_zero(alpha)) alpha = 0.0;  // alpha is at most 1
+            if (on[i]) alpha = imin_nan(alpha, q[i]);
+        if (nan64(alpha)) alpha = 1.0;  // no blend
+        if (lt_zero(alpha)) alpha = 0.0;
     }
     double uc = 0.0, vc = 0.0;
     if (lt64(alpha, 1.0)) {
         if (P.tight_slope_limiters == 0) hc = wk - zk;
-        if (P.use_centroid_velocities == 1 && lt64(eps, hc)) {
+        if (P.use_centroid_velocities == 1 && gt64_nan(hc, eps)) {
             const Two c = div2(uk, hc, vk, hc);
             uc = c.a;
             vc = c.b;
@@ -1278,13 +1346,13 @@ __global__ void __launch_bounds__(BS, PER_SM * 256 / BS) distribute_fp64(DevMesh
                         const double h0 = w0 - S.zc[k0];
                         const double h1 = w1 - S.zc[k1];
                         const double h2 = w2 - S.zc[k2];
-                        if (P.optimise_dry_cells && lt64(imax(h0, imax(h1, h2)), P.epsilon)) {
+                        if (P.optimise_dry_cells && dry_neighbours(h0, h1, h2, P.epsilon)) {
                             keep = true;
                         } else {
                             double hfactor = 0.0;
                             if (P.betas_differ) {
-                                const double hmin = imin(imin(h0, imin(h1, h2)), wk - zk);
-                                if (lt64(0.001, hmin))
+                                const double hmin = least_depth(h0, h1, h2, wk - zk);
+                                if (gt64_nan(hmin, 0.001))
                                     hfactor = fdiv64(hmin - 0.001, hmin + 0.004);
                             }
                             const double q0[3] = {w0, U[k0], V[k0]};
@@ -1341,7 +1409,7 @@ __global__ void __launch_bounds__(BS, PER_SM * 256 / BS) distribute_fp64(DevMesh
             // back from velocity to momentum with the vertex depth
 #pragma unroll
             for (int i = 0; i < 3; i++) {
-                const double dv = gt_zero(hv[i]) ? hv[i] : 0.0;
+                const double dv = above_zero(hv[i]);
                 ou[i] = ou[i] * dv;
                 ov[i] = ov[i] * dv;
             }
@@ -1492,13 +1560,13 @@ __global__ void __launch_bounds__(3 * kSplitTile) distribute_split_fp64(DevMesh 
                         const double h0 = S.w[k0n] - S.zc[k0n];
                         const double h1 = S.w[k1n] - S.zc[k1n];
                         const double h2 = S.w[k2n] - S.zc[k2n];
-                        if (P.optimise_dry_cells && lt64(imax(h0, imax(h1, h2)), P.epsilon)) {
+                        if (P.optimise_dry_cells && dry_neighbours(h0, h1, h2, P.epsilon)) {
                             keep = true;
                         } else {
                             double hfactor = 0.0;
                             if (P.betas_differ) {
-                                const double hmin = imin(imin(h0, imin(h1, h2)), wk - zk);
-                                if (lt64(0.001, hmin))
+                                const double hmin = least_depth(h0, h1, h2, wk - zk);
+                                if (gt64_nan(hmin, 0.001))
                                     hfactor = fdiv64(hmin - 0.001, hmin + 0.004);
                             }
                             double beta[3];
@@ -1548,7 +1616,7 @@ __global__ void __launch_bounds__(3 * kSplitTile) distribute_split_fp64(DevMesh 
         ou = vert[1][role][t];
         ov = vert[2][role][t];
         if (to_momentum) {
-            const double dv = gt_zero(h) ? h : 0.0;
+            const double dv = above_zero(h);
             ou = ou * dv;
             ov = ov * dv;
         }
@@ -1634,9 +1702,9 @@ __global__ void __launch_bounds__(3 * kSplitTile) distribute_de_split_fp64(DevMe
             }
             if (nbk <= 1) {
                 int k0 = M.surr[k], k1 = M.surr[N + k], k2 = M.surr[2 * N + k];
-                if (!lt64(S.zc[k2], S.w[k2])) k2 = k;
-                if (!lt64(S.zc[k0], S.w[k0])) k0 = k;
-                if (!lt64(S.zc[k1], S.w[k1])) k1 = k;
+                if (le64_nan(S.w[k2], S.zc[k2])) k2 = k;
+                if (le64_nan(S.w[k0], S.zc[k0])) k0 = k;
+                if (le64_nan(S.w[k1], S.zc[k1])) k1 = k;
                 const double x0 = M.cxy[k0], y0 = M.cxy[N + k0];
                 const double dx1 = M.cxy[k1] - x0, dx2 = M.cxy[k2] - x0;
                 const double dy1 = M.cxy[N + k1] - y0, dy2 = M.cxy[N + k2] - y0;
@@ -1648,9 +1716,10 @@ __global__ void __launch_bounds__(3 * kSplitTile) distribute_de_split_fp64(DevMe
                     const double h0 = S.w[k0] - S.zc[k0];
                     const double h1 = S.w[k1] - S.zc[k1];
                     const double h2 = S.w[k2] - S.zc[k2];
-                    const double hmin = imin(imin(h0, imin(h1, h2)), hc);
-                    const double hfactor = gt_zero(hmin) ? 1.0 : 0.0;
-                    if (P.optimise_dry_cells && lt64(imax(h0, imax(h1, h2)), P.epsilon)) {
+                    double hfactor = 0.0;
+                    if (P.betas_differ && gt64_nan(least_depth(h0, h1, h2, hc), 0.0))
+                        hfactor = 1.0;
+                    if (P.optimise_dry_cells && dry_neighbours(h0, h1, h2, P.epsilon)) {
                         keep = true;
                     } else {
                         double beta[3];
@@ -1701,12 +1770,10 @@ __global__ void __launch_bounds__(3 * kSplitTile) distribute_de_split_fp64(DevMe
         double ou = edge[1][a][t] + edge[1][b][t] - ue;
         double ov = edge[2][a][t] + edge[2][b][t] - ve;
         if (vel) {
-            double de = we - S.ze[role * N + k];
-            if (!gt_zero(de)) de = 0.0;
+            const double de = above_zero(we - S.ze[role * N + k]);
             ue = ue * de;
             ve = ve * de;
-            double dv = ow - S.zv[role * N + k];
-            if (!gt_zero(dv)) dv = 0.0;
+            const double dv = above_zero(ow - S.zv[role * N + k]);
             ou = ou * dv;
             ov = ov * dv;
         }

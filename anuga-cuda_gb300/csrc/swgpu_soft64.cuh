@@ -59,11 +59,27 @@ __device__ __forceinline__ bool nan64(double x) {
 __device__ __forceinline__ bool lt64_nan(double x, double y) { return lt64(x, y) && !nan64(x); }
 // x > y also where x may be NaN (then false)
 __device__ __forceinline__ bool gt64_nan(double x, double y) { return lt64(y, x) && !nan64(x); }
+// x <= y also where either may be NaN (then false)
+__device__ __forceinline__ bool le64_nan(double x, double y) {
+    return !lt64(y, x) && !nan64(x) && !nan64(y);
+}
+// x > 0 ? x : 0 (0 for a NaN)
+__device__ __forceinline__ double above_zero(double x) {
+    return bits64(x) - 1 < 0x7ff0000000000000ull ? x : 0.0;
+}
+// neither is an infinity or NaN
+__device__ __forceinline__ bool finite64(double x, double y) {
+    return max(hi32(x) & 0x7fffffffu, hi32(y) & 0x7fffffffu) < 0x7ff00000u;
+}
 
-// The larger and smaller of two, the second on ties (x > y ? x : y and
+// The larger and smaller of two numbers, the second on ties (x > y ? x : y and
 // x < y ? x : y, as src/anuga_HMPP/util_ext.h:45-59).
 __device__ __forceinline__ double imax(double x, double y) { return lt64(y, x) ? x : y; }
 __device__ __forceinline__ double imin(double x, double y) { return lt64(x, y) ? x : y; }
+// The smaller where either may be NaN (then the second).
+__device__ __forceinline__ double imin_nan(double x, double y) {
+    return lt64(x, y) && !nan64(x) && !nan64(y) ? x : y;
+}
 
 // 0.5 * x on the integer pipe where the halved number is normal (or x zero)
 static __device__ __noinline__ double half_any(double x) { return 0.5 * x; }
