@@ -233,7 +233,7 @@ __device__ __forceinline__ EdgeFlux central_flux(const EdgeState &s, const DevPa
 // triangle instead of three, and equal work for every lane.
 //
 // PER_SM: blocks of 256 that the registers leave room for, here and in the
-// distribute.  With three, at 80 registers (24 and 34 words spilled, which L1
+// distribute.  With three, at 80 registers (24 and 58 words spilled, which L1
 // holds), the FP64 pipe of a large mesh finds a ready warp more often than with
 // two at 97 and 127 (a million triangles: flux 224 -> 205 us, distribute 318 ->
 // 304; four: 202 and 310); a mesh without that many warps only has the spills
