@@ -125,13 +125,18 @@ __device__ __forceinline__ u64 mul_32x64(unsigned a, u64 b) {
 
 // a / b, correctly rounded.
 //
-// B in [2^52, 2^53), A in [B, 2B).  Estimates: the reciprocal r of B's leading
-// 24 bits is within 2^-23 (truncation) + 2^-23 (rcp.approx) of 1/B; scaled by
-// 1 - 2^-21 it never exceeds it, and is below it by at most 2^-20.4.
-//   q1 = floor(A r 2^21):   short by < 2^22 2^-20.4 + 3 (A's 24 bits, floor)
-//                           -> R1 = 2^21 A - q1 B in [0, 7B)
-//   q2 = floor(R1 r 2^20):  R1's 23 bits from 2^33 cut 2^-19 B: short by
-//                           < 7 2^20 2^-20.4 + 2 + 1 -> R2 in [0, 9B)
+// B in [2^52, 2^53), A in [B, 2B), b = B / 2^52.  The reciprocal of b's leading
+// 24 bits is off by at most 2^-23 / b^2 above (truncation) and 2^-23 either way
+// (rcp.approx); scaled by 1 - 2^-21, r never exceeds 1/b and is short of it by a
+// factor of at most 1 - (4.5 + b) 2^-23.  The two errors are not largest
+// together (the first at b = 1, the second at b = 2), which is what keeps R2
+// within the 56 bits that bits23<33> takes:
+//   q1 = floor(A r 2^21):   A's 24 bits, a product's rounding and the floor on
+//                           top: short by less than (6 + b) / 2 + 1
+//                           -> R1 = 2^21 A - q1 B in [0, 5B)
+//   q2 = floor(R1 r 2^20):  R1's bits from 2^33 cut up to 2 / b: short by less
+//                           than (4 + b / 2) (5 + b) / 8 + 2 / b + 1 <= 6.375
+//                           -> R2 in [0, 6.375 B), below 2^55.7
 //   q3 = floor(R2 r 2^11):  short by < 1.02 -> R3 in [0, 1.02 B)
 // N = 2^31 q1 + 2^11 q2 + q3 and R3 = 2^52 A - N B decide the rounding.
 //
