@@ -114,6 +114,8 @@ _SIGNATURES = [
     ("swgpu_get_tracking", C.c_int, [_VP, C.POINTER(C.c_float), C.POINTER(C.c_float)]),
     ("swgpu_get_launch_config", C.c_int, [_VP, C.POINTER(LaunchConfig_t)]),
     ("swgpu_set_launch_config", C.c_int, [_VP, C.POINTER(LaunchConfig_t)]),
+    ("swgpu_resolve_launch_config", C.c_int,
+     [_VP, C.POINTER(LaunchConfig_t), C.POINTER(LaunchConfig_t)]),
     ("swgpu_ensemble_get_state", C.c_int, [_VP, C.c_int, C.POINTER(State_t)]),
     ("swgpu_ensemble_set_finaltimes", C.c_int, [_VP, _f64p]),
     ("swgpu_ensemble_mass", C.c_int, [_VP, _f64p]),

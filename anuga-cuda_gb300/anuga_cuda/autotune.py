@@ -8,7 +8,9 @@ candidate shape runs whole steps through the device-resident loop (CUDA
 graphs, programmatic dependent launches, exactly as evolve issues them),
 timed with CUDA events on the handle's stream (``swgpu_evolve_run_timed``),
 one knob at a time from the current best; a candidate is kept when its step
-is at least 1% faster.  Timing kernels one by one instead would miss what the
+is at least 1% faster.  A candidate that comes to the same launches as one
+already timed (``swgpu_resolve_launch_config``: small meshes read few of the
+knobs) is not timed: a difference would be noise.  Timing kernels one by one instead would miss what the
 graph overlaps (a persistent flux that looks faster alone holds the SMs
 against the next kernel's early blocks).  The steps the measurement runs
 advance the model: tune a throwaway copy of a domain (``tune_domain``
@@ -28,7 +30,7 @@ import os
 from . import _lib
 from ._lib import check, lib
 
-__all__ = ["get_config", "set_config", "tune_handle", "tune_domain", "cache_path",
+__all__ = ["get_config", "set_config", "resolve_config", "tune_handle", "tune_domain", "cache_path",
            "cached_config", "DEFAULT_CANDIDATES", "STEPS_PER_GRAPH"]
 
 DEFAULT_CANDIDATES = {"flux": (64, 128, 256), "update": (128, 256, 512),
@@ -36,20 +38,37 @@ DEFAULT_CANDIDATES = {"flux": (64, 128, 256), "update": (128, 256, 512),
 _FIELD = {"flux": "flux_block", "update": "update_block", "distribute": "distribute_block"}
 
 
-def get_config(h) -> dict:
-    c = _lib.LaunchConfig_t()
-    check(lib().swgpu_get_launch_config(h, C.byref(c)), h)
+def _as_dict(c) -> dict:
     return {"flux_block": c.flux_block, "update_block": c.update_block,
             "distribute_block": c.distribute_block, "steps_per_graph": c.steps_per_graph,
             "flux_pipelined": c.flux_pipelined, "dependent_launch": c.dependent_launch}
 
 
+def _as_struct(h, cfg: dict):
+    return _lib.LaunchConfig_t(int(cfg["flux_block"]), int(cfg["update_block"]),
+                               int(cfg["distribute_block"]), int(cfg.get("steps_per_graph", 16)),
+                               int(cfg.get("flux_pipelined", 0)),
+                               int(cfg.get("dependent_launch",
+                                           get_config(h)["dependent_launch"])))
+
+
+def get_config(h) -> dict:
+    c = _lib.LaunchConfig_t()
+    check(lib().swgpu_get_launch_config(h, C.byref(c)), h)
+    return _as_dict(c)
+
+
 def set_config(h, cfg: dict) -> None:
-    c = _lib.LaunchConfig_t(int(cfg["flux_block"]), int(cfg["update_block"]),
-                            int(cfg["distribute_block"]), int(cfg.get("steps_per_graph", 16)),
-                            int(cfg.get("flux_pipelined", 0)),
-                            int(cfg.get("dependent_launch", get_config(h)["dependent_launch"])))
+    c = _as_struct(h, cfg)
     check(lib().swgpu_set_launch_config(h, C.byref(c)), h)
+
+
+def resolve_config(h, cfg: dict) -> dict:
+    """The launches that ``cfg`` comes to on this handle: block sizes as the
+    kernels take them, 0 for knobs that its steps do not read."""
+    c, r = _as_struct(h, cfg), _lib.LaunchConfig_t()
+    check(lib().swgpu_resolve_launch_config(h, C.byref(c), C.byref(r)), h)
+    return _as_dict(r)
 
 
 STEPS_PER_GRAPH = (8, 16, 32)
@@ -84,6 +103,7 @@ def tune_handle(h, steps=64, candidates=None, ensemble=False) -> dict:
         cand["distribute"] = tuple(b for b in cand["distribute"] if b <= 256)
     best = get_config(h)
     best_ms = start_ms = _time_shape(h, best, steps)
+    timed = [resolve_config(h, best)]
     trials = []
     for kernel, values in cand.items():
         trials += [{_FIELD[kernel]: v} for v in values]
@@ -98,6 +118,10 @@ def tune_handle(h, steps=64, candidates=None, ensemble=False) -> dict:
         if trial == best:
             continue
         try:
+            launches = resolve_config(h, trial)
+            if launches in timed:
+                continue
+            timed.append(launches)
             t = _time_shape(h, trial, steps)
         except _lib.SwgpuError:
             set_config(h, best)

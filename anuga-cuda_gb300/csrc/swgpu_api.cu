@@ -1403,9 +1403,7 @@ int swgpu_get_launch_config(void *handle, swgpu_launch_config *cfg) {
     return SWGPU_OK;
 }
 
-int swgpu_set_launch_config(void *handle, const swgpu_launch_config *cfg) {
-    Handle *h = static_cast<Handle *>(handle);
-    if (!h || !cfg) return fail(h, SWGPU_EINVAL, "null argument");
+static int check_launch_config(Handle *h, const swgpu_launch_config *cfg) {
     auto one_of = [](int v, std::initializer_list<int> ok) {
         for (int x : ok)
             if (v == x) return true;
@@ -1422,8 +1420,37 @@ int swgpu_set_launch_config(void *handle, const swgpu_launch_config *cfg) {
         return fail(h, SWGPU_EINVAL,
                     "launch config: flux 64/128/256 (at most 128 pipelined), update and "
                     "distribute 128/256/512 (at most 256 for an ensemble), 1..64 steps per graph");
-    int rc = edit_ctrl(h);
-    if (rc) return rc;
+    return SWGPU_OK;
+}
+
+int swgpu_resolve_launch_config(void *handle, const swgpu_launch_config *cfg,
+                                swgpu_launch_config *out) {
+    Handle *h = static_cast<Handle *>(handle);
+    if (!h || !cfg || !out) return fail(h, SWGPU_EINVAL, "null argument");
+    if (int rc = check_launch_config(h, cfg)) return rc;
+    swgpu_launch_config c = *cfg;
+    c.flux_pipelined = cfg->flux_pipelined ? 1 : 0;
+    c.dependent_launch = cfg->dependent_launch ? 1 : 0;
+    if (h->resident.kernel && c.dependent_launch) {
+        c = swgpu_launch_config{};
+        c.dependent_launch = 1;
+    } else if (h->precision == SWGPU_FP64) {
+        const int sms = h->M.shape.sms;
+        c.flux_block = fp64_block(cfg->flux_block, h->M.edges.E, sms);
+        c.update_block = fp64_block(cfg->update_block, h->M.N, sms);
+        c.distribute_block =
+            distribute_split(h->M.N, sms) ? 0 : fp64_block(cfg->distribute_block, h->M.N, sms);
+        c.flux_pipelined = 0;
+    }
+    *out = c;
+    return SWGPU_OK;
+}
+
+int swgpu_set_launch_config(void *handle, const swgpu_launch_config *cfg) {
+    Handle *h = static_cast<Handle *>(handle);
+    if (!h || !cfg) return fail(h, SWGPU_EINVAL, "null argument");
+    int rc = check_launch_config(h, cfg);
+    if (rc || (rc = edit_ctrl(h))) return rc;
     CK(cudaStreamSynchronize(h->stream));
     drop_graphs(h);  // recaptured with the new shape on the next run
     h->M.shape.flux = cfg->flux_block;

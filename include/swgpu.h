@@ -224,8 +224,10 @@ int swgpu_ensemble_mass(void *handle, double *masses);
  * is the same for every shape).  flux_block: threads per block of the FP64
  * flux, or triangles per TMA tile of the mixed flux (64, 128, 256);
  * update_block, distribute_block: 128, 256 or 512 (at most 256 for an
- * ensemble); steps_per_graph: 1..64 steps captured per CUDA graph.  No
- * counterpart in the reference (its block sizes are fixed per kernel,
+ * ensemble); steps_per_graph: 1..64 steps captured per CUDA graph.  The FP64
+ * kernels take their block sizes as upper bounds: blocks shrink until every SM
+ * has its share, and the distribute of a small mesh has a shape of its own.
+ * No counterpart in the reference (its block sizes are fixed per kernel,
  * gpu_domain_advanced.py:186-507). */
 typedef struct {
     int32_t flux_block;
@@ -234,10 +236,11 @@ typedef struct {
     int32_t steps_per_graph;
     int32_t flux_pipelined;   /* mixed flux: persistent blocks, double-buffered TMA
                                  tiles (flux_block 64 or 128) */
-    int32_t dependent_launch; /* mixed kernels: each step kernel is launched as a
-                                 programmatic dependent of the previous one, so
-                                 its blocks start (and fetch the static planes)
-                                 during that kernel's last wave; 0 also runs
+    int32_t dependent_launch; /* each step kernel is launched as a programmatic
+                                 dependent of the previous one, so that its
+                                 blocks start before that kernel has ended
+                                 (where in it depends on the mesh size, and FP64
+                                 meshes of some sizes do without); 0 also runs
                                  small mixed meshes kernel by kernel, which
                                  otherwise take whole steps in one resident
                                  launch, without the knobs above */
@@ -245,6 +248,12 @@ typedef struct {
 
 int swgpu_get_launch_config(void *handle, swgpu_launch_config *config);
 int swgpu_set_launch_config(void *handle, const swgpu_launch_config *config);
+/* What the handle's step kernels would run with under config: the block sizes
+ * that they take, and 0 for each knob that its steps do not read (all but
+ * dependent_launch in the resident step).  Two shapes that resolve to the same
+ * are the same launches. */
+int swgpu_resolve_launch_config(void *handle, const swgpu_launch_config *config,
+                                swgpu_launch_config *resolved);
 
 /* Per-triangle tracking over the device-resident loop: the maximum depth
  * since the call and the first model time (end of a whole step) at which
