@@ -603,16 +603,14 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     M.n_launch = (int)N;
     M.Nb = (int)Nb;
     int *d_nbr, *d_surr, *d_bcell, *d_bedge, *d_btag;
-    uint8_t *d_nb, *d_order, *d_full;
-    double *d_normals, *d_len, *d_radii, *d_areas, *d_vxy, *d_cxy;
+    uint8_t *d_nb, *d_order;
+    double *d_normals, *d_len, *d_areas, *d_vxy, *d_cxy;
     TRY(dalloc(h, &d_nbr, n3));
     TRY(dalloc(h, &d_surr, n3));
     TRY(dalloc(h, &d_nb, n1));
     TRY(dalloc(h, &d_order, n1));
-    TRY(dalloc(h, &d_full, n1));
     TRY(dalloc(h, &d_normals, n6));
     TRY(dalloc(h, &d_len, n3));
-    TRY(dalloc(h, &d_radii, n1));
     TRY(dalloc(h, &d_areas, n1));
     TRY(dalloc(h, &d_vxy, n6));
     TRY(dalloc(h, &d_cxy, 2 * n1));
@@ -623,7 +621,6 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     TRY(upload(h, d_surr, surr.data(), n3));
     TRY(upload(h, d_nb, nb.data(), n1));
     TRY(upload(h, d_order, order.data(), n1));
-    TRY(upload(h, d_full, full.data(), n1));
     h->h_normals = to_planes<double>(mesh->normals, N, 6);
     h->h_len = to_planes<double>(mesh->edgelengths, N, 3);
     h->h_vxy = to_planes<double>(mesh->vertex_coordinates, N, 6);
@@ -635,7 +632,6 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     h->h_nb = nb;
     TRY(upload(h, d_normals, h->h_normals.data(), n6));
     TRY(upload(h, d_len, h->h_len.data(), n3));
-    TRY(upload(h, d_radii, mesh->radii, n1));
     TRY(upload(h, d_areas, mesh->areas, n1));
     TRY(upload(h, d_vxy, h->h_vxy.data(), n6));
     TRY(upload(h, d_cxy, h->h_cxy.data(), 2 * n1));
@@ -654,10 +650,8 @@ static int create_impl(const swgpu_mesh *mesh, const swgpu_params *params, int p
     M.surr = d_surr;
     M.nb = d_nb;
     M.order = d_order;
-    M.full = d_full;
     M.normals = d_normals;
     M.len = d_len;
-    M.radii = d_radii;
     M.areas = d_areas;
     M.vxy = d_vxy;
     M.cxy = d_cxy;

@@ -69,10 +69,8 @@ struct DevMesh {
     const int *surr;           // [3][N] surrogate neighbours
     const uint8_t *nb;         // [N] number_of_boundaries
     const uint8_t *order;      // [N] flux summation order (2 bits per position)
-    const uint8_t *full;       // [N] tri_full_flag
     const double *normals;     // [6][N]
     const double *len;         // [3][N]
-    const double *radii;       // [N]
     const double *areas;       // [N]
     const double *vxy;         // [6][N]
     const double *cxy;         // [2][N]
