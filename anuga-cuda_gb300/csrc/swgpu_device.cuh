@@ -203,9 +203,10 @@ __device__ __forceinline__ bool last_block_done(unsigned int *counter, unsigned 
     return false;
 }
 
-// Once all atomicMins of the step are done (FP64: the flux kernel's last
-// block; mixed: step_clock_mixed, after the flux grid): evaluate
-// update_timestep once and publish it for the update kernel.
+// Once all atomicMins of the step are done: update_timestep evaluated and
+// published for the distribute, by the update (every block evaluates it, the
+// scenario's first publishes) or, on large meshes, once before it (FP64: by the
+// flux's last block; mixed: by step_clock_mixed).
 __device__ __forceinline__ void publish_step_clock(Ctrl *c, const StepClock &s) {
     c->clk_dt = s.dt;
     c->clk_ftmin = s.ftmin;

@@ -482,8 +482,9 @@ __device__ __forceinline__ void flux_body(const DevMesh &M, const DevMixed &X, c
     if (arrived && tid < cnt) t = flux_tile_triangle<TILE>(X, P, T, k0, cnt);
     if (LATE) pdl_launch_at(kStartEnd, flags);
     if (flags & kNoTimestep) return;  // later Runge-Kutta stage: the step's dt is set
-    // the step's clock is evaluated from the minimum by step_clock_mixed once
-    // this grid has completed: no block waits on a count of finished blocks
+    // the step's clock is evaluated from the minimum by the update (on large
+    // meshes by step_clock_mixed) once this grid has completed: no block waits
+    // on a count of finished blocks
     block_min_timestep_f<TILE>(t, ctrl, &ft_seen);
 }
 template <int TILE>
@@ -700,8 +701,9 @@ __device__ __forceinline__ void update_body(const DevMesh &M, const DevState &S,
     const float4 us = in ? ro(X.ust + k) : make_float4(0.f, 0.f, 0.f, 0.f);
     const float eta = us.x, zmoff = us.y, zhi = us.z, zlo = us.w;
     pdl_wait();
-    // a stopped scenario's threads load nothing more (the flag is settled:
-    // only the step's clock and the distribute change it)
+    // a stopped scenario's threads load nothing more (the flag is settled: the
+    // distribute before has completed, and a 2 that becomes 1 below or in the
+    // step's clock means the same here)
     if ((flags & kFused) && ctrl_halt_settled(ctrl)) {
         if (CLOCK && threadIdx.x == 0 && first_of_scenario(M) && ctrl->halt == 2)
             ctrl->halt = 1;  // the last step's distribute has run
@@ -1189,8 +1191,9 @@ __device__ __forceinline__ void distribute_body(const DevMesh &M, const DevState
     }
     pdl_wait();
     if (stopped_early) return;  // no copy was issued
-    // halt == 1 only from a step clock kernel, which has completed: the same
-    // for every thread (halt == 2: the scenario stops after this distribute)
+    // halt == 1 only from the update or the step clock kernel, which have
+    // completed: the same for every thread (halt == 2: the scenario stops after
+    // this distribute)
     const bool halted = fused && ctrl_halt_settled(ctrl) == 1;
     if (tid == 0) {
         if (halted) {

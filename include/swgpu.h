@@ -268,9 +268,10 @@ int swgpu_get_tracking(void *handle, float *max_depth, float *arrival_time);
  * and the 90% quantile of the first output's absolute error, from 9 scenario
  * parameters and the triangle's centroid, bed and distance to the inflow.
  * BF16 weights and activations, FP32 accumulation; every layer of width
- * 256 runs as tcgen05.mma tiles (128 rows x 256 units) accumulating in
- * tensor memory, in the forward and the backward pass; FP32 master weights
- * trained by Adam.  params is the flat FP32 vector W1 [16][256], b1 [256],
+ * 256 runs as tcgen05.mma tiles accumulating in tensor memory, in the forward
+ * and the backward pass (128 rows x 256 units in training; inference has
+ * products of 256 rows over a pair of CTAs); FP32 master weights trained by
+ * Adam.  params is the flat FP32 vector W1 [16][256], b1 [256],
  * W2 [256][256], b2, W3 [256][256], b3, W4 [256][3], b4 [3]
  * (swgpu_mlp_num_params() floats, in-major weights); the feature map is
  * (raw - mean) * inv_std over 16 features (the last 3 are zero).  Handles
