@@ -1745,15 +1745,20 @@ static int run_units(Handle *h, int64_t max_steps) {
             }
             // a budget's last unit: the caller waits for it
             if (steps == budget) return SWGPU_OK;
-            CK(cudaMemcpyAsync(h->h_summary, h->d_summary, sizeof(RunSummary),
-                               cudaMemcpyDeviceToHost, h->stream));
-            if (h->nscen > 1)
-                CK(cudaMemcpyAsync(h->h_halt_bits, h->d_halt_bits,
-                                   sizeof(unsigned) * ((h->nscen + 31) / 32),
-                                   cudaMemcpyDeviceToHost, h->stream));
-            if (watch)
+            // what the host follows: one mesh's control block, which has its stop
+            // too (a second copy for the summary cost units of one step 2.5 us),
+            // else the scenarios' summary
+            if (watch) {
                 CK(cudaMemcpyAsync(h->h_watch + slot, h->d_ctrl, sizeof(Ctrl),
                                    cudaMemcpyDeviceToHost, h->stream));
+            } else {
+                CK(cudaMemcpyAsync(h->h_summary, h->d_summary, sizeof(RunSummary),
+                                   cudaMemcpyDeviceToHost, h->stream));
+                if (h->nscen > 1)
+                    CK(cudaMemcpyAsync(h->h_halt_bits, h->d_halt_bits,
+                                       sizeof(unsigned) * ((h->nscen + 31) / 32),
+                                       cudaMemcpyDeviceToHost, h->stream));
+            }
             CK(cudaEventRecord(ev[slot], h->stream));
             if (budget != INT64_MAX) budget -= steps;
             issued[slot] = steps;
@@ -1768,6 +1773,8 @@ static int run_units(Handle *h, int64_t max_steps) {
         if (watch) {
             *h->h_ctrl = h->h_watch[oldest];
             ahead -= issued[oldest];
+            if (h->h_ctrl->halt) return SWGPU_OK;
+            continue;
         }
         if (h->h_summary->halted >= h->nscen || h->h_summary->status) return SWGPU_OK;
         if (h->nscen > 1 && !resident) {
