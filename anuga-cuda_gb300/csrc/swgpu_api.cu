@@ -236,7 +236,7 @@ static bool separate_clock(const Handle *h) { return h->M.N >= (1 << 20); }
 static void issue_stage(Handle *h, const Stage &stg) {
     const int flux_flags = kFused | (stg.kind == kStageMid || stg.kind == kStageLast
                                          ? kNoTimestep : 0);
-    const int update_flags = kFused | kFrictionInline | (h->S.hmax ? kTrack : 0);
+    const int update_flags = kFused | (h->S.hmax ? kTrack : 0);
     const int dist_flags = kFused | kWriteBoundary;
     if (h->precision == SWGPU_FP64) {
         launch_flux_fp64(h->M, h->S, h->P, h->d_ctrl, flux_flags, h->stream);
@@ -1666,11 +1666,10 @@ int swgpu_profile_steps(void *handle, int64_t nsteps, double *ms) {
             launch_step_clock_mixed(h->P, h->d_ctrl, h->nscen, h->M.shape.pdl, h->stream);
         CK(cudaEventRecord(ev[2], h->stream));
         if (!mixed)
-            launch_update_fp64(h->M, h->S, h->P, h->d_ctrl, 0.0, kFused | kFrictionInline,
-                               kEulerStage, h->stream);
+            launch_update_fp64(h->M, h->S, h->P, h->d_ctrl, 0.0, kFused, kEulerStage, h->stream);
         else
-            launch_update_mixed(h->M, h->S, h->X, h->P, h->d_ctrl, kFused | kFrictionInline,
-                                kEulerStage, !own_clock, h->d_tags, h->time_tags, h->stream);
+            launch_update_mixed(h->M, h->S, h->X, h->P, h->d_ctrl, kFused, kEulerStage,
+                                !own_clock, h->d_tags, h->time_tags, h->stream);
         CK(cudaEventRecord(ev[3], h->stream));
         if (!mixed)
             launch_distribute_fp64(h->M, h->S, h->P, h->d_tags, h->d_ctrl,

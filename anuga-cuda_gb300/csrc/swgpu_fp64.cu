@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
         }
         double su, sv;
         bool applied;
-        if (flags & kFrictionInline) {
+        if (FUSED) {
             const double Sf = manning_S(M, S, P, k, w, uh, vh, applied);
             su = applied ? Sf * uh : 0.0;
             sv = applied ? Sf * vh : 0.0;
@@ -667,7 +667,8 @@ __global__ void __launch_bounds__(BS) update_fp64(DevMesh M, DevState S, DevPara
         S.w[k] = w;
         S.uh[k] = uh;
         S.vh[k] = vh;
-        if ((flags & kTrack) && (stg.kind == kStageEuler || stg.kind == kStageLast))
+        if (FUSED && (flags & kTrack) &&
+            (stg.kind == kStageEuler || stg.kind == kStageLast))
             track_depth(S, k, w - zc, step_end_time(ctrl, dt, stg), P.track_threshold);
     }
     if (bad) set_status(ctrl, SWGPU_EDENOMINATOR);

@@ -216,7 +216,6 @@ enum : int {
     kFused = 1,           // part of the device-resident loop (reads/writes Ctrl)
     kWriteEdges = 2,      // distribute materialises edge values
     kWriteBoundary = 4,   // distribute evaluates boundary conditions
-    kFrictionInline = 8,  // update computes Manning friction itself
     kWriteMaxSpeed = 16,  // flux writes max_speed
     kNoTimestep = 32,     // flux skips the timestep reduction (later Runge-Kutta stages)
     kTrack = 64,          // update records maximum depth and arrival time (whole steps)
