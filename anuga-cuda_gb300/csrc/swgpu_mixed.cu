@@ -1433,8 +1433,12 @@ __device__ __forceinline__ void cluster_put(unsigned a, int v) {
 }
 // Every thread of the cluster; what was written before it is visible after.
 // (A hardware barrier of blocks that run side by side by construction: no
-// thread leaves the kernel, or the step loop, without the others.)
+// thread leaves the kernel, or the step loop, without the others.  The aligned
+// form asks for warps whose threads have come together, and they come here from
+// triangles that are in or out, wet or dry.  The form that is not aligned costs
+// 8,100 triangles 8.45 us a step instead of 8.3.)
 __device__ __forceinline__ void cluster_meet() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
