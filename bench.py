@@ -60,10 +60,10 @@ UNIT = "triangle-steps/s"
 
 # algorithmic bytes per triangle-step of each kernel (own arrays, neighbour
 # gathers counted as cache hits)
-MIXED_BYTES = {"flux": 128, "update": 104, "distribute": 114}
+MIXED_BYTES = {"flux": 128, "update": 108, "distribute": 129}
 # DRAM bytes (read + write) per launch from one ncu capture of the 4,000,000-
 # triangle mesh (1000x1000 cells); scaled by the triangles for other meshes
-NCU_TRAFFIC_4M = {"flux": 509.35e6, "update": 377.39e6, "distribute": 520.23e6}
+NCU_TRAFFIC_4M = {"flux": 502.91e6, "update": 374.97e6, "distribute": 530.88e6}
 MODEL_BYTES = {"mixed": 368, "fp64": 568}   # whole-step byte model
 ACC_STEPS = 1000                             # steps of the mixed-vs-FP64 accuracy check
 WET_FLOOR = 0.01                             # m: wet triangles of the per-element depth error
@@ -73,7 +73,7 @@ WET_FLOOR = 0.01                             # m: wet triangles of the per-eleme
 # FP64 at 1/64 of the FP32 rate, 2 thread instructions per SM per clock
 # (DADD, DMUL, DFMA and the pipe's other instructions one slot each):
 # 152 SMs x 2 x 2.07 GHz
-FP64_PIPE_INST = {"flux": 94.48, "update": 95.00, "distribute": 138.99}
+FP64_PIPE_INST = {"flux": 94.48, "update": 94.60, "distribute": 133.99}
 FP64_PIPE_PEAK = 152 * 2 * 2.07e9
 
 
